@@ -72,7 +72,7 @@ int32_t validate_matmul(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, 
 int32_t jq_matmul_device(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, const float* lhs, float* dst,
                          cudaStream_t s) {
     jq_ctx* ctx = w->ctx;
-    if (!ctx->force_f32 && jq::gemv_mma_supports(w->type, w->dev, n, k, m)) {
+    if (!ctx->force_f32 && jq::gemv_mma_dense_supports(w->type, w->dev, n, k, m)) {
         void* scratch = nullptr;
         JQ_CUDA(ctx->scratch_for(s, jq::gemv_mma_scratch_bytes(m, k), &scratch));
         JQ_CUDA(jq::launch_gemv_mma(w->type, w->dev, n, k, lhs, m, dst, scratch, ctx->status_dev, s));
@@ -80,9 +80,10 @@ int32_t jq_matmul_device(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n,
     }
     // Batches a little above the decode kernel's eight rows: eight rows at a time through the decode kernel
     // (the weights are read once per slice, from L2 when they fit) still beats the tile GEMM, whose K loop
-    // costs the same at any batch.
-    if (!ctx->force_f32 && m > jq::GEMV_MMA_MAX_M && m <= ctx->sliced_max_m &&
-        jq::gemv_mma_supports(w->type, w->dev, n, k, jq::GEMV_MMA_MAX_M)) {
+    // costs the same at any batch.  Q6_K has no tile GEMM: any batch goes in slices, which read packed bytes at
+    // terabytes per second where the exact-decode float kernel (the other route) reaches half of one.
+    if (!ctx->force_f32 && m > jq::GEMV_MMA_MAX_M && (m <= ctx->sliced_max_m || w->type == jq::T_Q6_K) &&
+        jq::gemv_mma_dense_supports(w->type, w->dev, n, k, jq::GEMV_MMA_MAX_M)) {
         void* scratch = nullptr;
         JQ_CUDA(ctx->scratch_for(s, jq::gemv_mma_scratch_bytes(jq::GEMV_MMA_MAX_M, k), &scratch));
         for (uint64_t r0 = 0; r0 < m; r0 += jq::GEMV_MMA_MAX_M) {

@@ -120,6 +120,9 @@ cudaError_t tables_gemv_mma();
 // bytes of scratch (activation planes) a launch with these sizes needs
 size_t gemv_mma_scratch_bytes(uint64_t m, uint64_t k);
 bool gemv_mma_supports(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, uint64_t m);
+// The same for plain products (launch_gemv_mma, launch_gemv_mma_fused), which also take Q6_K: the type a mixed file
+// keeps its output head and a few matrices in.  Expert banks and the allocation-free entry stay with the five types.
+bool gemv_mma_dense_supports(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, uint64_t m);
 // error_flag: device int set to 1 if a bounded wait inside the kernel gave up
 cudaError_t launch_gemv_mma(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, const float* lhs, uint64_t m,
                             float* dst, void* scratch, int* error_flag, cudaStream_t s);

@@ -65,7 +65,8 @@ int32_t jq_matmul_norm_dev(const jq_weight* w, uint64_t m, uint64_t k, uint64_t 
     jq_ctx* ctx = w->ctx;
     const bool shapes_ok = k % w->fmt.elems == 0 && w->n_blocks == n * (k / w->fmt.elems) && m > 0 && n > 0 &&
                            lhs_dev && dst_dev;
-    if (shapes_ok && !ctx->force_f32 && jq::gemv_mma_supports(w->type, w->dev, n, k, m) && jq::gemv_mma_fusable(m, k)) {
+    if (shapes_ok && !ctx->force_f32 && jq::gemv_mma_dense_supports(w->type, w->dev, n, k, m) &&
+        jq::gemv_mma_fusable(m, k)) {
         JQ_CUDA(jq::launch_gemv_mma_fused(w->type, w->dev, n, k, lhs_dev, m, dst_dev, norm_w_dev, eps, residual_dev,
                                           ctx->status_dev, s));
         return jq::OK;

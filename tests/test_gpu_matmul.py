@@ -55,6 +55,25 @@ def test_generic_path_types_match_oracle(type_id, mkn):
     assert np.array_equal(bits(got), bits(q.matmul_t(mkn, lhs)))      # run-to-run bit equality
 
 
+@pytest.mark.parametrize("mkn", [(1, 256, 1), (2, 512, 17), (4, 4096, 33), (8, 4352, 16), (3, 14336, 31), (5, 8192, 130), (9, 512, 40),
+                                 (70, 768, 47)])
+@pytest.mark.parametrize("skip", [0, 1])
+def test_q6_k_decode_kernel(mkn, skip):
+    """Q6_K on the decode kernel: one unit to several ring chunks per row, every row-count variant, batches in slices,
+    and tensors that start on an odd multiple of two bytes (a slice of `skip` blocks; blocks are 210 bytes).  The bound
+    is the activation split's 6.1e-8 of a unit's largest value per term and f32 sums of k / 256 units: 1e-5 of the
+    terms' 2-norm leaves a factor of ten."""
+    m, k, n = mkn
+    raw = synth.random_weight(synth.Q6_K, n + 1, k, seed=n + k)
+    lhs = synth.random_activations(m, k, seed=m)
+    rows = raw[skip * 210:skip * 210 + n * (k // 256) * 210]
+    got = QTensor.from_bytes(synth.Q6_K, raw).slice_blocks(skip, n * (k // 256)).matmul_t(mkn, lhs)
+    w = oracle.dequantize(synth.Q6_K, rows).reshape(n, k).astype(np.float64)
+    want = lhs.astype(np.float64).reshape(m, k) @ w.T
+    scale = np.sqrt((lhs.astype(np.float64).reshape(m, k) ** 2) @ (w.T ** 2))
+    assert np.all(np.abs(got - want) <= 1e-5 * scale + 1e-30)
+
+
 def test_iq2xxs_golden_block_fixture():
     for mkn, mult in [((3, 512, 7), 7919), ((3, 1024, 11), 7919), ((4, 1024, 23), 104729)]:
         m, k, n = mkn
