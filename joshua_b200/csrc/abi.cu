@@ -93,6 +93,12 @@ int32_t jq_matmul_device(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n,
         }
         return jq::OK;
     }
+    if (!ctx->force_f32 && m > jq::GEMV_MMA_MAX_M && jq::gemm_f16_supports(w->type, w->dev, n, k, m)) {
+        void* scratch = nullptr;
+        JQ_CUDA(ctx->scratch_for(reinterpret_cast<cudaStream_t>(reinterpret_cast<uintptr_t>(s) ^ 3), jq::gemm_f16_scratch_bytes(m, k), &scratch));
+        JQ_CUDA(jq::launch_gemm_f16(w->type, w->dev, n, k, lhs, m, dst, scratch, ctx->status_dev, s));
+        return jq::OK;
+    }
     if (!ctx->force_f32 && m > jq::GEMV_MMA_MAX_M && jq::gemm_tc_supports(w->type, w->dev, n, k, m)) {
         void* scratch = nullptr;
         JQ_CUDA(ctx->scratch_for(reinterpret_cast<cudaStream_t>(reinterpret_cast<uintptr_t>(s) ^ 3), jq::gemm_tc_scratch_bytes(m, k), &scratch));
@@ -169,6 +175,7 @@ int32_t jq_init(int32_t device, jq_ctx** out) {
     JQ_CUDA(jq::tables_gemv_f32());
     JQ_CUDA(jq::tables_gemv_mma());
     JQ_CUDA(jq::tables_gemm_tc());
+    JQ_CUDA(jq::tables_gemm_f16());
     jq_ctx* c = new (std::nothrow) jq_ctx();
     if (!c) return jq_fail(jq::E_NOMEM, "jq_init: out of host memory");
     c->device = device;

@@ -77,7 +77,15 @@ cudaError_t tables_gemv_f32();
 cudaError_t launch_matmul_f32(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, const float* lhs, uint64_t m,
                               float* dst, cudaStream_t s);
 
-// gemm_tc.cu: tcgen05 tile GEMM for m > 8 (prefill, batched decode)
+// gemm_f16.cu: tcgen05 tile GEMM in half-precision terms for m > 8 (prefill, batched decode)
+cudaError_t tables_gemm_f16();
+bool gemm_f16_supports(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, uint64_t m);
+// scratch: gemm_f16_scratch_bytes(m, k) bytes (the activations' two terms, group sums and scales), 256-byte aligned
+size_t gemm_f16_scratch_bytes(uint64_t m, uint64_t k);
+cudaError_t launch_gemm_f16(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, const float* lhs, uint64_t m,
+                            float* dst, void* scratch, int* error_flag, cudaStream_t s);
+
+// gemm_tc.cu: the same for the shapes gemm_f16.cu does not take
 cudaError_t tables_gemm_tc();
 bool gemm_tc_supports(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, uint64_t m);
 // scratch: gemm_tc_scratch_bytes(m, k) bytes (the activations' two TF32 terms), 256-byte aligned
@@ -93,15 +101,15 @@ cudaError_t launch_gemm_tc(uint32_t type, const uint8_t* w, uint64_t n, uint64_t
 // `narrow` (tiles of at most 32 rows, run as 32-token tiles) and `wide`, their lengths in counts[0] and counts[1]
 // (device memory, read by the kernels: the launches cover max_narrow / max_wide entries and the surplus CTAs
 // leave at once), so that no host read stands between the routing and the products.  False from
-// gemm_tc_grouped_supports = shapes this form does not take (the caller then runs one product per expert).
+// gemm_f16_grouped_supports = shapes this form does not take (the caller then runs one product per expert).
 struct GemmTile {
     uint32_t expert;
     uint32_t row0;  // first row of the tile in x / dst
     uint32_t cnt;   // rows, 1..128
     uint32_t pad;
 };
-bool gemm_tc_grouped_supports(uint32_t type, const uint8_t* bank, uint64_t n, uint64_t k);
-cudaError_t launch_gemm_tc_grouped(uint32_t type, const uint8_t* bank_a, const uint8_t* bank_b, uint64_t expert_bytes,
+bool gemm_f16_grouped_supports(uint32_t type, const uint8_t* bank, uint64_t n, uint64_t k);
+cudaError_t launch_gemm_f16_grouped(uint32_t type, const uint8_t* bank_a, const uint8_t* bank_b, uint64_t expert_bytes,
                                    uint64_t n, uint64_t k, const float* x, uint64_t rows, float* dst_a, float* dst_b,
                                    const GemmTile* narrow, uint32_t max_narrow, const GemmTile* wide, uint32_t max_wide,
                                    const uint32_t* counts, void* scratch, int* error_flag, cudaStream_t s);

@@ -91,31 +91,12 @@ __device__ __forceinline__ uint32_t ld_u32(const uint8_t* p) {  // p 4-byte alig
 }
 __device__ __forceinline__ uint32_t ld_u16_bytes(const uint8_t* p) { return ld_u8(p) | (ld_u8(p + 1) << 8); }
 
-// Where a decoder's block bytes live: global memory (read-only path) or this CTA's shared memory.
+// How a decoder reads its block bytes: global memory, read-only path.
 struct LdGlobal {
     static __device__ __forceinline__ uint32_t u8(const uint8_t* p) { return ld_u8(p); }
     static __device__ __forceinline__ uint32_t u16(const uint8_t* p) { return ld_u16(p); }
     static __device__ __forceinline__ uint32_t u32(const uint8_t* p) { return ld_u32(p); }
 };
-struct LdShared {
-    static __device__ __forceinline__ uint32_t addr(const uint8_t* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-    static __device__ __forceinline__ uint32_t u8(const uint8_t* p) {
-        uint32_t v;
-        asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(addr(p)));
-        return v;
-    }
-    static __device__ __forceinline__ uint32_t u16(const uint8_t* p) {  // p 2-byte aligned
-        uint32_t v;
-        asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(addr(p)));
-        return v;
-    }
-    static __device__ __forceinline__ uint32_t u32(const uint8_t* p) {  // p 4-byte aligned
-        uint32_t v;
-        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr(p)));
-        return v;
-    }
-};
-
 // The 8-bit sign pattern of a 7-bit IQ2_XXS sign index: bit 7 makes the
 // population count even (the reference's KSIGNS table, src/iq2xxs.rs:441-449).
 __device__ __forceinline__ uint32_t iq2_signs(uint32_t idx7) { return idx7 | ((__popc(idx7) & 1u) << 7); }

@@ -1,0 +1,865 @@
+// Prefill / batched matmul (m > 8) over raw GGUF blocks on the 5th-generation tensor cores, in half precision terms
+// that lose nothing against f32.
+//
+// dst[m, n] = lhs[m, k] . W[n, k]^T with W left in its GGUF bytes.  A CTA owns 128 rows of W and up to N_TILE rows of
+// lhs.  Per window of 256 columns (one super-block of the K formats) the weights of a row are one f32 factor times
+// numbers that f16 holds exactly, or as two terms:
+//
+//   Q4_K, Q2_K   d  * (scale * code)            <= 945, 45: one term; the minima below
+//   IQ2_XXS      d/8 * (2 s + 1) * (+-grid)     <= 1333: one term
+//   MXFP4        2^(e_max - 139) * (E2M1 * 2^(e - e_max + 12))   one term
+//   Q8_0         2^p * (code * d_block / 2^p)   18 bits: two terms, the second by an exact fused multiply-subtract
+//
+// The activations are split once per launch (`split_f16_kernel`): a row is scaled by a power of two that puts its
+// largest value just below 2^10, hi = f16(x), lo = f16(x - hi), so hi + lo carries 22 to 24 bits of every value within
+// 2^17 of the row's largest one and an absolute error below 2^-35 of it otherwise.  The tensor core's products of
+// f16 terms are exact; two or three products (hi*hi, hi*lo, lo*hi) replace the three TF32 products of the form
+// below at twice their rate: 32 to 48 instructions per window instead of 96.
+//
+// Minima (Q4_K, Q2_K): sum_c dmin m_g x_c = sum_g (dmin m_g) (sum of x over the group), an inner product of 16 terms per
+// window.  The split kernel also writes the sums of each 16 values as two f16 terms, the converters write
+// -(dmin / f) m_g as two f16 terms, and three more instructions add their product to the same accumulator.
+//
+// The tensor core adds into its f32 accumulator with truncation, so an accumulator only ever holds one window: the
+// converter warps read it back with tcgen05.ld and add f * acc, round-to-nearest, to running sums in registers while
+// the next window accumulates in the other half of tensor memory.
+//
+// Tensor memory, 512 columns: [0, 2N) two accumulators, then four stages of 64 columns: 32 columns the first terms of
+// 64 weights (two per column), 32 the second terms (or, in the last stage of a window, the minima), weight row r in
+// lane r.  The activation ring in shared memory has the same four stages, 64 columns each.
+//
+// Warps: 16 converters, warp (q = w % 4, g = w / 4) owns weight rows 32q .. 32q+31 (the tensor-memory lanes it may
+// touch) and the columns 64g .. 64g+63 of every window; the four warps of a quarter share the staged raw bytes of a
+// window and hand them over through pairs of mbarriers.  Warp 16 issues the MMAs, warp 17 the TMA copies.
+//
+// Few tiles (small n, or few rows of lhs) leave SMs idle: then a cluster of S CTAs splits k, every CTA leaves its
+// partial tile in its shared memory, and each adds a share of the tile over the cluster in rank order (distributed
+// shared memory), so results do not depend on timing.
+//
+// Every wait on an mbarrier is bounded; a wait that runs out raises the device status flag, and every thread still
+// reaches the common exit where tensor memory is released.
+#include <algorithm>
+
+#include <cudaTypedefs.h>
+
+#include "common.cuh"
+#include "tc5.cuh"
+
+namespace jq {
+
+cudaError_t tables_gemm_f16() { return upload_tables(); }
+
+namespace {
+
+constexpr int HM = 128;           // weight rows per CTA = MMA M = TMEM lanes
+constexpr int H_CONV = 16;        // converter / epilogue warps
+constexpr int H_THREADS = (H_CONV + 2) * 32;
+constexpr uint32_t H_STEPS = 4;   // 64-column steps per 256-column window = ring stages
+
+template <uint32_t TYPE>
+struct HT;  // UNIT: bytes of 256 columns of a row; UNITS: windows staged together (whole 32-bit words)
+template <>
+struct HT<T_Q4_K> {
+    static constexpr uint32_t UNIT = 144, UNITS = 1, BUFS = 2;
+    static constexpr bool TWO = false, MIN = true, VEC16 = true;
+};
+template <>
+struct HT<T_Q2_K> {
+    static constexpr uint32_t UNIT = 84, UNITS = 1, BUFS = 2;
+    static constexpr bool TWO = false, MIN = true, VEC16 = false;
+};
+template <>
+struct HT<T_IQ2_XXS> {
+    static constexpr uint32_t UNIT = 66, UNITS = 2, BUFS = 2;
+    static constexpr bool TWO = false, MIN = false, VEC16 = false;
+};
+template <>
+struct HT<T_MXFP4> {
+    static constexpr uint32_t UNIT = 136, UNITS = 1, BUFS = 2;
+    static constexpr bool TWO = false, MIN = false, VEC16 = false;
+};
+template <>
+struct HT<T_Q8_0> {
+    static constexpr uint32_t UNIT = 272, UNITS = 1, BUFS = 2;
+    static constexpr bool TWO = true, MIN = false, VEC16 = false;
+};
+// Row stride of the staged bytes in words: odd, so that 32 lanes reading the same word of their rows hit 32 banks;
+// Q4_K rows (nine 16-byte vectors) are read as vectors, which 36 words spread over the banks.
+template <uint32_t TYPE>
+constexpr uint32_t raw_stride() {
+    return HT<TYPE>::VEC16 ? HT<TYPE>::UNIT / 4 : (HT<TYPE>::UNIT * HT<TYPE>::UNITS / 4) | 1u;
+}
+template <uint32_t TYPE, int N_TILE>
+constexpr size_t h_smem_bytes() {
+    return (size_t)H_STEPS * 2 * N_TILE * 128 + (HT<TYPE>::MIN ? N_TILE * 128 : 0) +
+           (size_t)HT<TYPE>::BUFS * HM * raw_stride<TYPE>() * 4 + (TYPE == T_IQ2_XXS ? 2048 : 0) + 1024;
+}
+
+// Instruction descriptor: D f32, A and B f16, both K-major, M = 128, N = n_tile.
+__device__ __forceinline__ constexpr uint32_t h_idesc(uint32_t n_tile) {
+    return (1u << 4) | ((n_tile >> 3) << 17) | ((uint32_t)(HM >> 4) << 24);
+}
+// D (tensor memory) += A (tensor memory, 16 columns of k in 8 columns) * B (shared memory)
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
+                                            uint32_t accumulate) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t"
+        "}\n" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+        : "memory");
+}
+
+// ── activations ──
+// One CTA per row; a thread takes 16 consecutive values at a time.  hi / lo [m][k]; sums [m][k / 256][32]: the 16 group
+// sums of a window, first terms then second terms; inv[m]: the inverse of the row's scale.
+__global__ void __launch_bounds__(256) split_f16_kernel(const float* __restrict__ x, uint32_t k, __half* __restrict__ hi,
+                                                        __half* __restrict__ lo, __half* __restrict__ sums,
+                                                        float* __restrict__ inv) {
+    __shared__ float s_max[8];
+    pdl_trigger();
+    pdl_wait();
+    const uint32_t row = blockIdx.x, tid = threadIdx.x, groups = k / 16;
+    const float4* xr = reinterpret_cast<const float4*>(x + (uint64_t)row * k);
+    float amax = 0.0f;
+    for (uint32_t i = tid; i < k / 4; i += 256) {
+        const float4 v = __ldg(xr + i);
+        amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+    if ((tid & 31) == 0) s_max[tid >> 5] = amax;
+    __syncthreads();
+    amax = s_max[0];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) amax = fmaxf(amax, s_max[i]);
+    // scale 2^(136 - e): the largest value lands in [2^9, 2^10), 16 of them sum to less than 2^14.  Clamped where the
+    // scale itself would leave f32 (rows below 2^-118); a row with an infinity keeps it.
+    const uint32_t e = __float_as_uint(amax) >> 23;
+    const uint32_t se = e == 255 ? 127u : min(254u, 263u - e);
+    const float scale = __uint_as_float(se << 23);
+    if (tid == 0) inv[row] = se == 254 ? __uint_as_float(0x00400000u) : __uint_as_float((254u - se) << 23);
+    for (uint32_t g = tid; g < groups; g += 256) {
+        uint32_t h[8], l[8];
+        float sum = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float4 v = __ldg(xr + 4 * g + j);
+            v.x *= scale, v.y *= scale, v.z *= scale, v.w *= scale;
+            sum += (v.x + v.y) + (v.z + v.w);
+            const __half2 h0 = __floats2half2_rn(v.x, v.y), h1 = __floats2half2_rn(v.z, v.w);
+            const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
+            const __half2 l0 = __floats2half2_rn(v.x - f0.x, v.y - f0.y), l1 = __floats2half2_rn(v.z - f1.x, v.w - f1.y);
+            h[2 * j] = *reinterpret_cast<const uint32_t*>(&h0), h[2 * j + 1] = *reinterpret_cast<const uint32_t*>(&h1);
+            l[2 * j] = *reinterpret_cast<const uint32_t*>(&l0), l[2 * j + 1] = *reinterpret_cast<const uint32_t*>(&l1);
+        }
+        uint4* hp = reinterpret_cast<uint4*>(hi + (uint64_t)row * k + 16 * g);
+        uint4* lp = reinterpret_cast<uint4*>(lo + (uint64_t)row * k + 16 * g);
+        hp[0] = make_uint4(h[0], h[1], h[2], h[3]), hp[1] = make_uint4(h[4], h[5], h[6], h[7]);
+        lp[0] = make_uint4(l[0], l[1], l[2], l[3]), lp[1] = make_uint4(l[4], l[5], l[6], l[7]);
+        const __half sh = __float2half_rn(sum);
+        __half* sp = sums + ((uint64_t)row * (k / 256) + (g >> 4)) * 32 + (g & 15);
+        sp[0] = sh;
+        sp[16] = __float2half_rn(sum - __half2float(sh));
+    }
+}
+
+// ── weights: 32 columns of a row -> packed f16 terms ──
+__device__ __forceinline__ uint32_t s32(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ uint32_t s16(uint32_t addr) {
+    uint32_t v;
+    asm volatile("{\n\t.reg .u16 t;\n\tld.shared.u16 t, [%1];\n\tcvt.u32.u16 %0, t;\n\t}" : "=r"(v) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ uint32_t s8(uint32_t addr) { return (s32(addr & ~3u) >> ((addr & 3u) * 8)) & 0xFFu; }
+__device__ __forceinline__ uint4 s128(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+    return v;
+}
+// N consecutive words from any byte address
+template <int N>
+__device__ __forceinline__ void s_words(uint32_t addr, uint32_t (&w)[N]) {
+    const uint32_t al = addr & ~3u, sh = (addr & 3u) * 8;
+    uint32_t prev = s32(al);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        // the word behind an aligned run may lie outside the row: it is not needed and not read
+        const uint32_t next = (i + 1 < N || sh) ? s32(al + 4 * (i + 1)) : 0u;
+        w[i] = __funnelshift_r(prev, next, sh);
+        prev = next;
+    }
+}
+__device__ __forceinline__ __half2 as_h2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
+__device__ __forceinline__ uint32_t as_u32(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
+// Bytes b0..b3 (0..255) as two half2 of 1024 + byte: exact, and one fused multiply-add away from scale * byte.
+__device__ __forceinline__ void bytes_1024(uint32_t b, __half2* lo, __half2* hi) {
+    *lo = as_h2(__byte_perm(b, 0x64646464u, 0x4140));
+    *hi = as_h2(__byte_perm(b, 0x64646464u, 0x4342));
+}
+__device__ __forceinline__ float pow2_f32(int e) {  // 2^e for -149 <= e <= 127
+    return e >= -126 ? __uint_as_float((uint32_t)(e + 127) << 23) : __uint_as_float(1u << (e + 149));
+}
+
+// Per window and row: the f32 factor of the accumulated products, and what the terms need of it.
+struct RowWin {
+    float f;      // result = f * accumulator
+    float aux;    // Q4_K / Q2_K: scale of the codes (a power of two); Q8_0: 1 / f; MXFP4: e_max
+    float dmin;   // Q4_K / Q2_K: dmin / f
+};
+
+// The codes' factor f = d 2^e.  Usually e = 0; where dmin is 2^10 times d or more the codes are scaled down by 2^-e
+// (exact, f16 has subnormals down to 2^-24) so that the minima stay inside f16: |dmin / f * m| <= 1024 * 63.
+__device__ __forceinline__ RowWin min_factors(float d, float dmin) {
+    const float ratio = fabsf(dmin) / fabsf(d);
+    if (!(ratio >= 1024.0f)) {  // also d = dmin = 0 (and NaN)
+        const bool zero = d == 0.0f;
+        return {d, 1.0f, zero ? 0.0f : dmin / d};
+    }
+    if (d == 0.0f) return {dmin * (1.0f / 512.0f), 0.0f, 512.0f};
+    const int e = (int)(__float_as_uint(ratio) >> 23) - 127 - 9;
+    const float f = d * pow2_f32(min(e, 100));
+    return {f, e <= 24 ? pow2_f32(-e) : 0.0f, dmin / f};
+}
+
+template <uint32_t TYPE>
+__device__ __forceinline__ RowWin row_window(uint32_t u) {  // u: shared address of the row's 256 columns
+    if constexpr (TYPE == T_Q4_K) {
+        const uint32_t dd = s32(u);
+        return min_factors(f16_bits_to_f32(dd & 0xFFFF), f16_bits_to_f32(dd >> 16));
+    } else if constexpr (TYPE == T_Q2_K) {
+        const uint32_t dd = s32(u + 80);
+        return min_factors(f16_bits_to_f32(dd & 0xFFFF), f16_bits_to_f32(dd >> 16));
+    } else if constexpr (TYPE == T_IQ2_XXS) {
+        return {f16_bits_to_f32(s16(u)) * 0.125f, 0.0f, 0.0f};
+    } else if constexpr (TYPE == T_Q8_0) {
+        uint32_t mx = 0;
+#pragma unroll
+        for (int b = 0; b < 8; ++b) mx = max(mx, s16(u + 34 * b) & 0x7FFFu);
+        // the largest |d| / f lies in [128, 256): codes times it stay below 2^15
+        const float amax = f16_bits_to_f32(mx);
+        const int p = mx == 0 ? 0 : (int)(__float_as_uint(amax) >> 23) - 127 - 7;
+        return {pow2_f32(p), pow2_f32(-p), 0.0f};
+    } else {
+        uint32_t mx = 0;
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+            const uint32_t e = s8(u + 17 * b);
+            mx = max(mx, e == 255u ? 0u : e);
+        }
+        return {pow2_f32((int)mx - 139), (float)mx, 0.0f};
+    }
+}
+
+// Columns 32 G .. 32 G + 31 of the window: 16 packed first terms and (two-term types) 16 second terms.
+template <uint32_t TYPE>
+__device__ __forceinline__ void convert32(uint32_t u, uint32_t G, const RowWin& rw, const uint2* s_grid, uint32_t (&a)[16],
+                                          [[maybe_unused]] uint32_t (&b)[16]) {
+    if constexpr (TYPE == T_Q4_K) {
+        const uint4 hd = s128(u);
+        const uint32_t j = G & 3;
+        const uint32_t sc = G < 4 ? (hd.y >> (8 * j)) & 63u
+                                  : ((hd.w >> (8 * j)) & 15u) | (((hd.y >> (8 * j + 6)) & 3u) << 4);
+        const __half2 s2 = __float2half2_rn((float)sc * rw.aux), off = __hmul2(s2, __float2half2_rn(-1024.0f));
+        const uint32_t sh = 4 * (G & 1);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const uint4 v = s128(u + 16 + 32 * (G >> 1) + 16 * i);
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                __half2 lo, hi;
+                bytes_1024((w[q] >> sh) & 0x0F0F0F0Fu, &lo, &hi);
+                a[8 * i + 2 * q] = as_u32(__hfma2(lo, s2, off));
+                a[8 * i + 2 * q + 1] = as_u32(__hfma2(hi, s2, off));
+            }
+        }
+    } else if constexpr (TYPE == T_Q2_K) {
+        const uint32_t sh = 2 * (G & 3), qb = u + 16 + 32 * (G >> 2);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {  // 16-value group 2G + i
+            const uint32_t sc = s8(u + 2 * G + i) & 15u;
+            const __half2 s2 = __float2half2_rn((float)sc * rw.aux), off = __hmul2(s2, __float2half2_rn(-1024.0f));
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                __half2 lo, hi;
+                bytes_1024((s32(qb + 16 * i + 4 * q) >> sh) & 0x03030303u, &lo, &hi);
+                a[8 * i + 2 * q] = as_u32(__hfma2(lo, s2, off));
+                a[8 * i + 2 * q + 1] = as_u32(__hfma2(hi, s2, off));
+            }
+        }
+    } else if constexpr (TYPE == T_IQ2_XXS) {
+        uint32_t g2[2];
+        s_words<2>(u + 2 + 8 * G, g2);
+        const __half2 s2 = __float2half2_rn((float)(2 * (g2[1] >> 28) + 1)), off = __hmul2(s2, __float2half2_rn(-1024.0f));
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+            const uint2 gr = s_grid[(g2[0] >> (8 * l)) & 0xFFu];
+            const uint32_t sg = iq2_signs((g2[1] >> (7 * l)) & 127u);
+            __half2 v[4];
+            bytes_1024(gr.x, &v[0], &v[1]);
+            bytes_1024(gr.y, &v[2], &v[3]);
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {  // sign bits 2p and 2p + 1 -> bits 15 and 31
+                const uint32_t t = sg >> (2 * p);
+                a[4 * l + p] = as_u32(__hfma2(v[p], s2, off)) ^ (((t << 15) & 0x8000u) | ((t << 30) & 0x80000000u));
+            }
+        }
+    } else if constexpr (TYPE == T_MXFP4) {
+        const uint32_t e = s8(u + 17 * G);
+        uint32_t w[4];
+        s_words<4>(u + 17 * G + 1, w);
+        const int ex = (int)e - (int)rw.aux + 12;  // <= 12; below 2^-24 the block is less than 2^-35 of the largest
+        const __half2 s2 = __float2half2_rn(e == 255u || ex < -24 ? 0.0f : pow2_f32(ex));
+        // f16 of 0, .5, 1, 1.5, 2, 3, 4, 6 has a zero low byte: the table holds the high bytes
+        const uint32_t T0 = 0x3E3C3800u, T1 = 0x46444240u;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t m = w[q] & 0x77777777u;
+#pragma unroll
+            for (int hw = 0; hw < 2; ++hw) {  // two code bytes: values 4q + 2hw, + 1 (low nibbles) and those + 16
+                // bytes {low of byte 0, high of byte 0, low of byte 1, high of byte 1}; sign bits 3 and 7 go to bit 7
+                const uint32_t mag = __byte_perm(T0, T1, (m >> (16 * hw)) & 0xFFFFu);
+                const uint32_t by = w[q] >> (16 * hw), sg = (by << 4 & 0x80u) | (by << 8 & 0x8000u) | (by << 12 & 0x800000u) | (by << 16 & 0x80000000u);
+                const uint32_t v = mag | sg;
+                a[2 * q + hw] = as_u32(__hmul2(as_h2(__byte_perm(v, 0, 0x2404)), s2));
+                a[8 + 2 * q + hw] = as_u32(__hmul2(as_h2(__byte_perm(v, 0, 0x3414)), s2));
+            }
+        }
+    } else {  // Q8_0
+        const __half2 r2 = __float2half2_rn(f16_bits_to_f32(s16(u + 34 * G)) * rw.aux);
+        uint32_t w[8];
+        s_words<8>(u + 34 * G + 2, w);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            __half2 v[2];
+            bytes_1024(w[q] ^ 0x80808080u, &v[0], &v[1]);
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                const __half2 c = __hsub2(v[p], __float2half2_rn(1152.0f)), hi = __hmul2(c, r2);
+                a[2 * q + p] = as_u32(hi);
+                b[2 * q + p] = as_u32(__hfma2(c, r2, __hneg2(hi)));
+            }
+        }
+    }
+}
+
+// The window's 16 minima, -(dmin / f) m, as eight packed first and eight packed second terms.
+template <uint32_t TYPE>
+__device__ __forceinline__ void convert_minima(uint32_t u, const RowWin& rw, uint32_t (&a)[16]) {
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {  // groups of 16 values 2p, 2p + 1
+        float m0, m1;
+        if constexpr (TYPE == T_Q4_K) {  // one minimum per 32 values
+            const uint32_t m6 = p < 4 ? s8(u + 8 + p) & 63u : (s8(u + 8 + p) >> 4) | ((s8(u + 4 + p) >> 6) << 4);
+            m0 = m1 = (float)m6;
+        } else {
+            m0 = (float)(s8(u + 2 * p) >> 4);
+            m1 = (float)(s8(u + 2 * p + 1) >> 4);
+        }
+        m0 *= -rw.dmin, m1 *= -rw.dmin;
+        const __half2 h = __floats2half2_rn(m0, m1);
+        const float2 hf = __half22float2(h);
+        a[p] = as_u32(h);
+        a[8 + p] = as_u32(__floats2half2_rn(m0 - hf.x, m1 - hf.y));
+    }
+}
+
+template <uint32_t TYPE, int N_TILE>
+__global__ void __launch_bounds__(H_THREADS, 1)
+    gemm_f16_kernel(const uint8_t* __restrict__ w_a, uint64_t n, uint64_t k, const __grid_constant__ CUtensorMap map_hi,
+                    const __grid_constant__ CUtensorMap map_lo, const __grid_constant__ CUtensorMap map_sums,
+                    const float* __restrict__ inv, uint64_t m_rows, float* __restrict__ dst_a, int* __restrict__ error_flag,
+                    const GemmTile* __restrict__ tiles, const uint32_t* __restrict__ n_tiles, uint64_t expert_bytes,
+                    const uint8_t* __restrict__ w_b, float* __restrict__ dst_b, uint32_t split) {
+    using T = HT<TYPE>;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    constexpr uint32_t PLANE_B = N_TILE * 128;  // 64 f16 columns of N_TILE rows
+    constexpr uint32_t STAGE = 2 * PLANE_B;     // hi | lo
+    constexpr uint32_t A_COL0 = 2 * N_TILE;
+    constexpr uint32_t RAW_STRIDE = raw_stride<TYPE>();
+    constexpr uint32_t RAW_BUF = HM * RAW_STRIDE * 4;
+    constexpr uint32_t WIN_WORDS = T::UNIT * T::UNITS / 4;
+    constexpr int MY_COLS = N_TILE / 4;
+    static_assert(2 * N_TILE + 64 * H_STEPS <= 512 && MY_COLS % 8 == 0, "tile shape");
+    uint8_t* s_sums = smem + (size_t)H_STEPS * STAGE;
+    uint8_t* raw = s_sums + (T::MIN ? PLANE_B : 0);
+    uint2* s_grid = reinterpret_cast<uint2*>(raw + T::BUFS * RAW_BUF);
+    // full[s]: the step's four converter warps + the TMA thread (and the tiles' bytes); empty[s]: the MMAs' commit
+    __shared__ uint64_t full[H_STEPS], empty[H_STEPS], acc_full[2], acc_empty[2], raw_full[4][2], raw_empty[4][2];
+    __shared__ uint32_t tmem_base_slot;
+    __shared__ int abort_flag;
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    pdl_trigger();
+    // Grouped form: tile blockIdx.y of the list, its expert's slice of the bank (blockIdx.z picks the bank and its
+    // destination); rows of the tile box beyond the tile's count belong to other experts, are multiplied along and
+    // never stored.  The launch covers the list's capacity, not its length.
+    uint64_t tok0 = (uint64_t)blockIdx.y * N_TILE, m = m_rows;
+    const uint8_t* w = w_a;
+    float* dst = dst_a;
+    if (tiles != nullptr) {
+        pdl_wait();
+        if (blockIdx.y >= *n_tiles) return;
+        const GemmTile t = tiles[blockIdx.y];
+        if (blockIdx.z) w = w_b, dst = dst_b;
+        w += (uint64_t)t.expert * expert_bytes;
+        tok0 = t.row0;
+        m = (uint64_t)t.row0 + t.cnt;
+    }
+    const uint64_t row0 = (uint64_t)blockIdx.x * HM;
+    const uint64_t row_bytes = k / 256 * T::UNIT;
+    // this CTA's share of k, in staged windows
+    const uint32_t rank = split > 1 ? blockIdx.z : 0;
+    const uint32_t all_windows = (uint32_t)(k / (256 * T::UNITS));
+    const uint32_t win0 = (uint32_t)((uint64_t)all_windows * rank / split);
+    const uint32_t n_windows = (uint32_t)((uint64_t)all_windows * (rank + 1) / split) - win0;
+    const uint32_t n_chunks = n_windows * T::UNITS;  // accumulated windows of 256 columns
+
+    if (tid == 0) {
+        for (uint32_t s = 0; s < H_STEPS; ++s) {
+            mbar_init(&full[s], 4 + 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&acc_full[b], 1);
+            mbar_init(&acc_empty[b], H_CONV);
+        }
+        for (int q = 0; q < 4; ++q)
+            for (int b = 0; b < 2; ++b) {
+                mbar_init(&raw_full[q][b], 4);
+                mbar_init(&raw_empty[q][b], 4);
+            }
+        abort_flag = 0;
+        mbar_fence_init();
+    }
+    if (warp == H_CONV) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)),
+                     "r"(512u)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if constexpr (TYPE == T_IQ2_XXS)
+        for (int i = tid; i < 256; i += H_THREADS) s_grid[i] = g_iq2xxs_grid[i];
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_d = tmem_base_slot;
+
+    if (warp < H_CONV) {
+        const uint32_t q = warp & 3, g = warp >> 2;
+        const uint32_t lane_base = (q * 32) << 16;  // this warp's quarter of the tensor-memory lanes
+        float sums[MY_COLS];
+#pragma unroll
+        for (int c = 0; c < MY_COLS; ++c) sums[c] = 0.0f;
+        auto drain = [&](uint32_t c, float f) -> bool {
+            const uint32_t buf = c & 1;
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait(&acc_full[buf], (c >> 1) & 1))) return false;
+            tc_fence_after();
+            const uint32_t taddr = tmem_d + lane_base + buf * N_TILE + g * MY_COLS;
+            if constexpr (MY_COLS == 8) {
+                uint32_t rr[8];
+                tmem_ld8(taddr, rr);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) sums[i] = fmaf(f, __uint_as_float(rr[i]), sums[i]);
+            } else {
+#pragma unroll
+                for (int part = 0; part < MY_COLS / 16; ++part) {
+                    uint32_t rr[16];
+                    tmem_ld16(taddr + part * 16, rr);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) sums[part * 16 + i] = fmaf(f, __uint_as_float(rr[i]), sums[part * 16 + i]);
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[buf]);
+            return true;
+        };
+        // this warp's 8 of the quarter's 32 rows of window wn, consecutive lanes consecutive words (16-byte vectors
+        // where the rows are made of them)
+        const uint32_t raw_q = smem_u32(raw) + q * 32 * RAW_STRIDE * 4;
+        auto copy_window = [&](uint32_t wn) {
+            if (wn < n_windows) {
+                const uint64_t gr0 = row0 + q * 32 + g * 8;
+                const uint32_t dst0 = raw_q + (wn % T::BUFS) * RAW_BUF + g * 8 * RAW_STRIDE * 4;
+                const uint8_t* src0 = w + (uint64_t)(win0 + wn) * (WIN_WORDS * 4);
+                if constexpr (T::VEC16) {
+                    constexpr uint32_t V = T::UNIT / 16;
+#pragma unroll
+                    for (uint32_t i = lane; i < 8 * V; i += 32) {
+                        const uint32_t rr = i / V, c = i - rr * V;
+                        const uint64_t gr = gr0 + rr < n ? gr0 + rr : n - 1;
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst0 + rr * (RAW_STRIDE * 4) + 16 * c),
+                                     "l"(src0 + gr * row_bytes + 16 * c)
+                                     : "memory");
+                    }
+                } else {
+#pragma unroll 1
+                    for (uint32_t rr = 0; rr < 8; ++rr) {
+                        const uint64_t gr = gr0 + rr < n ? gr0 + rr : n - 1;
+                        const uint8_t* src = src0 + gr * row_bytes + lane * 4;
+                        const uint32_t dstp = dst0 + rr * (RAW_STRIDE * 4) + lane * 4;
+#pragma unroll
+                        for (uint32_t c = 0; c < WIN_WORDS; c += 32) {
+                            if (c + lane < WIN_WORDS)
+                                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dstp + c * 4), "l"(src + c * 4)
+                                             : "memory");
+                        }
+                    }
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");  // an empty group past the last window
+        };
+        bool ok = true;
+        float f_prev = 0.0f;
+#pragma unroll
+        for (uint32_t b = 0; b < T::BUFS; ++b) copy_window(b);
+        for (uint32_t wn = 0; wn < n_windows && ok; ++wn) {
+            const uint32_t buf = wn % T::BUFS, par = (wn / T::BUFS) & 1;
+            // my copies of this window have landed; hand them over and wait for the others'
+            asm volatile("cp.async.wait_group %0;" ::"n"(T::BUFS - 1) : "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&raw_full[q][buf]);
+            ok = __all_sync(0xFFFFFFFFu, mbar_wait(&raw_full[q][buf], par));
+            if (!ok) break;
+#pragma unroll 1
+            for (uint32_t cc = 0; cc < T::UNITS; ++cc) {
+                const uint32_t c = wn * T::UNITS + cc;
+                const uint32_t u = raw_q + buf * RAW_BUF + lane * RAW_STRIDE * 4 + cc * T::UNIT;
+                const RowWin rw = row_window<TYPE>(u);
+                // the stage's columns must have been read by the MMAs that used them last
+                ok = __all_sync(0xFFFFFFFFu, mbar_wait(&empty[g], (c & 1) ^ 1));
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t acol = tmem_d + lane_base + A_COL0 + g * 64;
+#pragma unroll
+                for (uint32_t h = 0; h < 2; ++h) {
+                    uint32_t a[16], b[16];
+                    convert32<TYPE>(u, 2 * g + h, rw, s_grid, a, b);
+                    tmem_st16(acol + 16 * h, a);
+                    if constexpr (T::TWO) tmem_st16(acol + 32 + 16 * h, b);
+                }
+                if constexpr (T::MIN) {
+                    if (g == H_STEPS - 1) {
+                        uint32_t a[16];
+                        convert_minima<TYPE>(u, rw, a);
+                        tmem_st16(acol + 32, a);
+                    }
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full[g]);
+                if (cc == T::UNITS - 1) {
+                    // once the quarter's other warps are through with this window too, bring in my rows of a later one
+                    if (wn + T::BUFS < n_windows) {
+                        if (lane == 0) mbar_arrive(&raw_empty[q][buf]);
+                        ok = __all_sync(0xFFFFFFFFu, mbar_wait(&raw_empty[q][buf], par));
+                        if (!ok) break;
+                    }
+                    copy_window(wn + T::BUFS);
+                }
+                // read back the window before this one while this one accumulates
+                if (c > 0) ok = drain(c - 1, f_prev);
+                if (!ok) break;
+                f_prev = rw.f;
+            }
+        }
+        if (ok && n_chunks > 0) ok = drain(n_chunks - 1, f_prev);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        if (!ok) abort_flag = 1;
+        pdl_wait();  // inv and dst belong to the kernels before this one
+        if (split == 1) {
+            const uint64_t out_row = row0 + q * 32 + lane;
+            if (ok && out_row < n) {
+#pragma unroll
+                for (int c = 0; c < MY_COLS; ++c) {
+                    const uint64_t tok = tok0 + g * MY_COLS + c;
+                    if (tok < m) dst[tok * n + out_row] = sums[c] * __ldg(inv + tok);
+                }
+            }
+        } else {
+            // the ring is idle (every MMA of this CTA was waited for): leave the partial tile there, [token][row]
+            float* red = reinterpret_cast<float*>(smem);
+#pragma unroll
+            for (int c = 0; c < MY_COLS; ++c) red[(g * MY_COLS + c) * HM + q * 32 + lane] = sums[c];
+        }
+    } else if (warp == H_CONV) {
+        // ── issuer ──
+        constexpr uint32_t idesc = h_idesc(N_TILE);
+        const uint32_t base0 = smem_u32(smem);
+        const uint64_t d0_hi = umma_desc(base0), d0_lo = umma_desc(base0 + PLANE_B);
+        [[maybe_unused]] const uint64_t d_sums = umma_desc(smem_u32(s_sums));
+        bool ok = true;
+        for (uint32_t c = 0; c < n_chunks && ok; ++c) {
+            const uint32_t buf = c & 1, d = tmem_d + buf * N_TILE;
+            if (c >= 2) {
+                ok = __all_sync(0xFFFFFFFFu, mbar_wait(&acc_empty[buf], ((c >> 1) - 1) & 1));
+                if (!ok) break;
+            }
+#pragma unroll
+            for (uint32_t s = 0; s < H_STEPS; ++s) {
+                ok = __all_sync(0xFFFFFFFFu, mbar_wait(&full[s], c & 1));
+                if (!ok) break;
+                tc_fence_after();  // the converters' tcgen05.st / .ld
+                if (elect_one()) {
+                    const uint64_t so = (uint64_t)s * (STAGE >> 4);
+                    const uint32_t a1 = tmem_d + A_COL0 + s * 64, a2 = a1 + 32;
+#pragma unroll
+                    for (uint32_t kk = 0; kk < 4; ++kk) {  // 16 columns: 8 columns of A, 32 bytes of B's swizzled rows
+                        umma_f16_ts(d, a1 + kk * 8, d0_hi + so + kk * 2, idesc, s != 0 || kk != 0);
+                        umma_f16_ts(d, a1 + kk * 8, d0_lo + so + kk * 2, idesc, 1);
+                        if constexpr (T::TWO) umma_f16_ts(d, a2 + kk * 8, d0_hi + so + kk * 2, idesc, 1);
+                    }
+                    if constexpr (T::MIN) {
+                        if (s == H_STEPS - 1) {
+                            // a tile of sums holds two windows, 64 bytes each: first terms, second terms
+                            const uint64_t ds = d_sums + ((win0 + c) & 1) * 4;
+                            umma_f16_ts(d, a2, ds, idesc, 1);
+                            umma_f16_ts(d, a2 + 8, ds, idesc, 1);
+                            umma_f16_ts(d, a2, ds + 2, idesc, 1);
+                        }
+                    }
+                    umma_commit(&empty[s]);  // both the weight columns and the activation tiles of the stage are free
+                    if (s == H_STEPS - 1) umma_commit(&acc_full[buf]);
+                }
+                __syncwarp();
+            }
+        }
+        if (!ok && lane == 0) abort_flag = 1;
+    } else {
+        // ── activation tiles: one lane keeps the ring of TMA copies full ──
+        if (lane == 0) {
+            pdl_wait();
+            bool ok = true;
+            for (uint32_t c = 0; c < n_chunks && ok; ++c) {
+                const uint32_t col = (win0 * T::UNITS + c) * 256;
+                for (uint32_t s = 0; s < H_STEPS; ++s) {
+                    ok = mbar_wait(&empty[s], (c & 1) ^ 1);
+                    if (!ok) break;
+                    uint8_t* st = smem + (size_t)s * STAGE;
+                    const bool with_sums = T::MIN && s == H_STEPS - 1;
+                    mbar_arrive_expect_tx(&full[s], (with_sums ? 3 : 2) * PLANE_B);
+                    tma_load_2d(st, &map_hi, col + 64 * s, (uint32_t)tok0, &full[s]);
+                    tma_load_2d(st + PLANE_B, &map_lo, col + 64 * s, (uint32_t)tok0, &full[s]);
+                    if (with_sums) tma_load_2d(s_sums, &map_sums, ((win0 + c) >> 1) * 64, (uint32_t)tok0, &full[s]);
+                }
+            }
+            if (!ok) abort_flag = 1;
+        }
+        __syncwarp();
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (split > 1) {
+        cluster_sync_all();
+        // tile element i = token * 128 + row; rank r adds the tokens t = r (mod split), over the ranks in order
+        const uint32_t red = smem_u32(smem);
+        if (abort_flag == 0) {
+            const uint32_t row = tid & (HM - 1);
+            for (uint32_t t = rank + split * (tid / HM); t < N_TILE; t += split * (H_CONV * 32 / HM)) {
+                if (tid >= H_CONV * 32) break;
+                const uint64_t tok = tok0 + t;
+                if (tok >= m || row0 + row >= n) continue;
+                float v = 0.0f;
+                for (uint32_t r = 0; r < split; ++r) v += ld_cluster_f32(red + (t * HM + row) * 4, r);
+                dst[tok * n + row0 + row] = v * __ldg(inv + tok);
+            }
+        }
+        cluster_sync_all();  // no CTA leaves while another reads its shared memory
+    }
+    if (abort_flag && tid == 0) *reinterpret_cast<volatile int*>(error_flag) = 1;
+    if (warp == H_CONV) {
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(512u) : "memory");
+    }
+}
+
+// ── host side ──
+PFN_cuTensorMapEncodeTiled g_encode_f16 = nullptr;
+
+cudaError_t f16_map(const __half* base, uint64_t rows, uint64_t cols, uint32_t n_tile, CUtensorMap* out) {
+    if (!g_encode_f16) {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult qres;
+        cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres);
+        if (e != cudaSuccess) return e;
+        if (qres != cudaDriverEntryPointSuccess || !fn) return cudaErrorNotSupported;
+        g_encode_f16 = reinterpret_cast<PFN_cuTensorMapEncodeTiled>(fn);
+    }
+    const cuuint64_t dims[2] = {cols, rows};
+    const cuuint64_t strides[1] = {cols * 2};  // a multiple of 64: cols is a multiple of 32
+    const cuuint32_t box[2] = {64, n_tile};    // 64 halves = one 128-byte swizzled row
+    const cuuint32_t estr[2] = {1, 1};
+    CUresult r = g_encode_f16(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(base), dims, strides, box, estr,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);  // rows and columns beyond the array read as zeros
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+struct SplitX {  // the split activations inside the caller's scratch
+    __half *hi, *lo, *sums;
+    float* inv;
+};
+uint64_t up128(uint64_t v) { return (v + 127) & ~(uint64_t)127; }
+SplitX split_in(void* scratch, uint64_t m, uint64_t k) {
+    SplitX x;
+    uint8_t* b = static_cast<uint8_t*>(scratch);
+    x.hi = reinterpret_cast<__half*>(b);
+    b += up128(2 * m * k);
+    x.lo = reinterpret_cast<__half*>(b);
+    b += up128(2 * m * k);
+    x.sums = reinterpret_cast<__half*>(b);
+    b += up128(m * k / 4);
+    x.inv = reinterpret_cast<float*>(b);
+    return x;
+}
+
+// Everything of a launch but the weights' type and the tile width.
+struct F16Launch {
+    const uint8_t *w_a, *w_b;
+    uint64_t n, k, rows, expert_bytes;
+    SplitX x;
+    float *dst_a, *dst_b;
+    const GemmTile* tiles;
+    uint32_t max_tiles;
+    const uint32_t* n_tiles;
+    int* error_flag;
+};
+
+template <uint32_t TYPE, int N_TILE>
+cudaError_t launch_f16_tile(const F16Launch& l, cudaStream_t s) {
+    constexpr size_t smem = h_smem_bytes<TYPE, N_TILE>();
+    static_assert(smem <= 226 * 1024, "shared memory of a tile");
+    auto kern = gemm_f16_kernel<TYPE, N_TILE>;
+    static bool configured[MAX_DEVICES] = {};
+    if (cudaError_t ce = set_max_smem_once(kern, 226 * 1024, configured); ce != cudaSuccess) return ce;
+    CUtensorMap hi, lo, sums;
+    cudaError_t e = f16_map(l.x.hi, l.rows, l.k, N_TILE, &hi);
+    if (e == cudaSuccess) e = f16_map(l.x.lo, l.rows, l.k, N_TILE, &lo);
+    if (e == cudaSuccess) e = f16_map(l.x.sums, l.rows, l.k / 8, N_TILE, &sums);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cfg.blockDim = dim3(H_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    const unsigned gx = (unsigned)((l.n + HM - 1) / HM);
+    uint32_t split = 1;
+    if (l.tiles) {
+        if (l.max_tiles > 65535) return cudaErrorInvalidValue;  // the tile list is walked along grid.y
+        cfg.gridDim = dim3(gx, l.max_tiles, l.w_b ? 2 : 1);
+    } else {
+        // Split k over a cluster where whole tiles fill the SMs badly: waves x (a CTA's windows + about three windows'
+        // worth of filling the pipeline and storing the tile).  Clusters of up to four pack the GPCs without loss.
+        const uint64_t gy = (l.rows + N_TILE - 1) / N_TILE, tiles = gx * gy, sms = (uint64_t)num_sms();
+        const uint64_t windows = l.k / (256 * HT<TYPE>::UNITS);
+        uint64_t best = ~0ull;
+        for (uint32_t c = 1; c <= 4 && c <= windows; ++c) {
+            const uint64_t waves = (tiles * c + sms - 1) / sms;
+            const uint64_t cost = waves * ((windows + c - 1) / c * HT<TYPE>::UNITS + 3 + (c > 1));
+            if (cost < best) best = cost, split = c;
+        }
+        cfg.gridDim = dim3(gx, (unsigned)gy, split);
+        if (gy > 65535) return cudaErrorInvalidValue;
+        if (split > 1) {
+            attr[1].id = cudaLaunchAttributeClusterDimension;
+            attr[1].val.clusterDim.x = 1;
+            attr[1].val.clusterDim.y = 1;
+            attr[1].val.clusterDim.z = split;
+            cfg.numAttrs = 2;
+        }
+    }
+    e = cudaLaunchKernelEx(&cfg, kern, l.w_a, l.n, l.k, hi, lo, sums, (const float*)l.x.inv, l.rows, l.dst_a, l.error_flag,
+                           l.tiles, l.n_tiles, l.expert_bytes, l.w_b, l.dst_b, split);
+    return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+template <int N_TILE>
+cudaError_t launch_f16_typed(uint32_t type, const F16Launch& l, cudaStream_t s) {
+    switch (type) {
+        case T_Q8_0: return launch_f16_tile<T_Q8_0, N_TILE>(l, s);
+        case T_Q2_K: return launch_f16_tile<T_Q2_K, N_TILE>(l, s);
+        case T_Q4_K: return launch_f16_tile<T_Q4_K, N_TILE>(l, s);
+        case T_IQ2_XXS: return launch_f16_tile<T_IQ2_XXS, N_TILE>(l, s);
+        case T_MXFP4: return launch_f16_tile<T_MXFP4, N_TILE>(l, s);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+cudaError_t split_activations_f16(const float* x, uint64_t m, uint64_t k, const SplitX& o, cudaStream_t s) {
+    return launch_pdl(split_f16_kernel, dim3((unsigned)m), 256, 0, s, x, (uint32_t)k, o.hi, o.lo, o.sums, o.inv);
+}
+
+}  // namespace
+
+// Whole staged windows of whole 32-bit words (Q4_K: 16-byte vectors) in every row.
+bool gemm_f16_supports(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, uint64_t m) {
+    if (m == 0 || n == 0 || k == 0 || k % 256 != 0 || k > 0x7FFFFFFFu || m > 0x7FFFFFFFu) return false;
+    const uintptr_t a = reinterpret_cast<uintptr_t>(w);
+    switch (type) {
+        case T_Q4_K: return a % 16 == 0;
+        case T_Q8_0:
+        case T_Q2_K:
+        case T_MXFP4: return a % 4 == 0;
+        case T_IQ2_XXS: return a % 4 == 0 && k % 512 == 0;
+        default: return false;
+    }
+}
+
+size_t gemm_f16_scratch_bytes(uint64_t m, uint64_t k) {
+    return (size_t)(2 * up128(2 * m * k) + up128(m * k / 4) + up128(4 * m));
+}
+
+cudaError_t launch_gemm_f16(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, const float* lhs, uint64_t m, float* dst,
+                            void* scratch, int* error_flag, cudaStream_t s) {
+    F16Launch l = {};
+    l.w_a = w;
+    l.n = n, l.k = k, l.rows = m;
+    l.x = split_in(scratch, m, k);
+    l.dst_a = dst;
+    l.error_flag = error_flag;
+    if (cudaError_t e = split_activations_f16(lhs, m, k, l.x, s); e != cudaSuccess) return e;
+    if (m <= 32) return launch_f16_typed<32>(type, l, s);
+    if (m <= 64) return launch_f16_typed<64>(type, l, s);
+    return launch_f16_typed<128>(type, l, s);
+}
+
+bool gemm_f16_grouped_supports(uint32_t type, const uint8_t* bank, uint64_t n, uint64_t k) {
+    return gemm_f16_supports(type, bank, n, k, 128);
+}
+
+cudaError_t launch_gemm_f16_grouped(uint32_t type, const uint8_t* bank_a, const uint8_t* bank_b, uint64_t expert_bytes,
+                                   uint64_t n, uint64_t k, const float* x, uint64_t rows, float* dst_a, float* dst_b,
+                                   const GemmTile* narrow, uint32_t max_narrow, const GemmTile* wide, uint32_t max_wide,
+                                   const uint32_t* counts, void* scratch, int* error_flag, cudaStream_t s) {
+    F16Launch l = {};
+    l.w_a = bank_a, l.w_b = bank_b;
+    l.n = n, l.k = k, l.rows = rows, l.expert_bytes = expert_bytes;
+    l.x = split_in(scratch, rows, k);
+    l.dst_a = dst_a, l.dst_b = dst_b;
+    l.error_flag = error_flag;
+    if (cudaError_t e = split_activations_f16(x, rows, k, l.x, s); e != cudaSuccess) return e;
+    if (max_narrow) {
+        l.tiles = narrow, l.max_tiles = max_narrow, l.n_tiles = counts;
+        if (cudaError_t e = launch_f16_typed<32>(type, l, s); e != cudaSuccess) return e;
+    }
+    if (max_wide) {
+        l.tiles = wide, l.max_tiles = max_wide, l.n_tiles = counts + 1;
+        return launch_f16_typed<128>(type, l, s);
+    }
+    return cudaSuccess;
+}
+
+}  // namespace jq

@@ -148,8 +148,8 @@ int32_t run_experts_bucketed(jq_moe* m, const float* x, uint64_t T, uint64_t P, 
     // them cut into tiles of up to 128 rows and runs on the tile GEMM, one grouped launch per phase and tile class
     // (gate and up together, then down); the other experts' jobs run on the grouped decode kernel in the same pass.
     // No host read: the launches cover the lists' capacity and the kernels read their lengths.
-    if (jq::gemm_tc_grouped_supports(m->gate->type, m->gate->dev, c.inter, c.hidden) && m->up->type == m->gate->type &&
-        jq::gemm_tc_grouped_supports(m->down->type, m->down->dev, c.hidden, c.inter) && P / 33 + 1 <= 65535) {
+    if (jq::gemm_f16_grouped_supports(m->gate->type, m->gate->dev, c.inter, c.hidden) && m->up->type == m->gate->type &&
+        jq::gemm_f16_grouped_supports(m->down->type, m->down->dev, c.hidden, c.inter) && P / 33 + 1 <= 65535) {
         // a narrow tile (<= 32 rows) is an expert's only tile (>= min rows) or the last piece behind full tiles; a wide
         // tile holds more than 32 rows
         // With 24 or more rows per expert on average hardly an expert is small: every expert then takes the tile
@@ -174,17 +174,17 @@ int32_t run_experts_bucketed(jq_moe* m, const float* x, uint64_t T, uint64_t P, 
         uint32_t* counts = reinterpret_cast<uint32_t*>(
             (reinterpret_cast<uintptr_t>(small_jobs + max_small) + 15) & ~(uintptr_t)15);
         void* scratch = nullptr;
-        const size_t need = std::max(jq::gemm_tc_scratch_bytes(P, c.hidden), jq::gemm_tc_scratch_bytes(P, c.inter));
+        const size_t need = std::max(jq::gemm_f16_scratch_bytes(P, c.hidden), jq::gemm_f16_scratch_bytes(P, c.inter));
         JQ_CUDA(m->ctx->scratch_for(reinterpret_cast<cudaStream_t>(reinterpret_cast<uintptr_t>(s) ^ 3), need, &scratch));
         JQ_CUDA(jq::launch_moe_gather(x, m->list_token, m->n_list, (uint32_t)P, c.hidden, xs, s));
         JQ_CUDA(jq::launch_moe_tiles(m->jobs, m->n_jobs, m->n_list, c.n_expert, min_rows, narrow, wide, small_jobs, counts, s));
-        JQ_CUDA(jq::launch_gemm_tc_grouped(m->gate->type, m->gate->dev, m->up->dev, m->gate_expert_bytes, c.inter, c.hidden, xs, P,
+        JQ_CUDA(jq::launch_gemm_f16_grouped(m->gate->type, m->gate->dev, m->up->dev, m->gate_expert_bytes, c.inter, c.hidden, xs, P,
                                            gbuf, ubuf, narrow, max_narrow, wide, max_wide, counts, scratch, m->ctx->status_dev, s));
         // SwiGLU over every list row (rows of the small experts hold nothing yet; the decode kernel writes them next)
         JQ_CUDA(jq::launch_swiglu_rows(gbuf, ubuf, counts + 2, (uint32_t)P, c.inter, c.clamp, m->hidden, s));
         if (!all_tiles)
             if (int32_t rc = run_experts(m, x, T, P, rows_per_job, s, nullptr, 0.0f, small_jobs, counts + 3, 1)) return rc;
-        JQ_CUDA(jq::launch_gemm_tc_grouped(m->down->type, m->down->dev, nullptr, m->down_expert_bytes, c.hidden, c.inter,
+        JQ_CUDA(jq::launch_gemm_f16_grouped(m->down->type, m->down->dev, nullptr, m->down_expert_bytes, c.hidden, c.inter,
                                            m->hidden, P, m->out, nullptr, narrow, max_narrow, wide, max_wide, counts, scratch,
                                            m->ctx->status_dev, s));
         return all_tiles ? jq::OK : run_experts(m, x, T, P, rows_per_job, s, nullptr, 0.0f, small_jobs, counts + 3, 2);

@@ -72,3 +72,56 @@ def test_sliced_batches_match_oracle(type_id, mkn):
     got = q.matmul_t(mkn, lhs)
     assert_close(got, oracle.matmul_t(type_id, mkn, lhs, raw), what=f"{synth.NAMES[type_id]} {mkn} sliced")
     assert np.array_equal(bits(got), bits(q.matmul_t(mkn, lhs)))
+
+
+def _edge_blocks(type_id, n, k, kind):
+    """Random blocks whose scales sit at an edge of the tile GEMM's per-window factors."""
+    raw = synth.random_weight(type_id, n, k, seed=n + k).reshape(-1, synth.BLOCK[type_id][1]).copy()
+    rng = np.random.default_rng(5)
+
+    def put(offset, values):
+        raw[:, offset:offset + 2] = np.asarray(values, np.float16).view(np.uint8).reshape(-1, 2)
+
+    blocks = raw.shape[0]
+    if type_id in (synth.Q4_K, synth.Q2_K):
+        at = 0 if type_id == synth.Q4_K else 80
+        if kind == "minima":   # dmin from nothing to far above d, and d = 0
+            put(at, np.where(rng.random(blocks) < 0.2, 0.0, 10.0 ** rng.uniform(-6, -1, blocks)))
+            put(at + 2, np.where(rng.random(blocks) < 0.2, 0.0, 10.0 ** rng.uniform(-6, 2, blocks)))
+        else:                  # negative and zero scales
+            put(at, rng.choice([-0.01, 0.0, 0.02, 6e-8], blocks))
+            put(at + 2, rng.choice([-0.01, 0.0, 0.05], blocks))
+    elif type_id == synth.MXFP4:
+        raw[:, 0] = rng.integers(90, 150, blocks) if kind == "minima" else rng.choice([0, 1, 100, 127, 255], blocks)
+    else:
+        put(0, np.where(rng.random(blocks) < 0.2, 0.0, 10.0 ** rng.uniform(-7, 1, blocks)))
+    return raw.reshape(-1)
+
+
+@pytest.mark.parametrize("type_id", [synth.Q4_K, synth.Q2_K, synth.Q8_0, synth.IQ2_XXS, synth.MXFP4])
+@pytest.mark.parametrize("mkn,kind", [((9, 512, 16), "minima"), ((33, 2560, 130), "minima"), ((129, 1536, 257), "signs"),
+                                      ((65, 7168, 128), "minima"), ((64, 512, 600), "signs")])
+def test_scales_and_rows_at_the_edges(type_id, mkn, kind, tc_ctx):
+    """The f16 terms of the tile GEMM against float64: block scales and minima decades apart inside a window, rows of lhs
+    from 1e-30 to 1e30 and rows of zeros, one to four CTAs along k.  Bound: at most 48 truncating additions of 2^-23 per
+    window and terms good to 2^-22, so 48 * 2^-23 + 2^-21 < 7e-6 of the sum of the terms' absolute values; a term below
+    2^-35 of its window's largest may go missing, inside the same bound."""
+    m, k, n = mkn
+    raw = _edge_blocks(type_id, n, k, kind)
+    lhs = synth.random_activations(m, k, seed=m).reshape(m, k).astype(np.float64)
+    lhs *= 10.0 ** np.random.default_rng(1).integers(-30, 31, m)[:, None]
+    lhs[m // 2] = 0.0
+    lhs = lhs.astype(np.float32)
+    got = QTensor.from_bytes(type_id, raw, tc_ctx).matmul_t(mkn, lhs).astype(np.float64)
+    w = oracle.dequantize(type_id, raw).reshape(n, k).astype(np.float64)
+    x = lhs.astype(np.float64)
+    parts = [w]
+    if type_id in (synth.Q4_K, synth.Q2_K):   # the codes' and the minima's terms are summed apart
+        at, parts = (0 if type_id == synth.Q4_K else 80), []
+        for gone in (at, at + 2):
+            blk = raw.reshape(-1, synth.BLOCK[type_id][1]).copy()
+            blk[:, gone:gone + 2] = 0
+            parts.append(oracle.dequantize(type_id, blk.reshape(-1)).reshape(n, k).astype(np.float64))
+    want, size = x @ w.T, np.abs(x) @ sum(np.abs(p) for p in parts).T
+    inside = size < 1e38   # f32 results
+    assert np.all(np.abs(got - want)[inside] <= 7e-6 * size[inside] + 1e-42)
