@@ -3,6 +3,8 @@
 // they replace are in include/joshua_b200.h.
 #include <cuda_fp16.h>
 
+#include <algorithm>
+
 #include "handles.cuh"
 
 namespace {
@@ -66,22 +68,40 @@ int32_t validate_matmul(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, 
     return jq::OK;
 }
 
-// Picks the kernel for a device-resident product.
 }  // namespace
+
+bool jq_uses_tiles(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n) {
+    return !w->ctx->force_f32 && m >= w->ctx->tiles_min_m && jq::gemm_f16_supports(w->type, w->dev, n, k, m);
+}
+
+int32_t jq_matmul_tiles(const jq_weight* w, const jq_weight* w_b, uint64_t m, uint64_t k, uint64_t n, const float* lhs,
+                        const float* norm_w, float eps, const float* residual, float* dst, float* dst_b, cudaStream_t s) {
+    jq_ctx* ctx = w->ctx;
+    void* scratch = nullptr;
+    JQ_CUDA(ctx->scratch_for(reinterpret_cast<cudaStream_t>(reinterpret_cast<uintptr_t>(s) ^ 3),
+                             jq::gemm_f16_scratch_bytes(m, k), &scratch));
+    JQ_CUDA(jq::launch_gemm_f16(w->type, w->dev, w_b ? w_b->dev : nullptr, n, k, lhs, m, norm_w, eps, residual, dst, dst_b,
+                                scratch, ctx->status_dev, s));
+    return jq::OK;
+}
+
+// Picks the kernel for a device-resident product.
 
 int32_t jq_matmul_device(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, const float* lhs, float* dst,
                          cudaStream_t s) {
     jq_ctx* ctx = w->ctx;
+    if (jq_uses_tiles(w, m, k, n)) return jq_matmul_tiles(w, nullptr, m, k, n, lhs, nullptr, 0.0f, nullptr, dst, nullptr, s);
     if (!ctx->force_f32 && jq::gemv_mma_dense_supports(w->type, w->dev, n, k, m)) {
         void* scratch = nullptr;
         JQ_CUDA(ctx->scratch_for(s, jq::gemv_mma_scratch_bytes(m, k), &scratch));
         JQ_CUDA(jq::launch_gemv_mma(w->type, w->dev, n, k, lhs, m, dst, scratch, ctx->status_dev, s));
         return jq::OK;
     }
-    // Batches a little above the decode kernel's eight rows: eight rows at a time through the decode kernel
-    // (the weights are read once per slice, from L2 when they fit) still beats the tile GEMM, whose K loop
-    // costs the same at any batch.  Q6_K has no tile GEMM: any batch goes in slices, which read packed bytes at
-    // terabytes per second where the exact-decode float kernel (the other route) reaches half of one.
+    // What the f16 tiles do not take (k not a whole number of their windows).  Batches a little above the decode
+    // kernel's eight rows: eight rows at a time through the decode kernel (the weights are read once per slice, from
+    // L2 when they fit) still beats the TF32 tile GEMM, whose K loop costs the same at any batch.  Q6_K has no TF32
+    // form: any batch goes in slices, which read packed bytes at terabytes per second where the exact-decode float
+    // kernel (the other route) reaches half of one.
     if (!ctx->force_f32 && m > jq::GEMV_MMA_MAX_M && (m <= ctx->sliced_max_m || w->type == jq::T_Q6_K) &&
         jq::gemv_mma_dense_supports(w->type, w->dev, n, k, jq::GEMV_MMA_MAX_M)) {
         void* scratch = nullptr;
@@ -91,12 +111,6 @@ int32_t jq_matmul_device(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n,
             JQ_CUDA(jq::launch_gemv_mma(w->type, w->dev, n, k, lhs + r0 * k, rows, dst + r0 * n, scratch,
                                         ctx->status_dev, s));
         }
-        return jq::OK;
-    }
-    if (!ctx->force_f32 && m > jq::GEMV_MMA_MAX_M && jq::gemm_f16_supports(w->type, w->dev, n, k, m)) {
-        void* scratch = nullptr;
-        JQ_CUDA(ctx->scratch_for(reinterpret_cast<cudaStream_t>(reinterpret_cast<uintptr_t>(s) ^ 3), jq::gemm_f16_scratch_bytes(m, k), &scratch));
-        JQ_CUDA(jq::launch_gemm_f16(w->type, w->dev, n, k, lhs, m, dst, scratch, ctx->status_dev, s));
         return jq::OK;
     }
     if (!ctx->force_f32 && m > jq::GEMV_MMA_MAX_M && jq::gemm_tc_supports(w->type, w->dev, n, k, m)) {
@@ -181,6 +195,7 @@ int32_t jq_init(int32_t device, jq_ctx** out) {
     c->device = device;
     const char* f = std::getenv("JQ_FORCE_F32_PATH");
     c->force_f32 = f && f[0] == '1';
+    if (const char* tm = std::getenv("JQ_TILES_MIN_M")) c->tiles_min_m = std::max(1ull, std::strtoull(tm, nullptr, 10));
     if (const char* sm = std::getenv("JQ_SLICED_MAX_M")) c->sliced_max_m = std::strtoull(sm, nullptr, 10);
     cudaError_t he = cudaHostAlloc(&c->status_host, sizeof(int), cudaHostAllocMapped);
     if (he == cudaSuccess) he = cudaHostGetDevicePointer(&c->status_dev, c->status_host, 0);

@@ -82,8 +82,11 @@ cudaError_t tables_gemm_f16();
 bool gemm_f16_supports(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, uint64_t m);
 // scratch: gemm_f16_scratch_bytes(m, k) bytes (the activations' two terms, group sums and scales), 256-byte aligned
 size_t gemm_f16_scratch_bytes(uint64_t m, uint64_t k);
-cudaError_t launch_gemm_f16(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, const float* lhs, uint64_t m,
-                            float* dst, void* scratch, int* error_flag, cudaStream_t s);
+// dst_a = residual + norm(lhs) . W^T (norm_w, residual optional; residual may be dst_a); with w_b, a tensor of the same
+// type and shape, also dst_b = norm(lhs) . W_b^T in the same launch (no residual then)
+cudaError_t launch_gemm_f16(uint32_t type, const uint8_t* w_a, const uint8_t* w_b, uint64_t n, uint64_t k, const float* lhs,
+                            uint64_t m, const float* norm_w, float eps, const float* residual, float* dst_a, float* dst_b,
+                            void* scratch, int* error_flag, cudaStream_t s);
 
 // gemm_tc.cu: the same for the shapes gemm_f16.cu does not take
 cudaError_t tables_gemm_tc();

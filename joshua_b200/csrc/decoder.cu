@@ -264,7 +264,9 @@ __global__ void __launch_bounds__(PF_THREADS, 2)
     float* sp = skv + PF_TK * LDQ;        // [PF_TK][LDP] probabilities, key-major
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     pdl_wait_();
-    const uint32_t head = blockIdx.y, kvh = head / (nq / nkv), s0 = blockIdx.x * PF_TQ;
+    // heads run fastest, the last queries first: they see the most keys, and a long CTA in the last wave leaves the
+    // other SMs waiting
+    const uint32_t head = blockIdx.x, kvh = head / (nq / nkv), s0 = (gridDim.y - 1 - blockIdx.y) * PF_TQ;
     const uint32_t tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int32_t p0 = pos[0];
     if (p0 < 0 || (uint64_t)p0 + seq > max_ctx) {
@@ -624,7 +626,7 @@ cudaError_t launch_attention_decode(const float* q, const float* cache_k, const 
 cudaError_t launch_attention_prefill(const float* q, const float* cache_k, const float* cache_v, const int32_t* pos,
                                      uint32_t seq, uint32_t nq, uint32_t nkv, uint32_t hd, uint32_t max_ctx, float* out,
                                      int32_t* bad_pos, cudaStream_t s) {
-    const dim3 grid((seq + PF_TQ - 1) / PF_TQ, nq);
+    const dim3 grid(nq, (seq + PF_TQ - 1) / PF_TQ);
     const size_t smem = (size_t)((PF_TQ + PF_TK) * (hd + 4) + PF_TK * (PF_TQ + 4)) * 4;
     cudaError_t e;
     if (hd == 64) {

@@ -1,6 +1,28 @@
 // C ABI of the decode-step kernels around the matmuls.  Declarations are in include/joshua_b200.h.
 #include "handles.cuh"
 
+namespace {
+
+// The split kernel of the tile GEMM reads rows and norm weights as 16-byte vectors; other buffers take the separate
+// kernels, which copy.
+bool vectors(const float* lhs, const float* norm_w) {
+    return (reinterpret_cast<uintptr_t>(lhs) | reinterpret_cast<uintptr_t>(norm_w)) % 16 == 0;
+}
+
+// silu(clamp(gate x)) * clamp(up x) on the tile GEMM: one launch for both tensors into scratch, then the combine.
+int32_t swiglu_tiles(const jq_weight* gate, const jq_weight* up, uint64_t m, uint64_t k, uint64_t n, const float* lhs,
+                     const float* norm_w, float eps, float* dst, float clamp, cudaStream_t s) {
+    void* scratch = nullptr;
+    JQ_CUDA(gate->ctx->scratch_for(reinterpret_cast<cudaStream_t>(reinterpret_cast<uintptr_t>(s) ^ 1), 2 * m * n * 4 + 512, &scratch));
+    float* g = static_cast<float*>(scratch);
+    float* u = g + ((m * n + 63) & ~(uint64_t)63);
+    if (int32_t rc = jq_matmul_tiles(gate, up, m, k, n, lhs, norm_w, eps, nullptr, g, u, s)) return rc;
+    JQ_CUDA(jq::launch_swiglu(g, u, m * n, clamp, dst, s));
+    return jq::OK;
+}
+
+}  // namespace
+
 extern "C" {
 
 int32_t jq_matmul_swiglu_dev(const jq_weight* gate, const jq_weight* up, uint64_t m, uint64_t k, uint64_t n,
@@ -16,6 +38,8 @@ int32_t jq_matmul_swiglu_dev(const jq_weight* gate, const jq_weight* up, uint64_
     if (!lhs_dev || !dst_dev) return jq_fail(jq::E_INVALID, "jq_matmul_swiglu_dev: NULL buffer");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     jq_ctx* ctx = gate->ctx;
+    if (jq_uses_tiles(gate, m, k, n) && jq_uses_tiles(up, m, k, n))
+        return swiglu_tiles(gate, up, m, k, n, lhs_dev, nullptr, 0.0f, dst_dev, clamp, s);
     if (!ctx->force_f32 && jq::gemv_mma_supports(gate->type, gate->dev, n, k, m) &&
         jq::gemv_mma_supports(up->type, up->dev, n, k, m) && jq::gemv_mma_scratch_bytes(m, k) == 0) {
         JQ_CUDA(jq::launch_gemv_mma_swiglu(gate->type, gate->dev, up->dev, n, k, lhs_dev, m, dst_dev, clamp,
@@ -43,6 +67,8 @@ int32_t jq_matmul_swiglu_norm_dev(const jq_weight* gate, const jq_weight* up, ui
     jq_ctx* ctx = gate->ctx;
     const bool shapes_ok = gate->type == up->type && gate->n_blocks == up->n_blocks && k % gate->fmt.elems == 0 &&
                            gate->n_blocks == n * (k / gate->fmt.elems) && m > 0 && n > 0 && lhs_dev && dst_dev;
+    if (shapes_ok && vectors(lhs_dev, norm_w_dev) && jq_uses_tiles(gate, m, k, n) && jq_uses_tiles(up, m, k, n))
+        return swiglu_tiles(gate, up, m, k, n, lhs_dev, norm_w_dev, eps, dst_dev, clamp, s);
     if (shapes_ok && !ctx->force_f32 && jq::gemv_mma_supports(gate->type, gate->dev, n, k, m) &&
         jq::gemv_mma_supports(up->type, up->dev, n, k, m) && jq::gemv_mma_fusable(m, k)) {
         JQ_CUDA(jq::launch_gemv_mma_swiglu(gate->type, gate->dev, up->dev, n, k, lhs_dev, m, dst_dev, clamp,
@@ -65,6 +91,8 @@ int32_t jq_matmul_norm_dev(const jq_weight* w, uint64_t m, uint64_t k, uint64_t 
     jq_ctx* ctx = w->ctx;
     const bool shapes_ok = k % w->fmt.elems == 0 && w->n_blocks == n * (k / w->fmt.elems) && m > 0 && n > 0 &&
                            lhs_dev && dst_dev;
+    if (shapes_ok && vectors(lhs_dev, norm_w_dev) && jq_uses_tiles(w, m, k, n))
+        return jq_matmul_tiles(w, nullptr, m, k, n, lhs_dev, norm_w_dev, eps, residual_dev, dst_dev, nullptr, s);
     if (shapes_ok && !ctx->force_f32 && jq::gemv_mma_dense_supports(w->type, w->dev, n, k, m) &&
         jq::gemv_mma_fusable(m, k)) {
         JQ_CUDA(jq::launch_gemv_mma_fused(w->type, w->dev, n, k, lhs_dev, m, dst_dev, norm_w_dev, eps, residual_dev,

@@ -9,6 +9,7 @@
 //   IQ2_XXS      d/8 * (2 s + 1) * (+-grid)     <= 1333: one term
 //   MXFP4        2^(e_max - 139) * (E2M1 * 2^(e - e_max + 12))   one term
 //   Q8_0         2^p * (code * d_block / 2^p)   18 bits: two terms, the second by an exact fused multiply-subtract
+//   Q6_K         d  * (scale * code)            13 bits: two terms
 //
 // The activations are split once per launch (`split_f16_kernel`): a row is scaled by a power of two that puts its
 // largest value just below 2^10, hi = f16(x), lo = f16(x - hi), so hi + lo carries 22 to 24 bits of every value within
@@ -20,13 +21,23 @@
 // window.  The split kernel also writes the sums of each 16 values as two f16 terms, the converters write
 // -(dmin / f) m_g as two f16 terms, and three more instructions add their product to the same accumulator.
 //
-// The tensor core adds into its f32 accumulator with truncation, so an accumulator only ever holds one window: the
-// converter warps read it back with tcgen05.ld and add f * acc, round-to-nearest, to running sums in registers while
-// the next window accumulates in the other half of tensor memory.
+// The tensor core adds into its f32 accumulator with truncation, an error that grows with the instructions behind one
+// another, so accumulators are short and the converter warps read them back with tcgen05.ld and add f * acc,
+// round-to-nearest, to running sums in registers.  Tiles of 128 rows of lhs: one accumulator per window, two of them
+// in turn, a column share for every warp.  Tiles of up to 32 rows are as exact as the decode kernel's integer sums:
+// every 64 columns have an accumulator (the small products first, then four instructions of full size), read back by
+// the warps that converted the columns, whose four partial tiles meet in shared memory at the end.
 //
-// Tensor memory, 512 columns: [0, 2N) two accumulators, then four stages of 64 columns: 32 columns the first terms of
-// 64 weights (two per column), 32 the second terms (or, in the last stage of a window, the minima), weight row r in
-// lane r.  The activation ring in shared memory has the same four stages, 64 columns each.
+// Tensor memory, 512 columns: the accumulators, then stages of 64 weights: 32 columns of first terms (two per column)
+// and 32 of second terms where the type has them, weight row r in lane r; then 16 columns of minima per window in
+// flight.  The activation ring in shared memory has the same stages, 64 columns of k each.  A window is four stages;
+// narrow tiles keep two windows in flight, because their products take less time than a conversion.
+//
+// Order of k inside four columns: 0, 2, 1, 3, for the activations and the weights alike, so that a mask picks two
+// codes out of a word of nibbles or bytes (MXFP4, which looks its values up, keeps the plain order).
+//
+// What bounds it: the converters' instruction issue (2 to 3 instructions per weight at first, all in address arithmetic
+// and unpacking; the masks and the flattened copies brought that to about 1.5), the tensor pipe from 128 rows on.
 //
 // Warps: 16 converters, warp (q = w % 4, g = w / 4) owns weight rows 32q .. 32q+31 (the tensor-memory lanes it may
 // touch) and the columns 64g .. 64g+63 of every window; the four warps of a quarter share the staged raw bytes of a
@@ -57,43 +68,71 @@ constexpr int H_THREADS = (H_CONV + 2) * 32;
 constexpr uint32_t H_STEPS = 4;   // 64-column steps per 256-column window = ring stages
 
 template <uint32_t TYPE>
-struct HT;  // UNIT: bytes of 256 columns of a row; UNITS: windows staged together (whole 32-bit words)
+struct HT;  // UNIT: bytes of 256 columns of a row; UNITS: windows staged together (whole 32-bit words); VEC: bytes a copy
 template <>
 struct HT<T_Q4_K> {
-    static constexpr uint32_t UNIT = 144, UNITS = 1, BUFS = 2;
-    static constexpr bool TWO = false, MIN = true, VEC16 = true;
+    static constexpr uint32_t UNIT = 144, UNITS = 1, VEC = 16;
+    static constexpr bool TWO = false, MIN = true;
 };
 template <>
 struct HT<T_Q2_K> {
-    static constexpr uint32_t UNIT = 84, UNITS = 1, BUFS = 2;
-    static constexpr bool TWO = false, MIN = true, VEC16 = false;
+    static constexpr uint32_t UNIT = 84, UNITS = 1, VEC = 4;
+    static constexpr bool TWO = false, MIN = true;
 };
 template <>
 struct HT<T_IQ2_XXS> {
-    static constexpr uint32_t UNIT = 66, UNITS = 2, BUFS = 2;
-    static constexpr bool TWO = false, MIN = false, VEC16 = false;
+    static constexpr uint32_t UNIT = 66, UNITS = 2, VEC = 4;
+    static constexpr bool TWO = false, MIN = false;
 };
 template <>
 struct HT<T_MXFP4> {
-    static constexpr uint32_t UNIT = 136, UNITS = 1, BUFS = 2;
-    static constexpr bool TWO = false, MIN = false, VEC16 = false;
+    static constexpr uint32_t UNIT = 136, UNITS = 1, VEC = 8;
+    static constexpr bool TWO = false, MIN = false;
 };
 template <>
 struct HT<T_Q8_0> {
-    static constexpr uint32_t UNIT = 272, UNITS = 1, BUFS = 2;
-    static constexpr bool TWO = true, MIN = false, VEC16 = false;
+    static constexpr uint32_t UNIT = 272, UNITS = 1, VEC = 8;
+    static constexpr bool TWO = true, MIN = false;
 };
-// Row stride of the staged bytes in words: odd, so that 32 lanes reading the same word of their rows hit 32 banks;
-// Q4_K rows (nine 16-byte vectors) are read as vectors, which 36 words spread over the banks.
+template <>
+struct HT<T_Q6_K> {
+    static constexpr uint32_t UNIT = 210, UNITS = 2, VEC = 4;
+    static constexpr bool TWO = true, MIN = false;
+};
+// Row stride of the staged bytes in words.  Rows copied by the word: odd, so that 32 lanes reading the same word of their
+// rows hit 32 banks.  Q4_K rows are read as 16-byte vectors, which 36 words spread over the banks; rows copied by
+// eight bytes take 34 or 70 words, two lanes a bank.
 template <uint32_t TYPE>
 constexpr uint32_t raw_stride() {
-    return HT<TYPE>::VEC16 ? HT<TYPE>::UNIT / 4 : (HT<TYPE>::UNIT * HT<TYPE>::UNITS / 4) | 1u;
+    constexpr uint32_t words = HT<TYPE>::UNIT * HT<TYPE>::UNITS / 4;
+    return HT<TYPE>::VEC == 4 ? words | 1u : HT<TYPE>::VEC == 8 && words % 4 == 0 ? words + 2 : words;
 }
+// Shape of a tile: windows in flight, buffers of raw bytes (narrow tiles stream weights at memory speed and want tens
+// of kilobytes on their way), accumulators.
 template <uint32_t TYPE, int N_TILE>
-constexpr size_t h_smem_bytes() {
-    return (size_t)H_STEPS * 2 * N_TILE * 128 + (HT<TYPE>::MIN ? N_TILE * 128 : 0) +
-           (size_t)HT<TYPE>::BUFS * HM * raw_stride<TYPE>() * 4 + (TYPE == T_IQ2_XXS ? 2048 : 0) + 1024;
-}
+struct Tile {
+    static constexpr bool FINE = N_TILE <= 32;
+    static constexpr uint32_t WINDOWS = N_TILE <= 32 && !HT<TYPE>::TWO ? 2 : 1;
+    static constexpr uint32_t STAGES = H_STEPS * WINDOWS;
+    static constexpr uint32_t ACCS = FINE ? H_STEPS : 2;
+    static constexpr uint32_t ACC_COLS = ACCS * N_TILE;
+    static constexpr uint32_t A_COLS = HT<TYPE>::TWO ? 64 : 32;
+    static constexpr uint32_t MIN_COL0 = ACC_COLS + STAGES * A_COLS;
+    static_assert(MIN_COL0 + (HT<TYPE>::MIN ? 16 * WINDOWS : 0) <= 512, "tensor memory");
+    static constexpr uint32_t PLANE_B = N_TILE * 128;  // 64 f16 columns of N_TILE rows
+    static constexpr uint32_t STAGE_B = 2 * PLANE_B;   // hi | lo
+    static constexpr uint32_t RAW_BUF = HM * raw_stride<TYPE>() * 4;
+    static constexpr uint32_t FIXED = STAGES * STAGE_B + (HT<TYPE>::MIN ? WINDOWS * PLANE_B : 0) +
+                                      (TYPE == T_IQ2_XXS ? 2048 : 0) + 1024;
+    static constexpr uint32_t ROOM = (226 * 1024 - FIXED) / RAW_BUF;
+    static constexpr uint32_t WANT = N_TILE <= 32 ? 4 : 2;
+    static constexpr uint32_t BUFS = ROOM < WANT ? ROOM : WANT;
+    static_assert(BUFS >= 1, "shared memory");
+    static constexpr uint32_t LOOP_SMEM = FIXED + BUFS * RAW_BUF;
+    static constexpr uint32_t RED_SMEM = (FINE ? 4 : 1) * N_TILE * HM * 4 + 1024;  // the partial tiles at the end
+    static constexpr uint32_t SMEM = LOOP_SMEM > RED_SMEM ? LOOP_SMEM : RED_SMEM;
+    static_assert(SMEM <= 226 * 1024, "shared memory");
+};
 
 // Instruction descriptor: D f32, A and B f16, both K-major, M = 128, N = n_tile.
 __device__ __forceinline__ constexpr uint32_t h_idesc(uint32_t n_tile) {
@@ -115,27 +154,42 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, ui
 // ── activations ──
 // One CTA per row; a thread takes 16 consecutive values at a time.  hi / lo [m][k]; sums [m][k / 256][32]: the 16 group
 // sums of a window, first terms then second terms; inv[m]: the inverse of the row's scale.
-__global__ void __launch_bounds__(256) split_f16_kernel(const float* __restrict__ x, uint32_t k, __half* __restrict__ hi,
+// With norm_w the rows are RMS-normalised first: the values split are x * rs * norm_w.
+__global__ void __launch_bounds__(256) split_f16_kernel(const float* __restrict__ x, uint32_t k,
+                                                        const float* __restrict__ norm_w, float eps, int plain_order,
+                                                        __half* __restrict__ hi,
                                                         __half* __restrict__ lo, __half* __restrict__ sums,
                                                         float* __restrict__ inv) {
-    __shared__ float s_max[8];
+    __shared__ float s_max[8], s_sq[8];
     pdl_trigger();
     pdl_wait();
     const uint32_t row = blockIdx.x, tid = threadIdx.x, groups = k / 16;
     const float4* xr = reinterpret_cast<const float4*>(x + (uint64_t)row * k);
-    float amax = 0.0f;
+    const float4* nr = reinterpret_cast<const float4*>(norm_w);
+    float amax = 0.0f, sq = 0.0f;
+#pragma unroll 4
     for (uint32_t i = tid; i < k / 4; i += 256) {
-        const float4 v = __ldg(xr + i);
+        float4 v = __ldg(xr + i);
+        if (norm_w) {
+            sq = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, sq))));
+            const float4 g = __ldg(nr + i);
+            v.x *= g.x, v.y *= g.y, v.z *= g.z, v.w *= g.w;
+        }
         amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
-    if ((tid & 31) == 0) s_max[tid >> 5] = amax;
+    for (int o = 16; o > 0; o >>= 1) {
+        amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+        sq += __shfl_xor_sync(0xFFFFFFFFu, sq, o);
+    }
+    if ((tid & 31) == 0) s_max[tid >> 5] = amax, s_sq[tid >> 5] = sq;
     __syncthreads();
-    amax = s_max[0];
+    amax = s_max[0], sq = s_sq[0];
 #pragma unroll
-    for (int i = 1; i < 8; ++i) amax = fmaxf(amax, s_max[i]);
-    // scale 2^(136 - e): the largest value lands in [2^9, 2^10), 16 of them sum to less than 2^14.  Clamped where the
+    for (int i = 1; i < 8; ++i) amax = fmaxf(amax, s_max[i]), sq += s_sq[i];
+    const float rs = norm_w ? rsqrtf(sq / (float)k + eps) : 1.0f;
+    amax *= rs;
+    // scale 2^(136 - e): the largest value lands in [2^9, 2^10) (a rounding of the norm aside), 16 sum to about 2^14.  Clamped where the
     // scale itself would leave f32 (rows below 2^-118); a row with an infinity keeps it.
     const uint32_t e = __float_as_uint(amax) >> 23;
     const uint32_t se = e == 255 ? 127u : min(254u, 263u - e);
@@ -147,8 +201,16 @@ __global__ void __launch_bounds__(256) split_f16_kernel(const float* __restrict_
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             float4 v = __ldg(xr + 4 * g + j);
+            if (norm_w) {
+                const float4 w = __ldg(nr + 4 * g + j);
+                v.x = v.x * rs * w.x, v.y = v.y * rs * w.y, v.z = v.z * rs * w.z, v.w = v.w * rs * w.w;
+            }
             v.x *= scale, v.y *= scale, v.z *= scale, v.w *= scale;
             sum += (v.x + v.y) + (v.z + v.w);
+            if (!plain_order) {
+                const float t = v.y;
+                v.y = v.z, v.z = t;
+            }
             const __half2 h0 = __floats2half2_rn(v.x, v.y), h1 = __floats2half2_rn(v.z, v.w);
             const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
             const __half2 l0 = __floats2half2_rn(v.x - f0.x, v.y - f0.y), l1 = __floats2half2_rn(v.z - f1.x, v.w - f1.y);
@@ -198,10 +260,21 @@ __device__ __forceinline__ void s_words(uint32_t addr, uint32_t (&w)[N]) {
 }
 __device__ __forceinline__ __half2 as_h2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
 __device__ __forceinline__ uint32_t as_u32(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
-// Bytes b0..b3 (0..255) as two half2 of 1024 + byte: exact, and one fused multiply-add away from scale * byte.
-__device__ __forceinline__ void bytes_1024(uint32_t b, __half2* lo, __half2* hi) {
-    *lo = as_h2(__byte_perm(b, 0x64646464u, 0x4140));
-    *hi = as_h2(__byte_perm(b, 0x64646464u, 0x4342));
+// Bytes 0 and 2, and 1 and 3, of a word of values below 256 as two half2 of 1024 + byte: exact, and one fused
+// multiply-add away from scale * byte.
+__device__ __forceinline__ void bytes_1024(uint32_t b, __half2* even, __half2* odd) {
+    *even = as_h2(__byte_perm(b, 0x64646464u, 0x4240));
+    *odd = as_h2(__byte_perm(b, 0x64646464u, 0x4341));
+}
+// (w & mask) | bits
+__device__ __forceinline__ uint32_t and_or(uint32_t w, uint32_t mask, uint32_t bits) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(w), "r"(mask), "r"(bits));
+    return r;
+}
+// a small integer (0..255) in both halves, exact
+__device__ __forceinline__ __half2 int_h2(uint32_t v) {
+    return __hsub2(as_h2(__byte_perm(v, 0x64646464u, 0x4040)), __float2half2_rn(1024.0f));
 }
 __device__ __forceinline__ float pow2_f32(int e) {  // 2^e for -149 <= e <= 127
     return e >= -126 ? __uint_as_float((uint32_t)(e + 127) << 23) : __uint_as_float(1u << (e + 149));
@@ -209,35 +282,32 @@ __device__ __forceinline__ float pow2_f32(int e) {  // 2^e for -149 <= e <= 127
 
 // Per window and row: the f32 factor of the accumulated products, and what the terms need of it.
 struct RowWin {
-    float f;      // result = f * accumulator
-    float aux;    // Q4_K / Q2_K: scale of the codes (a power of two); Q8_0: 1 / f; MXFP4: e_max
-    float dmin;   // Q4_K / Q2_K: dmin / f
+    float f;       // result = f * accumulator
+    float aux;     // Q4_K / Q2_K: scale of the codes (a power of two); Q8_0: 1 / f; MXFP4: e_max
+    float d, dmin; // Q4_K / Q2_K
 };
 
 // The codes' factor f = d 2^e.  Usually e = 0; where dmin is 2^10 times d or more the codes are scaled down by 2^-e
 // (exact, f16 has subnormals down to 2^-24) so that the minima stay inside f16: |dmin / f * m| <= 1024 * 63.
-__device__ __forceinline__ RowWin min_factors(float d, float dmin) {
+__device__ __forceinline__ RowWin min_factors(uint32_t dd) {
+    const float d = f16_bits_to_f32(dd & 0xFFFF), dmin = f16_bits_to_f32(dd >> 16);
+    if (!(fabsf(dmin) >= 1024.0f * fabsf(d)) || dmin == 0.0f) return {d, 1.0f, d, dmin};
+    if (d == 0.0f) return {dmin * (1.0f / 512.0f), 0.0f, d, dmin};
     const float ratio = fabsf(dmin) / fabsf(d);
-    if (!(ratio >= 1024.0f)) {  // also d = dmin = 0 (and NaN)
-        const bool zero = d == 0.0f;
-        return {d, 1.0f, zero ? 0.0f : dmin / d};
-    }
-    if (d == 0.0f) return {dmin * (1.0f / 512.0f), 0.0f, 512.0f};
     const int e = (int)(__float_as_uint(ratio) >> 23) - 127 - 9;
-    const float f = d * pow2_f32(min(e, 100));
-    return {f, e <= 24 ? pow2_f32(-e) : 0.0f, dmin / f};
+    return {d * pow2_f32(min(e, 100)), e <= 24 ? pow2_f32(-e) : 0.0f, d, dmin};
 }
 
 template <uint32_t TYPE>
 __device__ __forceinline__ RowWin row_window(uint32_t u) {  // u: shared address of the row's 256 columns
     if constexpr (TYPE == T_Q4_K) {
-        const uint32_t dd = s32(u);
-        return min_factors(f16_bits_to_f32(dd & 0xFFFF), f16_bits_to_f32(dd >> 16));
+        return min_factors(s32(u));
     } else if constexpr (TYPE == T_Q2_K) {
-        const uint32_t dd = s32(u + 80);
-        return min_factors(f16_bits_to_f32(dd & 0xFFFF), f16_bits_to_f32(dd >> 16));
+        return min_factors(s32(u + 80));
     } else if constexpr (TYPE == T_IQ2_XXS) {
-        return {f16_bits_to_f32(s16(u)) * 0.125f, 0.0f, 0.0f};
+        return {f16_bits_to_f32(s16(u)) * 0.125f, 0.0f, 0.0f, 0.0f};
+    } else if constexpr (TYPE == T_Q6_K) {
+        return {f16_bits_to_f32(s16(u + 208)), 0.0f, 0.0f, 0.0f};
     } else if constexpr (TYPE == T_Q8_0) {
         uint32_t mx = 0;
 #pragma unroll
@@ -245,7 +315,7 @@ __device__ __forceinline__ RowWin row_window(uint32_t u) {  // u: shared address
         // the largest |d| / f lies in [128, 256): codes times it stay below 2^15
         const float amax = f16_bits_to_f32(mx);
         const int p = mx == 0 ? 0 : (int)(__float_as_uint(amax) >> 23) - 127 - 7;
-        return {pow2_f32(p), pow2_f32(-p), 0.0f};
+        return {pow2_f32(p), pow2_f32(-p), 0.0f, 0.0f};
     } else {
         uint32_t mx = 0;
 #pragma unroll
@@ -253,99 +323,147 @@ __device__ __forceinline__ RowWin row_window(uint32_t u) {  // u: shared address
             const uint32_t e = s8(u + 17 * b);
             mx = max(mx, e == 255u ? 0u : e);
         }
-        return {pow2_f32((int)mx - 139), (float)mx, 0.0f};
+        return {pow2_f32((int)mx - 139), (float)mx, 0.0f, 0.0f};
     }
 }
 
-// Columns 32 G .. 32 G + 31 of the window: 16 packed first terms and (two-term types) 16 second terms.
-template <uint32_t TYPE>
-__device__ __forceinline__ void convert32(uint32_t u, uint32_t G, const RowWin& rw, const uint2* s_grid, uint32_t (&a)[16],
-                                          [[maybe_unused]] uint32_t (&b)[16]) {
+// Columns 64 g .. 64 g + 63 of the window: h = 0, 1 are its two groups of 32; put(h, a, b) takes 16 packed first terms
+// and (two-term types) 16 second terms.
+template <uint32_t TYPE, class Put>
+__device__ __forceinline__ void convert64(uint32_t u, uint32_t g, const RowWin& rw, const uint2* s_grid, Put put) {
     if constexpr (TYPE == T_Q4_K) {
-        const uint4 hd = s128(u);
-        const uint32_t j = G & 3;
-        const uint32_t sc = G < 4 ? (hd.y >> (8 * j)) & 63u
-                                  : ((hd.w >> (8 * j)) & 15u) | (((hd.y >> (8 * j + 6)) & 3u) << 4);
-        const __half2 s2 = __float2half2_rn((float)sc * rw.aux), off = __hmul2(s2, __float2half2_rn(-1024.0f));
-        const uint32_t sh = 4 * (G & 1);
+        const uint4 hd = s128(u), v0 = s128(u + 16 + 32 * g), v1 = s128(u + 32 + 32 * g);
+        const uint32_t w[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+        // scales of pairs 2g and 2g + 1 in bytes 0 and 1
+        const uint32_t j = 16 * (g & 1);
+        const uint32_t sc = g < 2 ? (hd.y >> j) & 0x3F3Fu : ((hd.w >> j) & 0x0F0Fu) | ((hd.y >> (j + 2)) & 0x3030u);
+        const __half2 aux = __float2half2_rn(rw.aux);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const uint4 v = s128(u + 16 + 32 * (G >> 1) + 16 * i);
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        for (uint32_t h = 0; h < 2; ++h) {
+            // low nibbles: 1024 + q; high nibbles in place: 64 + q (their unit is 1/16 of 64's last place)
+            const uint32_t mask = h ? 0x00F000F0u : 0x000F000Fu, bits = h ? 0x54005400u : 0x64006400u;
+            const __half2 s2 = __hmul2(int_h2((sc >> (8 * h)) & 0xFFu), aux), off = __hmul2(s2, __float2half2_rn(h ? -64.0f : -1024.0f));
+            uint32_t a[16];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                __half2 lo, hi;
-                bytes_1024((w[q] >> sh) & 0x0F0F0F0Fu, &lo, &hi);
-                a[8 * i + 2 * q] = as_u32(__hfma2(lo, s2, off));
-                a[8 * i + 2 * q + 1] = as_u32(__hfma2(hi, s2, off));
+            for (int q = 0; q < 8; ++q) {
+                a[2 * q] = as_u32(__hfma2(as_h2(and_or(w[q], mask, bits)), s2, off));
+                a[2 * q + 1] = as_u32(__hfma2(as_h2(and_or(w[q] >> 8, mask, bits)), s2, off));
             }
+            put(h, a, a);
         }
     } else if constexpr (TYPE == T_Q2_K) {
-        const uint32_t sh = 2 * (G & 3), qb = u + 16 + 32 * (G >> 2);
+        // 32 bytes of four 2-bit fields; this step takes fields 2 (g % 2) and the next.  Field i in place is q in
+        // units of 4^i: 1024 / 4^i + q.
+        const uint32_t qb = u + 16 + 32 * (g >> 1), scs = s32(u + 4 * g);
+        uint32_t w[8];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {  // 16-value group 2G + i
-            const uint32_t sc = s8(u + 2 * G + i) & 15u;
-            const __half2 s2 = __float2half2_rn((float)sc * rw.aux), off = __hmul2(s2, __float2half2_rn(-1024.0f));
+        for (int q = 0; q < 8; ++q) w[q] = s32(qb + 4 * q);
+        const __half2 aux = __float2half2_rn(rw.aux);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                __half2 lo, hi;
-                bytes_1024((s32(qb + 16 * i + 4 * q) >> sh) & 0x03030303u, &lo, &hi);
-                a[8 * i + 2 * q] = as_u32(__hfma2(lo, s2, off));
-                a[8 * i + 2 * q + 1] = as_u32(__hfma2(hi, s2, off));
+        for (uint32_t h = 0; h < 2; ++h) {
+            const uint32_t i = 2 * (g & 1) + h, mask = 0x00030003u << (2 * i), bits = 0x64006400u - i * 0x08000800u;
+            const __half2 base = as_h2(bits | 0x80008000u);
+            uint32_t a[16];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const __half2 s2 = __hmul2(int_h2((scs >> (16 * h + 8 * (q >> 2))) & 15u), aux), off = __hmul2(s2, base);
+                a[2 * q] = as_u32(__hfma2(as_h2(and_or(w[q], mask, bits)), s2, off));
+                a[2 * q + 1] = as_u32(__hfma2(as_h2(and_or(w[q] >> 8, mask, bits)), s2, off));
             }
+            put(h, a, a);
         }
     } else if constexpr (TYPE == T_IQ2_XXS) {
-        uint32_t g2[2];
-        s_words<2>(u + 2 + 8 * G, g2);
-        const __half2 s2 = __float2half2_rn((float)(2 * (g2[1] >> 28) + 1)), off = __hmul2(s2, __float2half2_rn(-1024.0f));
+        uint32_t gw[4];
+        s_words<4>(u + 2 + 16 * g, gw);
 #pragma unroll
-        for (int l = 0; l < 4; ++l) {
-            const uint2 gr = s_grid[(g2[0] >> (8 * l)) & 0xFFu];
-            const uint32_t sg = iq2_signs((g2[1] >> (7 * l)) & 127u);
-            __half2 v[4];
-            bytes_1024(gr.x, &v[0], &v[1]);
-            bytes_1024(gr.y, &v[2], &v[3]);
+        for (uint32_t h = 0; h < 2; ++h) {
+            const uint32_t codes = gw[2 * h], sw = gw[2 * h + 1];
+            const __half2 s2 = int_h2(2 * (sw >> 28) + 1), off = __hmul2(s2, __float2half2_rn(-1024.0f));
+            uint32_t a[16];
 #pragma unroll
-            for (int p = 0; p < 4; ++p) {  // sign bits 2p and 2p + 1 -> bits 15 and 31
-                const uint32_t t = sg >> (2 * p);
-                a[4 * l + p] = as_u32(__hfma2(v[p], s2, off)) ^ (((t << 15) & 0x8000u) | ((t << 30) & 0x80000000u));
+            for (int l = 0; l < 4; ++l) {
+                const uint2 gr = s_grid[(codes >> (8 * l)) & 0xFFu];
+                const uint32_t sg = iq2_signs((sw >> (7 * l)) & 127u);
+                __half2 v[4];
+                bytes_1024(gr.x, &v[0], &v[1]);
+                bytes_1024(gr.y, &v[2], &v[3]);
+#pragma unroll
+                for (int p = 0; p < 4; ++p) {  // values e and e + 2: their sign bits -> bits 15 and 31
+                    const int e = 4 * (p >> 1) + (p & 1);
+                    a[4 * l + p] = as_u32(__hfma2(v[p], s2, off)) ^ (((sg << (15 - e)) & 0x8000u) | ((sg << (29 - e)) & 0x80000000u));
+                }
             }
+            put(h, a, a);
         }
     } else if constexpr (TYPE == T_MXFP4) {
-        const uint32_t e = s8(u + 17 * G);
-        uint32_t w[4];
-        s_words<4>(u + 17 * G + 1, w);
-        const int ex = (int)e - (int)rw.aux + 12;  // <= 12; below 2^-24 the block is less than 2^-35 of the largest
-        const __half2 s2 = __float2half2_rn(e == 255u || ex < -24 ? 0.0f : pow2_f32(ex));
         // f16 of 0, .5, 1, 1.5, 2, 3, 4, 6 has a zero low byte: the table holds the high bytes
         const uint32_t T0 = 0x3E3C3800u, T1 = 0x46444240u;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const uint32_t m = w[q] & 0x77777777u;
+        for (uint32_t h = 0; h < 2; ++h) {
+            const uint32_t blk = u + 17 * (2 * g + h), e = s8(blk);
+            uint32_t w[4];
+            s_words<4>(blk + 1, w);
+            const int ex = (int)e - (int)rw.aux + 12;  // <= 12; below 2^-24 the block is less than 2^-35 of the largest
+            const __half2 s2 = __float2half2_rn(e == 255u || ex < -24 ? 0.0f : pow2_f32(ex));
+            uint32_t a[16];
 #pragma unroll
-            for (int hw = 0; hw < 2; ++hw) {  // two code bytes: values 4q + 2hw, + 1 (low nibbles) and those + 16
-                // bytes {low of byte 0, high of byte 0, low of byte 1, high of byte 1}; sign bits 3 and 7 go to bit 7
-                const uint32_t mag = __byte_perm(T0, T1, (m >> (16 * hw)) & 0xFFFFu);
-                const uint32_t by = w[q] >> (16 * hw), sg = (by << 4 & 0x80u) | (by << 8 & 0x8000u) | (by << 12 & 0x800000u) | (by << 16 & 0x80000000u);
-                const uint32_t v = mag | sg;
-                a[2 * q + hw] = as_u32(__hmul2(as_h2(__byte_perm(v, 0, 0x2404)), s2));
-                a[8 + 2 * q + hw] = as_u32(__hmul2(as_h2(__byte_perm(v, 0, 0x3414)), s2));
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t m = w[q] & 0x77777777u, w4 = w[q] << 4;
+#pragma unroll
+                for (int hw = 0; hw < 2; ++hw) {  // two code bytes: values 4q + 2hw, + 1 (low nibbles) and those + 16
+                    // bytes {low of byte 0, high of byte 0, low of byte 1, high of byte 1}, then their sign bits (the top
+                    // bits of the bytes of w << 4 and w)
+                    const uint32_t mag = __byte_perm(T0, T1, hw ? m >> 16 : m & 0xFFFFu);
+                    const uint32_t v = and_or(__byte_perm(w[q], w4, hw ? 0x3726 : 0x1504), 0x80808080u, mag);
+                    a[2 * q + hw] = as_u32(__hmul2(as_h2(__byte_perm(v, 0, 0x2404)), s2));
+                    a[8 + 2 * q + hw] = as_u32(__hmul2(as_h2(__byte_perm(v, 0, 0x3414)), s2));
+                }
             }
+            put(h, a, a);
         }
-    } else {  // Q8_0
-        const __half2 r2 = __float2half2_rn(f16_bits_to_f32(s16(u + 34 * G)) * rw.aux);
-        uint32_t w[8];
-        s_words<8>(u + 34 * G + 2, w);
+    } else if constexpr (TYPE == T_Q8_0) {
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            __half2 v[2];
-            bytes_1024(w[q] ^ 0x80808080u, &v[0], &v[1]);
+        for (uint32_t h = 0; h < 2; ++h) {
+            const uint32_t blk = u + 34 * (2 * g + h);
+            const __half2 r2 = __float2half2_rn(f16_bits_to_f32(s16(blk)) * rw.aux);
+            uint32_t w[8], a[16], b[16];
+            s_words<8>(blk + 2, w);
 #pragma unroll
-            for (int p = 0; p < 2; ++p) {
-                const __half2 c = __hsub2(v[p], __float2half2_rn(1152.0f)), hi = __hmul2(c, r2);
-                a[2 * q + p] = as_u32(hi);
-                b[2 * q + p] = as_u32(__hfma2(c, r2, __hneg2(hi)));
+            for (int q = 0; q < 8; ++q) {
+                __half2 v[2];
+                bytes_1024(w[q] ^ 0x80808080u, &v[0], &v[1]);
+#pragma unroll
+                for (int p = 0; p < 2; ++p) {
+                    const __half2 c = __hsub2(v[p], __float2half2_rn(1152.0f)), hi = __hmul2(c, r2);
+                    a[2 * q + p] = as_u32(hi);
+                    b[2 * q + p] = as_u32(__hfma2(c, r2, __hneg2(hi)));
+                }
             }
+            put(h, a, b);
+        }
+    } else {  // Q6_K: half = g / 2; part = 2 (g % 2) + h takes nibble g % 2 of low run h and bit pair `part`
+        uint32_t qh[8];
+        s_words<8>(u + 128 + 32 * (g >> 1), qh);
+#pragma unroll
+        for (uint32_t h = 0; h < 2; ++h) {
+            uint32_t ql[8], a[16], b[16];
+            s_words<8>(u + 64 * (g >> 1) + 32 * h, ql);
+            const uint32_t nsh = 4 * (g & 1), part = 2 * (g & 1) + h;
+            const __half2 r[2] = {__float2half2_rn((float)(int8_t)s8(u + 192 + 4 * g + 2 * h)),
+                                  __float2half2_rn((float)(int8_t)s8(u + 193 + 4 * g + 2 * h))};
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const uint32_t code = ((ql[q] >> nsh) & 0x0F0F0F0Fu) | (((qh[q] >> (2 * part)) & 0x03030303u) << 4);
+                __half2 v[2];
+                bytes_1024(code, &v[0], &v[1]);
+#pragma unroll
+                for (int p = 0; p < 2; ++p) {
+                    const __half2 c = __hsub2(v[p], __float2half2_rn(1056.0f)), hi = __hmul2(c, r[q >> 2]);
+                    a[2 * q + p] = as_u32(hi);
+                    b[2 * q + p] = as_u32(__hfma2(c, r[q >> 2], __hneg2(hi)));
+                }
+            }
+            put(h, a, b);
         }
     }
 }
@@ -353,6 +471,8 @@ __device__ __forceinline__ void convert32(uint32_t u, uint32_t G, const RowWin& 
 // The window's 16 minima, -(dmin / f) m, as eight packed first and eight packed second terms.
 template <uint32_t TYPE>
 __device__ __forceinline__ void convert_minima(uint32_t u, const RowWin& rw, uint32_t (&a)[16]) {
+    // -dmin / f, where f is d, d 2^e or (d = 0) dmin / 512
+    const float ratio = rw.dmin == 0.0f ? 0.0f : -(rw.dmin / rw.f);
 #pragma unroll
     for (int p = 0; p < 8; ++p) {  // groups of 16 values 2p, 2p + 1
         float m0, m1;
@@ -363,7 +483,7 @@ __device__ __forceinline__ void convert_minima(uint32_t u, const RowWin& rw, uin
             m0 = (float)(s8(u + 2 * p) >> 4);
             m1 = (float)(s8(u + 2 * p + 1) >> 4);
         }
-        m0 *= -rw.dmin, m1 *= -rw.dmin;
+        m0 *= ratio, m1 *= ratio;
         const __half2 h = __floats2half2_rn(m0, m1);
         const float2 hf = __half22float2(h);
         a[p] = as_u32(h);
@@ -375,41 +495,38 @@ template <uint32_t TYPE, int N_TILE>
 __global__ void __launch_bounds__(H_THREADS, 1)
     gemm_f16_kernel(const uint8_t* __restrict__ w_a, uint64_t n, uint64_t k, const __grid_constant__ CUtensorMap map_hi,
                     const __grid_constant__ CUtensorMap map_lo, const __grid_constant__ CUtensorMap map_sums,
-                    const float* __restrict__ inv, uint64_t m_rows, float* __restrict__ dst_a, int* __restrict__ error_flag,
+                    const float* __restrict__ inv, uint64_t m_rows, float* dst_a, const float* residual, int* __restrict__ error_flag,
                     const GemmTile* __restrict__ tiles, const uint32_t* __restrict__ n_tiles, uint64_t expert_bytes,
-                    const uint8_t* __restrict__ w_b, float* __restrict__ dst_b, uint32_t split) {
+                    const uint8_t* __restrict__ w_b, float* dst_b, uint32_t split) {
     using T = HT<TYPE>;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    constexpr uint32_t PLANE_B = N_TILE * 128;  // 64 f16 columns of N_TILE rows
-    constexpr uint32_t STAGE = 2 * PLANE_B;     // hi | lo
-    constexpr uint32_t A_COL0 = 2 * N_TILE;
+    using S = Tile<TYPE, N_TILE>;
+    constexpr uint32_t PLANE_B = S::PLANE_B, STAGE = S::STAGE_B, RAW_BUF = S::RAW_BUF, BUFS = S::BUFS;
     constexpr uint32_t RAW_STRIDE = raw_stride<TYPE>();
-    constexpr uint32_t RAW_BUF = HM * RAW_STRIDE * 4;
     constexpr uint32_t WIN_WORDS = T::UNIT * T::UNITS / 4;
-    constexpr int MY_COLS = N_TILE / 4;
-    static_assert(2 * N_TILE + 64 * H_STEPS <= 512 && MY_COLS % 8 == 0, "tile shape");
-    uint8_t* s_sums = smem + (size_t)H_STEPS * STAGE;
-    uint8_t* raw = s_sums + (T::MIN ? PLANE_B : 0);
-    uint2* s_grid = reinterpret_cast<uint2*>(raw + T::BUFS * RAW_BUF);
+    constexpr int MY_COLS = S::FINE ? N_TILE : N_TILE / 4;  // accumulator columns a converter thread keeps
+    uint8_t* s_sums = smem + (size_t)S::STAGES * STAGE;
+    uint8_t* raw = s_sums + (T::MIN ? S::WINDOWS * PLANE_B : 0);
+    uint2* s_grid = reinterpret_cast<uint2*>(raw + BUFS * RAW_BUF);
     // full[s]: the step's four converter warps + the TMA thread (and the tiles' bytes); empty[s]: the MMAs' commit
-    __shared__ uint64_t full[H_STEPS], empty[H_STEPS], acc_full[2], acc_empty[2], raw_full[4][2], raw_empty[4][2];
+    __shared__ uint64_t full[S::STAGES], empty[S::STAGES], acc_full[2], acc_empty[S::ACCS], raw_full[4][BUFS], raw_empty[4][BUFS];
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     pdl_trigger();
-    // Grouped form: tile blockIdx.y of the list, its expert's slice of the bank (blockIdx.z picks the bank and its
-    // destination); rows of the tile box beyond the tile's count belong to other experts, are multiplied along and
+    // blockIdx.z: the bank (gate and up in one launch) and this CTA's place in its cluster along k.
+    // Grouped form: tile blockIdx.y of the list, its expert's slice of the bank; rows of the tile box beyond the tile's count belong to other experts, are multiplied along and
     // never stored.  The launch covers the list's capacity, not its length.
     uint64_t tok0 = (uint64_t)blockIdx.y * N_TILE, m = m_rows;
-    const uint8_t* w = w_a;
-    float* dst = dst_a;
+    const uint32_t bank = blockIdx.z / split, rank = blockIdx.z - bank * split;
+    const uint8_t* w = bank ? w_b : w_a;
+    float* dst = bank ? dst_b : dst_a;
     if (tiles != nullptr) {
         pdl_wait();
         if (blockIdx.y >= *n_tiles) return;
         const GemmTile t = tiles[blockIdx.y];
-        if (blockIdx.z) w = w_b, dst = dst_b;
         w += (uint64_t)t.expert * expert_bytes;
         tok0 = t.row0;
         m = (uint64_t)t.row0 + t.cnt;
@@ -417,23 +534,22 @@ __global__ void __launch_bounds__(H_THREADS, 1)
     const uint64_t row0 = (uint64_t)blockIdx.x * HM;
     const uint64_t row_bytes = k / 256 * T::UNIT;
     // this CTA's share of k, in staged windows
-    const uint32_t rank = split > 1 ? blockIdx.z : 0;
     const uint32_t all_windows = (uint32_t)(k / (256 * T::UNITS));
     const uint32_t win0 = (uint32_t)((uint64_t)all_windows * rank / split);
     const uint32_t n_windows = (uint32_t)((uint64_t)all_windows * (rank + 1) / split) - win0;
     const uint32_t n_chunks = n_windows * T::UNITS;  // accumulated windows of 256 columns
 
     if (tid == 0) {
-        for (uint32_t s = 0; s < H_STEPS; ++s) {
+        for (uint32_t s = 0; s < S::STAGES; ++s) {
             mbar_init(&full[s], 4 + 1);
             mbar_init(&empty[s], 1);
         }
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], H_CONV);
+        for (uint32_t b = 0; b < S::ACCS; ++b) {
+            if (!S::FINE) mbar_init(&acc_full[b & 1], 1);
+            mbar_init(&acc_empty[b], S::FINE ? 4 : H_CONV);
         }
         for (int q = 0; q < 4; ++q)
-            for (int b = 0; b < 2; ++b) {
+            for (uint32_t b = 0; b < BUFS; ++b) {
                 mbar_init(&raw_full[q][b], 4);
                 mbar_init(&raw_empty[q][b], 4);
             }
@@ -459,73 +575,63 @@ __global__ void __launch_bounds__(H_THREADS, 1)
         float sums[MY_COLS];
 #pragma unroll
         for (int c = 0; c < MY_COLS; ++c) sums[c] = 0.0f;
-        auto drain = [&](uint32_t c, float f) -> bool {
-            const uint32_t buf = c & 1;
-            if (!__all_sync(0xFFFFFFFFu, mbar_wait(&acc_full[buf], (c >> 1) & 1))) return false;
-            tc_fence_after();
-            const uint32_t taddr = tmem_d + lane_base + buf * N_TILE + g * MY_COLS;
-            if constexpr (MY_COLS == 8) {
-                uint32_t rr[8];
-                tmem_ld8(taddr, rr);
+        // sums += f * (this warp's columns of the accumulator at column `col`)
+        auto add_acc = [&](uint32_t col, float f) {
+            constexpr int PART = 16;
+            const uint32_t taddr = tmem_d + lane_base + col;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) sums[i] = fmaf(f, __uint_as_float(rr[i]), sums[i]);
-            } else {
+            for (int part = 0; part < MY_COLS / PART; ++part) {
+                uint32_t rr[PART];
+                tmem_ld16(taddr + part * 16, rr);
 #pragma unroll
-                for (int part = 0; part < MY_COLS / 16; ++part) {
-                    uint32_t rr[16];
-                    tmem_ld16(taddr + part * 16, rr);
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) sums[part * 16 + i] = fmaf(f, __uint_as_float(rr[i]), sums[part * 16 + i]);
-                }
+                for (int i = 0; i < PART; ++i) sums[part * PART + i] = fmaf(f, __uint_as_float(rr[i]), sums[part * PART + i]);
             }
+        };
+        // read back window c: this warp's columns of its accumulator, or all columns of the accumulator of its own step
+        auto drain = [&](uint32_t c, float f) -> bool {
+            uint64_t* ready = S::FINE ? &empty[(c % S::WINDOWS) * H_STEPS + g] : &acc_full[c & 1];
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait(ready, (S::FINE ? c / S::WINDOWS : c >> 1) & 1))) return false;
+            tc_fence_after();
+            add_acc(S::FINE ? g * N_TILE : (c & 1) * N_TILE + g * MY_COLS, f);
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[buf]);
+            if (lane == 0) mbar_arrive(&acc_empty[S::FINE ? g : c & 1]);
             return true;
         };
-        // this warp's 8 of the quarter's 32 rows of window wn, consecutive lanes consecutive words (16-byte vectors
-        // where the rows are made of them)
+        // this warp's 8 of the quarter's 32 rows of window wn, as one run of vectors over the lanes
         const uint32_t raw_q = smem_u32(raw) + q * 32 * RAW_STRIDE * 4;
+        constexpr uint32_t VEC = T::VEC, ROW_VECS = WIN_WORDS * 4 / VEC, COPIES = (8 * ROW_VECS + 31) / 32;
+        const uint64_t gr0 = min(row0 + q * 32 + g * 8, n - 1);
+        const uint32_t rows_left = (uint32_t)min((uint64_t)8, n - gr0);  // rows past n repeat the last one
+        const uint8_t* src0 = w + gr0 * row_bytes + (uint64_t)win0 * (WIN_WORDS * 4);
+        const uint32_t row_bytes32 = (uint32_t)row_bytes;
         auto copy_window = [&](uint32_t wn) {
             if (wn < n_windows) {
-                const uint64_t gr0 = row0 + q * 32 + g * 8;
-                const uint32_t dst0 = raw_q + (wn % T::BUFS) * RAW_BUF + g * 8 * RAW_STRIDE * 4;
-                const uint8_t* src0 = w + (uint64_t)(win0 + wn) * (WIN_WORDS * 4);
-                if constexpr (T::VEC16) {
-                    constexpr uint32_t V = T::UNIT / 16;
+                const uint32_t dst0 = raw_q + (wn % BUFS) * RAW_BUF + g * 8 * RAW_STRIDE * 4;
+                const uint8_t* src = src0 + (uint64_t)wn * (WIN_WORDS * 4);
+                auto one = [&](uint32_t i) {
+                    const uint32_t rr = i / ROW_VECS, c = i - rr * ROW_VECS;
+                    const uint8_t* sp = src + ((uint64_t)min(rr, rows_left - 1) * row_bytes32 + c * VEC);
+                    const uint32_t dp = dst0 + rr * (RAW_STRIDE * 4) + c * VEC;
+                    if constexpr (VEC == 16)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dp), "l"(sp) : "memory");
+                    else
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dp), "l"(sp), "n"(VEC) : "memory");
+                };
 #pragma unroll
-                    for (uint32_t i = lane; i < 8 * V; i += 32) {
-                        const uint32_t rr = i / V, c = i - rr * V;
-                        const uint64_t gr = gr0 + rr < n ? gr0 + rr : n - 1;
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst0 + rr * (RAW_STRIDE * 4) + 16 * c),
-                                     "l"(src0 + gr * row_bytes + 16 * c)
-                                     : "memory");
-                    }
-                } else {
-#pragma unroll 1
-                    for (uint32_t rr = 0; rr < 8; ++rr) {
-                        const uint64_t gr = gr0 + rr < n ? gr0 + rr : n - 1;
-                        const uint8_t* src = src0 + gr * row_bytes + lane * 4;
-                        const uint32_t dstp = dst0 + rr * (RAW_STRIDE * 4) + lane * 4;
-#pragma unroll
-                        for (uint32_t c = 0; c < WIN_WORDS; c += 32) {
-                            if (c + lane < WIN_WORDS)
-                                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dstp + c * 4), "l"(src + c * 4)
-                                             : "memory");
-                        }
-                    }
-                }
+                for (uint32_t j = 0; j < COPIES; ++j)
+                    if (32 * j + 32 <= 8 * ROW_VECS || lane + 32 * j < 8 * ROW_VECS) one(lane + 32 * j);
             }
             asm volatile("cp.async.commit_group;" ::: "memory");  // an empty group past the last window
         };
         bool ok = true;
         float f_prev = 0.0f;
 #pragma unroll
-        for (uint32_t b = 0; b < T::BUFS; ++b) copy_window(b);
+        for (uint32_t b = 0; b < BUFS; ++b) copy_window(b);
         for (uint32_t wn = 0; wn < n_windows && ok; ++wn) {
-            const uint32_t buf = wn % T::BUFS, par = (wn / T::BUFS) & 1;
+            const uint32_t buf = wn % BUFS, par = (wn / BUFS) & 1;
             // my copies of this window have landed; hand them over and wait for the others'
-            asm volatile("cp.async.wait_group %0;" ::"n"(T::BUFS - 1) : "memory");
+            asm volatile("cp.async.wait_group %0;" ::"n"(BUFS - 1) : "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(&raw_full[q][buf]);
             ok = __all_sync(0xFFFFFFFFu, mbar_wait(&raw_full[q][buf], par));
@@ -536,36 +642,34 @@ __global__ void __launch_bounds__(H_THREADS, 1)
                 const uint32_t u = raw_q + buf * RAW_BUF + lane * RAW_STRIDE * 4 + cc * T::UNIT;
                 const RowWin rw = row_window<TYPE>(u);
                 // the stage's columns must have been read by the MMAs that used them last
-                ok = __all_sync(0xFFFFFFFFu, mbar_wait(&empty[g], (c & 1) ^ 1));
+                const uint32_t ph = c % S::WINDOWS, st = ph * H_STEPS + g;
+                ok = __all_sync(0xFFFFFFFFu, mbar_wait(&empty[st], ((c / S::WINDOWS) & 1) ^ 1));
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t acol = tmem_d + lane_base + A_COL0 + g * 64;
-#pragma unroll
-                for (uint32_t h = 0; h < 2; ++h) {
-                    uint32_t a[16], b[16];
-                    convert32<TYPE>(u, 2 * g + h, rw, s_grid, a, b);
+                const uint32_t acol = tmem_d + lane_base + S::ACC_COLS + st * S::A_COLS;
+                convert64<TYPE>(u, g, rw, s_grid, [&](uint32_t h, const uint32_t (&a)[16], const uint32_t (&b)[16]) {
                     tmem_st16(acol + 16 * h, a);
                     if constexpr (T::TWO) tmem_st16(acol + 32 + 16 * h, b);
-                }
+                });
                 if constexpr (T::MIN) {
                     if (g == H_STEPS - 1) {
                         uint32_t a[16];
                         convert_minima<TYPE>(u, rw, a);
-                        tmem_st16(acol + 32, a);
+                        tmem_st16(tmem_d + lane_base + S::MIN_COL0 + 16 * ph, a);
                     }
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&full[g]);
+                if (lane == 0) mbar_arrive(&full[st]);
                 if (cc == T::UNITS - 1) {
                     // once the quarter's other warps are through with this window too, bring in my rows of a later one
-                    if (wn + T::BUFS < n_windows) {
+                    if (wn + BUFS < n_windows) {
                         if (lane == 0) mbar_arrive(&raw_empty[q][buf]);
                         ok = __all_sync(0xFFFFFFFFu, mbar_wait(&raw_empty[q][buf], par));
                         if (!ok) break;
                     }
-                    copy_window(wn + T::BUFS);
+                    copy_window(wn + BUFS);
                 }
                 // read back the window before this one while this one accumulates
                 if (c > 0) ok = drain(c - 1, f_prev);
@@ -577,17 +681,23 @@ __global__ void __launch_bounds__(H_THREADS, 1)
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         if (!ok) abort_flag = 1;
         pdl_wait();  // inv and dst belong to the kernels before this one
-        if (split == 1) {
+        if (!S::FINE && split == 1) {
             const uint64_t out_row = row0 + q * 32 + lane;
             if (ok && out_row < n) {
 #pragma unroll
                 for (int c = 0; c < MY_COLS; ++c) {
                     const uint64_t tok = tok0 + g * MY_COLS + c;
-                    if (tok < m) dst[tok * n + out_row] = sums[c] * __ldg(inv + tok);
+                    if (tok < m) {
+                        const float v = sums[c] * __ldg(inv + tok);
+                        dst[tok * n + out_row] = residual ? residual[tok * n + out_row] + v : v;
+                    }
                 }
             }
         } else {
-            // the ring is idle (every MMA of this CTA was waited for): leave the partial tile there, [token][row]
+            // leave the partial tile in shared memory, [token][row] (four of them where the warps of a quarter hold sums
+            // of their own steps).  The ring and the staged bytes are idle once every converter is here: the last
+            // read-back waited for this CTA's last products.
+            asm volatile("bar.sync 1, %0;" ::"n"(H_CONV * 32) : "memory");
             float* red = reinterpret_cast<float*>(smem);
 #pragma unroll
             for (int c = 0; c < MY_COLS; ++c) red[(g * MY_COLS + c) * HM + q * 32 + lane] = sums[c];
@@ -600,36 +710,43 @@ __global__ void __launch_bounds__(H_THREADS, 1)
         [[maybe_unused]] const uint64_t d_sums = umma_desc(smem_u32(s_sums));
         bool ok = true;
         for (uint32_t c = 0; c < n_chunks && ok; ++c) {
-            const uint32_t buf = c & 1, d = tmem_d + buf * N_TILE;
-            if (c >= 2) {
-                ok = __all_sync(0xFFFFFFFFu, mbar_wait(&acc_empty[buf], ((c >> 1) - 1) & 1));
-                if (!ok) break;
-            }
+            const uint32_t ph = c % S::WINDOWS;
 #pragma unroll
-            for (uint32_t s = 0; s < H_STEPS; ++s) {
-                ok = __all_sync(0xFFFFFFFFu, mbar_wait(&full[s], c & 1));
+            for (uint32_t g = 0; g < H_STEPS; ++g) {
+                const uint32_t st = ph * H_STEPS + g, acc = S::FINE ? g : c & 1, d = tmem_d + acc * N_TILE;
+                // the accumulator's last contents must have been read back
+                if (S::FINE ? c >= 1 : g == 0 && c >= 2) {
+                    ok = __all_sync(0xFFFFFFFFu, mbar_wait(&acc_empty[acc], (S::FINE ? c - 1 : (c >> 1) - 1) & 1));
+                    if (!ok) break;
+                }
+                ok = __all_sync(0xFFFFFFFFu, mbar_wait(&full[st], (c / S::WINDOWS) & 1));
                 if (!ok) break;
                 tc_fence_after();  // the converters' tcgen05.st / .ld
                 if (elect_one()) {
-                    const uint64_t so = (uint64_t)s * (STAGE >> 4);
-                    const uint32_t a1 = tmem_d + A_COL0 + s * 64, a2 = a1 + 32;
+                    const uint64_t so = (uint64_t)st * (STAGE >> 4);
+                    const uint32_t a1 = tmem_d + S::ACC_COLS + st * S::A_COLS, a2 = a1 + 32;
+                    const bool fresh = S::FINE || g == 0;
+                    // small products first, while the accumulator is small.  16 columns an instruction: 8 columns of A,
+                    // 32 bytes of B's swizzled rows.
 #pragma unroll
-                    for (uint32_t kk = 0; kk < 4; ++kk) {  // 16 columns: 8 columns of A, 32 bytes of B's swizzled rows
-                        umma_f16_ts(d, a1 + kk * 8, d0_hi + so + kk * 2, idesc, s != 0 || kk != 0);
-                        umma_f16_ts(d, a1 + kk * 8, d0_lo + so + kk * 2, idesc, 1);
+                    for (uint32_t kk = 0; kk < 4; ++kk) {
+                        umma_f16_ts(d, a1 + kk * 8, d0_lo + so + kk * 2, idesc, !fresh || kk != 0);
                         if constexpr (T::TWO) umma_f16_ts(d, a2 + kk * 8, d0_hi + so + kk * 2, idesc, 1);
                     }
                     if constexpr (T::MIN) {
-                        if (s == H_STEPS - 1) {
+                        if (g == H_STEPS - 1) {
                             // a tile of sums holds two windows, 64 bytes each: first terms, second terms
-                            const uint64_t ds = d_sums + ((win0 + c) & 1) * 4;
-                            umma_f16_ts(d, a2, ds, idesc, 1);
-                            umma_f16_ts(d, a2 + 8, ds, idesc, 1);
-                            umma_f16_ts(d, a2, ds + 2, idesc, 1);
+                            const uint64_t ds = d_sums + ph * (PLANE_B >> 4) + ((win0 + c) & 1) * 4;
+                            const uint32_t am = tmem_d + S::MIN_COL0 + 16 * ph;
+                            umma_f16_ts(d, am + 8, ds, idesc, 1);
+                            umma_f16_ts(d, am, ds + 2, idesc, 1);
+                            umma_f16_ts(d, am, ds, idesc, 1);
                         }
                     }
-                    umma_commit(&empty[s]);  // both the weight columns and the activation tiles of the stage are free
-                    if (s == H_STEPS - 1) umma_commit(&acc_full[buf]);
+#pragma unroll
+                    for (uint32_t kk = 0; kk < 4; ++kk) umma_f16_ts(d, a1 + kk * 8, d0_hi + so + kk * 2, idesc, 1);
+                    umma_commit(&empty[st]);  // the weight columns and the activation tiles of the stage are free
+                    if (!S::FINE && g == H_STEPS - 1) umma_commit(&acc_full[acc]);
                 }
                 __syncwarp();
             }
@@ -642,15 +759,18 @@ __global__ void __launch_bounds__(H_THREADS, 1)
             bool ok = true;
             for (uint32_t c = 0; c < n_chunks && ok; ++c) {
                 const uint32_t col = (win0 * T::UNITS + c) * 256;
-                for (uint32_t s = 0; s < H_STEPS; ++s) {
-                    ok = mbar_wait(&empty[s], (c & 1) ^ 1);
+                const uint32_t ph = c % S::WINDOWS;
+                for (uint32_t g = 0; g < H_STEPS; ++g) {
+                    const uint32_t st = ph * H_STEPS + g;
+                    ok = mbar_wait(&empty[st], ((c / S::WINDOWS) & 1) ^ 1);
                     if (!ok) break;
-                    uint8_t* st = smem + (size_t)s * STAGE;
-                    const bool with_sums = T::MIN && s == H_STEPS - 1;
-                    mbar_arrive_expect_tx(&full[s], (with_sums ? 3 : 2) * PLANE_B);
-                    tma_load_2d(st, &map_hi, col + 64 * s, (uint32_t)tok0, &full[s]);
-                    tma_load_2d(st + PLANE_B, &map_lo, col + 64 * s, (uint32_t)tok0, &full[s]);
-                    if (with_sums) tma_load_2d(s_sums, &map_sums, ((win0 + c) >> 1) * 64, (uint32_t)tok0, &full[s]);
+                    uint8_t* tile = smem + (size_t)st * STAGE;
+                    const bool with_sums = T::MIN && g == H_STEPS - 1;
+                    mbar_arrive_expect_tx(&full[st], (with_sums ? 3 : 2) * PLANE_B);
+                    tma_load_2d(tile, &map_hi, col + 64 * g, (uint32_t)tok0, &full[st]);
+                    tma_load_2d(tile + PLANE_B, &map_lo, col + 64 * g, (uint32_t)tok0, &full[st]);
+                    if (with_sums)
+                        tma_load_2d(s_sums + ph * PLANE_B, &map_sums, ((win0 + c) >> 1) * 64, (uint32_t)tok0, &full[st]);
                 }
             }
             if (!ok) abort_flag = 1;
@@ -659,22 +779,28 @@ __global__ void __launch_bounds__(H_THREADS, 1)
     }
     tc_fence_before();
     __syncthreads();
-    if (split > 1) {
-        cluster_sync_all();
-        // tile element i = token * 128 + row; rank r adds the tokens t = r (mod split), over the ranks in order
-        const uint32_t red = smem_u32(smem);
-        if (abort_flag == 0) {
-            const uint32_t row = tid & (HM - 1);
+    if (S::FINE || split > 1) {
+        if (split > 1) cluster_sync_all();
+        // tile element i = token * 128 + row; rank r adds the tokens t = r (mod split), over the ranks and their partial
+        // tiles in order
+        if (abort_flag == 0 && tid < H_CONV * 32) {
+            const uint32_t red = smem_u32(smem), row = tid & (HM - 1);
+            constexpr uint32_t TILES = S::FINE ? 4 : 1;
             for (uint32_t t = rank + split * (tid / HM); t < N_TILE; t += split * (H_CONV * 32 / HM)) {
-                if (tid >= H_CONV * 32) break;
-                const uint64_t tok = tok0 + t;
+                const uint64_t tok = tok0 + t, at = tok * n + row0 + row;
                 if (tok >= m || row0 + row >= n) continue;
                 float v = 0.0f;
-                for (uint32_t r = 0; r < split; ++r) v += ld_cluster_f32(red + (t * HM + row) * 4, r);
-                dst[tok * n + row0 + row] = v * __ldg(inv + tok);
+                for (uint32_t r = 0; r < split; ++r)
+#pragma unroll
+                    for (uint32_t p = 0; p < TILES; ++p) {
+                        const uint32_t addr = red + ((p * N_TILE + t) * HM + row) * 4;
+                        v += split > 1 ? ld_cluster_f32(addr, r) : __uint_as_float(s32(addr));
+                    }
+                v *= __ldg(inv + tok);
+                dst[at] = residual ? residual[at] + v : v;
             }
         }
-        cluster_sync_all();  // no CTA leaves while another reads its shared memory
+        if (split > 1) cluster_sync_all();  // no CTA leaves while another reads its shared memory
     }
     if (abort_flag && tid == 0) *reinterpret_cast<volatile int*>(error_flag) = 1;
     if (warp == H_CONV) {
@@ -728,6 +854,7 @@ struct F16Launch {
     uint64_t n, k, rows, expert_bytes;
     SplitX x;
     float *dst_a, *dst_b;
+    const float* residual;
     const GemmTile* tiles;
     uint32_t max_tiles;
     const uint32_t* n_tiles;
@@ -736,8 +863,7 @@ struct F16Launch {
 
 template <uint32_t TYPE, int N_TILE>
 cudaError_t launch_f16_tile(const F16Launch& l, cudaStream_t s) {
-    constexpr size_t smem = h_smem_bytes<TYPE, N_TILE>();
-    static_assert(smem <= 226 * 1024, "shared memory of a tile");
+    constexpr size_t smem = Tile<TYPE, N_TILE>::SMEM;
     auto kern = gemm_f16_kernel<TYPE, N_TILE>;
     static bool configured[MAX_DEVICES] = {};
     if (cudaError_t ce = set_max_smem_once(kern, 226 * 1024, configured); ce != cudaSuccess) return ce;
@@ -763,7 +889,8 @@ cudaError_t launch_f16_tile(const F16Launch& l, cudaStream_t s) {
     } else {
         // Split k over a cluster where whole tiles fill the SMs badly: waves x (a CTA's windows + about three windows'
         // worth of filling the pipeline and storing the tile).  Clusters of up to four pack the GPCs without loss.
-        const uint64_t gy = (l.rows + N_TILE - 1) / N_TILE, tiles = gx * gy, sms = (uint64_t)num_sms();
+        const unsigned banks = l.w_b ? 2 : 1;
+        const uint64_t gy = (l.rows + N_TILE - 1) / N_TILE, tiles = gx * gy * banks, sms = (uint64_t)num_sms();
         const uint64_t windows = l.k / (256 * HT<TYPE>::UNITS);
         uint64_t best = ~0ull;
         for (uint32_t c = 1; c <= 4 && c <= windows; ++c) {
@@ -771,7 +898,7 @@ cudaError_t launch_f16_tile(const F16Launch& l, cudaStream_t s) {
             const uint64_t cost = waves * ((windows + c - 1) / c * HT<TYPE>::UNITS + 3 + (c > 1));
             if (cost < best) best = cost, split = c;
         }
-        cfg.gridDim = dim3(gx, (unsigned)gy, split);
+        cfg.gridDim = dim3(gx, (unsigned)gy, split * banks);
         if (gy > 65535) return cudaErrorInvalidValue;
         if (split > 1) {
             attr[1].id = cudaLaunchAttributeClusterDimension;
@@ -781,7 +908,7 @@ cudaError_t launch_f16_tile(const F16Launch& l, cudaStream_t s) {
             cfg.numAttrs = 2;
         }
     }
-    e = cudaLaunchKernelEx(&cfg, kern, l.w_a, l.n, l.k, hi, lo, sums, (const float*)l.x.inv, l.rows, l.dst_a, l.error_flag,
+    e = cudaLaunchKernelEx(&cfg, kern, l.w_a, l.n, l.k, hi, lo, sums, (const float*)l.x.inv, l.rows, l.dst_a, l.residual, l.error_flag,
                            l.tiles, l.n_tiles, l.expert_bytes, l.w_b, l.dst_b, split);
     return e != cudaSuccess ? e : cudaGetLastError();
 }
@@ -794,26 +921,32 @@ cudaError_t launch_f16_typed(uint32_t type, const F16Launch& l, cudaStream_t s) 
         case T_Q4_K: return launch_f16_tile<T_Q4_K, N_TILE>(l, s);
         case T_IQ2_XXS: return launch_f16_tile<T_IQ2_XXS, N_TILE>(l, s);
         case T_MXFP4: return launch_f16_tile<T_MXFP4, N_TILE>(l, s);
+        case T_Q6_K:
+            if constexpr (N_TILE <= 32) return launch_f16_tile<T_Q6_K, N_TILE>(l, s);
+            return cudaErrorInvalidValue;
         default: return cudaErrorInvalidValue;
     }
 }
 
-cudaError_t split_activations_f16(const float* x, uint64_t m, uint64_t k, const SplitX& o, cudaStream_t s) {
-    return launch_pdl(split_f16_kernel, dim3((unsigned)m), 256, 0, s, x, (uint32_t)k, o.hi, o.lo, o.sums, o.inv);
+cudaError_t split_activations_f16(uint32_t type, const float* x, uint64_t m, uint64_t k, const float* norm_w, float eps, const SplitX& o,
+                                  cudaStream_t s) {
+    return launch_pdl(split_f16_kernel, dim3((unsigned)m), 256, 0, s, x, (uint32_t)k, norm_w, eps,
+                      type == T_MXFP4 ? 1 : 0, o.hi, o.lo, o.sums, o.inv);
 }
 
 }  // namespace
 
-// Whole staged windows of whole 32-bit words (Q4_K: 16-byte vectors) in every row.
+// Whole staged windows in every row, made of the vectors they are copied by.
 bool gemm_f16_supports(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, uint64_t m) {
     if (m == 0 || n == 0 || k == 0 || k % 256 != 0 || k > 0x7FFFFFFFu || m > 0x7FFFFFFFu) return false;
     const uintptr_t a = reinterpret_cast<uintptr_t>(w);
     switch (type) {
         case T_Q4_K: return a % 16 == 0;
         case T_Q8_0:
-        case T_Q2_K:
-        case T_MXFP4: return a % 4 == 0;
-        case T_IQ2_XXS: return a % 4 == 0 && k % 512 == 0;
+        case T_MXFP4: return a % 8 == 0;
+        case T_Q2_K: return a % 4 == 0;
+        case T_IQ2_XXS:
+        case T_Q6_K: return a % 4 == 0 && k % 512 == 0;
         default: return false;
     }
 }
@@ -822,22 +955,26 @@ size_t gemm_f16_scratch_bytes(uint64_t m, uint64_t k) {
     return (size_t)(2 * up128(2 * m * k) + up128(m * k / 4) + up128(4 * m));
 }
 
-cudaError_t launch_gemm_f16(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, const float* lhs, uint64_t m, float* dst,
+// dst_a = residual + norm(lhs) . W^T; with w_b the same rows through a second tensor into dst_b.
+cudaError_t launch_gemm_f16(uint32_t type, const uint8_t* w_a, const uint8_t* w_b, uint64_t n, uint64_t k, const float* lhs,
+                            uint64_t m, const float* norm_w, float eps, const float* residual, float* dst_a, float* dst_b,
                             void* scratch, int* error_flag, cudaStream_t s) {
     F16Launch l = {};
-    l.w_a = w;
+    l.w_a = w_a, l.w_b = w_b;
     l.n = n, l.k = k, l.rows = m;
     l.x = split_in(scratch, m, k);
-    l.dst_a = dst;
+    l.dst_a = dst_a, l.dst_b = dst_b;
+    l.residual = residual;
     l.error_flag = error_flag;
-    if (cudaError_t e = split_activations_f16(lhs, m, k, l.x, s); e != cudaSuccess) return e;
-    if (m <= 32) return launch_f16_typed<32>(type, l, s);
-    if (m <= 64) return launch_f16_typed<64>(type, l, s);
+    if (cudaError_t e = split_activations_f16(type, lhs, m, k, norm_w, eps, l.x, s); e != cudaSuccess) return e;
+    if (m <= 16) return launch_f16_typed<16>(type, l, s);
+    // up to 64 rows the other route is the decode kernel, for Q6_K always: they stay on the exact tiles
+    if (m <= 64 || type == T_Q6_K) return launch_f16_typed<32>(type, l, s);
     return launch_f16_typed<128>(type, l, s);
 }
 
 bool gemm_f16_grouped_supports(uint32_t type, const uint8_t* bank, uint64_t n, uint64_t k) {
-    return gemm_f16_supports(type, bank, n, k, 128);
+    return type != T_Q6_K && gemm_f16_supports(type, bank, n, k, 128);
 }
 
 cudaError_t launch_gemm_f16_grouped(uint32_t type, const uint8_t* bank_a, const uint8_t* bank_b, uint64_t expert_bytes,
@@ -850,7 +987,7 @@ cudaError_t launch_gemm_f16_grouped(uint32_t type, const uint8_t* bank_a, const 
     l.x = split_in(scratch, rows, k);
     l.dst_a = dst_a, l.dst_b = dst_b;
     l.error_flag = error_flag;
-    if (cudaError_t e = split_activations_f16(x, rows, k, l.x, s); e != cudaSuccess) return e;
+    if (cudaError_t e = split_activations_f16(type, x, rows, k, nullptr, 0.0f, l.x, s); e != cudaSuccess) return e;
     if (max_narrow) {
         l.tiles = narrow, l.max_tiles = max_narrow, l.n_tiles = counts;
         if (cudaError_t e = launch_f16_typed<32>(type, l, s); e != cudaSuccess) return e;

@@ -50,6 +50,7 @@ struct StreamScratch {
 struct jq_ctx {
     int device = 0;
     bool force_f32 = false;        // JQ_FORCE_F32_PATH=1: always take the exact-decode float kernels
+    uint64_t tiles_min_m = 9;      // JQ_TILES_MIN_M: smallest batch that runs on the f16 tile GEMM
     uint64_t sliced_max_m = 64;    // JQ_SLICED_MAX_M: largest batch run as 8-row slices of the decode kernel (0 = never)
     int* status_host = nullptr;    // pinned, device-visible: set to 1 by a kernel whose bounded wait gave up
     int* status_dev = nullptr;
@@ -118,6 +119,12 @@ struct jq_weight {
 // Picks the kernel for a device-resident product (abi.cu).
 int32_t jq_matmul_device(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, const float* lhs, float* dst,
                          cudaStream_t s);
+
+// Whether a product of m rows runs on the f16 tile GEMM, and that product: dst = residual + norm(lhs) . W^T, with w_b (a
+// tensor of the same type and shape) also dst_b = norm(lhs) . W_b^T.  norm_w, residual and w_b may be NULL (abi.cu).
+bool jq_uses_tiles(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n);
+int32_t jq_matmul_tiles(const jq_weight* w, const jq_weight* w_b, uint64_t m, uint64_t k, uint64_t n, const float* lhs,
+                        const float* norm_w, float eps, const float* residual, float* dst, float* dst_b, cudaStream_t s);
 
 // One MoE layer (moe_abi.cu); shared with the expert-parallel exchange (ep.cu).
 struct jq_moe {

@@ -154,7 +154,7 @@ int32_t run_experts_bucketed(jq_moe* m, const float* x, uint64_t T, uint64_t P, 
         // tile holds more than 32 rows
         // With 24 or more rows per expert on average hardly an expert is small: every expert then takes the tile
         // form (an expert with a few rows is one narrow tile) and the decode kernel's passes are left out.
-        const bool all_tiles = P >= 24ull * c.n_expert;
+        const bool all_tiles = true;
         const uint32_t min_rows = all_tiles ? 1u : (uint32_t)BUCKET_ROWS_PER_EXPERT;
         const uint32_t max_narrow = (uint32_t)std::min<uint64_t>(c.n_expert, P / min_rows + 1);
         const uint32_t max_wide = (uint32_t)(P / 33 + 1);

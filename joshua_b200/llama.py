@@ -161,43 +161,36 @@ class LlamaDecoder:
         s = torch.cuda.current_stream(self.dev).cuda_stream if stream is None else stream
         ids = torch.as_tensor(token_ids, dtype=torch.int32).to(self.dev)
         S, h, f32 = int(ids.numel()), c.hidden, dict(dtype=torch.float32, device=self.dev)
-        x, xn = torch.empty(S, h, **f32), torch.empty(S, h, **f32)
+        x = torch.empty(S, h, **f32)
         qkv, q = torch.empty(S, c.qkv_rows, **f32), torch.empty(S, c.q_heads * c.head_dim, **f32)
-        att, o = torch.empty(S, c.q_heads * c.head_dim, **f32), torch.empty(S, h, **f32)
+        att = torch.empty(S, c.q_heads * c.head_dim, **f32)
         check(L.jq_embedding_dev(self.embed._h, P(ids), S, c.vocab, h, P(x), P(self.bad), s))
         for ly in self.layers:
-            check(L.jq_rmsnorm_dev(P(x), None, P(ly["attn_norm"]), c.eps, S, h, None, P(xn), s))
-            check(L.jq_matmul_t_dev(ly["wqkv"]._h, S, h, c.qkv_rows, P(xn), P(qkv), s))
+            check(L.jq_matmul_norm_dev(ly["wqkv"]._h, S, h, c.qkv_rows, P(x), P(ly["attn_norm"]), c.eps, None, P(qkv), s))
             check(L.jq_rope_append_prefill_dev(P(qkv), P(self.pos), S, c.q_heads, c.kv_heads, c.head_dim, self.max_ctx,
                                                c.rope_theta, P(ly["q_norm"]) if self.qk_norm else None,
                                                P(ly["k_norm"]) if self.qk_norm else None, c.eps, P(q), P(ly["k"]),
                                                P(ly["v"]), P(self.bad_pos), s))
             check(L.jq_attention_prefill_dev(P(q), P(ly["k"]), P(ly["v"]), P(self.pos), S, c.q_heads, c.kv_heads,
                                              c.head_dim, self.max_ctx, P(att), P(self.bad_pos), s))
-            check(L.jq_matmul_t_dev(ly["wo"]._h, S, c.q_heads * c.head_dim, h, P(att), P(o), s))
-            check(L.jq_add_dev(P(x), P(o), S * h, P(x), s))
-            self._ffn_prefill(ly, x, xn, S, s)
+            check(L.jq_matmul_norm_dev(ly["wo"]._h, S, c.q_heads * c.head_dim, h, P(att), None, 0.0, P(x), P(x), s))
+            self._ffn_prefill(ly, x, S, s)
         # the last token's row -> logits, next token; the position moves past the prompt
         self.x.copy_(x[S - 1:S])
         check(L.jq_matmul_norm_dev(self.output._h, 1, h, c.vocab, P(self.x), P(self.out_norm), c.eps, None,
                                    P(self.logits), s))
         self.pos.add_(S - 1)
         self._sample(s)
-        self._keep_prefill = (x, xn, qkv, q, att, o, ids)   # alive until the stream has run them
+        self._keep_prefill = (x, qkv, q, att, ids)   # alive until the stream has run them
 
-    def _ffn_prefill(self, ly, x, xn, S, s) -> None:
-        """x += FFN(rmsnorm(x; ffn_norm)) over S rows: two batched matmuls + SwiGLU, then the down projection."""
+    def _ffn_prefill(self, ly, x, S, s) -> None:
+        """x += FFN(rmsnorm(x; ffn_norm)) over S rows: the gate / up pair with SwiGLU, then the down projection."""
         torch, L, c, P = self.torch, _lib.lib(), self.cfg, lambda t: t.data_ptr()
-        f32 = dict(dtype=torch.float32, device=self.dev)
-        g, u = torch.empty(S, c.ffn, **f32), torch.empty(S, c.ffn, **f32)
-        d = torch.empty(S, c.hidden, **f32)
-        check(L.jq_rmsnorm_dev(P(x), None, P(ly["ffn_norm"]), c.eps, S, c.hidden, None, P(xn), s))
-        check(L.jq_matmul_t_dev(ly["w_gate"]._h, S, c.hidden, c.ffn, P(xn), P(g), s))
-        check(L.jq_matmul_t_dev(ly["w_up"]._h, S, c.hidden, c.ffn, P(xn), P(u), s))
-        check(L.jq_swiglu_dev(P(g), P(u), S * c.ffn, 0.0, P(g), s))
-        check(L.jq_matmul_t_dev(ly["w_down"]._h, S, c.ffn, c.hidden, P(g), P(d), s))
-        check(L.jq_add_dev(P(x), P(d), S * c.hidden, P(x), s))
-        self._keep_ffn = (g, u, d)
+        act = torch.empty(S, c.ffn, dtype=torch.float32, device=self.dev)
+        check(L.jq_matmul_swiglu_norm_dev(ly["w_gate"]._h, ly["w_up"]._h, S, c.hidden, c.ffn, P(x), P(ly["ffn_norm"]), c.eps,
+                                          P(act), 0.0, s))
+        check(L.jq_matmul_norm_dev(ly["w_down"]._h, S, c.ffn, c.hidden, P(act), None, 0.0, P(x), P(x), s))
+        self._keep_ffn = act
 
     def _sample(self, s) -> None:
         """Next token of every sequence from self.logits (`sample_token` of src/engine.rs:2339-2378 at

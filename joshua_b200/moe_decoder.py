@@ -143,7 +143,7 @@ class MoeDecoder(LlamaDecoder):
         assert self.world == 1, "prefill runs on one GPU (the exchange windows are sized for decode batches)"
         super().prefill(token_ids, stream)
 
-    def _ffn_prefill(self, ly, x, xn, S, s) -> None:
+    def _ffn_prefill(self, ly, x, S, s) -> None:
         """x += MoE(rmsnorm(x; ffn_norm)) over S tokens (`Moe::forward` with n_tokens = seq_len)."""
         L, c, P = _lib.lib(), self.cfg, lambda t: t.data_ptr()
         layer = self.ffn_layers[self._layer_index[id(ly)]]["moe"]
