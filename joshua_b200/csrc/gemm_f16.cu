@@ -41,7 +41,9 @@
 //
 // Warps: 16 converters, warp (q = w % 4, g = w / 4) owns weight rows 32q .. 32q+31 (the tensor-memory lanes it may
 // touch) and the columns 64g .. 64g+63 of every window; the four warps of a quarter share the staged raw bytes of a
-// window and hand them over through pairs of mbarriers.  Warp 16 issues the MMAs, warp 17 the TMA copies.
+// window and meet once per window on a named barrier (an mbarrier round trip costs some 200 cycles here).  Warps 16 to
+// 19 issue the MMAs: an instruction takes about 30 cycles to issue, so narrow tiles have an issuer per step (wide ones
+// one in all, their steps share an accumulator).  Warp 20 issues the TMA copies.
 //
 // Few tiles (small n, or few rows of lhs) leave SMs idle: then a cluster of S CTAs splits k, every CTA leaves its
 // partial tile in its shared memory, and each adds a share of the tile over the cluster in rank order (distributed
@@ -50,6 +52,7 @@
 // Every wait on an mbarrier is bounded; a wait that runs out raises the device status flag, and every thread still
 // reaches the common exit where tensor memory is released.
 #include <algorithm>
+#include <type_traits>
 
 #include <cudaTypedefs.h>
 
@@ -64,7 +67,8 @@ namespace {
 
 constexpr int HM = 128;           // weight rows per CTA = MMA M = TMEM lanes
 constexpr int H_CONV = 16;        // converter / epilogue warps
-constexpr int H_THREADS = (H_CONV + 2) * 32;
+constexpr int H_ISSUE = 4;        // issuing warps: one per 64-column step where the steps have their own accumulators
+constexpr int H_THREADS = (H_CONV + H_ISSUE + 1) * 32;
 constexpr uint32_t H_STEPS = 4;   // 64-column steps per 256-column window = ring stages
 
 template <uint32_t TYPE>
@@ -510,7 +514,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
     uint8_t* raw = s_sums + (T::MIN ? S::WINDOWS * PLANE_B : 0);
     uint2* s_grid = reinterpret_cast<uint2*>(raw + BUFS * RAW_BUF);
     // full[s]: the step's four converter warps + the TMA thread (and the tiles' bytes); empty[s]: the MMAs' commit
-    __shared__ uint64_t full[S::STAGES], empty[S::STAGES], acc_full[2], acc_empty[S::ACCS], raw_full[4][BUFS], raw_empty[4][BUFS];
+    __shared__ uint64_t full[S::STAGES], empty[S::STAGES], acc_full[2], acc_empty[S::ACCS];
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
 
@@ -548,11 +552,6 @@ __global__ void __launch_bounds__(H_THREADS, 1)
             if (!S::FINE) mbar_init(&acc_full[b & 1], 1);
             mbar_init(&acc_empty[b], S::FINE ? 4 : H_CONV);
         }
-        for (int q = 0; q < 4; ++q)
-            for (uint32_t b = 0; b < BUFS; ++b) {
-                mbar_init(&raw_full[q][b], 4);
-                mbar_init(&raw_empty[q][b], 4);
-            }
         abort_flag = 0;
         mbar_fence_init();
     }
@@ -590,7 +589,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
         // read back window c: this warp's columns of its accumulator, or all columns of the accumulator of its own step
         auto drain = [&](uint32_t c, float f) -> bool {
             uint64_t* ready = S::FINE ? &empty[(c % S::WINDOWS) * H_STEPS + g] : &acc_full[c & 1];
-            if (!__all_sync(0xFFFFFFFFu, mbar_wait(ready, (S::FINE ? c / S::WINDOWS : c >> 1) & 1))) return false;
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait_polling(ready, (S::FINE ? c / S::WINDOWS : c >> 1) & 1))) return false;
             tc_fence_after();
             add_acc(S::FINE ? g * N_TILE : (c & 1) * N_TILE + g * MY_COLS, f);
             tc_fence_before();
@@ -627,23 +626,23 @@ __global__ void __launch_bounds__(H_THREADS, 1)
         bool ok = true;
         float f_prev = 0.0f;
 #pragma unroll
-        for (uint32_t b = 0; b < BUFS; ++b) copy_window(b);
-        for (uint32_t wn = 0; wn < n_windows && ok; ++wn) {
-            const uint32_t buf = wn % BUFS, par = (wn / BUFS) & 1;
-            // my copies of this window have landed; hand them over and wait for the others'
-            asm volatile("cp.async.wait_group %0;" ::"n"(BUFS - 1) : "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&raw_full[q][buf]);
-            ok = __all_sync(0xFFFFFFFFu, mbar_wait(&raw_full[q][buf], par));
-            if (!ok) break;
+        for (uint32_t b = 0; b + 1 < BUFS || b == 0; ++b) copy_window(b);
+        for (uint32_t wn = 0; wn < n_windows; ++wn) {
+            const uint32_t buf = wn % BUFS;
+            // my copies of this window have landed; meet the quarter's other warps, which also means that all four are
+            // through with the window before: its buffer takes a later one.  A warp whose wait ran out keeps coming
+            // here, so that no other waits for it.
+            asm volatile("cp.async.wait_group %0;" ::"n"(BUFS > 1 ? BUFS - 2 : 0) : "memory");
+            asm volatile("bar.sync %0, 128;" ::"r"(2 + q) : "memory");
+            if constexpr (BUFS > 1) copy_window(wn + BUFS - 1);
 #pragma unroll 1
-            for (uint32_t cc = 0; cc < T::UNITS; ++cc) {
+            for (uint32_t cc = 0; cc < T::UNITS && ok; ++cc) {
                 const uint32_t c = wn * T::UNITS + cc;
                 const uint32_t u = raw_q + buf * RAW_BUF + lane * RAW_STRIDE * 4 + cc * T::UNIT;
                 const RowWin rw = row_window<TYPE>(u);
                 // the stage's columns must have been read by the MMAs that used them last
                 const uint32_t ph = c % S::WINDOWS, st = ph * H_STEPS + g;
-                ok = __all_sync(0xFFFFFFFFu, mbar_wait(&empty[st], ((c / S::WINDOWS) & 1) ^ 1));
+                ok = __all_sync(0xFFFFFFFFu, mbar_wait_polling(&empty[st], ((c / S::WINDOWS) & 1) ^ 1));
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t acol = tmem_d + lane_base + S::ACC_COLS + st * S::A_COLS;
@@ -662,19 +661,13 @@ __global__ void __launch_bounds__(H_THREADS, 1)
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&full[st]);
-                if (cc == T::UNITS - 1) {
-                    // once the quarter's other warps are through with this window too, bring in my rows of a later one
-                    if (wn + BUFS < n_windows) {
-                        if (lane == 0) mbar_arrive(&raw_empty[q][buf]);
-                        ok = __all_sync(0xFFFFFFFFu, mbar_wait(&raw_empty[q][buf], par));
-                        if (!ok) break;
-                    }
-                    copy_window(wn + BUFS);
-                }
                 // read back the window before this one while this one accumulates
                 if (c > 0) ok = drain(c - 1, f_prev);
-                if (!ok) break;
                 f_prev = rw.f;
+            }
+            if constexpr (BUFS == 1) {  // one buffer: everyone must be through with it before it is refilled
+                asm volatile("bar.sync %0, 128;" ::"r"(2 + q) : "memory");
+                copy_window(wn + 1);
             }
         }
         if (ok && n_chunks > 0) ok = drain(n_chunks - 1, f_prev);
@@ -702,54 +695,67 @@ __global__ void __launch_bounds__(H_THREADS, 1)
 #pragma unroll
             for (int c = 0; c < MY_COLS; ++c) red[(g * MY_COLS + c) * HM + q * 32 + lane] = sums[c];
         }
-    } else if (warp == H_CONV) {
-        // ── issuer ──
+    } else if (warp < H_CONV + H_ISSUE) {
+        // ── issuers ──
         constexpr uint32_t idesc = h_idesc(N_TILE);
         const uint32_t base0 = smem_u32(smem);
         const uint64_t d0_hi = umma_desc(base0), d0_lo = umma_desc(base0 + PLANE_B);
         [[maybe_unused]] const uint64_t d_sums = umma_desc(smem_u32(s_sums));
         bool ok = true;
-        for (uint32_t c = 0; c < n_chunks && ok; ++c) {
-            const uint32_t ph = c % S::WINDOWS;
+        // steps G0 .. G1 - 1 of every window; compile-time, so that the descriptors need no arithmetic but a stage's offset
+        auto issue = [&](auto G0, auto G1) {
+            for (uint32_t c = 0; c < n_chunks && ok; ++c) {
+                const uint32_t ph = c % S::WINDOWS;
 #pragma unroll
-            for (uint32_t g = 0; g < H_STEPS; ++g) {
-                const uint32_t st = ph * H_STEPS + g, acc = S::FINE ? g : c & 1, d = tmem_d + acc * N_TILE;
-                // the accumulator's last contents must have been read back
-                if (S::FINE ? c >= 1 : g == 0 && c >= 2) {
-                    ok = __all_sync(0xFFFFFFFFu, mbar_wait(&acc_empty[acc], (S::FINE ? c - 1 : (c >> 1) - 1) & 1));
+                for (uint32_t g = G0.value; g < G1.value; ++g) {
+                    const uint32_t st = ph * H_STEPS + g, acc = S::FINE ? g : c & 1, d = tmem_d + acc * N_TILE;
+                    // the accumulator's last contents must have been read back
+                    if (S::FINE ? c >= 1 : g == 0 && c >= 2) {
+                        ok = __all_sync(0xFFFFFFFFu, mbar_wait_polling(&acc_empty[acc], (S::FINE ? c - 1 : (c >> 1) - 1) & 1));
+                        if (!ok) break;
+                    }
+                    ok = __all_sync(0xFFFFFFFFu, mbar_wait_polling(&full[st], (c / S::WINDOWS) & 1));
                     if (!ok) break;
-                }
-                ok = __all_sync(0xFFFFFFFFu, mbar_wait(&full[st], (c / S::WINDOWS) & 1));
-                if (!ok) break;
-                tc_fence_after();  // the converters' tcgen05.st / .ld
-                if (elect_one()) {
-                    const uint64_t so = (uint64_t)st * (STAGE >> 4);
-                    const uint32_t a1 = tmem_d + S::ACC_COLS + st * S::A_COLS, a2 = a1 + 32;
-                    const bool fresh = S::FINE || g == 0;
-                    // small products first, while the accumulator is small.  16 columns an instruction: 8 columns of A,
-                    // 32 bytes of B's swizzled rows.
+                    tc_fence_after();  // the converters' tcgen05.st / .ld
+                    if (elect_one()) {
+                        const uint64_t so = (uint64_t)st * (STAGE >> 4);
+                        const uint32_t a1 = tmem_d + S::ACC_COLS + st * S::A_COLS, a2 = a1 + 32;
+                        const bool fresh = S::FINE || g == 0;
+                        // small products first, while the accumulator is small.  16 columns an instruction: 8 columns of A,
+                        // 32 bytes of B's swizzled rows.
 #pragma unroll
-                    for (uint32_t kk = 0; kk < 4; ++kk) {
-                        umma_f16_ts(d, a1 + kk * 8, d0_lo + so + kk * 2, idesc, !fresh || kk != 0);
-                        if constexpr (T::TWO) umma_f16_ts(d, a2 + kk * 8, d0_hi + so + kk * 2, idesc, 1);
-                    }
-                    if constexpr (T::MIN) {
-                        if (g == H_STEPS - 1) {
-                            // a tile of sums holds two windows, 64 bytes each: first terms, second terms
-                            const uint64_t ds = d_sums + ph * (PLANE_B >> 4) + ((win0 + c) & 1) * 4;
-                            const uint32_t am = tmem_d + S::MIN_COL0 + 16 * ph;
-                            umma_f16_ts(d, am + 8, ds, idesc, 1);
-                            umma_f16_ts(d, am, ds + 2, idesc, 1);
-                            umma_f16_ts(d, am, ds, idesc, 1);
+                        for (uint32_t kk = 0; kk < 4; ++kk) {
+                            umma_f16_ts(d, a1 + kk * 8, d0_lo + so + kk * 2, idesc, !fresh || kk != 0);
+                            if constexpr (T::TWO) umma_f16_ts(d, a2 + kk * 8, d0_hi + so + kk * 2, idesc, 1);
                         }
-                    }
+                        if constexpr (T::MIN) {
+                            if (g == H_STEPS - 1) {
+                                // a tile of sums holds two windows, 64 bytes each: first terms, second terms
+                                const uint64_t ds = d_sums + ph * (PLANE_B >> 4) + ((win0 + c) & 1) * 4;
+                                const uint32_t am = tmem_d + S::MIN_COL0 + 16 * ph;
+                                umma_f16_ts(d, am + 8, ds, idesc, 1);
+                                umma_f16_ts(d, am, ds + 2, idesc, 1);
+                                umma_f16_ts(d, am, ds, idesc, 1);
+                            }
+                        }
 #pragma unroll
-                    for (uint32_t kk = 0; kk < 4; ++kk) umma_f16_ts(d, a1 + kk * 8, d0_hi + so + kk * 2, idesc, 1);
-                    umma_commit(&empty[st]);  // the weight columns and the activation tiles of the stage are free
-                    if (!S::FINE && g == H_STEPS - 1) umma_commit(&acc_full[acc]);
+                        for (uint32_t kk = 0; kk < 4; ++kk) umma_f16_ts(d, a1 + kk * 8, d0_hi + so + kk * 2, idesc, 1);
+                        umma_commit(&empty[st]);  // the weight columns and the activation tiles of the stage are free
+                        if (!S::FINE && g == H_STEPS - 1) umma_commit(&acc_full[acc]);
+                    }
+                    __syncwarp();
                 }
-                __syncwarp();
             }
+        };
+        using std::integral_constant;
+        const uint32_t mine = warp - H_CONV;
+        if constexpr (S::FINE) {
+            if (mine == 0) issue(integral_constant<uint32_t, 0>{}, integral_constant<uint32_t, 1>{});
+            else if (mine == 1) issue(integral_constant<uint32_t, 1>{}, integral_constant<uint32_t, 2>{});
+            else if (mine == 2) issue(integral_constant<uint32_t, 2>{}, integral_constant<uint32_t, 3>{});
+            else issue(integral_constant<uint32_t, 3>{}, integral_constant<uint32_t, 4>{});
+        } else if (mine == 0) {
+            issue(integral_constant<uint32_t, 0>{}, integral_constant<uint32_t, H_STEPS>{});
         }
         if (!ok && lane == 0) abort_flag = 1;
     } else {
@@ -762,7 +768,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
                 const uint32_t ph = c % S::WINDOWS;
                 for (uint32_t g = 0; g < H_STEPS; ++g) {
                     const uint32_t st = ph * H_STEPS + g;
-                    ok = mbar_wait(&empty[st], ((c / S::WINDOWS) & 1) ^ 1);
+                    ok = mbar_wait_polling(&empty[st], ((c / S::WINDOWS) & 1) ^ 1);
                     if (!ok) break;
                     uint8_t* tile = smem + (size_t)st * STAGE;
                     const bool with_sums = T::MIN && g == H_STEPS - 1;

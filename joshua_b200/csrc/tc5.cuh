@@ -8,6 +8,24 @@
 
 namespace jq {
 
+// mbar_wait for phases that usually are complete: the non-blocking test answers faster than a try_wait, which may put
+// the thread to sleep.  Bounded like mbar_wait.
+__device__ __forceinline__ bool mbar_wait_polling(uint64_t* bar, uint32_t parity) {
+    const uint32_t addr = smem_u32(bar);
+    for (int i = 0; i < 32; ++i) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(addr), "r"(parity)
+            : "memory");
+        if (done) return true;
+    }
+    return mbar_wait(bar, parity);
+}
+
 // One box of a 2-D tensor map into shared memory (x = element offset along the row, 16-byte aligned; y = row).
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint32_t x, uint32_t y, uint64_t* bar) {
     asm volatile(
