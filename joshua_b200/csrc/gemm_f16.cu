@@ -472,26 +472,25 @@ __device__ __forceinline__ void convert64(uint32_t u, uint32_t g, const RowWin& 
     }
 }
 
-// The window's 16 minima, -(dmin / f) m, as eight packed first and eight packed second terms.
+// The window's 16 minima, -(dmin / f) m, as eight packed first and eight packed second terms.  The ratio is two f16
+// terms, m at most six bits: the first products' remainders are exact.
 template <uint32_t TYPE>
 __device__ __forceinline__ void convert_minima(uint32_t u, const RowWin& rw, uint32_t (&a)[16]) {
     // -dmin / f, where f is d, d 2^e or (d = 0) dmin / 512
     const float ratio = rw.dmin == 0.0f ? 0.0f : -(rw.dmin / rw.f);
+    const __half2 rh = __float2half2_rn(ratio), rl = __float2half2_rn(ratio - __low2float(rh));
+    const uint4 hd = TYPE == T_Q4_K ? s128(u) : make_uint4(s32(u), s32(u + 4), s32(u + 8), s32(u + 12));
+    // Q4_K: eight minima of 32 values, a byte each; Q2_K: sixteen of 16 values in the high nibbles
+    const uint32_t m4[4] = {TYPE == T_Q4_K ? hd.z & 0x3F3F3F3Fu : hd.x >> 4 & 0x0F0F0F0Fu,
+                            TYPE == T_Q4_K ? (hd.w >> 4 & 0x0F0F0F0Fu) | (hd.z >> 2 & 0x30303030u) : hd.y >> 4 & 0x0F0F0F0Fu,
+                            hd.z >> 4 & 0x0F0F0F0Fu, hd.w >> 4 & 0x0F0F0F0Fu};
 #pragma unroll
     for (int p = 0; p < 8; ++p) {  // groups of 16 values 2p, 2p + 1
-        float m0, m1;
-        if constexpr (TYPE == T_Q4_K) {  // one minimum per 32 values
-            const uint32_t m6 = p < 4 ? s8(u + 8 + p) & 63u : (s8(u + 8 + p) >> 4) | ((s8(u + 4 + p) >> 6) << 4);
-            m0 = m1 = (float)m6;
-        } else {
-            m0 = (float)(s8(u + 2 * p) >> 4);
-            m1 = (float)(s8(u + 2 * p + 1) >> 4);
-        }
-        m0 *= ratio, m1 *= ratio;
-        const __half2 h = __floats2half2_rn(m0, m1);
-        const float2 hf = __half22float2(h);
-        a[p] = as_u32(h);
-        a[8 + p] = as_u32(__floats2half2_rn(m0 - hf.x, m1 - hf.y));
+        const uint32_t pair = TYPE == T_Q4_K ? __byte_perm(m4[p >> 2], 0x64646464u, 0x4040 + 0x0101 * (p & 3))
+                                             : __byte_perm(m4[p >> 1], 0x64646464u, p & 1 ? 0x4342 : 0x4140);
+        const __half2 m = __hsub2(as_h2(pair), __float2half2_rn(1024.0f)), hi = __hmul2(m, rh);
+        a[p] = as_u32(hi);
+        a[8 + p] = as_u32(__hfma2(m, rl, __hfma2(m, rh, __hneg2(hi))));
     }
 }
 
@@ -696,7 +695,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
             for (int c = 0; c < MY_COLS; ++c) red[(g * MY_COLS + c) * HM + q * 32 + lane] = sums[c];
         }
     } else if (warp < H_CONV + H_ISSUE) {
-        // ── issuers ──
+        // ── issuers (their waits sleep: polling warps take issue slots from the converters) ──
         constexpr uint32_t idesc = h_idesc(N_TILE);
         const uint32_t base0 = smem_u32(smem);
         const uint64_t d0_hi = umma_desc(base0), d0_lo = umma_desc(base0 + PLANE_B);
@@ -711,10 +710,10 @@ __global__ void __launch_bounds__(H_THREADS, 1)
                     const uint32_t st = ph * H_STEPS + g, acc = S::FINE ? g : c & 1, d = tmem_d + acc * N_TILE;
                     // the accumulator's last contents must have been read back
                     if (S::FINE ? c >= 1 : g == 0 && c >= 2) {
-                        ok = __all_sync(0xFFFFFFFFu, mbar_wait_polling(&acc_empty[acc], (S::FINE ? c - 1 : (c >> 1) - 1) & 1));
+                        ok = __all_sync(0xFFFFFFFFu, mbar_wait(&acc_empty[acc], (S::FINE ? c - 1 : (c >> 1) - 1) & 1));
                         if (!ok) break;
                     }
-                    ok = __all_sync(0xFFFFFFFFu, mbar_wait_polling(&full[st], (c / S::WINDOWS) & 1));
+                    ok = __all_sync(0xFFFFFFFFu, mbar_wait(&full[st], (c / S::WINDOWS) & 1));
                     if (!ok) break;
                     tc_fence_after();  // the converters' tcgen05.st / .ld
                     if (elect_one()) {
@@ -768,7 +767,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
                 const uint32_t ph = c % S::WINDOWS;
                 for (uint32_t g = 0; g < H_STEPS; ++g) {
                     const uint32_t st = ph * H_STEPS + g;
-                    ok = mbar_wait_polling(&empty[st], ((c / S::WINDOWS) & 1) ^ 1);
+                    ok = mbar_wait(&empty[st], ((c / S::WINDOWS) & 1) ^ 1);
                     if (!ok) break;
                     uint8_t* tile = smem + (size_t)st * STAGE;
                     const bool with_sums = T::MIN && g == H_STEPS - 1;
