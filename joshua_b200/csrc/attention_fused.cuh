@@ -81,7 +81,11 @@ __device__ __forceinline__ void att_sync() {
 
 // One (chunk, kv head, sequence) item.  tid = 0..255 inside the group of threads; s_f: the item's shared
 // memory (attention_fused_smem_floats floats); s_last: one shared word.
-template <int BAR, uint32_t HD, uint32_t G>
+//
+// MANY: the launch holds more items than SMs.  An item then looks at the position first and leaves, without a load, if
+// its chunk lies behind it: with one wave the extra trip to L2 costs more than the loads, with several the dead items'
+// rows are most of the traffic (16 of 17 chunks of a 1056-position cache at the start of a sequence).
+template <int BAR, uint32_t HD, uint32_t G, bool MANY>
 __device__ __forceinline__ void attention_fused_item_t(const AttnArgs& a, uint32_t chunk, uint32_t kvh, uint32_t sg,
                                                        uint32_t b, uint32_t tid, float* s_f, uint32_t* s_last) {
     constexpr uint32_t NW = ATT_FUSED_THREADS / 32;
@@ -115,6 +119,7 @@ __device__ __forceinline__ void attention_fused_item_t(const AttnArgs& a, uint32
 
     // ── every independent load first: position, rotary inputs, the chunk's K rows and V rows ──
     const int32_t p_raw = __ldcg(a.pos + b);
+    if (MANY && p_raw >= 0 && (uint32_t)p_raw < max_ctx && t0 > (uint32_t)p_raw) return;
     float ra[ROT_PER], rb[ROT_PER];
 #pragma unroll
     for (uint32_t r = 0; r < ROT_PER; ++r) {
@@ -360,28 +365,6 @@ __device__ __forceinline__ void attention_fused_item_t(const AttnArgs& a, uint32
             a.out[((uint64_t)b * nq + hb + g) * HD + i] = acc / sden[g];
         }
     }
-}
-
-// Dispatch on the head size and the heads per item (attention_fused_shape_ok).
-template <int BAR>
-__device__ __forceinline__ void attention_fused_item(const AttnArgs& a, uint32_t chunk, uint32_t kvh, uint32_t sg,
-                                                     uint32_t b, uint32_t tid, float* s_f, uint32_t* s_last) {
-    const uint32_t G = a.nq / a.nkv / a.gsplit;
-#define JQ_ATT_CASE(HDV, GV) \
-    if (a.hd == HDV && G == GV) return attention_fused_item_t<BAR, HDV, GV>(a, chunk, kvh, sg, b, tid, s_f, s_last);
-    JQ_ATT_CASE(128, 4)
-    JQ_ATT_CASE(128, 8)
-    JQ_ATT_CASE(128, 1)
-    JQ_ATT_CASE(128, 2)
-    JQ_ATT_CASE(64, 1)
-    JQ_ATT_CASE(64, 2)
-    JQ_ATT_CASE(64, 4)
-    JQ_ATT_CASE(64, 8)
-    JQ_ATT_CASE(256, 1)
-    JQ_ATT_CASE(256, 2)
-    JQ_ATT_CASE(256, 4)
-    JQ_ATT_CASE(256, 8)
-#undef JQ_ATT_CASE
 }
 
 }  // namespace jq
