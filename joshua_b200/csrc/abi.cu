@@ -70,16 +70,27 @@ int32_t validate_matmul(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, 
 
 }  // namespace
 
-bool jq_uses_tiles(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n) {
-    return !w->ctx->force_f32 && m >= w->ctx->tiles_min_m && jq::gemm_f16_supports(w->type, w->dev, n, k, m);
+static cudaStream_t tiles_scratch_key(cudaStream_t s) {
+    return reinterpret_cast<cudaStream_t>(reinterpret_cast<uintptr_t>(s) ^ 3);
+}
+
+// From nine rows on the other route is the decode kernel once per eight rows.  From five rows on, where the decode
+// kernel's activation planes do not fit its shared memory, it reads them from L2 for every 16 weight rows; Q4_K, bound
+// by its consumers' instructions, is behind the tiles from five rows on in any case.  Measured, eight rows, tiles /
+// decode kernel: Q4_K 28672 x 4096 53 / 66 us, 4096 x 14336 31 / 35 us, 7168 x 2048 12 / 19 us, Q8_0 69 / 96, 38 / 59
+// and 13 / 15 us; five rows, planes in shared memory: Q4_K 28672 x 4096 52 / 64 us, Q8_0 69 / 50 us; four rows, Q4_K:
+// 53 / 28 us.
+bool jq_uses_tiles(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, cudaStream_t s) {
+    if (w->ctx->force_f32 || m < 5 || !jq::gemm_f16_supports(w->type, w->dev, n, k, m)) return false;
+    if (m <= jq::GEMV_MMA_MAX_M && w->type != jq::T_Q4_K && jq::gemv_mma_scratch_bytes(m, k) == 0) return false;
+    return w->ctx->scratch_available(tiles_scratch_key(s), jq::gemm_f16_scratch_bytes(m, k), s);
 }
 
 int32_t jq_matmul_tiles(const jq_weight* w, const jq_weight* w_b, uint64_t m, uint64_t k, uint64_t n, const float* lhs,
                         const float* norm_w, float eps, const float* residual, float* dst, float* dst_b, cudaStream_t s) {
     jq_ctx* ctx = w->ctx;
     void* scratch = nullptr;
-    JQ_CUDA(ctx->scratch_for(reinterpret_cast<cudaStream_t>(reinterpret_cast<uintptr_t>(s) ^ 3),
-                             jq::gemm_f16_scratch_bytes(m, k), &scratch));
+    JQ_CUDA(ctx->scratch_for(tiles_scratch_key(s), jq::gemm_f16_scratch_bytes(m, k), &scratch));
     JQ_CUDA(jq::launch_gemm_f16(w->type, w->dev, w_b ? w_b->dev : nullptr, n, k, lhs, m, norm_w, eps, residual, dst, dst_b,
                                 scratch, ctx->status_dev, s));
     return jq::OK;
@@ -90,7 +101,7 @@ int32_t jq_matmul_tiles(const jq_weight* w, const jq_weight* w_b, uint64_t m, ui
 int32_t jq_matmul_device(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, const float* lhs, float* dst,
                          cudaStream_t s) {
     jq_ctx* ctx = w->ctx;
-    if (jq_uses_tiles(w, m, k, n)) return jq_matmul_tiles(w, nullptr, m, k, n, lhs, nullptr, 0.0f, nullptr, dst, nullptr, s);
+    if (jq_uses_tiles(w, m, k, n, s)) return jq_matmul_tiles(w, nullptr, m, k, n, lhs, nullptr, 0.0f, nullptr, dst, nullptr, s);
     if (!ctx->force_f32 && jq::gemv_mma_dense_supports(w->type, w->dev, n, k, m)) {
         void* scratch = nullptr;
         JQ_CUDA(ctx->scratch_for(s, jq::gemv_mma_scratch_bytes(m, k), &scratch));
@@ -195,7 +206,6 @@ int32_t jq_init(int32_t device, jq_ctx** out) {
     c->device = device;
     const char* f = std::getenv("JQ_FORCE_F32_PATH");
     c->force_f32 = f && f[0] == '1';
-    if (const char* tm = std::getenv("JQ_TILES_MIN_M")) c->tiles_min_m = std::max(1ull, std::strtoull(tm, nullptr, 10));
     if (const char* sm = std::getenv("JQ_SLICED_MAX_M")) c->sliced_max_m = std::strtoull(sm, nullptr, 10);
     cudaError_t he = cudaHostAlloc(&c->status_host, sizeof(int), cudaHostAllocMapped);
     if (he == cudaSuccess) he = cudaHostGetDevicePointer(&c->status_dev, c->status_host, 0);

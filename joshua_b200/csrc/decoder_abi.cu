@@ -9,11 +9,20 @@ bool vectors(const float* lhs, const float* norm_w) {
     return (reinterpret_cast<uintptr_t>(lhs) | reinterpret_cast<uintptr_t>(norm_w)) % 16 == 0;
 }
 
+size_t swiglu_scratch_bytes(uint64_t m, uint64_t n) { return 2 * m * n * 4 + 512; }
+cudaStream_t swiglu_scratch_key(cudaStream_t s) {
+    return reinterpret_cast<cudaStream_t>(reinterpret_cast<uintptr_t>(s) ^ 1);
+}
+bool pair_uses_tiles(const jq_weight* gate, const jq_weight* up, uint64_t m, uint64_t k, uint64_t n, cudaStream_t s) {
+    return jq_uses_tiles(gate, m, k, n, s) && jq_uses_tiles(up, m, k, n, s) &&
+           gate->ctx->scratch_available(swiglu_scratch_key(s), swiglu_scratch_bytes(m, n), s);
+}
+
 // silu(clamp(gate x)) * clamp(up x) on the tile GEMM: one launch for both tensors into scratch, then the combine.
 int32_t swiglu_tiles(const jq_weight* gate, const jq_weight* up, uint64_t m, uint64_t k, uint64_t n, const float* lhs,
                      const float* norm_w, float eps, float* dst, float clamp, cudaStream_t s) {
     void* scratch = nullptr;
-    JQ_CUDA(gate->ctx->scratch_for(reinterpret_cast<cudaStream_t>(reinterpret_cast<uintptr_t>(s) ^ 1), 2 * m * n * 4 + 512, &scratch));
+    JQ_CUDA(gate->ctx->scratch_for(swiglu_scratch_key(s), swiglu_scratch_bytes(m, n), &scratch));
     float* g = static_cast<float*>(scratch);
     float* u = g + ((m * n + 63) & ~(uint64_t)63);
     if (int32_t rc = jq_matmul_tiles(gate, up, m, k, n, lhs, norm_w, eps, nullptr, g, u, s)) return rc;
@@ -38,7 +47,7 @@ int32_t jq_matmul_swiglu_dev(const jq_weight* gate, const jq_weight* up, uint64_
     if (!lhs_dev || !dst_dev) return jq_fail(jq::E_INVALID, "jq_matmul_swiglu_dev: NULL buffer");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     jq_ctx* ctx = gate->ctx;
-    if (jq_uses_tiles(gate, m, k, n) && jq_uses_tiles(up, m, k, n))
+    if (pair_uses_tiles(gate, up, m, k, n, s))
         return swiglu_tiles(gate, up, m, k, n, lhs_dev, nullptr, 0.0f, dst_dev, clamp, s);
     if (!ctx->force_f32 && jq::gemv_mma_supports(gate->type, gate->dev, n, k, m) &&
         jq::gemv_mma_supports(up->type, up->dev, n, k, m) && jq::gemv_mma_scratch_bytes(m, k) == 0) {
@@ -48,8 +57,7 @@ int32_t jq_matmul_swiglu_dev(const jq_weight* gate, const jq_weight* up, uint64_
     }
     // two products into scratch, then the element-wise combine
     void* scratch = nullptr;
-    size_t need = 2 * m * n * 4 + 512;
-    JQ_CUDA(ctx->scratch_for(reinterpret_cast<cudaStream_t>(reinterpret_cast<uintptr_t>(s) ^ 1), need, &scratch));
+    JQ_CUDA(ctx->scratch_for(swiglu_scratch_key(s), swiglu_scratch_bytes(m, n), &scratch));
     float* g = static_cast<float*>(scratch);
     float* u = g + ((m * n + 63) & ~(uint64_t)63);
     if (int32_t rc = jq_matmul_device(gate, m, k, n, lhs_dev, g, s)) return rc;
@@ -67,7 +75,7 @@ int32_t jq_matmul_swiglu_norm_dev(const jq_weight* gate, const jq_weight* up, ui
     jq_ctx* ctx = gate->ctx;
     const bool shapes_ok = gate->type == up->type && gate->n_blocks == up->n_blocks && k % gate->fmt.elems == 0 &&
                            gate->n_blocks == n * (k / gate->fmt.elems) && m > 0 && n > 0 && lhs_dev && dst_dev;
-    if (shapes_ok && vectors(lhs_dev, norm_w_dev) && jq_uses_tiles(gate, m, k, n) && jq_uses_tiles(up, m, k, n))
+    if (shapes_ok && vectors(lhs_dev, norm_w_dev) && pair_uses_tiles(gate, up, m, k, n, s))
         return swiglu_tiles(gate, up, m, k, n, lhs_dev, norm_w_dev, eps, dst_dev, clamp, s);
     if (shapes_ok && !ctx->force_f32 && jq::gemv_mma_supports(gate->type, gate->dev, n, k, m) &&
         jq::gemv_mma_supports(up->type, up->dev, n, k, m) && jq::gemv_mma_fusable(m, k)) {
@@ -91,7 +99,7 @@ int32_t jq_matmul_norm_dev(const jq_weight* w, uint64_t m, uint64_t k, uint64_t 
     jq_ctx* ctx = w->ctx;
     const bool shapes_ok = k % w->fmt.elems == 0 && w->n_blocks == n * (k / w->fmt.elems) && m > 0 && n > 0 &&
                            lhs_dev && dst_dev;
-    if (shapes_ok && vectors(lhs_dev, norm_w_dev) && jq_uses_tiles(w, m, k, n))
+    if (shapes_ok && vectors(lhs_dev, norm_w_dev) && jq_uses_tiles(w, m, k, n, s))
         return jq_matmul_tiles(w, nullptr, m, k, n, lhs_dev, norm_w_dev, eps, residual_dev, dst_dev, nullptr, s);
     if (shapes_ok && !ctx->force_f32 && jq::gemv_mma_dense_supports(w->type, w->dev, n, k, m) &&
         jq::gemv_mma_fusable(m, k)) {

@@ -50,8 +50,7 @@ struct StreamScratch {
 struct jq_ctx {
     int device = 0;
     bool force_f32 = false;        // JQ_FORCE_F32_PATH=1: always take the exact-decode float kernels
-    uint64_t tiles_min_m = 9;      // JQ_TILES_MIN_M: smallest batch that runs on the f16 tile GEMM
-    uint64_t sliced_max_m = 64;    // JQ_SLICED_MAX_M: largest batch run as 8-row slices of the decode kernel (0 = never)
+    uint64_t sliced_max_m = 64;    // JQ_SLICED_MAX_M: largest batch run as 8-row slices of the decode kernel where the f16 tiles do not apply (0 = never)
     int* status_host = nullptr;    // pinned, device-visible: set to 1 by a kernel whose bounded wait gave up
     int* status_dev = nullptr;
     std::mutex mu;
@@ -79,6 +78,18 @@ struct jq_ctx {
         }
         *out = sc.dev;
         return cudaSuccess;
+    }
+
+    // Whether `stream`'s scratch can be had now: it is large enough, or may be allocated because `capture` (the stream the
+    // work goes to) is not being captured.  Routes that need scratch where an older one did not ask this first.
+    bool scratch_available(cudaStream_t stream, size_t bytes, cudaStream_t capture) {
+        {
+            std::lock_guard<std::mutex> g(mu);
+            auto it = scratch.find(stream);
+            if (it != scratch.end() && it->second.cap >= bytes) return true;
+        }
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        return cudaStreamIsCapturing(capture, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
     }
 
     Workspace* acquire() {
@@ -122,7 +133,7 @@ int32_t jq_matmul_device(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n,
 
 // Whether a product of m rows runs on the f16 tile GEMM, and that product: dst = residual + norm(lhs) . W^T, with w_b (a
 // tensor of the same type and shape) also dst_b = norm(lhs) . W_b^T.  norm_w, residual and w_b may be NULL (abi.cu).
-bool jq_uses_tiles(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n);
+bool jq_uses_tiles(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, cudaStream_t s);
 int32_t jq_matmul_tiles(const jq_weight* w, const jq_weight* w_b, uint64_t m, uint64_t k, uint64_t n, const float* lhs,
                         const float* norm_w, float eps, const float* residual, float* dst, float* dst_b, cudaStream_t s);
 

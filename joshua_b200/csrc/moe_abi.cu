@@ -131,6 +131,35 @@ int32_t run_experts(jq_moe* m, const float* x, uint64_t R, uint64_t P, uint32_t 
 // launch per phase over a list of (expert, row range) tiles built on the device.
 constexpr uint64_t BUCKET_ROWS_PER_EXPERT = 12;  // rows from which an expert runs on the tile GEMM
 constexpr uint64_t BUCKET_MIN_TOKENS = 128;      // tokens from which the prefill form (tile GEMM + decode kernel) is used
+constexpr uint64_t TILES_MIN_TOKENS = 32;        // the same for the types whose experts all run on tiles
+
+// Banks whose experts run on the tile GEMM whatever their row count.  Measured, 384 MXFP4 experts of 7168 x 2048, eight a
+// token, tiles / decode kernel: 3.87 / 4.85 ms at 100 tokens, 2.13 / 2.17 at 32, 1.35 / 1.19 at 16; 48 layers of 128
+// Q4_K experts of 2048 x 768: 14.0 / 27.6 ms at 100 tokens, 11.6 / 14.5 at 40, 13.8 / 10.1 (a decode step) at 16.
+bool all_experts_on_tiles(const jq_moe* m) {
+    auto one = [](const jq_weight* w) { return w->type == jq::T_Q4_K || w->type == jq::T_MXFP4; };
+    return one(m->gate) && one(m->up) && one(m->down);
+}
+
+cudaStream_t bucket_scratch_key(cudaStream_t s) {
+    return reinterpret_cast<cudaStream_t>(reinterpret_cast<uintptr_t>(s) ^ 3);
+}
+size_t bucket_scratch_bytes(const jq_moe_config& c, uint64_t P) {
+    return std::max(jq::gemm_f16_scratch_bytes(P, c.hidden), jq::gemm_f16_scratch_bytes(P, c.inter));
+}
+// The device form of run_experts_bucketed: no host read.
+bool grouped_tiles_ok(const jq_moe* m, uint64_t P) {
+    const jq_moe_config& c = m->cfg;
+    return jq::gemm_f16_grouped_supports(m->gate->type, m->gate->dev, c.inter, c.hidden) && m->up->type == m->gate->type &&
+           jq::gemm_f16_grouped_supports(m->up->type, m->up->dev, c.inter, c.hidden) &&
+           jq::gemm_f16_grouped_supports(m->down->type, m->down->dev, c.hidden, c.inter) && P / 33 + 1 <= 65535;
+}
+
+uint32_t max_narrow_tiles(const jq_moe* m, uint64_t P) { return (uint32_t)std::min<uint64_t>(m->cfg.n_expert, P + 1); }
+uint64_t bucket_lists_bytes(const jq_moe* m, uint64_t P, uint32_t rows_per_job) {
+    return ((uint64_t)max_narrow_tiles(m, P) + P / 33 + 1) * sizeof(jq::GemmTile) +
+           std::min<uint64_t>(P, P / rows_per_job + m->cfg.n_expert) * sizeof(jq::MoeJob) + 32;
+}
 
 int32_t run_experts_bucketed(jq_moe* m, const float* x, uint64_t T, uint64_t P, uint32_t rows_per_job, cudaStream_t s) {
     const jq_moe_config& c = m->cfg;
@@ -148,18 +177,17 @@ int32_t run_experts_bucketed(jq_moe* m, const float* x, uint64_t T, uint64_t P, 
     // them cut into tiles of up to 128 rows and runs on the tile GEMM, one grouped launch per phase and tile class
     // (gate and up together, then down); the other experts' jobs run on the grouped decode kernel in the same pass.
     // No host read: the launches cover the lists' capacity and the kernels read their lengths.
-    if (jq::gemm_f16_grouped_supports(m->gate->type, m->gate->dev, c.inter, c.hidden) && m->up->type == m->gate->type &&
-        jq::gemm_f16_grouped_supports(m->down->type, m->down->dev, c.hidden, c.inter) && P / 33 + 1 <= 65535) {
+    if (grouped_tiles_ok(m, P)) {
         // a narrow tile (<= 32 rows) is an expert's only tile (>= min rows) or the last piece behind full tiles; a wide
         // tile holds more than 32 rows
         // With 24 or more rows per expert on average hardly an expert is small: every expert then takes the tile
-        // form (an expert with a few rows is one narrow tile) and the decode kernel's passes are left out.
-        const bool all_tiles = true;
+        // form (an expert with a few rows is one narrow tile) and the decode kernel's passes are left out; so do the
+        // types whose narrow tiles are ahead of the decode kernel at any row count.
+        const bool all_tiles = all_experts_on_tiles(m) || P >= 24ull * c.n_expert;
         const uint32_t min_rows = all_tiles ? 1u : (uint32_t)BUCKET_ROWS_PER_EXPERT;
-        const uint32_t max_narrow = (uint32_t)std::min<uint64_t>(c.n_expert, P / min_rows + 1);
-        const uint32_t max_wide = (uint32_t)(P / 33 + 1);
+        const uint32_t max_narrow = max_narrow_tiles(m, P), max_wide = (uint32_t)(P / 33 + 1);
         const uint32_t max_small = (uint32_t)std::min<uint64_t>(P, P / rows_per_job + c.n_expert);
-        const uint64_t need_bytes = ((uint64_t)max_narrow + max_wide) * sizeof(jq::GemmTile) + (uint64_t)max_small * sizeof(jq::MoeJob) + 32;
+        const uint64_t need_bytes = bucket_lists_bytes(m, P, rows_per_job);
         if (need_bytes > m->tiles_cap) {
             if (m->tiles) cudaFree(m->tiles);
             m->tiles = nullptr;
@@ -174,8 +202,7 @@ int32_t run_experts_bucketed(jq_moe* m, const float* x, uint64_t T, uint64_t P, 
         uint32_t* counts = reinterpret_cast<uint32_t*>(
             (reinterpret_cast<uintptr_t>(small_jobs + max_small) + 15) & ~(uintptr_t)15);
         void* scratch = nullptr;
-        const size_t need = std::max(jq::gemm_f16_scratch_bytes(P, c.hidden), jq::gemm_f16_scratch_bytes(P, c.inter));
-        JQ_CUDA(m->ctx->scratch_for(reinterpret_cast<cudaStream_t>(reinterpret_cast<uintptr_t>(s) ^ 3), need, &scratch));
+        JQ_CUDA(m->ctx->scratch_for(bucket_scratch_key(s), bucket_scratch_bytes(c, P), &scratch));
         JQ_CUDA(jq::launch_moe_gather(x, m->list_token, m->n_list, (uint32_t)P, c.hidden, xs, s));
         JQ_CUDA(jq::launch_moe_tiles(m->jobs, m->n_jobs, m->n_list, c.n_expert, min_rows, narrow, wide, small_jobs, counts, s));
         JQ_CUDA(jq::launch_gemm_f16_grouped(m->gate->type, m->gate->dev, m->up->dev, m->gate_expert_bytes, c.inter, c.hidden, xs, P,
@@ -542,20 +569,27 @@ int32_t jq_moe_forward_norm_add_dev(jq_moe* m, const float* x_dev, uint64_t T, c
         JQ_CUDA(jq::launch_moe_jobs(m->ids, (uint32_t)T, c.n_used, c.n_expert, rpj, m->list_token, m->inv, m->jobs,
                                     m->n_jobs, m->n_list, m->bad_dev, s));
     }
-    // From BUCKET_MIN_TOKENS tokens on, the prefill form: experts with at least BUCKET_ROWS_PER_EXPERT rows on the
-    // tile GEMM, the others on the grouped decode kernel, decided per expert on the device.  Measured crossovers of
-    // the two kernels (uniform routing): 128 Q4_K experts of 2048 x 768 between 8 and 16 rows per expert (tile GEMM /
-    // decode kernel 0.91 / 0.68 ms at 8, 0.78 / 1.13 ms at 16), 384 MXFP4 experts of 7168 x 2048 near 11
-    // (20.8 / 19.2 ms), 256 IQ2_XXS experts of the same shape above 8 (13.3 / 9.2 ms).
+    // From BUCKET_MIN_TOKENS tokens on, the prefill form: the experts on the tile GEMM, or (types that are not
+    // all_experts_on_tiles) those with at least BUCKET_ROWS_PER_EXPERT rows and the others on the grouped decode kernel,
+    // decided per expert on the device.  From TILES_MIN_TOKENS on where every expert takes tiles, unless that would
+    // allocate while the stream is captured (the decode form needs nothing beyond jq_moe_reserve).
     uint64_t min_tokens = BUCKET_MIN_TOKENS;
+    if (T >= TILES_MIN_TOKENS && T < BUCKET_MIN_TOKENS && all_experts_on_tiles(m) && grouped_tiles_ok(m, P)) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &st) == cudaSuccess &&
+            (st == cudaStreamCaptureStatusNone ||
+             (P <= m->bucket_pairs && bucket_lists_bytes(m, P, rpj) <= m->tiles_cap &&
+              m->ctx->scratch_available(bucket_scratch_key(s), bucket_scratch_bytes(c, P), s))))
+            min_tokens = TILES_MIN_TOKENS;
+    }
 #ifdef JQ_PROFILING
     if (const char* thr_env = std::getenv("JQ_MOE_BUCKET_TOKENS")) min_tokens = std::strtoull(thr_env, nullptr, 10);  // measurement switch
 #endif
     const bool bucketed = !fused && !m->ctx->force_f32 && T >= min_tokens;
+    if (T < BUCKET_MIN_TOKENS || !bucketed) m->last_rows = T, m->last_pairs = P, m->last_rpj = rpj;  // the replay entry's list
     if (bucketed) {
         if (int32_t rc = run_experts_bucketed(m, x_in, T, P, rpj, s)) return rc;
     } else {
-        m->last_rows = T, m->last_pairs = P, m->last_rpj = rpj;
         if (int32_t rc = run_experts(m, x_in, T, P, rpj, s, nw, eps)) return rc;
     }
     const float* shared = nullptr;
