@@ -143,8 +143,8 @@ cudaError_t launch_gemv_mma_swiglu(uint32_t type, const uint8_t* w_gate, const u
                                    const float* lhs, uint64_t m, float* dst, float clamp, int* error_flag,
                                    cudaStream_t s, const float* norm_w = nullptr, float eps = 0.0f);
 // dst = residual + rmsnorm(lhs; norm_w, eps) . W^T in one launch (norm_w, residual optional; residual may be
-// dst).  Valid when gemv_mma_fusable(m, k).
-bool gemv_mma_fusable(uint64_t m, uint64_t k);
+// dst).  Valid when gemv_mma_fusable(type, m, k).
+bool gemv_mma_fusable(uint32_t type, uint64_t m, uint64_t k);
 cudaError_t launch_gemv_mma_fused(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, const float* lhs,
                                   uint64_t m, float* dst, const float* norm_w, float eps, const float* residual,
                                   int* error_flag, cudaStream_t s);

@@ -100,13 +100,17 @@ __global__ void __launch_bounds__(128) rope_append_kernel(const float* __restric
                                                           float* __restrict__ cache_k, float* __restrict__ cache_v,
                                                           int32_t* __restrict__ bad_pos, uint32_t seq,
                                                           const float* __restrict__ q_norm,
-                                                          const float* __restrict__ k_norm, float qk_eps) {
+                                                          const float* __restrict__ k_norm, float qk_eps,
+                                                          uint32_t heads_per_cta) {
     __shared__ float red[4];
+    extern __shared__ float2 s_rot[];  // hd / 2 (sine, cosine)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     pdl_wait_();
     // decode (seq == 0): blockIdx.y is the sequence, its position pos[b].  Prefill (seq > 0): one sequence,
     // blockIdx.y is the token, its position pos[0] + token; the cache is sequence 0's.
-    const uint32_t b = blockIdx.y, head = blockIdx.x;  // heads 0..nq-1: q; nq..nq+nkv-1: k; then v
+    // heads 0..nq-1: q; nq..nq+nkv-1: k; then v.  A CTA takes heads_per_cta consecutive heads: the angles of a position
+    // (a power, a sine and a cosine per pair) are the same for all of them.
+    const uint32_t b = blockIdx.y, heads = nq + 2 * nkv, h0 = blockIdx.x * heads_per_cta;
     const int32_t p_raw = seq ? pos[0] + (int32_t)b : pos[b];
     const uint32_t cb = seq ? 0u : b;  // cache block
     if (p_raw < 0 || (uint32_t)p_raw >= max_ctx) {
@@ -114,31 +118,36 @@ __global__ void __launch_bounds__(128) rope_append_kernel(const float* __restric
         if (threadIdx.x == 0 && bad_pos) atomicExch(bad_pos, 1);
         return;
     }
-    const uint32_t p = (uint32_t)p_raw;
-    const float* src = qkv + ((uint64_t)b * (nq + 2 * nkv) + head) * hd;
-    const uint32_t half = hd / 2;
-    if (head < nq + nkv) {
-        float* dst = head < nq ? q_out + ((uint64_t)b * nq + head) * hd
-                               : cache_k + (((uint64_t)cb * nkv + (head - nq)) * max_ctx + p) * hd;
-        const float* nw = head < nq ? q_norm : k_norm;
-        float sc = 1.0f;
-        if (nw != nullptr) {  // per-head RMS norm in front of the rotary embedding
-            float ss = 0.0f;
-            for (uint32_t i = threadIdx.x; i < hd; i += blockDim.x) ss = fmaf(src[i], src[i], ss);
-            sc = rsqrtf(block_sum(ss, red) / (float)hd + qk_eps);
+    const uint32_t p = (uint32_t)p_raw, half = hd / 2;
+    for (uint32_t i = threadIdx.x; i < half; i += blockDim.x) {
+        if (h0 >= nq + nkv) break;  // v heads only
+        float s, c;
+        sincosf((float)p * rope_freq(theta, i, hd), &s, &c);
+        s_rot[i] = make_float2(s, c);  // read back by this thread alone
+    }
+    for (uint32_t head = h0; head < min(h0 + heads_per_cta, heads); ++head) {
+        const float* src = qkv + ((uint64_t)b * heads + head) * hd;
+        if (head < nq + nkv) {
+            float* dst = head < nq ? q_out + ((uint64_t)b * nq + head) * hd
+                                   : cache_k + (((uint64_t)cb * nkv + (head - nq)) * max_ctx + p) * hd;
+            const float* nw = head < nq ? q_norm : k_norm;
+            float sc = 1.0f;
+            if (nw != nullptr) {  // per-head RMS norm in front of the rotary embedding
+                float ss = 0.0f;
+                for (uint32_t i = threadIdx.x; i < hd; i += blockDim.x) ss = fmaf(src[i], src[i], ss);
+                sc = rsqrtf(block_sum(ss, red) / (float)hd + qk_eps);
+            }
+            for (uint32_t i = threadIdx.x; i < half; i += blockDim.x) {
+                const float s = s_rot[i].x, c = s_rot[i].y;
+                float a = src[i], bb = src[i + half];
+                if (nw != nullptr) a = a * sc * nw[i], bb = bb * sc * nw[i + half];
+                dst[i] = a * c - bb * s;
+                dst[i + half] = a * s + bb * c;
+            }
+        } else {
+            float* dst = cache_v + (((uint64_t)cb * nkv + (head - nq - nkv)) * max_ctx + p) * hd;
+            for (uint32_t i = threadIdx.x; i < hd; i += blockDim.x) dst[i] = src[i];
         }
-        for (uint32_t i = threadIdx.x; i < half; i += blockDim.x) {
-            float freq = rope_freq(theta, i, hd);
-            float s, c;
-            sincosf((float)p * freq, &s, &c);
-            float a = src[i], bb = src[i + half];
-            if (nw != nullptr) a = a * sc * nw[i], bb = bb * sc * nw[i + half];
-            dst[i] = a * c - bb * s;
-            dst[i + half] = a * s + bb * c;
-        }
-    } else {
-        float* dst = cache_v + (((uint64_t)cb * nkv + (head - nq - nkv)) * max_ctx + p) * hd;
-        for (uint32_t i = threadIdx.x; i < hd; i += blockDim.x) dst[i] = src[i];
     }
 }
 
@@ -548,8 +557,11 @@ cudaError_t launch_rope_append(const float* qkv, const int32_t* pos, uint32_t ba
                                uint32_t hd, uint32_t max_ctx, float theta, float* q_out, float* cache_k, float* cache_v,
                                int32_t* bad_pos, cudaStream_t s, uint32_t seq, const float* q_norm, const float* k_norm,
                                float qk_eps) {
-    cudaError_t le2__ = launch_pdl(rope_append_kernel, dim3(nq + 2 * nkv, seq ? seq : batch), 128, 0, s, qkv, pos, nq, nkv, hd, max_ctx, theta, q_out, cache_k,
-                                                                 cache_v, bad_pos, seq, q_norm, k_norm, qk_eps);
+    // one head a CTA while the grid is small (a decode step: latency), eight once every SM has its CTAs
+    const uint32_t heads = nq + 2 * nkv, rows = seq ? seq : batch;
+    const uint32_t per = (uint64_t)heads * rows >= 8ull * 16 * num_sms() ? 8 : 1;
+    cudaError_t le2__ = launch_pdl(rope_append_kernel, dim3((heads + per - 1) / per, rows), 128, hd / 2 * sizeof(float2), s, qkv, pos, nq,
+                                   nkv, hd, max_ctx, theta, q_out, cache_k, cache_v, bad_pos, seq, q_norm, k_norm, qk_eps, per);
     if (le2__ != cudaSuccess) return le2__;
     return cudaGetLastError();
 }

@@ -978,6 +978,9 @@ __global__ void __launch_bounds__((NCW + 2) * 32, 1) gemv_mma_kernel(const __gri
         a.n_groups = n_groups;
         float colacc[NH][2][2], minacc[NB][2];
         uint32_t job = 0, red_it = 0;
+        // Units are dealt to the warps in turn over the CTA's whole stream of chunks and tiles: a chunk of eight units
+        // (Q8_0), a last chunk or a row of three units occupies some warps and the next one the others.
+        uint32_t first = cw;  // this warp's first unit of the chunk: (cw - units dealt so far) mod NCW
         for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
             uint32_t rt;
             const MoeJob jd = job_of(tile, &rt);
@@ -1003,11 +1006,12 @@ __global__ void __launch_bounds__((NCW + 2) * 32, 1) gemv_mma_kernel(const __gri
                     const uint8_t* st = ring + s * stage_bytes;
                     const uint32_t u_lo = chunk * Tr::CHUNK_UNITS;
                     const uint32_t cnt = min(units_per_row - u_lo, Tr::CHUNK_UNITS);
-                    for (uint32_t u = cw; u < cnt; u += NCW) {
+                    for (uint32_t u = first; u < cnt; u += NCW) {
                         const uint8_t* u0 = st + ro.g * plan.row_stride + sh0 + u * Tr::UNIT_BYTES;
                         const uint8_t* u1 = st + (ro.g + 8) * plan.row_stride + sh1 + u * Tr::UNIT_BYTES;
                         process_unit<TYPE, MB, NH, ACT>(u0, u1, u_lo + u, a, ro, s_grid, s_mask, colacc, minacc);
                     }
+                    first = (first - cnt) & (NCW - 1);
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&empty[s]);
                 }
@@ -1310,7 +1314,11 @@ __global__ void __launch_bounds__((16 + 2) * 32, 1) gemv_narrow_kernel(const __g
 }
 
 constexpr uint32_t SMEM_BUDGET = 220 * 1024;  // of the 227 KB a CTA may use
-constexpr uint32_t ACT_SMEM_MAX = 96 * 1024;  // measured: 116 KB (8 rows of k = 4096 in shared memory, two ring stages left) is slower than planes in global memory with a deeper ring
+// Activation planes kept in shared memory, at most.  Measured: 116 KB (8 rows of k = 4096, two ring stages left) is slower
+// than planes in global memory with a deeper ring.  Four rows of k = 7168 (98 KB), 2048 weight rows, shared / global:
+// Q8_0 13.7 / 14.9 us, Q4_K 12.6 / 9.6 us, IQ2_XXS 14.0 / 9.0 us: only Q8_0, whose units take the fewest instructions,
+// gains.
+constexpr uint32_t ACT_SMEM_MAX = 96 * 1024, ACT_SMEM_MAX_Q8_0 = 100 * 1024;
 
 template <uint32_t TYPE>
 uint32_t row_stride_for(uint64_t k) {
@@ -1383,7 +1391,9 @@ cudaError_t launch_typed(uint32_t type, GemvArgs& ga, uint32_t rows_per_job, uin
 }  // namespace
 
 // Activation planes live in the kernel's shared memory when they fit; only larger products need scratch.
-static bool acts_fit_in_smem(uint64_t rows, uint64_t k) { return rows * (k / 32) * 112 <= ACT_SMEM_MAX; }
+static bool acts_fit_in_smem(uint64_t rows, uint64_t k, uint32_t type = 0) {
+    return rows * (k / 32) * 112 <= (type == T_Q8_0 ? ACT_SMEM_MAX_Q8_0 : ACT_SMEM_MAX);
+}
 
 size_t gemv_mma_scratch_bytes(uint64_t rows, uint64_t k) {
     if (acts_fit_in_smem(rows, k)) return 0;
@@ -1429,13 +1439,15 @@ cudaError_t launch_quantize_acts(uint32_t type, const float* x, uint64_t rows, u
                       const_cast<float2*>(act.meta), const_cast<float*>(act.sum16));
 }
 
-bool gemv_mma_fusable(uint64_t m, uint64_t k) { return m <= GEMV_MMA_MAX_M && acts_fit_in_smem(m, k); }
+bool gemv_mma_fusable(uint32_t type, uint64_t m, uint64_t k) {
+    return m <= GEMV_MMA_MAX_M && acts_fit_in_smem(m, k, type);
+}
 
 // dst = residual + rmsnorm(lhs; norm_w, eps) . W^T in one launch; norm_w and residual are optional.
 cudaError_t launch_gemv_mma_fused(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, const float* lhs,
                                   uint64_t m, float* dst, const float* norm_w, float eps, const float* residual,
                                   int* error_flag, cudaStream_t s) {
-    if (!gemv_mma_fusable(m, k)) return cudaErrorInvalidValue;
+    if (!gemv_mma_fusable(type, m, k)) return cudaErrorInvalidValue;
     GemvArgs ga = {};
     ga.w[0] = ga.w[1] = w;
     ga.n = n;
@@ -1463,7 +1475,7 @@ cudaError_t launch_gemv_mma(uint32_t type, const uint8_t* w, uint64_t n, uint64_
     ga.dst = dst;
     ga.error_flag = error_flag;
     uint64_t tiles = (n + ROWS - 1) / ROWS;
-    if (acts_fit_in_smem(m, k)) return launch_typed<1, 0>(type, ga, (uint32_t)m, tiles, s);
+    if (acts_fit_in_smem(m, k, type)) return launch_typed<1, 0>(type, ga, (uint32_t)m, tiles, s);
     cudaError_t e = launch_quantize_acts(type, lhs, m, k, scratch, s);
     if (e != cudaSuccess) return e;
     ga.act = planes_in(scratch, m, k);
@@ -1474,7 +1486,7 @@ cudaError_t launch_gemv_mma(uint32_t type, const uint8_t* w, uint64_t n, uint64_
 cudaError_t launch_gemv_mma_swiglu(uint32_t type, const uint8_t* w_gate, const uint8_t* w_up, uint64_t n, uint64_t k,
                                    const float* lhs, uint64_t m, float* dst, float clamp, int* error_flag,
                                    cudaStream_t s, const float* norm_w, float eps) {
-    if (!acts_fit_in_smem(m, k)) return cudaErrorInvalidValue;
+    if (!acts_fit_in_smem(m, k, type)) return cudaErrorInvalidValue;
     GemvArgs ga = {};
     ga.w[0] = w_gate;
     ga.w[1] = w_up;

@@ -10,40 +10,56 @@ namespace jq {
 
 namespace {
 
-// logits[t, e] = sum_j x[t, j] * router[e, j], f32: one warp per (token, four consecutive experts), so that a token's
-// row is read once for four dot products; each dot product sums its lane's strided pieces in column order and
-// then across the lanes, the same order for every batch size.
+// logits[t, e] = sum_j x[t, j] * router[e, j], f32: one warp per (TT consecutive tokens, four consecutive experts), so
+// that a token's row is read once for four dot products and an expert's for TT; each dot product sums its lane's
+// strided pieces in column order and then across the lanes, the same order for every batch size.  Bound by the loads
+// from L1 and L2: with one token a warp five vectors feed 16 multiply-adds a lane, with four eight feed 64.
+template <int TT>
 __global__ void __launch_bounds__(256) moe_logits_kernel(const float* __restrict__ x, const float* __restrict__ router,
                                                          uint32_t T, uint32_t E, uint32_t h,
                                                          float* __restrict__ logits) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const uint32_t lane = threadIdx.x & 31, E4 = (E + 3) / 4;
-    const uint64_t total = (uint64_t)T * E4;
+    const uint32_t lane = threadIdx.x & 31, E4 = (E + 3) / 4, TG = (T + TT - 1) / TT;
+    const uint64_t total = (uint64_t)TG * E4;
     for (uint64_t p = blockIdx.x * 8ull + (threadIdx.x >> 5); p < total; p += gridDim.x * 8ull) {
-        const uint32_t t = (uint32_t)(p / E4), e0 = (uint32_t)(p % E4) * 4;
-        const float4* a = reinterpret_cast<const float4*>(x + (uint64_t)t * h);
+        const uint32_t t0 = (uint32_t)(p / E4) * TT, e0 = (uint32_t)(p % E4) * 4;
+        const float4* a[TT];
+#pragma unroll
+        for (int r = 0; r < TT; ++r) a[r] = reinterpret_cast<const float4*>(x + (uint64_t)min(t0 + r, T - 1) * h);
         const float4* b[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) b[q] = reinterpret_cast<const float4*>(router + (uint64_t)min(e0 + q, E - 1) * h);
-        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        float acc[TT][4];
+#pragma unroll
+        for (int r = 0; r < TT; ++r)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[r][q] = 0.0f;
         for (uint32_t j = lane; j < h / 4; j += 32) {
-            const float4 u = __ldg(a + j);
+            float4 u[TT];
+#pragma unroll
+            for (int r = 0; r < TT; ++r) u[r] = __ldg(a[r] + j);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const float4 v = __ldg(b[q] + j);
-                acc[q] = fmaf(u.x, v.x, acc[q]);
-                acc[q] = fmaf(u.y, v.y, acc[q]);
-                acc[q] = fmaf(u.z, v.z, acc[q]);
-                acc[q] = fmaf(u.w, v.w, acc[q]);
+#pragma unroll
+                for (int r = 0; r < TT; ++r) {
+                    acc[r][q] = fmaf(u[r].x, v.x, acc[r][q]);
+                    acc[r][q] = fmaf(u[r].y, v.y, acc[r][q]);
+                    acc[r][q] = fmaf(u[r].z, v.z, acc[r][q]);
+                    acc[r][q] = fmaf(u[r].w, v.w, acc[r][q]);
+                }
             }
         }
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int r = 0; r < TT; ++r)
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_xor_sync(0xFFFFFFFFu, acc[q], o);
-            if (lane == 0 && e0 + q < E) logits[(uint64_t)t * E + e0 + q] = acc[q];
-        }
+            for (int q = 0; q < 4; ++q) {
+                float v = acc[r][q];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+                if (lane == 0 && t0 + r < T && e0 + q < E) logits[(uint64_t)(t0 + r) * E + e0 + q] = v;
+            }
     }
 }
 
@@ -743,7 +759,11 @@ unsigned blocks_for(uint64_t work, unsigned per_block) {
 
 cudaError_t launch_moe_logits(const float* x, const float* router, uint32_t T, uint32_t E, uint32_t h, float* logits,
                               cudaStream_t s) {
-    cudaError_t le1__ = launch_pdl(moe_logits_kernel, blocks_for((uint64_t)T * ((E + 3) / 4), 8), 256, 0, s, x, router, T, E, h, logits);
+    // four tokens a warp once that still leaves every SM eight warps
+    const uint64_t e4 = (E + 3) / 4, groups4 = (uint64_t)((T + 3) / 4) * e4;
+    cudaError_t le1__ = groups4 >= 8ull * num_sms()
+                            ? launch_pdl(moe_logits_kernel<4>, blocks_for(groups4, 8), 256, 0, s, x, router, T, E, h, logits)
+                            : launch_pdl(moe_logits_kernel<1>, blocks_for((uint64_t)T * e4, 8), 256, 0, s, x, router, T, E, h, logits);
     if (le1__ != cudaSuccess) return le1__;
     return cudaGetLastError();
 }
