@@ -978,9 +978,6 @@ __global__ void __launch_bounds__((NCW + 2) * 32, 1) gemv_mma_kernel(const __gri
         a.n_groups = n_groups;
         float colacc[NH][2][2], minacc[NB][2];
         uint32_t job = 0, red_it = 0;
-        // Units are dealt to the warps in turn over the CTA's whole stream of chunks and tiles: a chunk of eight units
-        // (Q8_0), a last chunk or a row of three units occupies some warps and the next one the others.
-        uint32_t first = cw;  // this warp's first unit of the chunk: (cw - units dealt so far) mod NCW
         for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
             uint32_t rt;
             const MoeJob jd = job_of(tile, &rt);
@@ -1006,12 +1003,11 @@ __global__ void __launch_bounds__((NCW + 2) * 32, 1) gemv_mma_kernel(const __gri
                     const uint8_t* st = ring + s * stage_bytes;
                     const uint32_t u_lo = chunk * Tr::CHUNK_UNITS;
                     const uint32_t cnt = min(units_per_row - u_lo, Tr::CHUNK_UNITS);
-                    for (uint32_t u = first; u < cnt; u += NCW) {
+                    for (uint32_t u = cw; u < cnt; u += NCW) {
                         const uint8_t* u0 = st + ro.g * plan.row_stride + sh0 + u * Tr::UNIT_BYTES;
                         const uint8_t* u1 = st + (ro.g + 8) * plan.row_stride + sh1 + u * Tr::UNIT_BYTES;
                         process_unit<TYPE, MB, NH, ACT>(u0, u1, u_lo + u, a, ro, s_grid, s_mask, colacc, minacc);
                     }
-                    first = (first - cnt) & (NCW - 1);
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&empty[s]);
                 }
