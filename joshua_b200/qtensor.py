@@ -50,6 +50,17 @@ def default_context(device: int = 0) -> Context:
     return _default_ctx[device]
 
 
+_calls: dict = {}  # torch and the C entry of the device product, looked up once: a small product costs microseconds
+
+
+def _device_call():
+    if not _calls:
+        import torch
+
+        _calls.update(torch=torch, raw_stream=torch._C._cuda_getCurrentRawStream, matmul_t_dev=_lib.lib().jq_matmul_t_dev)
+    return _calls
+
+
 def _np_ptr(a: np.ndarray):
     return a.ctypes.data_as(ctypes.c_void_p)
 
@@ -146,11 +157,12 @@ class QTensor:
     # ── device-resident product ─────────────────────────────────────────
     def matmul_t_dev(self, mkn, lhs, dst, stream=None) -> None:
         """Same product on torch CUDA tensors (f32, contiguous), on torch's current stream."""
-        import torch
-
+        c = _calls or _device_call()
         m, k, n = mkn
-        s = torch.cuda.current_stream(lhs.device).cuda_stream if stream is None else stream
-        check(_lib.lib().jq_matmul_t_dev(self._h, m, k, n, lhs.data_ptr(), dst.data_ptr(), s))
+        s = c["raw_stream"](lhs.device.index) if stream is None else stream
+        rc = c["matmul_t_dev"](self._h, m, k, n, lhs.data_ptr(), dst.data_ptr(), s)
+        if rc:
+            check(rc)
 
     def dequantize_dev(self, out, two_step: bool = True, stream=None) -> None:
         import torch
@@ -175,11 +187,15 @@ class QMatMul:
         return cls(qtensor, shape[0], shape[1])
 
     def forward(self, xs):
-        import torch
-
+        torch = (_calls or _device_call())["torch"]
         if xs.dtype != torch.float32 or not xs.is_cuda:
             raise JoshuaB200Error(_lib.E_INVALID, "QMatMul.forward expects an f32 CUDA tensor")
-        x2 = xs.reshape(-1, self.k).contiguous()
-        out = torch.empty((x2.shape[0], self.n), dtype=torch.float32, device=xs.device)
-        self.w.matmul_t_dev((x2.shape[0], self.k, self.n), x2, out)
-        return out.reshape(*xs.shape[:-1], self.n)
+        shape, k, n = xs.shape, self.k, self.n
+        if len(shape) > 0 and shape[-1] == k and xs.is_contiguous():  # the usual case: no views, no copies
+            out = torch.empty((*shape[:-1], n), dtype=torch.float32, device=xs.device)
+            self.w.matmul_t_dev((xs.numel() // k, k, n), xs, out)
+            return out
+        x2 = xs.reshape(-1, k).contiguous()
+        out = torch.empty((x2.shape[0], n), dtype=torch.float32, device=xs.device)
+        self.w.matmul_t_dev((x2.shape[0], k, n), x2, out)
+        return out.reshape(*shape[:-1], n)

@@ -151,5 +151,18 @@ def test_qmatmul_forward_on_device_tensors():
     assert y.shape == (2, 3, n)
     want = oracle.matmul_t(synth.Q4_K, (6, k, n), x.reshape(6, k).cpu().numpy(), raw)
     assert_close(y.reshape(6, n).cpu().numpy(), want)
+    # views and other layouts: the same values through a copy; one row; no rows; a side stream
+    want = mm.forward(x)
+    xt = x.transpose(0, 1)
+    assert torch.equal(mm.forward(xt), want.transpose(0, 1)) and torch.equal(mm.forward(x[0, 0]), mm.forward(x[:1, :1])[0, 0])
+    assert mm.forward(x[:0]).shape == (0, 3, n) and mm.forward(x.reshape(-1, k)[:, :]).shape == (6, n)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        y2 = mm.forward(x)
+    side.synchronize()
+    assert torch.equal(y2, want)
+    with pytest.raises(JoshuaB200Error):
+        mm.forward(x.half())
     with pytest.raises(JoshuaB200Error):
         QMatMul.from_qtensor(QTensor.from_bytes(synth.Q4_K, raw), (n + 1, k))
