@@ -125,3 +125,61 @@ def test_scales_and_rows_at_the_edges(type_id, mkn, kind, tc_ctx):
     want, size = x @ w.T, np.abs(x) @ sum(np.abs(p) for p in parts).T
     inside = size < 1e38   # f32 results
     assert np.all(np.abs(got - want)[inside] <= 7e-6 * size[inside] + 1e-42)
+
+
+@pytest.mark.parametrize("m", [5, 8, 9, 40])
+def test_a_stream_under_capture_without_scratch_takes_the_older_route(m):
+    """The tile GEMM needs scratch; a capture on a stream that has none yet must not allocate, so the decode kernel runs
+    there (its planes fit shared memory at this k) as it did before the tiles took these batches."""
+    import torch
+
+    from joshua_b200.qtensor import Context
+
+    n, k = 384, 1024
+    raw = synth.random_weight(synth.Q4_K, n, k, seed=6)
+    lhs = synth.random_activations(m, k, seed=7).reshape(m, k)
+    want = oracle.matmul_t(synth.Q4_K, (m, k, n), lhs, raw)
+    x, out = torch.from_numpy(lhs).cuda(), torch.zeros(m, n, device="cuda")
+    QTensor.from_bytes(synth.Q4_K, raw).matmul_t((m, k, n), lhs)   # kernels of this process are loaded
+    warm = torch.cuda.Stream()
+    with torch.cuda.stream(warm):
+        for rows in range(1, 9):                                    # every row-count variant of the decode kernel
+            QTensor.from_bytes(synth.Q4_K, raw, Context(0)).matmul_t_dev((min(rows, m), k, n), x, out)
+    torch.cuda.synchronize()
+    q = QTensor.from_bytes(synth.Q4_K, raw, Context(0))
+    s = torch.cuda.Stream()
+    out.zero_()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        q.matmul_t_dev((m, k, n), x, out)
+    g.replay()
+    torch.cuda.synchronize()
+    assert_close(out.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("type_id", [synth.Q4_K, synth.Q8_0, synth.Q2_K, synth.Q6_K])
+@pytest.mark.parametrize("m", [5, 7, 16, 17, 33, 64, 65, 128, 130])
+def test_norm_and_residual_inside_the_tile_gemm(type_id, m):
+    """dst = residual + rmsnorm(x) . W^T with dst = residual, over the tile widths and both sides of their edges, k split
+    over a cluster (n = 96 is one tile), against float64.  Bound as in the test above, plus the norm's own rounding."""
+    import torch
+
+    from joshua_b200 import _lib
+
+    n, k = 96, 4608 if type_id != synth.Q6_K else 4096
+    raw = synth.random_weight(type_id, n, k, seed=11)
+    w = oracle.dequantize(type_id, raw).reshape(n, k).astype(np.float64)
+    rng = np.random.default_rng(m)
+    x, nw, res = rng.standard_normal((m, k)), rng.uniform(0.5, 1.5, k), rng.standard_normal((m, n))
+    x, nw, res = (v.astype(np.float32) for v in (x, nw, res))
+    q = QTensor.from_bytes(type_id, raw)
+    xd, nd, rd = (torch.from_numpy(v).cuda() for v in (x, nw, res))
+    _lib.check(_lib.lib().jq_matmul_norm_dev(q._h, m, k, n, xd.data_ptr(), nd.data_ptr(), 1e-5, rd.data_ptr(), rd.data_ptr(),
+                                             torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    x64 = x.astype(np.float64)
+    xn = x64 / np.sqrt((x64 ** 2).mean(1, keepdims=True) + 1e-5) * nw.astype(np.float64)
+    want = res + xn @ w.T
+    size = np.abs(res) + np.abs(xn) @ np.abs(w.T) * (3 if type_id in (synth.Q4_K, synth.Q2_K) else 1)
+    assert np.all(np.abs(rd.cpu().numpy() - want) <= 8e-6 * size)

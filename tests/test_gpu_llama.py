@@ -182,6 +182,73 @@ def test_fused_attention_matches_rope_append_attention(nq, nkv, hd, ctx):
     assert float((got - want).abs().max()) <= 2e-5 * max(1.0, float(want.abs().max()))
 
 
+@pytest.mark.parametrize("nq,nkv,hd", [(32, 8, 128), (32, 4, 128), (8, 8, 64), (16, 8, 256)])
+def test_fused_attention_with_more_items_than_sms(nq, nkv, hd):
+    """Eight sequences over a 17-chunk cache: items look at the position before they load, dead chunks leave.  Positions
+    at both ends of a chunk and of the cache, and one outside it."""
+    import torch
+
+    from joshua_b200 import _lib
+
+    L = _lib.lib()
+    B, max_ctx, theta = 8, 1056, 10000.0
+    g = torch.Generator(device="cuda").manual_seed(hd)
+    qkv = torch.randn(B, (nq + 2 * nkv) * hd, device="cuda", generator=g)
+    ck = torch.randn(B, nkv, max_ctx, hd, device="cuda", generator=g)
+    cv = torch.randn(B, nkv, max_ctx, hd, device="cuda", generator=g)
+    ck2, cv2 = ck.clone(), cv.clone()
+    pos = torch.tensor([0, 63, 64, 512, 1055, 1023, 1056, 1], dtype=torch.int32, device="cuda")
+    s = torch.cuda.current_stream().cuda_stream
+    flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+    q, want = torch.empty(B, nq * hd, device="cuda"), torch.empty(B, nq * hd, device="cuda")
+    scratch = torch.empty(L.jq_attention_scratch_bytes(B, nq, hd, max_ctx) // 4 + 1, device="cuda")
+    _lib.check(L.jq_rope_append_dev(qkv.data_ptr(), pos.data_ptr(), B, nq, nkv, hd, max_ctx, theta, q.data_ptr(),
+                                    ck.data_ptr(), cv.data_ptr(), flag.data_ptr(), s))
+    _lib.check(L.jq_attention_decode_dev(q.data_ptr(), ck.data_ptr(), cv.data_ptr(), pos.data_ptr(), B, nq, nkv, hd,
+                                         max_ctx, want.data_ptr(), scratch.data_ptr(), flag.data_ptr(), s))
+    got = torch.full((B, nq * hd), 123.0, device="cuda")
+    fscratch = torch.zeros(L.jq_attention_fused_scratch_bytes(B, nq, nkv, hd, max_ctx) // 4 + 1, device="cuda")
+    flag.zero_()
+    for _ in range(2):   # twice: the arrival counters must come back to zero
+        _lib.check(L.jq_attention_fused_dev(qkv.data_ptr(), pos.data_ptr(), B, nq, nkv, hd, max_ctx, theta, ck2.data_ptr(),
+                                            cv2.data_ptr(), got.data_ptr(), fscratch.data_ptr(), flag.data_ptr(), s))
+    torch.cuda.synchronize()
+    live = [0, 1, 2, 3, 4, 5, 7]
+    assert int(flag.item()) == 1 and bool((got[6] == 123.0).all())
+    assert torch.equal(ck, ck2) and torch.equal(cv, cv2)
+    # the bound of the one-wave test: f32 sums of up to 1056 terms in another order
+    assert float((got[live] - want[live]).abs().max()) <= 2e-5 * max(1.0, float(want[live].abs().max()))
+
+
+@pytest.mark.parametrize("nq,nkv,hd,norms", [(32, 8, 128, False), (32, 4, 64, True), (5, 5, 128, True)])
+def test_rotary_append_of_a_long_prompt_equals_short_pieces(nq, nkv, hd, norms):
+    """A CTA takes eight heads when the grid is large and one when it is small: the same bits."""
+    import torch
+
+    from joshua_b200 import _lib
+
+    L = _lib.lib()
+    seq, max_ctx, theta = 1300, 1400, 10000.0
+    g = torch.Generator(device="cuda").manual_seed(3)
+    qkv = torch.randn(seq, (nq + 2 * nkv) * hd, device="cuda", generator=g)
+    w = torch.rand(2, hd, device="cuda", generator=g) if norms else None
+    nw = (w[0].data_ptr(), w[1].data_ptr()) if norms else (None, None)
+    s = torch.cuda.current_stream().cuda_stream
+    outs = []
+    for piece in (seq, 50):
+        q = torch.zeros(seq, nq * hd, device="cuda")
+        k, v = torch.zeros(nkv, max_ctx, hd, device="cuda"), torch.zeros(nkv, max_ctx, hd, device="cuda")
+        for a in range(0, seq, piece):
+            pos = torch.tensor([7 + a], dtype=torch.int32, device="cuda")
+            _lib.check(L.jq_rope_append_prefill_dev(qkv[a:].data_ptr(), pos.data_ptr(), min(piece, seq - a), nq, nkv, hd,
+                                                    max_ctx, theta, *nw, 1e-6, q[a:].data_ptr(), k.data_ptr(),
+                                                    v.data_ptr(), None, s))
+            torch.cuda.synchronize()
+        outs.append((q, k, v))
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
+
+
 def test_positions_beyond_the_cache_store_nothing_and_raise_the_flag():
     """Stepping past max_ctx: the kernels skip the append and the attention for that sequence, the flag is set,
     the memory behind the cache is untouched (the cache is the front part of a larger canary-filled buffer),

@@ -267,3 +267,48 @@ def test_forward_with_norm_and_residual_folded_in(T, shared):
     torch.cuda.synchronize()
     moe.status()
     assert float((got - want).abs().max()) <= 1e-4 * max(1.0, float(want.abs().max()))
+
+
+@pytest.mark.parametrize("hidden,n_expert", [(512, 130), (1024, 128)])
+def test_routing_of_many_tokens_equals_small_batches(hidden, n_expert):
+    """The router's logits take four tokens a warp in large batches and one in small ones: the same sums, bit for bit."""
+    import torch
+
+    rng = np.random.default_rng(hidden)
+    banks = [QTensor.from_bytes(synth.Q4_K, synth.random_weight(synth.Q4_K, n_expert * r, c, 1))
+             for r, c in ((256, hidden), (256, hidden), (hidden, 256))]
+    layer = Moe(MoeConfig(gating=GATE_SOFTMAX, n_expert=n_expert, n_used=4, hidden=hidden, inter=256),
+                rng.standard_normal((n_expert, hidden)).astype(np.float32), *banks)
+    T = 301
+    layer.reserve(T)
+    x = torch.randn(T, hidden, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+    got = []
+    for piece in (T, 43):
+        ids = torch.zeros(T, 4, dtype=torch.int32, device="cuda")
+        wts = torch.zeros(T, 4, device="cuda")
+        for a in range(0, T, piece):
+            layer.route_dev(x[a:a + piece], ids[a:a + piece], wts[a:a + piece])
+        got.append((ids, wts))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("tokens", [31, 32, 90])
+def test_experts_on_tiles_match_the_oracle_and_replay(tokens):
+    """From 32 tokens the experts of Q4_K and MXFP4 banks run on tiles; the replay entry still finds the job list."""
+    import torch
+
+    E, K, hidden, inter = 24, 4, 512, 256
+    cfg = MoeConfig(gating=GATE_SOFTMAX, n_expert=E, n_used=K, hidden=hidden, inter=inter)
+    rng = np.random.default_rng(tokens)
+    router = rng.standard_normal((E, hidden)).astype(np.float32) * 0.5
+    raw = [synth.random_weight(synth.Q4_K, E * r, c, i) for i, (r, c) in enumerate([(inter, hidden), (inter, hidden), (hidden, inter)])]
+    layer = Moe(cfg, router, *[QTensor.from_bytes(synth.Q4_K, b) for b in raw])
+    x = (rng.standard_normal((tokens, hidden)) * 0.02).astype(np.float32)
+    got = layer.forward(x)
+    ids, wts = layer.last_routing(tokens)
+    ocfg = oracle.moe_cfg(gating=cfg.gating, n_expert=E, n_used=K, hidden=hidden, inter=inter, decode_path=True)
+    want = oracle.moe_dispatch(ocfg, x, ids, wts, [synth.Q4_K] * 3, raw, None, None)
+    assert_close(got, want)
+    layer.experts_replay_dev(torch.from_numpy(x).cuda())
+    torch.cuda.synchronize()
+    layer.status()
