@@ -757,7 +757,8 @@ __device__ __forceinline__ void process_unit(const uint8_t* u0, const uint8_t* u
         // 2i of the high word, and its two 16-groups are the two runs hf.  The codes minus 32 are the A operand, the
         // int8 scales multiply the exact integer sums (|sum| <= 16 groups * 16 * 32 * 127 * 128 < 2^31).
         // Bound by the consumers' instructions like the other formats.  Measured, 128256 x 4096, one row: 101 us
-        // (4.3 TB/s); the exact-decode float kernel, which served the type before, 847 us.  A block starts on any even address: every word is two aligned words and a shift.
+        // (4.3 TB/s); the exact-decode float kernel, which served the type before, 847 us.  A block starts on any even
+        // address: every word is two aligned words and a shift.
         const uint32_t s0 = 8 * (uint32_t)(reinterpret_cast<uintptr_t>(u0) & 2);
         const uint32_t s1 = 8 * (uint32_t)(reinterpret_cast<uintptr_t>(u1) & 2);
         const uint8_t* a0 = u0 - (s0 >> 3) + 4 * ro.t;
