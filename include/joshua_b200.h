@@ -121,7 +121,15 @@ int32_t jq_matmul_t_f16(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, 
 /* Same product with DEVICE buffers on a caller stream (cudaStream_t passed as
  * void*), no synchronisation: the device-resident insertion point that
  * `Weight::Zc` / ZcWeight::forward occupies in the reference
- * (src/quantized_qwen3_moe.rs:215-227, src/zero_copy_metal.rs:374-408). */
+ * (src/quantized_qwen3_moe.rs:215-227, src/zero_copy_metal.rs:374-408).
+ *   Scratch of this and the other *_dev products (split activations, gate and up
+ * results) belongs to the context, one set per stream, allocated when a stream
+ * first needs it and grown by larger calls.  A buffer that a capture has used is
+ * kept when the stream outgrows it, until jq_free: a graph stays valid whatever
+ * the stream runs later.  A graph replays into the scratch of the stream it was
+ * captured on, so work on that stream, and other graphs captured on it, must not
+ * run at the same time on another stream.  Growth allocates: warm a stream up
+ * before capturing it. */
 int32_t jq_matmul_t_dev(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, const float* lhs_dev,
                         float* dst_dev, void* stream);
 

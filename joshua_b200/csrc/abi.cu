@@ -70,10 +70,6 @@ int32_t validate_matmul(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, 
 
 }  // namespace
 
-static cudaStream_t tiles_scratch_key(cudaStream_t s) {
-    return reinterpret_cast<cudaStream_t>(reinterpret_cast<uintptr_t>(s) ^ 3);
-}
-
 // From nine rows on the other route is the decode kernel once per eight rows.  From five rows on, where the decode
 // kernel's activation planes do not fit its shared memory, it reads them from L2 for every 16 weight rows; Q4_K, bound
 // by its consumers' instructions, is behind the tiles from five rows on in any case.  Measured, eight rows, tiles /
@@ -86,28 +82,27 @@ bool jq_uses_tiles(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, cudaS
     // in a near tie change places (logits 2 % off in a third of the batches tried).
     if (w->type == jq::T_Q8_0 && m <= 2 * jq::GEMV_MMA_MAX_M) return false;
     if (m <= jq::GEMV_MMA_MAX_M && w->type != jq::T_Q4_K && jq::gemv_mma_scratch_bytes(m, k) == 0) return false;
-    return w->ctx->scratch_available(tiles_scratch_key(s), jq::gemm_f16_scratch_bytes(m, k), s);
+    return w->ctx->scratch_available(s, SLOT_TILES, jq::gemm_f16_scratch_bytes(m, k));
 }
 
 int32_t jq_matmul_tiles(const jq_weight* w, const jq_weight* w_b, uint64_t m, uint64_t k, uint64_t n, const float* lhs,
                         const float* norm_w, float eps, const float* residual, float* dst, float* dst_b, cudaStream_t s) {
     jq_ctx* ctx = w->ctx;
     void* scratch = nullptr;
-    JQ_CUDA(ctx->scratch_for(tiles_scratch_key(s), jq::gemm_f16_scratch_bytes(m, k), &scratch));
+    JQ_CUDA(ctx->scratch_for(s, SLOT_TILES, jq::gemm_f16_scratch_bytes(m, k), &scratch));
     JQ_CUDA(jq::launch_gemm_f16(w->type, w->dev, w_b ? w_b->dev : nullptr, n, k, lhs, m, norm_w, eps, residual, dst, dst_b,
                                 scratch, ctx->status_dev, s));
     return jq::OK;
 }
 
 // Picks the kernel for a device-resident product.
-
 int32_t jq_matmul_device(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, const float* lhs, float* dst,
                          cudaStream_t s) {
     jq_ctx* ctx = w->ctx;
     if (jq_uses_tiles(w, m, k, n, s)) return jq_matmul_tiles(w, nullptr, m, k, n, lhs, nullptr, 0.0f, nullptr, dst, nullptr, s);
     if (!ctx->force_f32 && jq::gemv_mma_dense_supports(w->type, w->dev, n, k, m)) {
         void* scratch = nullptr;
-        JQ_CUDA(ctx->scratch_for(s, jq::gemv_mma_scratch_bytes(m, k), &scratch));
+        JQ_CUDA(ctx->scratch_for(s, SLOT_PLANES, jq::gemv_mma_scratch_bytes(m, k), &scratch));
         JQ_CUDA(jq::launch_gemv_mma(w->type, w->dev, n, k, lhs, m, dst, scratch, ctx->status_dev, s));
         return jq::OK;
     }
@@ -119,7 +114,7 @@ int32_t jq_matmul_device(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n,
     if (!ctx->force_f32 && m > jq::GEMV_MMA_MAX_M && (m <= ctx->sliced_max_m || w->type == jq::T_Q6_K) &&
         jq::gemv_mma_dense_supports(w->type, w->dev, n, k, jq::GEMV_MMA_MAX_M)) {
         void* scratch = nullptr;
-        JQ_CUDA(ctx->scratch_for(s, jq::gemv_mma_scratch_bytes(jq::GEMV_MMA_MAX_M, k), &scratch));
+        JQ_CUDA(ctx->scratch_for(s, SLOT_PLANES, jq::gemv_mma_scratch_bytes(jq::GEMV_MMA_MAX_M, k), &scratch));
         for (uint64_t r0 = 0; r0 < m; r0 += jq::GEMV_MMA_MAX_M) {
             const uint64_t rows = std::min<uint64_t>(jq::GEMV_MMA_MAX_M, m - r0);
             JQ_CUDA(jq::launch_gemv_mma(w->type, w->dev, n, k, lhs + r0 * k, rows, dst + r0 * n, scratch,
@@ -129,7 +124,7 @@ int32_t jq_matmul_device(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n,
     }
     if (!ctx->force_f32 && m > jq::GEMV_MMA_MAX_M && jq::gemm_tc_supports(w->type, w->dev, n, k, m)) {
         void* scratch = nullptr;
-        JQ_CUDA(ctx->scratch_for(reinterpret_cast<cudaStream_t>(reinterpret_cast<uintptr_t>(s) ^ 3), jq::gemm_tc_scratch_bytes(m, k), &scratch));
+        JQ_CUDA(ctx->scratch_for(s, SLOT_TILES, jq::gemm_tc_scratch_bytes(m, k), &scratch));
         JQ_CUDA(jq::launch_gemm_tc(w->type, w->dev, n, k, lhs, m, dst, scratch, ctx->status_dev, s));
         return jq::OK;
     }
@@ -226,6 +221,7 @@ void jq_free(jq_ctx* ctx) {
     cudaSetDevice(ctx->device);
     cudaDeviceSynchronize();
     for (auto& kv : ctx->scratch) cudaFree(kv.second.dev);
+    for (void* p : ctx->retired) cudaFree(p);
     for (int i = 0; i < 8; ++i) {
         if (ctx->aux[i]) cudaStreamDestroy(ctx->aux[i]);
         if (ctx->join_ev[i]) cudaEventDestroy(ctx->join_ev[i]);

@@ -10,19 +10,16 @@ bool vectors(const float* lhs, const float* norm_w) {
 }
 
 size_t swiglu_scratch_bytes(uint64_t m, uint64_t n) { return 2 * m * n * 4 + 512; }
-cudaStream_t swiglu_scratch_key(cudaStream_t s) {
-    return reinterpret_cast<cudaStream_t>(reinterpret_cast<uintptr_t>(s) ^ 1);
-}
 bool pair_uses_tiles(const jq_weight* gate, const jq_weight* up, uint64_t m, uint64_t k, uint64_t n, cudaStream_t s) {
     return jq_uses_tiles(gate, m, k, n, s) && jq_uses_tiles(up, m, k, n, s) &&
-           gate->ctx->scratch_available(swiglu_scratch_key(s), swiglu_scratch_bytes(m, n), s);
+           gate->ctx->scratch_available(s, SLOT_PAIR, swiglu_scratch_bytes(m, n));
 }
 
 // silu(clamp(gate x)) * clamp(up x) on the tile GEMM: one launch for both tensors into scratch, then the combine.
 int32_t swiglu_tiles(const jq_weight* gate, const jq_weight* up, uint64_t m, uint64_t k, uint64_t n, const float* lhs,
                      const float* norm_w, float eps, float* dst, float clamp, cudaStream_t s) {
     void* scratch = nullptr;
-    JQ_CUDA(gate->ctx->scratch_for(swiglu_scratch_key(s), swiglu_scratch_bytes(m, n), &scratch));
+    JQ_CUDA(gate->ctx->scratch_for(s, SLOT_PAIR, swiglu_scratch_bytes(m, n), &scratch));
     float* g = static_cast<float*>(scratch);
     float* u = g + ((m * n + 63) & ~(uint64_t)63);
     if (int32_t rc = jq_matmul_tiles(gate, up, m, k, n, lhs, norm_w, eps, nullptr, g, u, s)) return rc;
@@ -57,7 +54,7 @@ int32_t jq_matmul_swiglu_dev(const jq_weight* gate, const jq_weight* up, uint64_
     }
     // two products into scratch, then the element-wise combine
     void* scratch = nullptr;
-    JQ_CUDA(ctx->scratch_for(swiglu_scratch_key(s), swiglu_scratch_bytes(m, n), &scratch));
+    JQ_CUDA(ctx->scratch_for(s, SLOT_PAIR, swiglu_scratch_bytes(m, n), &scratch));
     float* g = static_cast<float*>(scratch);
     float* u = g + ((m * n + 63) & ~(uint64_t)63);
     if (int32_t rc = jq_matmul_device(gate, m, k, n, lhs_dev, g, s)) return rc;
@@ -85,7 +82,7 @@ int32_t jq_matmul_swiglu_norm_dev(const jq_weight* gate, const jq_weight* up, ui
     }
     // separate kernels: normalise into scratch, then the plain entry (which validates)
     void* scratch = nullptr;
-    JQ_CUDA(ctx->scratch_for(reinterpret_cast<cudaStream_t>(reinterpret_cast<uintptr_t>(s) ^ 2), m * k * 4 + 256, &scratch));
+    JQ_CUDA(ctx->scratch_for(s, SLOT_NORM, m * k * 4 + 256, &scratch));
     JQ_CUDA(jq::launch_rmsnorm(lhs_dev, nullptr, norm_w_dev, eps, m, (uint32_t)k, nullptr, static_cast<float*>(scratch), s));
     return jq_matmul_swiglu_dev(gate, up, m, k, n, static_cast<const float*>(scratch), dst_dev, clamp, stream);
 }
@@ -111,7 +108,7 @@ int32_t jq_matmul_norm_dev(const jq_weight* w, uint64_t m, uint64_t k, uint64_t 
     if (m == 0 || n == 0) return jq_matmul_t_dev(w, m, k, n, lhs_dev, dst_dev, stream);
     void* scratch = nullptr;
     const uint64_t xk = (m * k + 63) & ~(uint64_t)63;
-    JQ_CUDA(ctx->scratch_for(reinterpret_cast<cudaStream_t>(reinterpret_cast<uintptr_t>(s) ^ 2), (xk + m * n) * 4 + 256, &scratch));
+    JQ_CUDA(ctx->scratch_for(s, SLOT_NORM, (xk + m * n) * 4 + 256, &scratch));
     float* xn = static_cast<float*>(scratch);
     float* prod = xn + xk;
     const float* in = lhs_dev;

@@ -1,11 +1,13 @@
 // Internal definitions shared by the translation units that implement the C ABI.
 #pragma once
 
+#include <algorithm>
 #include <cstdlib>
 #include <map>
 #include <mutex>
 #include <new>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/joshua_b200.h"
@@ -41,10 +43,17 @@ struct Workspace {
     }
 };
 
-// Scratch of the decode kernels (activation planes), one per caller stream.
+// Scratch of a stream: one buffer per role, because a call may hold several at once.
+enum ScratchSlot : uint32_t {
+    SLOT_PLANES,  // activation planes of the decode kernel
+    SLOT_PAIR,    // gate and up products in front of their combine
+    SLOT_NORM,    // normalised rows and the product of the separate kernels
+    SLOT_TILES,   // split activations of the tile GEMMs
+};
 struct StreamScratch {
     void* dev = nullptr;
     size_t cap = 0;
+    bool in_graph = false;  // handed out during a capture: a graph may hold its address
 };
 
 struct jq_ctx {
@@ -60,36 +69,57 @@ struct jq_ctx {
     cudaStream_t aux[8] = {};
     cudaEvent_t fork_ev = nullptr, join_ev[8] = {};
     std::vector<Workspace*> idle;
-    std::map<cudaStream_t, StreamScratch> scratch;
+    std::map<std::pair<cudaStream_t, uint32_t>, StreamScratch> scratch;
+    std::vector<void*> retired;  // outgrown buffers whose addresses captured graphs hold; freed with the context
 
-    // Scratch for `stream`, at least `bytes` large.  Growing it frees the old buffer (cudaFree
-    // waits for the device), so warm a stream up at its largest shape before capturing it.
-    cudaError_t scratch_for(cudaStream_t stream, size_t bytes, void** out) {
+    // Scratch of `stream` in a role, at least `bytes` large.  Growing it frees the old buffer (cudaFree waits for the
+    // device), unless it was handed out while the stream was being captured: then a graph may replay into it, so it stays
+    // until the context goes, and the new one is at least twice as large (the retired ones together stay below the live one).
+    cudaError_t scratch_for(cudaStream_t stream, ScratchSlot slot, size_t bytes, void** out) {
+        *out = nullptr;
+        if (bytes == 0) return cudaSuccess;
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        if (cudaError_t e = cudaStreamIsCapturing(stream, &st); e != cudaSuccess) return e;
         std::lock_guard<std::mutex> g(mu);
-        StreamScratch& sc = scratch[stream];
+        StreamScratch& sc = scratch[{stream, slot}];
         if (bytes > sc.cap) {
-            if (sc.dev) cudaFree(sc.dev);
-            sc.dev = nullptr;
-            sc.cap = 0;
-            size_t want = (bytes + (1u << 20) - 1) & ~((size_t)(1u << 20) - 1);
+            constexpr size_t MB = 1u << 20;
+            const size_t need = (bytes + MB - 1) / MB * MB;
+            size_t want = need;
+            if (sc.in_graph) {
+                retired.push_back(sc.dev);
+                want = std::max(need, 2 * sc.cap);
+            } else if (sc.dev) {
+                cudaFree(sc.dev);
+            }
+            sc = StreamScratch{};
             cudaError_t e = cudaMalloc(&sc.dev, want);
-            if (e != cudaSuccess) return e;
+            if (e != cudaSuccess && want > need) {
+                cudaGetLastError();
+                want = need;
+                e = cudaMalloc(&sc.dev, want);
+            }
+            if (e != cudaSuccess) {
+                sc.dev = nullptr;
+                return e;
+            }
             sc.cap = want;
         }
+        sc.in_graph |= st != cudaStreamCaptureStatusNone;
         *out = sc.dev;
         return cudaSuccess;
     }
 
-    // Whether `stream`'s scratch can be had now: it is large enough, or may be allocated because `capture` (the stream the
-    // work goes to) is not being captured.  Routes that need scratch where an older one did not ask this first.
-    bool scratch_available(cudaStream_t stream, size_t bytes, cudaStream_t capture) {
+    // Whether that scratch can be had now: it is large enough, or may be allocated because the stream is not being
+    // captured.  Routes that need scratch where an older one did not ask this first.
+    bool scratch_available(cudaStream_t stream, ScratchSlot slot, size_t bytes) {
         {
             std::lock_guard<std::mutex> g(mu);
-            auto it = scratch.find(stream);
+            auto it = scratch.find({stream, slot});
             if (it != scratch.end() && it->second.cap >= bytes) return true;
         }
         cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-        return cudaStreamIsCapturing(capture, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
+        return cudaStreamIsCapturing(stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
     }
 
     Workspace* acquire() {

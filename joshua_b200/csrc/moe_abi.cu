@@ -141,9 +141,6 @@ bool all_experts_on_tiles(const jq_moe* m) {
     return one(m->gate) && one(m->up) && one(m->down);
 }
 
-cudaStream_t bucket_scratch_key(cudaStream_t s) {
-    return reinterpret_cast<cudaStream_t>(reinterpret_cast<uintptr_t>(s) ^ 3);
-}
 size_t bucket_scratch_bytes(const jq_moe_config& c, uint64_t P) {
     return std::max(jq::gemm_f16_scratch_bytes(P, c.hidden), jq::gemm_f16_scratch_bytes(P, c.inter));
 }
@@ -202,7 +199,7 @@ int32_t run_experts_bucketed(jq_moe* m, const float* x, uint64_t T, uint64_t P, 
         uint32_t* counts = reinterpret_cast<uint32_t*>(
             (reinterpret_cast<uintptr_t>(small_jobs + max_small) + 15) & ~(uintptr_t)15);
         void* scratch = nullptr;
-        JQ_CUDA(m->ctx->scratch_for(bucket_scratch_key(s), bucket_scratch_bytes(c, P), &scratch));
+        JQ_CUDA(m->ctx->scratch_for(s, SLOT_TILES, bucket_scratch_bytes(c, P), &scratch));
         JQ_CUDA(jq::launch_moe_gather(x, m->list_token, m->n_list, (uint32_t)P, c.hidden, xs, s));
         JQ_CUDA(jq::launch_moe_tiles(m->jobs, m->n_jobs, m->n_list, c.n_expert, min_rows, narrow, wide, small_jobs, counts, s));
         JQ_CUDA(jq::launch_gemm_f16_grouped(m->gate->type, m->gate->dev, m->up->dev, m->gate_expert_bytes, c.inter, c.hidden, xs, P,
@@ -579,7 +576,7 @@ int32_t jq_moe_forward_norm_add_dev(jq_moe* m, const float* x_dev, uint64_t T, c
         if (cudaStreamIsCapturing(s, &st) == cudaSuccess &&
             (st == cudaStreamCaptureStatusNone ||
              (P <= m->bucket_pairs && bucket_lists_bytes(m, P, rpj) <= m->tiles_cap &&
-              m->ctx->scratch_available(bucket_scratch_key(s), bucket_scratch_bytes(c, P), s))))
+              m->ctx->scratch_available(s, SLOT_TILES, bucket_scratch_bytes(c, P)))))
             min_tokens = TILES_MIN_TOKENS;
     }
 #ifdef JQ_PROFILING

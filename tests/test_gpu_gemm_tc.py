@@ -158,6 +158,54 @@ def test_a_stream_under_capture_without_scratch_takes_the_older_route(m):
     assert_close(out.cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("type_id,m", [(synth.Q4_K, 8), (synth.Q4_K, 16), (synth.Q8_0, 20), (synth.Q8_0, 12), (synth.MXFP4, 40)])
+def test_a_graph_survives_larger_calls_on_its_stream(type_id, m):
+    """A captured product and a captured gate / up pair hold addresses of the stream's scratch.  Larger eager calls on
+    the stream outgrow every role of it; replays then still give the captured batch's values, bit for bit."""
+    import torch
+
+    from joshua_b200 import _lib
+    from joshua_b200.qtensor import Context
+
+    n, k, big = 384, 4096, 700
+    L, ctx = _lib.lib(), Context(0)
+    raw = [synth.random_weight(type_id, n, k, seed=s) for s in (1, 2)]
+    q = [QTensor.from_bytes(type_id, r, ctx) for r in raw]
+    lhs = synth.random_activations(big, k, seed=3).reshape(big, k)
+    x, nw = torch.from_numpy(lhs).cuda(), torch.ones(k, device="cuda")
+    s = torch.cuda.Stream()
+
+    def calls(rows, out):
+        q[0].matmul_t_dev((rows, k, n), x, out[0], stream=s.cuda_stream)
+        _lib.check(L.jq_matmul_swiglu_norm_dev(q[0]._h, q[1]._h, rows, k, n, x.data_ptr(), nw.data_ptr(), 1e-5,
+                                               out[1].data_ptr(), 0.0, s.cuda_stream))
+        _lib.check(L.jq_matmul_norm_dev(q[0]._h, rows, k, n, x.data_ptr(), nw.data_ptr(), 1e-5, out[1].data_ptr(),
+                                        out[2].data_ptr(), s.cuda_stream))
+
+    small, large = torch.zeros(3, m, n, device="cuda"), torch.zeros(3, big, n, device="cuda")
+    torch.cuda.synchronize()
+    calls(m, small)
+    s.synchronize()
+    want = small.clone()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        calls(m, small)
+    for rows in (200, big):
+        calls(rows, large)
+    s.synchronize()
+    junk = [torch.full((1 << 20,), float("nan"), device="cuda") for _ in range(64)]   # what was freed gets new owners
+    for _ in range(2):
+        small.zero_()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(s):
+            g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(small, want)
+        calls(big, large)
+    assert all(bool(torch.isnan(j).all()) for j in junk)
+    assert_close(small[0].cpu().numpy(), oracle.matmul_t(type_id, (m, k, n), lhs[:m], raw[0]))
+
+
 @pytest.mark.parametrize("type_id", [synth.Q4_K, synth.Q8_0, synth.Q2_K, synth.Q6_K])
 @pytest.mark.parametrize("m", [5, 7, 16, 17, 33, 64, 65, 128, 130])
 def test_norm_and_residual_inside_the_tile_gemm(type_id, m):
