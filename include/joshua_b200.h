@@ -370,13 +370,18 @@ void jq_moe_free(jq_moe* m);
 int32_t jq_moe_forward(jq_moe* m, const float* x, uint64_t n_tokens, const uint32_t* forced_ids, float* y);
 
 /* Sizes the layer's device workspace for up to n_tokens tokens (and n_rows rows
- * for jq_moe_experts_dev).  The *_dev entries never allocate: call this first
- * (and before capturing a stream). */
+ * for jq_moe_experts_dev).  The *_dev entries allocate nothing but the stream's
+ * scratch (see jq_matmul_t_dev), which batches of 32 and more tokens need: call
+ * this first, and run the largest batch once before capturing a stream.  A
+ * workspace that a capture has used is kept until jq_moe_free when a later call
+ * outgrows it, so the graph stays valid. */
 int32_t jq_moe_reserve(jq_moe* m, uint64_t n_tokens, uint64_t n_rows);
 
-/* The same with DEVICE buffers on a caller stream.  No synchronisation for decode-sized and moderate batches;
- * when n_tokens * n_used >= 64 * n_expert (192 * n_expert for experts under 8 M weights; prefill) the call reads the expert histogram back once, which
- * synchronises the stream, and may allocate: such batches cannot be captured in a CUDA graph. */
+/* The same with DEVICE buffers on a caller stream, without synchronisation: routing, job lists and tile lists stay on the
+ * device.  Only banks that the grouped tile GEMM does not take (IQ2_XXS with a width that is no multiple of 512) read the
+ * job list back from 128 tokens on, which synchronises the stream; such batches cannot be captured in a CUDA graph.
+ * A capture of 32 to 127 tokens on a stream without scratch takes the decode kernel instead of the tile GEMM (another
+ * summation order). */
 int32_t jq_moe_forward_dev(jq_moe* m, const float* x_dev, uint64_t n_tokens, const uint32_t* forced_ids_dev,
                            float* y_dev, void* stream);
 

@@ -189,11 +189,12 @@ struct jq_moe {
     uint32_t* counter = nullptr;  // arrival counter of the fused router kernel (zero between calls)
     float* xn = nullptr;          // normalised tokens, for the paths that cannot fold the norm in
     float* bucket = nullptr;      // prefill path: gathered rows [P, hidden] + gate and up products [2][P, inter]
-    uint64_t bucket_pairs = 0;
+    uint64_t bucket_pairs = 0;    // P the prefill path's buffers (in ws, like the rest) are sized for
+    bool in_graph = false;        // a capture has used ws: a graph may hold its addresses
+    std::vector<void*> retired;   // outgrown workspaces of captured graphs; freed with the layer
     uint64_t last_rows = 0, last_pairs = 0;  // shape of the job list the last decode-sized call left (replay entry)
     uint32_t last_rpj = 0;
     jq::GemmTile* tiles = nullptr;  // prefill path: narrow and wide tile lists, the small experts' job list, 4 counts
-    uint64_t tiles_cap = 0;         // bytes allocated behind `tiles`
     int* bad_host = nullptr;  // pinned, device-visible: an expert id was out of range
     int* bad_dev = nullptr;
     std::mutex mu;

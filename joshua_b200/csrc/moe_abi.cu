@@ -15,14 +15,54 @@ uint32_t rows_per_job_for(uint64_t pairs, uint64_t tokens, uint32_t n_expert) {
     return 8;
 }
 
+constexpr uint64_t BUCKET_ROWS_PER_EXPERT = 12;  // rows from which an expert runs on the tile GEMM
+constexpr uint64_t BUCKET_MIN_TOKENS = 128;      // tokens from which the prefill form (tile GEMM + decode kernel) is used
+constexpr uint64_t TILES_MIN_TOKENS = 32;        // the same for the types whose experts all run on tiles
+
+// Banks whose experts run on the tile GEMM whatever their row count.  Measured, 384 MXFP4 experts of 7168 x 2048, eight a
+// token, tiles / decode kernel: 3.87 / 4.85 ms at 100 tokens, 2.13 / 2.17 at 32, 1.35 / 1.19 at 16; 48 layers of 128
+// Q4_K experts of 2048 x 768: 14.0 / 27.6 ms at 100 tokens, 11.6 / 14.5 at 40, 13.8 / 10.1 (a decode step) at 16.
+bool all_experts_on_tiles(const jq_moe* m) {
+    auto one = [](const jq_weight* w) { return w->type == jq::T_Q4_K || w->type == jq::T_MXFP4; };
+    return one(m->gate) && one(m->up) && one(m->down);
+}
+
+size_t bucket_scratch_bytes(const jq_moe_config& c, uint64_t P) {
+    return std::max(jq::gemm_f16_scratch_bytes(P, c.hidden), jq::gemm_f16_scratch_bytes(P, c.inter));
+}
+// The device form of run_experts_bucketed: no host read.
+bool grouped_tiles_ok(const jq_moe* m, uint64_t P) {
+    const jq_moe_config& c = m->cfg;
+    return jq::gemm_f16_grouped_supports(m->gate->type, m->gate->dev, c.inter, c.hidden) && m->up->type == m->gate->type &&
+           jq::gemm_f16_grouped_supports(m->up->type, m->up->dev, c.inter, c.hidden) &&
+           jq::gemm_f16_grouped_supports(m->down->type, m->down->dev, c.hidden, c.inter) && P / 33 + 1 <= 65535;
+}
+
+uint32_t max_narrow_tiles(const jq_moe* m, uint64_t P) { return (uint32_t)std::min<uint64_t>(m->cfg.n_expert, P + 1); }
+// narrow and wide tiles, the small experts' jobs (any rows per job), four counts
+uint64_t bucket_lists_bytes(const jq_moe* m, uint64_t P) {
+    return ((uint64_t)max_narrow_tiles(m, P) + P / 33 + 1) * sizeof(jq::GemmTile) + P * sizeof(jq::MoeJob) + 32;
+}
+// Tokens from which a layer may take the prefill form.
+uint64_t bucket_min_tokens(const jq_moe* m, uint64_t P) {
+    return all_experts_on_tiles(m) && grouped_tiles_ok(m, P) ? TILES_MIN_TOKENS : BUCKET_MIN_TOKENS;
+}
+
+// The layer's workspace for T tokens and P list positions, the prefill form's buffers included where such a batch takes it.
+// Growing it by a few tokens at a time would allocate every time: it grows by a quarter at least.  A workspace that a
+// capture has used stays for the graph that holds its addresses.
 int32_t reserve(jq_moe* m, uint64_t T, uint64_t P) {
     if (T <= m->cap_tokens && P <= m->cap_pairs) return jq::OK;
-    T = std::max(T, m->cap_tokens);
-    P = std::max(P, m->cap_pairs);
+    T = T > m->cap_tokens ? std::max(T, m->cap_tokens + m->cap_tokens / 4) : m->cap_tokens;
+    P = P > m->cap_pairs ? std::max(P, m->cap_pairs + m->cap_pairs / 4) : m->cap_pairs;
     const jq_moe_config& c = m->cfg;
-    if (m->ws) cudaFree(m->ws);
+    if (m->in_graph)
+        m->retired.push_back(m->ws);
+    else if (m->ws)
+        cudaFree(m->ws);
     m->ws = nullptr;
-    m->cap_tokens = m->cap_pairs = 0;
+    m->in_graph = false;
+    m->cap_tokens = m->cap_pairs = m->bucket_pairs = 0;
     size_t off = 0;
     auto take = [&](size_t bytes) {
         size_t o = off;
@@ -35,6 +75,12 @@ int32_t reserve(jq_moe* m, uint64_t T, uint64_t P) {
            o_sho = take(T * c.hidden * 4), o_ones = take(P * 4), o_xn = take(T * c.hidden * 4),
            o_px = take(jq::gemv_mma_scratch_bytes(T, c.hidden) + (T * (c.hidden / 32) * 112) + 256),
            o_ph = take(jq::gemv_mma_scratch_bytes(P, c.inter) + (P * (c.inter / 32) * 112) + 256);
+    size_t o_bucket = 0, o_tiles = 0;
+    bool bucket = m->gate && !m->ctx->force_f32 && T >= bucket_min_tokens(m, P);
+#ifdef JQ_PROFILING
+    bucket |= m->gate != nullptr;  // the measurement switch of the forward entry sends any batch to the prefill form
+#endif
+    if (bucket) o_bucket = take(P * (c.hidden + 2ull * c.inter) * sizeof(float)), o_tiles = take(bucket_lists_bytes(m, P));
     JQ_CUDA(cudaMalloc(&m->ws, off));
     uint8_t* b = m->ws;
     m->logits = (float*)(b + o_logits);
@@ -53,10 +99,24 @@ int32_t reserve(jq_moe* m, uint64_t T, uint64_t P) {
     m->xn = (float*)(b + o_xn);
     m->planes_x = b + o_px;
     m->planes_h = b + o_ph;
+    if (bucket) {
+        m->bucket = (float*)(b + o_bucket);
+        m->tiles = (jq::GemmTile*)(b + o_tiles);
+        m->bucket_pairs = P;
+    }
     std::vector<float> ones(P, 1.0f);
     JQ_CUDA(cudaMemcpy(m->ones, ones.data(), P * 4, cudaMemcpyHostToDevice));
     m->cap_tokens = T;
     m->cap_pairs = P;
+    return jq::OK;
+}
+
+// Called by every entry that gives the layer's buffers to a stream.
+int32_t note_capture(jq_moe* m, cudaStream_t s) {
+    if (m->in_graph) return jq::OK;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    JQ_CUDA(cudaStreamIsCapturing(s, &st));
+    m->in_graph = st != cudaStreamCaptureStatusNone;
     return jq::OK;
 }
 
@@ -129,44 +189,9 @@ int32_t run_experts(jq_moe* m, const float* x, uint64_t R, uint64_t P, uint32_t 
 // bucket (src/quantized_qwen3_moe.rs:455-520): when an expert sees dozens of rows, its rows are gathered into
 // bucket order and the experts' gate / up / down products run on the tile GEMM (tensor cores), as one grouped
 // launch per phase over a list of (expert, row range) tiles built on the device.
-constexpr uint64_t BUCKET_ROWS_PER_EXPERT = 12;  // rows from which an expert runs on the tile GEMM
-constexpr uint64_t BUCKET_MIN_TOKENS = 128;      // tokens from which the prefill form (tile GEMM + decode kernel) is used
-constexpr uint64_t TILES_MIN_TOKENS = 32;        // the same for the types whose experts all run on tiles
-
-// Banks whose experts run on the tile GEMM whatever their row count.  Measured, 384 MXFP4 experts of 7168 x 2048, eight a
-// token, tiles / decode kernel: 3.87 / 4.85 ms at 100 tokens, 2.13 / 2.17 at 32, 1.35 / 1.19 at 16; 48 layers of 128
-// Q4_K experts of 2048 x 768: 14.0 / 27.6 ms at 100 tokens, 11.6 / 14.5 at 40, 13.8 / 10.1 (a decode step) at 16.
-bool all_experts_on_tiles(const jq_moe* m) {
-    auto one = [](const jq_weight* w) { return w->type == jq::T_Q4_K || w->type == jq::T_MXFP4; };
-    return one(m->gate) && one(m->up) && one(m->down);
-}
-
-size_t bucket_scratch_bytes(const jq_moe_config& c, uint64_t P) {
-    return std::max(jq::gemm_f16_scratch_bytes(P, c.hidden), jq::gemm_f16_scratch_bytes(P, c.inter));
-}
-// The device form of run_experts_bucketed: no host read.
-bool grouped_tiles_ok(const jq_moe* m, uint64_t P) {
-    const jq_moe_config& c = m->cfg;
-    return jq::gemm_f16_grouped_supports(m->gate->type, m->gate->dev, c.inter, c.hidden) && m->up->type == m->gate->type &&
-           jq::gemm_f16_grouped_supports(m->up->type, m->up->dev, c.inter, c.hidden) &&
-           jq::gemm_f16_grouped_supports(m->down->type, m->down->dev, c.hidden, c.inter) && P / 33 + 1 <= 65535;
-}
-
-uint32_t max_narrow_tiles(const jq_moe* m, uint64_t P) { return (uint32_t)std::min<uint64_t>(m->cfg.n_expert, P + 1); }
-uint64_t bucket_lists_bytes(const jq_moe* m, uint64_t P, uint32_t rows_per_job) {
-    return ((uint64_t)max_narrow_tiles(m, P) + P / 33 + 1) * sizeof(jq::GemmTile) +
-           std::min<uint64_t>(P, P / rows_per_job + m->cfg.n_expert) * sizeof(jq::MoeJob) + 32;
-}
-
+// P is at most m->bucket_pairs.
 int32_t run_experts_bucketed(jq_moe* m, const float* x, uint64_t T, uint64_t P, uint32_t rows_per_job, cudaStream_t s) {
     const jq_moe_config& c = m->cfg;
-    if (P > m->bucket_pairs) {
-        if (m->bucket) cudaFree(m->bucket);
-        m->bucket = nullptr;
-        m->bucket_pairs = 0;
-        JQ_CUDA(cudaMalloc(&m->bucket, (P * c.hidden + 2 * P * c.inter) * sizeof(float)));
-        m->bucket_pairs = P;
-    }
     float* xs = m->bucket;
     float* gbuf = xs + P * c.hidden;
     float* ubuf = gbuf + P * c.inter;
@@ -184,14 +209,6 @@ int32_t run_experts_bucketed(jq_moe* m, const float* x, uint64_t T, uint64_t P, 
         const uint32_t min_rows = all_tiles ? 1u : (uint32_t)BUCKET_ROWS_PER_EXPERT;
         const uint32_t max_narrow = max_narrow_tiles(m, P), max_wide = (uint32_t)(P / 33 + 1);
         const uint32_t max_small = (uint32_t)std::min<uint64_t>(P, P / rows_per_job + c.n_expert);
-        const uint64_t need_bytes = bucket_lists_bytes(m, P, rows_per_job);
-        if (need_bytes > m->tiles_cap) {
-            if (m->tiles) cudaFree(m->tiles);
-            m->tiles = nullptr;
-            m->tiles_cap = 0;
-            JQ_CUDA(cudaMalloc(&m->tiles, need_bytes));
-            m->tiles_cap = need_bytes;
-        }
         jq::GemmTile* narrow = m->tiles;
         jq::GemmTile* wide = narrow + max_narrow;
         jq::MoeJob* small_jobs = reinterpret_cast<jq::MoeJob*>(wide + max_wide);
@@ -378,10 +395,12 @@ uint32_t jq_moe_rows_per_job(uint64_t live_rows, uint32_t n_expert) {
 int32_t jq_moe_experts_list(jq_moe* m, const float* x_dev, uint64_t n_rows, const uint32_t* expert_ids_dev,
                             uint64_t live_rows, cudaStream_t s) {
     const jq_moe_config& c = m->cfg;
+    if (int32_t rc = note_capture(m, s)) return rc;
     uint32_t rpj = jq_moe_rows_per_job(live_rows, c.n_expert);
     JQ_CUDA(jq::launch_moe_jobs(expert_ids_dev, (uint32_t)n_rows, 1, c.n_expert, rpj, m->list_token, m->inv, m->jobs,
                                 m->n_jobs, m->n_list, m->bad_dev, s));
-    if (!m->ctx->force_f32 && live_rows >= BUCKET_MIN_TOKENS) return run_experts_bucketed(m, x_dev, n_rows, n_rows, rpj, s);
+    if (!m->ctx->force_f32 && live_rows >= BUCKET_MIN_TOKENS && n_rows <= m->bucket_pairs)
+        return run_experts_bucketed(m, x_dev, n_rows, n_rows, rpj, s);
     m->last_rows = m->last_pairs = n_rows, m->last_rpj = rpj;
     return run_experts(m, x_dev, n_rows, n_rows, rpj, s);
 }
@@ -464,8 +483,7 @@ void jq_moe_free(jq_moe* m) {
     cudaFree(m->router);
     cudaFree(m->bias);
     cudaFree(m->ws);
-    cudaFree(m->bucket);
-    cudaFree(m->tiles);
+    for (void* p : m->retired) cudaFree(p);
     cudaFree(m->dense_jobs);
     cudaFree(m->one);
     if (m->bad_host) cudaFreeHost(m->bad_host);
@@ -492,6 +510,7 @@ int32_t jq_moe_route_norm_dev(jq_moe* m, const float* x_dev, uint64_t T, const f
     if (!x_dev || !ids_dev || !wts_dev) return jq_fail(jq::E_INVALID, "jq_moe_route_dev: NULL buffer");
     if (T > m->cap_tokens) return jq_fail(jq::E_TOO_LARGE, "jq_moe_route_dev: call jq_moe_reserve for this many tokens first");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (int32_t rc = note_capture(m, s)) return rc;
     const jq_moe_config& c = m->cfg;
     if (T <= 8 && c.hidden % 4 == 0) {
         JQ_CUDA(jq::launch_moe_route_fused(x_dev, norm_w_dev, eps, m->router, (uint32_t)T, c.hidden, m->logits, m->rp,
@@ -546,6 +565,7 @@ int32_t jq_moe_forward_norm_add_dev(jq_moe* m, const float* x_dev, uint64_t T, c
     if (T > m->cap_tokens || P > m->cap_pairs)
         return jq_fail(jq::E_TOO_LARGE, "jq_moe_forward_dev: call jq_moe_reserve for this many tokens first");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (int32_t rc = note_capture(m, s)) return rc;
     const uint32_t rpj = rows_per_job_for(P, T, c.n_expert);
     // Decode-sized batches: router, routing and job list in one launch, the RMS norm folded into it and into
     // the expert (and shared-expert) matmuls' activation split.
@@ -569,20 +589,14 @@ int32_t jq_moe_forward_norm_add_dev(jq_moe* m, const float* x_dev, uint64_t T, c
     // From BUCKET_MIN_TOKENS tokens on, the prefill form: the experts on the tile GEMM, or (types that are not
     // all_experts_on_tiles) those with at least BUCKET_ROWS_PER_EXPERT rows and the others on the grouped decode kernel,
     // decided per expert on the device.  From TILES_MIN_TOKENS on where every expert takes tiles, unless that would
-    // allocate while the stream is captured (the decode form needs nothing beyond jq_moe_reserve).
-    uint64_t min_tokens = BUCKET_MIN_TOKENS;
-    if (T >= TILES_MIN_TOKENS && T < BUCKET_MIN_TOKENS && all_experts_on_tiles(m) && grouped_tiles_ok(m, P)) {
-        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(s, &st) == cudaSuccess &&
-            (st == cudaStreamCaptureStatusNone ||
-             (P <= m->bucket_pairs && bucket_lists_bytes(m, P, rpj) <= m->tiles_cap &&
-              m->ctx->scratch_available(s, SLOT_TILES, bucket_scratch_bytes(c, P)))))
-            min_tokens = TILES_MIN_TOKENS;
-    }
+    // allocate the stream's scratch while it is captured (the decode form needs nothing beyond jq_moe_reserve).
+    uint64_t min_tokens = bucket_min_tokens(m, P);
+    if (T >= min_tokens && T < BUCKET_MIN_TOKENS && !m->ctx->scratch_available(s, SLOT_TILES, bucket_scratch_bytes(c, P)))
+        min_tokens = BUCKET_MIN_TOKENS;
 #ifdef JQ_PROFILING
     if (const char* thr_env = std::getenv("JQ_MOE_BUCKET_TOKENS")) min_tokens = std::strtoull(thr_env, nullptr, 10);  // measurement switch
 #endif
-    const bool bucketed = !fused && !m->ctx->force_f32 && T >= min_tokens;
+    const bool bucketed = !fused && !m->ctx->force_f32 && T >= min_tokens && P <= m->bucket_pairs;
     if (T < BUCKET_MIN_TOKENS || !bucketed) m->last_rows = T, m->last_pairs = P, m->last_rpj = rpj;  // the replay entry's list
     if (bucketed) {
         if (int32_t rc = run_experts_bucketed(m, x_in, T, P, rpj, s)) return rc;
@@ -602,6 +616,7 @@ int32_t jq_moe_experts_replay_dev(jq_moe* m, const float* x_dev, void* stream) {
     if (!m || !x_dev) return jq_fail(jq::E_INVALID, "jq_moe_experts_replay_dev: NULL argument");
     if (!m->gate || m->last_rpj == 0)
         return jq_fail(jq::E_INVALID, "jq_moe_experts_replay_dev: no decode-sized call has left a job list on this layer");
+    if (int32_t rc = note_capture(m, static_cast<cudaStream_t>(stream))) return rc;
     return run_experts(m, x_dev, m->last_rows, m->last_pairs, m->last_rpj, static_cast<cudaStream_t>(stream));
 }
 

@@ -312,3 +312,42 @@ def test_experts_on_tiles_match_the_oracle_and_replay(tokens):
     layer.experts_replay_dev(torch.from_numpy(x).cuda())
     torch.cuda.synchronize()
     layer.status()
+
+
+@pytest.mark.parametrize("kind,tokens_", [(synth.Q4_K, 4), (synth.Q4_K, 40), (synth.MXFP4, 64), (synth.Q8_0, 12), (synth.Q8_0, 140)])
+def test_a_captured_layer_survives_larger_batches(kind, tokens_):
+    """A graph of the layer holds addresses of its workspace and of the stream's scratch; reserving and running larger
+    batches afterwards outgrows both.  Replays still give the captured batch's values, bit for bit."""
+    import torch
+
+    cfg = MoeConfig(gating=GATE_SOFTMAX, n_expert=16, n_used=4, hidden=512, inter=256)
+    moe, router, banks, types, _ = build(cfg, kind, seed=61)
+    moe.reserve(tokens_)
+    s = torch.cuda.Stream()
+    x = torch.from_numpy(tokens(400, cfg.hidden, 6)).cuda()
+    small, large = torch.zeros(tokens_, cfg.hidden, device="cuda"), torch.zeros(400, cfg.hidden, device="cuda")
+    torch.cuda.synchronize()
+    moe.forward_dev(x[:tokens_], small, stream=s.cuda_stream)
+    s.synchronize()
+    want = small.clone()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        moe.forward_dev(x[:tokens_], small, stream=s.cuda_stream)
+    for T in (tokens_ + 1, 150, 400):
+        moe.reserve(T)
+        moe.forward_dev(x[:T], large, stream=s.cuda_stream)
+    s.synchronize()
+    junk = [torch.full((1 << 20,), float("nan"), device="cuda") for _ in range(32)]   # what was freed gets new owners
+    for _ in range(2):
+        small.zero_()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(s):
+            g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(small, want)
+        moe.forward_dev(x, large, stream=s.cuda_stream)
+    s.synchronize()
+    moe.status()
+    assert all(bool(torch.isnan(j).all()) for j in junk)
+    _, _, ref = oracle_forward(cfg, x[:tokens_].cpu().numpy(), router, banks, types)
+    assert_close(want.cpu().numpy(), ref)
