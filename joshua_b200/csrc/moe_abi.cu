@@ -63,6 +63,7 @@ int32_t reserve(jq_moe* m, uint64_t T, uint64_t P) {
     m->ws = nullptr;
     m->in_graph = false;
     m->cap_tokens = m->cap_pairs = m->bucket_pairs = 0;
+    m->last_rpj = 0;  // the replay entry's list goes with the workspace
     size_t off = 0;
     auto take = [&](size_t bytes) {
         size_t o = off;
@@ -399,8 +400,10 @@ int32_t jq_moe_experts_list(jq_moe* m, const float* x_dev, uint64_t n_rows, cons
     uint32_t rpj = jq_moe_rows_per_job(live_rows, c.n_expert);
     JQ_CUDA(jq::launch_moe_jobs(expert_ids_dev, (uint32_t)n_rows, 1, c.n_expert, rpj, m->list_token, m->inv, m->jobs,
                                 m->n_jobs, m->n_list, m->bad_dev, s));
-    if (!m->ctx->force_f32 && live_rows >= BUCKET_MIN_TOKENS && n_rows <= m->bucket_pairs)
+    if (!m->ctx->force_f32 && live_rows >= BUCKET_MIN_TOKENS && n_rows <= m->bucket_pairs) {
+        m->last_rpj = 0;
         return run_experts_bucketed(m, x_dev, n_rows, n_rows, rpj, s);
+    }
     m->last_rows = m->last_pairs = n_rows, m->last_rpj = rpj;
     return run_experts(m, x_dev, n_rows, n_rows, rpj, s);
 }
@@ -597,7 +600,8 @@ int32_t jq_moe_forward_norm_add_dev(jq_moe* m, const float* x_dev, uint64_t T, c
     if (const char* thr_env = std::getenv("JQ_MOE_BUCKET_TOKENS")) min_tokens = std::strtoull(thr_env, nullptr, 10);  // measurement switch
 #endif
     const bool bucketed = !fused && !m->ctx->force_f32 && T >= min_tokens && P <= m->bucket_pairs;
-    if (T < BUCKET_MIN_TOKENS || !bucketed) m->last_rows = T, m->last_pairs = P, m->last_rpj = rpj;  // the replay entry's list
+    // the replay entry's list: a prompt's list replaces it and is not offered, callers replay with a decode batch's rows
+    m->last_rows = T, m->last_pairs = P, m->last_rpj = T < BUCKET_MIN_TOKENS || !bucketed ? rpj : 0;
     if (bucketed) {
         if (int32_t rc = run_experts_bucketed(m, x_in, T, P, rpj, s)) return rc;
     } else {

@@ -227,6 +227,30 @@ def test_replay_needs_a_previous_call():
         moe.experts_replay_dev(torch.zeros(1, cfg.hidden, device="cuda"))
 
 
+def test_replay_is_refused_where_its_job_list_is_gone():
+    """The list lives in the workspace: a larger reserve takes it away, and a prompt writes its own over it, whose rows a
+    decode batch does not have."""
+    import torch
+
+    cfg = MoeConfig(gating=GATE_SOFTMAX, n_expert=16, n_used=4, hidden=512, inter=256)
+    moe, *_ = build(cfg, synth.Q4_K, seed=43)
+    x = torch.from_numpy(tokens(200, cfg.hidden, 9)).cuda()
+    y = torch.empty_like(x)
+    moe.reserve(5)
+    moe.forward_dev(x[:5], y[:5])
+    moe.experts_replay_dev(x[:5])
+    moe.reserve(200)
+    with pytest.raises(JoshuaB200Error, match="job list"):
+        moe.experts_replay_dev(x[:5])
+    moe.forward_dev(x[:5], y[:5])
+    moe.experts_replay_dev(x[:5])
+    moe.forward_dev(x, y)
+    with pytest.raises(JoshuaB200Error, match="job list"):
+        moe.experts_replay_dev(x[:5])
+    torch.cuda.synchronize()
+    moe.status()
+
+
 def test_create_rejects_bad_banks():
     cfg = MoeConfig(gating=GATE_SOFTMAX, n_expert=4, n_used=2, hidden=256, inter=256)
     g = QTensor.from_bytes(synth.Q4_K, synth.random_weight(synth.Q4_K, 4 * 256, 256, 1))
