@@ -3,10 +3,10 @@
 
 namespace {
 
-// The split kernel of the tile GEMM reads rows and norm weights as 16-byte vectors; other buffers take the separate
-// kernels, which copy.
-bool vectors(const float* lhs, const float* norm_w) {
-    return (reinterpret_cast<uintptr_t>(lhs) | reinterpret_cast<uintptr_t>(norm_w)) % 16 == 0;
+// Every kernel behind these entries reads rows and norm weights as 16-byte vectors.
+int32_t check_vectors(const char* who, const float* lhs, const float* norm_w) {
+    if ((reinterpret_cast<uintptr_t>(lhs) | reinterpret_cast<uintptr_t>(norm_w)) % 16 == 0) return jq::OK;
+    return jq_fail(jq::E_INVALID, std::string(who) + ": lhs and norm weights must be 16-byte aligned");
 }
 
 size_t swiglu_scratch_bytes(uint64_t m, uint64_t n) { return 2 * m * n * 4 + 512; }
@@ -42,6 +42,7 @@ int32_t jq_matmul_swiglu_dev(const jq_weight* gate, const jq_weight* up, uint64_
                                           std::to_string(k % gate->fmt.elems ? 0 : n * (k / gate->fmt.elems)));
     if (m == 0 || n == 0) return jq::OK;
     if (!lhs_dev || !dst_dev) return jq_fail(jq::E_INVALID, "jq_matmul_swiglu_dev: NULL buffer");
+    if (int32_t rc = check_vectors("jq_matmul_swiglu_dev", lhs_dev, nullptr)) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     jq_ctx* ctx = gate->ctx;
     if (pair_uses_tiles(gate, up, m, k, n, s))
@@ -72,15 +73,18 @@ int32_t jq_matmul_swiglu_norm_dev(const jq_weight* gate, const jq_weight* up, ui
     jq_ctx* ctx = gate->ctx;
     const bool shapes_ok = gate->type == up->type && gate->n_blocks == up->n_blocks && k % gate->fmt.elems == 0 &&
                            gate->n_blocks == n * (k / gate->fmt.elems) && m > 0 && n > 0 && lhs_dev && dst_dev;
-    if (shapes_ok && vectors(lhs_dev, norm_w_dev) && pair_uses_tiles(gate, up, m, k, n, s))
+    // the plain entry names the fault (or finds nothing to do) before anything is launched
+    if (!shapes_ok) return jq_matmul_swiglu_dev(gate, up, m, k, n, lhs_dev, dst_dev, clamp, stream);
+    if (int32_t rc = check_vectors("jq_matmul_swiglu_norm_dev", lhs_dev, norm_w_dev)) return rc;
+    if (pair_uses_tiles(gate, up, m, k, n, s))
         return swiglu_tiles(gate, up, m, k, n, lhs_dev, norm_w_dev, eps, dst_dev, clamp, s);
-    if (shapes_ok && !ctx->force_f32 && jq::gemv_mma_supports(gate->type, gate->dev, n, k, m) &&
+    if (!ctx->force_f32 && jq::gemv_mma_supports(gate->type, gate->dev, n, k, m) &&
         jq::gemv_mma_supports(up->type, up->dev, n, k, m) && jq::gemv_mma_fusable(gate->type, m, k)) {
         JQ_CUDA(jq::launch_gemv_mma_swiglu(gate->type, gate->dev, up->dev, n, k, lhs_dev, m, dst_dev, clamp,
                                            ctx->status_dev, s, norm_w_dev, eps));
         return jq::OK;
     }
-    // separate kernels: normalise into scratch, then the plain entry (which validates)
+    // separate kernels: normalise into scratch, then the plain entry
     void* scratch = nullptr;
     JQ_CUDA(ctx->scratch_for(s, SLOT_NORM, m * k * 4 + 256, &scratch));
     JQ_CUDA(jq::launch_rmsnorm(lhs_dev, nullptr, norm_w_dev, eps, m, (uint32_t)k, nullptr, static_cast<float*>(scratch), s));
@@ -96,16 +100,17 @@ int32_t jq_matmul_norm_dev(const jq_weight* w, uint64_t m, uint64_t k, uint64_t 
     jq_ctx* ctx = w->ctx;
     const bool shapes_ok = k % w->fmt.elems == 0 && w->n_blocks == n * (k / w->fmt.elems) && m > 0 && n > 0 &&
                            lhs_dev && dst_dev;
-    if (shapes_ok && vectors(lhs_dev, norm_w_dev) && jq_uses_tiles(w, m, k, n, s))
+    if (!shapes_ok) return jq_matmul_t_dev(w, m, k, n, lhs_dev, dst_dev, stream);  // as above
+    if (int32_t rc = check_vectors("jq_matmul_norm_dev", lhs_dev, norm_w_dev)) return rc;
+    if (jq_uses_tiles(w, m, k, n, s))
         return jq_matmul_tiles(w, nullptr, m, k, n, lhs_dev, norm_w_dev, eps, residual_dev, dst_dev, nullptr, s);
-    if (shapes_ok && !ctx->force_f32 && jq::gemv_mma_dense_supports(w->type, w->dev, n, k, m) &&
+    if (!ctx->force_f32 && jq::gemv_mma_dense_supports(w->type, w->dev, n, k, m) &&
         jq::gemv_mma_fusable(w->type, m, k)) {
         JQ_CUDA(jq::launch_gemv_mma_fused(w->type, w->dev, n, k, lhs_dev, m, dst_dev, norm_w_dev, eps, residual_dev,
                                           ctx->status_dev, s));
         return jq::OK;
     }
     // separate kernels: norm into scratch, product into scratch, then the add
-    if (m == 0 || n == 0) return jq_matmul_t_dev(w, m, k, n, lhs_dev, dst_dev, stream);
     void* scratch = nullptr;
     const uint64_t xk = (m * k + 63) & ~(uint64_t)63;
     JQ_CUDA(ctx->scratch_for(s, SLOT_NORM, (xk + m * n) * 4 + 256, &scratch));
@@ -113,7 +118,6 @@ int32_t jq_matmul_norm_dev(const jq_weight* w, uint64_t m, uint64_t k, uint64_t 
     float* prod = xn + xk;
     const float* in = lhs_dev;
     if (norm_w_dev) {
-        if (!lhs_dev) return jq_fail(jq::E_INVALID, "jq_matmul_norm_dev: NULL buffer");
         JQ_CUDA(jq::launch_rmsnorm(lhs_dev, nullptr, norm_w_dev, eps, m, (uint32_t)k, nullptr, xn, s));
         in = xn;
     }

@@ -71,3 +71,35 @@ def test_swiglu_pair_with_norm(type_id, m):
                                            0.0, s))
     torch.cuda.synchronize()
     _close(got, want, 1e-4)
+
+
+@pytest.mark.parametrize("type_id", [synth.Q4_K, synth.Q6_K, synth.Q8_0, synth.Q5_0])
+@pytest.mark.parametrize("m", [1, 7, 40])
+def test_bad_buffers_are_refused_before_a_launch(type_id, m):
+    """Rows and norm weights are read as 16-byte vectors: other addresses, NULL and wrong sizes are errors of the host, with
+    and without norm and residual, whatever kernel the batch would take."""
+    import torch
+
+    from joshua_b200 import _lib
+    from joshua_b200.qtensor import QTensor
+
+    L, k, n = _lib.lib(), 512, 96
+    w = QTensor.from_bytes(type_id, np.zeros(synth.tensor_bytes(type_id, n, k), np.uint8))
+    x, nw, res, out = (torch.zeros(size, device="cuda") for size in (m * k + 4, k + 4, m * n, m * n))
+    s = torch.cuda.current_stream().cuda_stream
+
+    def norm(lhs, norm_w, residual, kk=k):
+        return L.jq_matmul_norm_dev(w._h, m, kk, n, lhs, norm_w, 1e-5, residual, out.data_ptr(), s)
+
+    def pair(lhs, norm_w, kk=k):
+        return L.jq_matmul_swiglu_norm_dev(w._h, w._h, m, kk, n, lhs, norm_w, 1e-5, out.data_ptr(), 0.0, s)
+
+    X, N, R = x.data_ptr(), nw.data_ptr(), res.data_ptr()
+    for lhs, norm_w, residual, kk in [(X + 4, None, R, k), (X + 8, N, None, k), (X, N + 4, R, k), (X + 4, N, R, k),
+                                      (None, N, R, k), (None, None, R, k), (X, N, R, 2 * k)]:
+        assert norm(lhs, norm_w, residual, kk) == _lib.E_INVALID
+    for lhs, norm_w, kk in [(X + 4, None, k), (X + 8, N, k), (X, N + 4, k), (None, N, k), (None, None, k), (X, N, 2 * k)]:
+        assert pair(lhs, norm_w, kk) == _lib.E_INVALID
+    assert norm(X, N, R) == 0 and pair(X, N) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(out, torch.zeros_like(out))
