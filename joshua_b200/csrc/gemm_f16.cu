@@ -904,7 +904,6 @@ cudaError_t launch_f16_tile(const F16Launch& l, cudaStream_t s) {
             if (cost < best) best = cost, split = c;
         }
         cfg.gridDim = dim3(gx, (unsigned)gy, split * banks);
-        if (gy > 65535) return cudaErrorInvalidValue;
         if (split > 1) {
             attr[1].id = cudaLaunchAttributeClusterDimension;
             attr[1].val.clusterDim.x = 1;
@@ -941,9 +940,13 @@ cudaError_t split_activations_f16(uint32_t type, const float* x, uint64_t m, uin
 
 }  // namespace
 
-// Whole staged windows in every row, made of the vectors they are copied by.
+// Rows of a tile for m rows of lhs.  Up to 64 rows the other route is the decode kernel: they stay on the exact tiles.
+// Q6_K always does (no 128-row form of it was built).
+static uint32_t tile_rows(uint32_t type, uint64_t m) { return m <= 16 ? 16 : m <= 64 || type == T_Q6_K ? 32 : 128; }
+
+// Whole staged windows in every row, made of the vectors they are copied by; the tiles of lhs fit grid.y.
 bool gemm_f16_supports(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, uint64_t m) {
-    if (m == 0 || n == 0 || k == 0 || k % 256 != 0 || k > 0x7FFFFFFFu || m > 0x7FFFFFFFu) return false;
+    if (m == 0 || n == 0 || k == 0 || k % 256 != 0 || k > 0x7FFFFFFFu || m > 65535ull * tile_rows(type, m)) return false;
     const uintptr_t a = reinterpret_cast<uintptr_t>(w);
     switch (type) {
         case T_Q4_K: return a % 16 == 0;
@@ -972,10 +975,11 @@ cudaError_t launch_gemm_f16(uint32_t type, const uint8_t* w_a, const uint8_t* w_
     l.residual = residual;
     l.error_flag = error_flag;
     if (cudaError_t e = split_activations_f16(type, lhs, m, k, norm_w, eps, l.x, s); e != cudaSuccess) return e;
-    if (m <= 16) return launch_f16_typed<16>(type, l, s);
-    // up to 64 rows the other route is the decode kernel, for Q6_K always: they stay on the exact tiles
-    if (m <= 64 || type == T_Q6_K) return launch_f16_typed<32>(type, l, s);
-    return launch_f16_typed<128>(type, l, s);
+    switch (tile_rows(type, m)) {
+        case 16: return launch_f16_typed<16>(type, l, s);
+        case 32: return launch_f16_typed<32>(type, l, s);
+        default: return launch_f16_typed<128>(type, l, s);
+    }
 }
 
 bool gemm_f16_grouped_supports(uint32_t type, const uint8_t* bank, uint64_t n, uint64_t k) {

@@ -166,3 +166,21 @@ def test_qmatmul_forward_on_device_tensors():
         mm.forward(x.half())
     with pytest.raises(JoshuaB200Error):
         QMatMul.from_qtensor(QTensor.from_bytes(synth.Q4_K, raw), (n + 1, k))
+
+
+def test_q6_k_takes_more_rows_than_a_grid_of_tiles():
+    """A tile launch covers 65535 tiles of 32 rows of lhs; larger batches of Q6_K go through the decode kernel in slices."""
+    import torch
+
+    n, k, m = 2, 256, 65535 * 32 + 9
+    raw = synth.random_weight(synth.Q6_K, n, k, seed=4)
+    w = torch.from_numpy(oracle.dequantize(synth.Q6_K, raw).reshape(n, k)).cuda().double()
+    x = torch.randn(m, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(5))
+    out = torch.empty(m, n, device="cuda")
+    QTensor.from_bytes(synth.Q6_K, raw).matmul_t_dev((m, k, n), x, out)
+    torch.cuda.synchronize()
+    for a in (0, m // 2, m - 64):
+        rows = x[a:a + 64].double()
+        # one unit a row: 6.1e-8 of its largest value per term, f32 sums of the pieces (the bound above, per 2-norm)
+        scale = ((rows ** 2) @ (w.T ** 2)).sqrt()
+        assert bool(((out[a:a + 64].double() - rows @ w.T).abs() <= 1e-5 * scale).all())
