@@ -38,10 +38,14 @@ bool grouped_tiles_ok(const jq_moe* m, uint64_t P) {
            jq::gemm_f16_grouped_supports(m->down->type, m->down->dev, c.hidden, c.inter) && P / 33 + 1 <= 65535;
 }
 
-uint32_t max_narrow_tiles(const jq_moe* m, uint64_t P) { return (uint32_t)std::min<uint64_t>(m->cfg.n_expert, P + 1); }
+// One narrow tile at most for an expert, and none for one with fewer than min_rows rows.  The launch covers them all: with
+// one for every expert (256 of Q2_K, 2048 x 1024, 128 tokens) the surplus CTAs took the layer from 1069 to 1095 us.
+uint32_t max_narrow_tiles(const jq_moe* m, uint64_t P, uint32_t min_rows) {
+    return (uint32_t)std::min<uint64_t>(m->cfg.n_expert, P / min_rows + 1);
+}
 // narrow and wide tiles, the small experts' jobs (any rows per job), four counts
 uint64_t bucket_lists_bytes(const jq_moe* m, uint64_t P) {
-    return ((uint64_t)max_narrow_tiles(m, P) + P / 33 + 1) * sizeof(jq::GemmTile) + P * sizeof(jq::MoeJob) + 32;
+    return ((uint64_t)max_narrow_tiles(m, P, 1) + P / 33 + 1) * sizeof(jq::GemmTile) + P * sizeof(jq::MoeJob) + 32;
 }
 // Tokens from which a layer may take the prefill form.
 uint64_t bucket_min_tokens(const jq_moe* m, uint64_t P) {
@@ -208,7 +212,7 @@ int32_t run_experts_bucketed(jq_moe* m, const float* x, uint64_t T, uint64_t P, 
         // types whose narrow tiles are ahead of the decode kernel at any row count.
         const bool all_tiles = all_experts_on_tiles(m) || P >= 24ull * c.n_expert;
         const uint32_t min_rows = all_tiles ? 1u : (uint32_t)BUCKET_ROWS_PER_EXPERT;
-        const uint32_t max_narrow = max_narrow_tiles(m, P), max_wide = (uint32_t)(P / 33 + 1);
+        const uint32_t max_narrow = max_narrow_tiles(m, P, min_rows), max_wide = (uint32_t)(P / 33 + 1);
         const uint32_t max_small = (uint32_t)std::min<uint64_t>(P, P / rows_per_job + c.n_expert);
         jq::GemmTile* narrow = m->tiles;
         jq::GemmTile* wide = narrow + max_narrow;
