@@ -1312,9 +1312,11 @@ __global__ void __launch_bounds__((16 + 2) * 32, 1) gemv_narrow_kernel(const __g
 
 constexpr uint32_t SMEM_BUDGET = 220 * 1024;  // of the 227 KB a CTA may use
 // Activation planes kept in shared memory, at most.  Measured: 116 KB (8 rows of k = 4096, two ring stages left) is slower
-// than planes in global memory with a deeper ring.  Four rows of k = 7168 (98 KB), 2048 weight rows, shared / global:
-// Q8_0 13.7 / 14.9 us, Q4_K 12.6 / 9.6 us, IQ2_XXS 14.0 / 9.0 us: only Q8_0, whose units take the fewest instructions,
-// gains.
+// than planes in global memory with a deeper ring.  Between 96 and 100 KB, 2048 weight rows, shared / global: four rows of
+// k = 7168, Q8_0 13.4 / 15.9 us, Q4_K 12.6 / 9.6 us, IQ2_XXS 14.0 / 9.0 us: only Q8_0, whose units take the fewest
+// instructions, gains, and from three rows on: three of 9472 14.3 / 18.4, seven of 4096 13.6 / 14.2, two of 14336
+// 15.3 / 11.3 (few rows take little from L2, and every CTA splits all of them first).  At 512 weight rows 14.2 / 16.5,
+// 13.4 / 13.2, 14.9 / 10.1; at 4096 18.8 / 28.1, 17.0 / 20.9, 21.4 / 17.6.
 constexpr uint32_t ACT_SMEM_MAX = 96 * 1024, ACT_SMEM_MAX_Q8_0 = 100 * 1024;
 
 template <uint32_t TYPE>
@@ -1389,7 +1391,7 @@ cudaError_t launch_typed(uint32_t type, GemvArgs& ga, uint32_t rows_per_job, uin
 
 // Activation planes live in the kernel's shared memory when they fit; only larger products need scratch.
 static bool acts_fit_in_smem(uint64_t rows, uint64_t k, uint32_t type = 0) {
-    return rows * (k / 32) * 112 <= (type == T_Q8_0 ? ACT_SMEM_MAX_Q8_0 : ACT_SMEM_MAX);
+    return rows * (k / 32) * 112 <= (type == T_Q8_0 && rows >= 3 ? ACT_SMEM_MAX_Q8_0 : ACT_SMEM_MAX);
 }
 
 size_t gemv_mma_scratch_bytes(uint64_t rows, uint64_t k) {

@@ -184,3 +184,27 @@ def test_q6_k_takes_more_rows_than_a_grid_of_tiles():
         # one unit a row: 6.1e-8 of its largest value per term, f32 sums of the pieces (the bound above, per 2-norm)
         scale = ((rows ** 2) @ (w.T ** 2)).sqrt()
         assert bool(((out[a:a + 64].double() - rows @ w.T).abs() <= 1e-5 * scale).all())
+
+
+@pytest.mark.parametrize("m,k", [(1, 28160), (1, 28672), (2, 13824), (2, 14336), (3, 8960), (3, 9472), (4, 7168), (5, 5632), (7, 4096),
+                                 (8, 3328), (8, 3584), (8, 4096)])
+def test_q8_0_planes_around_the_shared_memory_limit(m, k):
+    """Q8_0 keeps up to 100 KB of activation planes in shared memory from three rows on and 96 KB below: both sides of either
+    line, with a residual (fused where the planes are in shared memory).  The bound is that of the split and of f32 sums, as
+    for Q6_K above."""
+    import torch
+
+    from joshua_b200 import _lib
+
+    n = 70
+    raw = synth.random_weight(synth.Q8_0, n, k, seed=m)
+    x = synth.random_activations(m, k, seed=k).reshape(m, k)
+    res = np.random.default_rng(m).standard_normal((m, n)).astype(np.float32)
+    q = QTensor.from_bytes(synth.Q8_0, raw)
+    xd, out = torch.from_numpy(x).cuda(), torch.from_numpy(res).cuda()
+    _lib.check(_lib.lib().jq_matmul_norm_dev(q._h, m, k, n, xd.data_ptr(), None, 0.0, out.data_ptr(), out.data_ptr(),
+                                             torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    w, x64 = oracle.dequantize(synth.Q8_0, raw).reshape(n, k).astype(np.float64), x.astype(np.float64)
+    scale = np.sqrt((x64 ** 2) @ (w.T ** 2)) + np.abs(res)
+    assert np.all(np.abs(out.cpu().numpy() - (res + x64 @ w.T)) <= 1e-5 * scale)
