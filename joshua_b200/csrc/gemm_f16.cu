@@ -11,15 +11,19 @@
 //   Q8_0         2^p * (code * d_block / 2^p)   18 bits: two terms, the second by an exact fused multiply-subtract
 //   Q6_K         d  * (scale * code)            13 bits: two terms
 //
-// The activations are split once per launch (`split_f16_kernel`): a row is scaled by a power of two that puts its
-// largest value just below 2^10, hi = f16(x), lo = f16(x - hi), so hi + lo carries 22 to 24 bits of every value within
-// 2^17 of the row's largest one and an absolute error below 2^-35 of it otherwise.  The tensor core's products of
-// f16 terms are exact; two or three products (hi*hi, hi*lo, lo*hi) replace the three TF32 products of the form
-// below at twice their rate: 32 to 48 instructions per window instead of 96.
+// The activations are split once per launch (`split_f16_kernel`): a row is scaled by a power of two that puts its largest
+// value just below 2^15, hi = f16(x), lo = f16(x - hi): 22 to 24 bits of every value within 2^17 of the largest one, an
+// absolute error below 2^-39 of it otherwise.  A window whose own largest value lies more than 2^8 below the row's (an
+// outlier elsewhere) is scaled further by itself, so the error stays below 2^-31 of the window's largest value (the int8
+// planes of the decode kernel, scaled over the same 256 values: 2^-24 of it), and the read-back undoes that scale token
+// by token.  Rows with such a window say so by the sign of their scale; a tile without one, the usual one, never asks.  The tensor core's products of f16
+// terms are exact; two or three products (hi*hi, hi*lo, lo*hi) replace three TF32 products (gemm_tc.cu) at twice their
+// rate: 32 to 48 instructions per window instead of 96.
 //
 // Minima (Q4_K, Q2_K): sum_c dmin m_g x_c = sum_g (dmin m_g) (sum of x over the group), an inner product of 16 terms per
-// window.  The split kernel also writes the sums of each 16 values as two f16 terms, the converters write
-// -(dmin / f) m_g as two f16 terms, and three more instructions add their product to the same accumulator.
+// window.  The split kernel also writes the sums of each 16 values, times 2^-5 so that they fit, as two f16 terms, the
+// converters write -2^5 (dmin / f) m_g as two f16 terms, and three more instructions add their product to the same
+// accumulator.
 //
 // The tensor core adds into its f32 accumulator with truncation, an error that grows with the instructions behind one
 // another, so accumulators are short and the converter warps read them back with tcgen05.ld and add f * acc,
@@ -42,8 +46,9 @@
 // Warps: 16 converters, warp (q = w % 4, g = w / 4) owns weight rows 32q .. 32q+31 (the tensor-memory lanes it may
 // touch) and the columns 64g .. 64g+63 of every window; the four warps of a quarter share the staged raw bytes of a
 // window and meet once per window on a named barrier (an mbarrier round trip costs some 200 cycles here).  Warps 16 to
-// 19 issue the MMAs: an instruction takes about 30 cycles to issue, so narrow tiles have an issuer per step (wide ones
-// one in all, their steps share an accumulator).  Warp 20 issues the TMA copies.
+// 19 issue the MMAs and the TMA copies: an instruction takes about 30 cycles to issue, so narrow tiles have an issuer per
+// step, which also copies its step's activation tiles; wide ones, whose steps share an accumulator, have one, and another
+// warp copies.
 //
 // Few tiles (small n, or few rows of lhs) leave SMs idle: then a cluster of S CTAs splits k, every CTA leaves its
 // partial tile in its shared memory, and each adds a share of the tile over the cluster in rank order (distributed
@@ -68,7 +73,7 @@ namespace {
 constexpr int HM = 128;           // weight rows per CTA = MMA M = TMEM lanes
 constexpr int H_CONV = 16;        // converter / epilogue warps
 constexpr int H_ISSUE = 4;        // issuing warps: one per 64-column step where the steps have their own accumulators
-constexpr int H_THREADS = (H_CONV + H_ISSUE + 1) * 32;
+constexpr int H_THREADS = (H_CONV + H_ISSUE) * 32;  // five warps a scheduler: 96 registers a thread (six: 80, and spills)
 constexpr uint32_t H_STEPS = 4;   // 64-column steps per 256-column window = ring stages
 
 template <uint32_t TYPE>
@@ -126,12 +131,13 @@ struct Tile {
     static constexpr uint32_t PLANE_B = N_TILE * 128;  // 64 f16 columns of N_TILE rows
     static constexpr uint32_t STAGE_B = 2 * PLANE_B;   // hi | lo
     static constexpr uint32_t RAW_BUF = HM * raw_stride<TYPE>() * 4;
+    static constexpr uint32_t SCALE_B = H_CONV * 32 * 16;  // every converter warp's tokens: what scales of windows need
     static constexpr uint32_t FIXED = STAGES * STAGE_B + (HT<TYPE>::MIN ? WINDOWS * PLANE_B : 0) +
-                                      (TYPE == T_IQ2_XXS ? 2048 : 0) + 1024;
+                                      (TYPE == T_IQ2_XXS ? 2048 : 0) + SCALE_B + 1024;
     static constexpr uint32_t ROOM = (226 * 1024 - FIXED) / RAW_BUF;
     static constexpr uint32_t WANT = N_TILE <= 32 ? 4 : 2;
     static constexpr uint32_t BUFS = ROOM < WANT ? ROOM : WANT;
-    static_assert(BUFS >= 1, "shared memory");
+    static_assert(BUFS >= 2, "shared memory");
     static constexpr uint32_t LOOP_SMEM = FIXED + BUFS * RAW_BUF;
     static constexpr uint32_t RED_SMEM = (FINE ? 4 : 1) * N_TILE * HM * 4 + 1024;  // the partial tiles at the end
     static constexpr uint32_t SMEM = LOOP_SMEM > RED_SMEM ? LOOP_SMEM : RED_SMEM;
@@ -156,21 +162,21 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, ui
 }
 
 // ── activations ──
-// One CTA per row; a thread takes 16 consecutive values at a time.  hi / lo [m][k]; sums [m][k / 256][32]: the 16 group
-// sums of a window, first terms then second terms; inv[m]: the inverse of the row's scale.
-// With norm_w the rows are RMS-normalised first: the values split are x * rs * norm_w.
+// One CTA per row; a thread takes 16 consecutive values at a time, half a warp a window.  hi / lo [m][k];
+// sums [m][k / 256][32]: the 16 group sums of a window, first terms then second terms; inv[m]: the inverse of the row's
+// scale, negative where some window has one of its own; rel[k / 256][m]: the inverse of that.  With norm_w the rows are RMS-normalised first: the values split are x * rs * norm_w.
 __global__ void __launch_bounds__(256) split_f16_kernel(const float* __restrict__ x, uint32_t k,
                                                         const float* __restrict__ norm_w, float eps, int plain_order,
                                                         __half* __restrict__ hi,
                                                         __half* __restrict__ lo, __half* __restrict__ sums,
-                                                        float* __restrict__ inv) {
+                                                        float* __restrict__ inv, float* __restrict__ rel) {
     __shared__ float s_max[8], s_sq[8];
     pdl_trigger();
     pdl_wait();
     const uint32_t row = blockIdx.x, tid = threadIdx.x, groups = k / 16;
     const float4* xr = reinterpret_cast<const float4*>(x + (uint64_t)row * k);
     const float4* nr = reinterpret_cast<const float4*>(norm_w);
-    float amax = 0.0f, sq = 0.0f;
+    float row_max = 0.0f, sq = 0.0f;
 #pragma unroll 4
     for (uint32_t i = tid; i < k / 4; i += 256) {
         float4 v = __ldg(xr + i);
@@ -179,29 +185,30 @@ __global__ void __launch_bounds__(256) split_f16_kernel(const float* __restrict_
             const float4 g = __ldg(nr + i);
             v.x *= g.x, v.y *= g.y, v.z *= g.z, v.w *= g.w;
         }
-        amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+        row_max = fmaxf(row_max, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+        row_max = fmaxf(row_max, __shfl_xor_sync(0xFFFFFFFFu, row_max, o));
         sq += __shfl_xor_sync(0xFFFFFFFFu, sq, o);
     }
-    if ((tid & 31) == 0) s_max[tid >> 5] = amax, s_sq[tid >> 5] = sq;
+    if ((tid & 31) == 0) s_max[tid >> 5] = row_max, s_sq[tid >> 5] = sq;
     __syncthreads();
-    amax = s_max[0], sq = s_sq[0];
+    row_max = s_max[0], sq = s_sq[0];
 #pragma unroll
-    for (int i = 1; i < 8; ++i) amax = fmaxf(amax, s_max[i]), sq += s_sq[i];
+    for (int i = 1; i < 8; ++i) row_max = fmaxf(row_max, s_max[i]), sq += s_sq[i];
     const float rs = norm_w ? rsqrtf(sq / (float)k + eps) : 1.0f;
-    amax *= rs;
-    // scale 2^(136 - e): the largest value lands in [2^9, 2^10) (a rounding of the norm aside), 16 sum to about 2^14.  Clamped where the
-    // scale itself would leave f32 (rows below 2^-118); a row with an infinity keeps it.
-    const uint32_t e = __float_as_uint(amax) >> 23;
-    const uint32_t se = e == 255 ? 127u : min(254u, 263u - e);
-    const float scale = __uint_as_float(se << 23);
-    if (tid == 0) inv[row] = se == 254 ? __uint_as_float(0x00400000u) : __uint_as_float((254u - se) << 23);
-    for (uint32_t g = tid; g < groups; g += 256) {
-        uint32_t h[8], l[8];
-        float sum = 0.0f;
+    // scale 2^(141 - e): the largest value lands in [2^14, 2^15) (a rounding of the norm aside).  Clamped where the scale
+    // itself would leave f32 (below 2^-113); infinities keep theirs.
+    auto scale_bits = [](float amax) {
+        const uint32_t e = __float_as_uint(amax) >> 23;
+        return e == 255 ? 127u : min(254u, 268u - e);
+    };
+    const uint32_t row_bits = scale_bits(row_max * rs);
+    bool own = false;  // a window of this thread has a scale of its own
+    for (uint32_t g = tid; g < groups; g += 256) {  // groups is a multiple of 16: whole half-warps
+        float4 val[4];
+        float amax = 0.0f;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             float4 v = __ldg(xr + 4 * g + j);
@@ -209,6 +216,21 @@ __global__ void __launch_bounds__(256) split_f16_kernel(const float* __restrict_
                 const float4 w = __ldg(nr + 4 * g + j);
                 v.x = v.x * rs * w.x, v.y = v.y * rs * w.y, v.z = v.z * rs * w.z, v.w = v.w * rs * w.w;
             }
+            amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+            val[j] = v;
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFu << (tid & 16), amax, o));
+        int extra = amax == 0.0f ? 0 : (int)scale_bits(amax) - (int)row_bits;
+        extra = extra <= 8 ? 0 : min(extra, 60);
+        own |= extra != 0;
+        const float scale = __uint_as_float((row_bits + extra) << 23);
+        if ((g & 15) == 0) rel[(uint64_t)(g >> 4) * gridDim.x + row] = __uint_as_float((uint32_t)(127 - extra) << 23);
+        uint32_t h[8], l[8];
+        float sum = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float4 v = val[j];
             v.x *= scale, v.y *= scale, v.z *= scale, v.w *= scale;
             sum += (v.x + v.y) + (v.z + v.w);
             if (!plain_order) {
@@ -225,10 +247,16 @@ __global__ void __launch_bounds__(256) split_f16_kernel(const float* __restrict_
         uint4* lp = reinterpret_cast<uint4*>(lo + (uint64_t)row * k + 16 * g);
         hp[0] = make_uint4(h[0], h[1], h[2], h[3]), hp[1] = make_uint4(h[4], h[5], h[6], h[7]);
         lp[0] = make_uint4(l[0], l[1], l[2], l[3]), lp[1] = make_uint4(l[4], l[5], l[6], l[7]);
+        sum *= 0.03125f;  // 16 values below 2^15: at most 2^14
         const __half sh = __float2half_rn(sum);
         __half* sp = sums + ((uint64_t)row * (k / 256) + (g >> 4)) * 32 + (g & 15);
         sp[0] = sh;
         sp[16] = __float2half_rn(sum - __half2float(sh));
+    }
+    const int any_own = __syncthreads_or(own);
+    if (tid == 0) {
+        const float v = row_bits == 254 ? __uint_as_float(0x00400000u) : __uint_as_float((254u - row_bits) << 23);
+        inv[row] = any_own ? -v : v;
     }
 }
 
@@ -291,14 +319,14 @@ struct RowWin {
     float d, dmin; // Q4_K / Q2_K
 };
 
-// The codes' factor f = d 2^e.  Usually e = 0; where dmin is 2^10 times d or more the codes are scaled down by 2^-e
-// (exact, f16 has subnormals down to 2^-24) so that the minima stay inside f16: |dmin / f * m| <= 1024 * 63.
+// The codes' factor f = d 2^e.  Usually e = 0; where dmin is 32 times d or more the codes are scaled down by 2^-e
+// (exact, f16 has subnormals down to 2^-24) so that the minima stay inside f16: |2^5 dmin / f * m| <= 1024 * 63.
 __device__ __forceinline__ RowWin min_factors(uint32_t dd) {
     const float d = f16_bits_to_f32(dd & 0xFFFF), dmin = f16_bits_to_f32(dd >> 16);
-    if (!(fabsf(dmin) >= 1024.0f * fabsf(d)) || dmin == 0.0f) return {d, 1.0f, d, dmin};
-    if (d == 0.0f) return {dmin * (1.0f / 512.0f), 0.0f, d, dmin};
+    if (!(fabsf(dmin) >= 32.0f * fabsf(d)) || dmin == 0.0f) return {d, 1.0f, d, dmin};
+    if (d == 0.0f) return {dmin * (1.0f / 16.0f), 0.0f, d, dmin};
     const float ratio = fabsf(dmin) / fabsf(d);
-    const int e = (int)(__float_as_uint(ratio) >> 23) - 127 - 9;
+    const int e = (int)(__float_as_uint(ratio) >> 23) - 127 - 4;
     return {d * pow2_f32(min(e, 100)), e <= 24 ? pow2_f32(-e) : 0.0f, d, dmin};
 }
 
@@ -472,12 +500,12 @@ __device__ __forceinline__ void convert64(uint32_t u, uint32_t g, const RowWin& 
     }
 }
 
-// The window's 16 minima, -(dmin / f) m, as eight packed first and eight packed second terms.  The ratio is two f16
+// The window's 16 minima, -2^5 (dmin / f) m, as eight packed first and eight packed second terms.  The ratio is two f16
 // terms, m at most six bits: the first products' remainders are exact.
 template <uint32_t TYPE>
 __device__ __forceinline__ void convert_minima(uint32_t u, const RowWin& rw, uint32_t (&a)[16]) {
-    // -dmin / f, where f is d, d 2^e or (d = 0) dmin / 512
-    const float ratio = rw.dmin == 0.0f ? 0.0f : -(rw.dmin / rw.f);
+    // f is d, d 2^e or (d = 0) dmin / 16
+    const float ratio = rw.dmin == 0.0f ? 0.0f : -32.0f * (rw.dmin / rw.f);
     const __half2 rh = __float2half2_rn(ratio), rl = __float2half2_rn(ratio - __low2float(rh));
     const uint4 hd = TYPE == T_Q4_K ? s128(u) : make_uint4(s32(u), s32(u + 4), s32(u + 8), s32(u + 12));
     // Q4_K: eight minima of 32 values, a byte each; Q2_K: sixteen of 16 values in the high nibbles
@@ -498,7 +526,7 @@ template <uint32_t TYPE, int N_TILE>
 __global__ void __launch_bounds__(H_THREADS, 1)
     gemm_f16_kernel(const uint8_t* __restrict__ w_a, uint64_t n, uint64_t k, const __grid_constant__ CUtensorMap map_hi,
                     const __grid_constant__ CUtensorMap map_lo, const __grid_constant__ CUtensorMap map_sums,
-                    const float* __restrict__ inv, uint64_t m_rows, float* dst_a, const float* residual, int* __restrict__ error_flag,
+                    const float* __restrict__ inv, const float* __restrict__ rel, uint64_t m_rows, float* dst_a, const float* residual, int* __restrict__ error_flag,
                     const GemmTile* __restrict__ tiles, const uint32_t* __restrict__ n_tiles, uint64_t expert_bytes,
                     const uint8_t* __restrict__ w_b, float* dst_b, uint32_t split) {
     using T = HT<TYPE>;
@@ -511,7 +539,8 @@ __global__ void __launch_bounds__(H_THREADS, 1)
     constexpr int MY_COLS = S::FINE ? N_TILE : N_TILE / 4;  // accumulator columns a converter thread keeps
     uint8_t* s_sums = smem + (size_t)S::STAGES * STAGE;
     uint8_t* raw = s_sums + (T::MIN ? S::WINDOWS * PLANE_B : 0);
-    uint2* s_grid = reinterpret_cast<uint2*>(raw + BUFS * RAW_BUF);
+    const uint32_t scales = smem_u32(raw + BUFS * RAW_BUF);
+    uint2* s_grid = reinterpret_cast<uint2*>(raw + BUFS * RAW_BUF + S::SCALE_B);
     // full[s]: the step's four converter warps + the TMA thread (and the tiles' bytes); empty[s]: the MMAs' commit
     __shared__ uint64_t full[S::STAGES], empty[S::STAGES], acc_full[2], acc_empty[S::ACCS];
     __shared__ uint32_t tmem_base_slot;
@@ -573,6 +602,32 @@ __global__ void __launch_bounds__(H_THREADS, 1)
         float sums[MY_COLS];
 #pragma unroll
         for (int c = 0; c < MY_COLS; ++c) sums[c] = 0.0f;
+        // Some token of this warp's columns has windows with scales of their own.  Its running sum then is in units of the
+        // scale of the window that was added last (the first one's, to begin with), and is brought to the next one's where
+        // they differ.  What that needs lies in shared memory and in a loop of its own, so that the usual tile spends no
+        // registers on it (in one loop Q6_K, 28672 x 4096, 40 rows took 202 us instead of 172).
+        bool scaled = false;
+        const uint32_t slot = scales + warp * 32 * 16;  // per token: its address in rel, its scale so far, its change
+        auto find_scales = [&] {
+            const uint64_t tok = min(tok0 + (S::FINE ? 0 : g * MY_COLS) + lane % MY_COLS, m_rows - 1);  // the last row, past it
+            scaled = __any_sync(0xFFFFFFFFu, __ldg(inv + tok) < 0.0f);
+            if (!scaled) return;
+            const float* p = rel + (uint64_t)win0 * T::UNITS * m_rows + tok;
+            asm volatile("st.shared.u64 [%0], %1;" ::"r"(slot + lane * 8), "l"(p) : "memory");
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(slot + 256 + lane * 4), "f"(__ldg(p)) : "memory");
+        };
+        auto rescale = [&](uint32_t c) {  // to window c's scales; c = n_chunks: to the rows'
+            const float* p;
+            asm volatile("ld.shared.u64 %0, [%1];" : "=l"(p) : "r"(slot + lane * 8));
+            const float was = __uint_as_float(s32(slot + 256 + lane * 4)), now = c < n_chunks ? __ldg(p + (uint64_t)c * m_rows) : 1.0f;
+            if (!__any_sync(0xFFFFFFFFu, was != now)) return;
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(slot + 256 + lane * 4), "f"(now) : "memory");
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(slot + 384 + lane * 4), "f"(was / now) : "memory");  // powers of two
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < MY_COLS; ++i) sums[i] *= __uint_as_float(s32(slot + 384 + i * 4));
+            __syncwarp();
+        };
         // sums += f * (this warp's columns of the accumulator at column `col`)
         auto add_acc = [&](uint32_t col, float f) {
             constexpr int PART = 16;
@@ -625,15 +680,15 @@ __global__ void __launch_bounds__(H_THREADS, 1)
         bool ok = true;
         float f_prev = 0.0f;
 #pragma unroll
-        for (uint32_t b = 0; b + 1 < BUFS || b == 0; ++b) copy_window(b);
-        for (uint32_t wn = 0; wn < n_windows; ++wn) {
+        for (uint32_t b = 0; b + 1 < BUFS; ++b) copy_window(b);
+        auto window = [&](uint32_t wn, auto with_scales) {
             const uint32_t buf = wn % BUFS;
             // my copies of this window have landed; meet the quarter's other warps, which also means that all four are
             // through with the window before: its buffer takes a later one.  A warp whose wait ran out keeps coming
             // here, so that no other waits for it.
-            asm volatile("cp.async.wait_group %0;" ::"n"(BUFS > 1 ? BUFS - 2 : 0) : "memory");
+            asm volatile("cp.async.wait_group %0;" ::"n"(BUFS - 2) : "memory");
             asm volatile("bar.sync %0, 128;" ::"r"(2 + q) : "memory");
-            if constexpr (BUFS > 1) copy_window(wn + BUFS - 1);
+            copy_window(wn + BUFS - 1);
 #pragma unroll 1
             for (uint32_t cc = 0; cc < T::UNITS && ok; ++cc) {
                 const uint32_t c = wn * T::UNITS + cc;
@@ -661,18 +716,25 @@ __global__ void __launch_bounds__(H_THREADS, 1)
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&full[st]);
                 // read back the window before this one while this one accumulates
-                if (c > 0) ok = drain(c - 1, f_prev);
+                if (c > 0) {
+                    if constexpr (with_scales.value) rescale(c - 1);
+                    ok = drain(c - 1, f_prev);
+                } else {
+                    pdl_wait();  // the scales, and dst, belong to the kernels before this one
+                    find_scales();
+                }
                 f_prev = rw.f;
             }
-            if constexpr (BUFS == 1) {  // one buffer: everyone must be through with it before it is refilled
-                asm volatile("bar.sync %0, 128;" ::"r"(2 + q) : "memory");
-                copy_window(wn + 1);
-            }
-        }
+        };
+        uint32_t wn = 0;
+        for (; wn < n_windows && !scaled; ++wn) window(wn, std::false_type{});  // the first window tells
+        for (; wn < n_windows; ++wn) window(wn, std::true_type{});
+        if (scaled) rescale(n_chunks - 1);
         if (ok && n_chunks > 0) ok = drain(n_chunks - 1, f_prev);
+        if (scaled) rescale(n_chunks);
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         if (!ok) abort_flag = 1;
-        pdl_wait();  // inv and dst belong to the kernels before this one
+        pdl_wait();  // (a warp that gave up in its first window)
         if (!S::FINE && split == 1) {
             const uint64_t out_row = row0 + q * 32 + lane;
             if (ok && out_row < n) {
@@ -680,7 +742,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
                 for (int c = 0; c < MY_COLS; ++c) {
                     const uint64_t tok = tok0 + g * MY_COLS + c;
                     if (tok < m) {
-                        const float v = sums[c] * __ldg(inv + tok);
+                        const float v = sums[c] * fabsf(__ldg(inv + tok));
                         dst[tok * n + out_row] = residual ? residual[tok * n + out_row] + v : v;
                     }
                 }
@@ -694,15 +756,36 @@ __global__ void __launch_bounds__(H_THREADS, 1)
 #pragma unroll
             for (int c = 0; c < MY_COLS; ++c) red[(g * MY_COLS + c) * HM + q * 32 + lane] = sums[c];
         }
-    } else if (warp < H_CONV + H_ISSUE) {
+    } else {
         // ── issuers (their waits sleep: polling warps take issue slots from the converters) ──
         constexpr uint32_t idesc = h_idesc(N_TILE);
         const uint32_t base0 = smem_u32(smem);
         const uint64_t d0_hi = umma_desc(base0), d0_lo = umma_desc(base0 + PLANE_B);
         [[maybe_unused]] const uint64_t d_sums = umma_desc(smem_u32(s_sums));
         bool ok = true;
+        // the activation tiles of window c's step g, once the products that read the stage last are through
+        auto load = [&](uint32_t c, uint32_t g) -> bool {
+            const uint32_t ph = c % S::WINDOWS, st = ph * H_STEPS + g;
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait(&empty[st], ((c / S::WINDOWS) & 1) ^ 1))) return false;
+            if (lane == 0) {
+                uint8_t* tile = smem + (size_t)st * STAGE;
+                const uint32_t col = (win0 * T::UNITS + c) * 256 + 64 * g;
+                const bool with_sums = T::MIN && g == H_STEPS - 1;
+                mbar_arrive_expect_tx(&full[st], (with_sums ? 3 : 2) * PLANE_B);
+                tma_load_2d(tile, &map_hi, col, (uint32_t)tok0, &full[st]);
+                tma_load_2d(tile + PLANE_B, &map_lo, col, (uint32_t)tok0, &full[st]);
+                if (with_sums)
+                    tma_load_2d(s_sums + ph * PLANE_B, &map_sums, ((win0 + c) >> 1) * 64, (uint32_t)tok0, &full[st]);
+            }
+            __syncwarp();
+            return true;
+        };
         // steps G0 .. G1 - 1 of every window; compile-time, so that the descriptors need no arithmetic but a stage's offset
         auto issue = [&](auto G0, auto G1) {
+            if (S::FINE) {
+                pdl_wait();
+                for (uint32_t c = 0; c < S::WINDOWS && c < n_chunks && ok; ++c) ok = load(c, G0.value);
+            }
             for (uint32_t c = 0; c < n_chunks && ok; ++c) {
                 const uint32_t ph = c % S::WINDOWS;
 #pragma unroll
@@ -744,6 +827,8 @@ __global__ void __launch_bounds__(H_THREADS, 1)
                     }
                     __syncwarp();
                 }
+                // the next window's tiles: its stage's last products are a window behind, or (one window) the ones above
+                if (S::FINE && ok && c + 1 >= S::WINDOWS && c + 1 < n_chunks) ok = load(c + 1, G0.value);
             }
         };
         using std::integral_constant;
@@ -755,32 +840,12 @@ __global__ void __launch_bounds__(H_THREADS, 1)
             else issue(integral_constant<uint32_t, 3>{}, integral_constant<uint32_t, 4>{});
         } else if (mine == 0) {
             issue(integral_constant<uint32_t, 0>{}, integral_constant<uint32_t, H_STEPS>{});
+        } else if (mine == 1) {
+            pdl_wait();
+            for (uint32_t c = 0; c < n_chunks && ok; ++c)
+                for (uint32_t g = 0; g < H_STEPS && ok; ++g) ok = load(c, g);
         }
         if (!ok && lane == 0) abort_flag = 1;
-    } else {
-        // ── activation tiles: one lane keeps the ring of TMA copies full ──
-        if (lane == 0) {
-            pdl_wait();
-            bool ok = true;
-            for (uint32_t c = 0; c < n_chunks && ok; ++c) {
-                const uint32_t col = (win0 * T::UNITS + c) * 256;
-                const uint32_t ph = c % S::WINDOWS;
-                for (uint32_t g = 0; g < H_STEPS; ++g) {
-                    const uint32_t st = ph * H_STEPS + g;
-                    ok = mbar_wait(&empty[st], ((c / S::WINDOWS) & 1) ^ 1);
-                    if (!ok) break;
-                    uint8_t* tile = smem + (size_t)st * STAGE;
-                    const bool with_sums = T::MIN && g == H_STEPS - 1;
-                    mbar_arrive_expect_tx(&full[st], (with_sums ? 3 : 2) * PLANE_B);
-                    tma_load_2d(tile, &map_hi, col + 64 * g, (uint32_t)tok0, &full[st]);
-                    tma_load_2d(tile + PLANE_B, &map_lo, col + 64 * g, (uint32_t)tok0, &full[st]);
-                    if (with_sums)
-                        tma_load_2d(s_sums + ph * PLANE_B, &map_sums, ((win0 + c) >> 1) * 64, (uint32_t)tok0, &full[st]);
-                }
-            }
-            if (!ok) abort_flag = 1;
-        }
-        __syncwarp();
     }
     tc_fence_before();
     __syncthreads();
@@ -801,7 +866,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
                         const uint32_t addr = red + ((p * N_TILE + t) * HM + row) * 4;
                         v += split > 1 ? ld_cluster_f32(addr, r) : __uint_as_float(s32(addr));
                     }
-                v *= __ldg(inv + tok);
+                v *= fabsf(__ldg(inv + tok));
                 dst[at] = residual ? residual[at] + v : v;
             }
         }
@@ -837,7 +902,7 @@ cudaError_t f16_map(const __half* base, uint64_t rows, uint64_t cols, uint32_t n
 
 struct SplitX {  // the split activations inside the caller's scratch
     __half *hi, *lo, *sums;
-    float* inv;
+    float *inv, *rel;
 };
 uint64_t up128(uint64_t v) { return (v + 127) & ~(uint64_t)127; }
 SplitX split_in(void* scratch, uint64_t m, uint64_t k) {
@@ -850,6 +915,8 @@ SplitX split_in(void* scratch, uint64_t m, uint64_t k) {
     x.sums = reinterpret_cast<__half*>(b);
     b += up128(m * k / 4);
     x.inv = reinterpret_cast<float*>(b);
+    b += up128(4 * m);
+    x.rel = reinterpret_cast<float*>(b);
     return x;
 }
 
@@ -912,7 +979,7 @@ cudaError_t launch_f16_tile(const F16Launch& l, cudaStream_t s) {
             cfg.numAttrs = 2;
         }
     }
-    e = cudaLaunchKernelEx(&cfg, kern, l.w_a, l.n, l.k, hi, lo, sums, (const float*)l.x.inv, l.rows, l.dst_a, l.residual, l.error_flag,
+    e = cudaLaunchKernelEx(&cfg, kern, l.w_a, l.n, l.k, hi, lo, sums, (const float*)l.x.inv, (const float*)l.x.rel, l.rows, l.dst_a, l.residual, l.error_flag,
                            l.tiles, l.n_tiles, l.expert_bytes, l.w_b, l.dst_b, split);
     return e != cudaSuccess ? e : cudaGetLastError();
 }
@@ -935,7 +1002,7 @@ cudaError_t launch_f16_typed(uint32_t type, const F16Launch& l, cudaStream_t s) 
 cudaError_t split_activations_f16(uint32_t type, const float* x, uint64_t m, uint64_t k, const float* norm_w, float eps, const SplitX& o,
                                   cudaStream_t s) {
     return launch_pdl(split_f16_kernel, dim3((unsigned)m), 256, 0, s, x, (uint32_t)k, norm_w, eps,
-                      type == T_MXFP4 ? 1 : 0, o.hi, o.lo, o.sums, o.inv);
+                      type == T_MXFP4 ? 1 : 0, o.hi, o.lo, o.sums, o.inv, o.rel);
 }
 
 }  // namespace
@@ -960,7 +1027,7 @@ bool gemm_f16_supports(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, 
 }
 
 size_t gemm_f16_scratch_bytes(uint64_t m, uint64_t k) {
-    return (size_t)(2 * up128(2 * m * k) + up128(m * k / 4) + up128(4 * m));
+    return (size_t)(2 * up128(2 * m * k) + up128(m * k / 4) + up128(4 * m) + up128(m * k / 64));
 }
 
 // dst_a = residual + norm(lhs) . W^T; with w_b the same rows through a second tensor into dst_b.

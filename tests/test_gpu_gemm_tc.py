@@ -127,6 +127,28 @@ def test_scales_and_rows_at_the_edges(type_id, mkn, kind, tc_ctx):
     assert np.all(np.abs(got - want)[inside] <= 7e-6 * size[inside] + 1e-42)
 
 
+@pytest.mark.parametrize("type_id", [synth.Q4_K, synth.Q2_K, synth.Q8_0, synth.IQ2_XXS, synth.MXFP4, synth.Q6_K])
+@pytest.mark.parametrize("m,n", [(9, 130), (20, 70), (33, 300), (70, 129)])
+@pytest.mark.parametrize("outlier", [1e3, 1e6])
+def test_one_large_value_costs_the_others_no_bits(type_id, m, n, outlier):
+    """Rows of N(0, 1) with one value far above the rest, whose weights are zeros: nothing of it is in the result, all of it
+    is in the activations' scale.  The split keeps 2^-39 of the largest value of the same 256 columns, 2e-6 here, for
+    those columns alone; a window's sum is at most 48 additions that truncate in the last of 24 places, half of it on
+    average: 48 * 2^-24 = 3e-6 of the result's 2-norm.  Types with blocks of 32 columns have other weights beside the zeros."""
+    k = 4096
+    if type_id == synth.Q8_0:
+        m = max(m, 17)   # below, the type runs on the decode kernel
+    elems, nbytes = synth.BLOCK[type_id]
+    raw = synth.random_weight(type_id, n, k, seed=n).reshape(n, k // elems, nbytes).copy()
+    raw[:, 1024 // elems] = 0
+    raw = raw.reshape(-1)
+    lhs = np.random.default_rng(m).standard_normal((m, k)).astype(np.float32)
+    lhs[:, 1030] = outlier
+    got = QTensor.from_bytes(type_id, raw).matmul_t((m, k, n), lhs).astype(np.float64)
+    want = lhs.astype(np.float64) @ oracle.dequantize(type_id, raw).reshape(n, k).astype(np.float64).T
+    assert np.linalg.norm(got - want) <= 3e-6 * np.linalg.norm(want)
+
+
 @pytest.mark.parametrize("m", [5, 8, 9, 40])
 def test_a_stream_under_capture_without_scratch_takes_the_older_route(m):
     """The tile GEMM needs scratch; a capture on a stream that has none yet must not allocate, so the decode kernel runs
