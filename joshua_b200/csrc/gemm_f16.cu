@@ -11,6 +11,11 @@
 //   Q8_0         2^p * (code * d_block / 2^p)   18 bits: two terms, the second by an exact fused multiply-subtract
 //   Q6_K         d  * (scale * code)            13 bits: two terms
 //
+// f16 has 40 powers of two.  What lies further apart than that inside one factor (MXFP4 blocks 2^-35 below the largest
+// beside them, Q8_0 blocks 2^-22 below it, a dmin 2^28 times d or 2^-9 of it) would lose bits: such a block, or such a
+// window of the K formats, is converted as zeros, and the CTA that met one adds its f32 weights' products at the end on
+// the CUDA cores (`add_lost`).  Weights of one layer do not differ that much; the check rides in branches not taken.
+//
 // The activations are split once per launch (`split_f16_kernel`): a row is scaled by a power of two that puts its largest
 // value just below 2^15, hi = f16(x), lo = f16(x - hi): 22 to 24 bits of every value within 2^17 of the largest one, an
 // absolute error below 2^-39 of it otherwise.  A window whose own largest value lies more than 2^8 below the row's (an
@@ -81,32 +86,32 @@ struct HT;  // UNIT: bytes of 256 columns of a row; UNITS: windows staged togeth
 template <>
 struct HT<T_Q4_K> {
     static constexpr uint32_t UNIT = 144, UNITS = 1, VEC = 16;
-    static constexpr bool TWO = false, MIN = true;
+    static constexpr bool TWO = false, MIN = true, LOSES = true;
 };
 template <>
 struct HT<T_Q2_K> {
     static constexpr uint32_t UNIT = 84, UNITS = 1, VEC = 4;
-    static constexpr bool TWO = false, MIN = true;
+    static constexpr bool TWO = false, MIN = true, LOSES = true;
 };
 template <>
 struct HT<T_IQ2_XXS> {
     static constexpr uint32_t UNIT = 66, UNITS = 2, VEC = 4;
-    static constexpr bool TWO = false, MIN = false;
+    static constexpr bool TWO = false, MIN = false, LOSES = false;
 };
 template <>
 struct HT<T_MXFP4> {
     static constexpr uint32_t UNIT = 136, UNITS = 1, VEC = 8;
-    static constexpr bool TWO = false, MIN = false;
+    static constexpr bool TWO = false, MIN = false, LOSES = true;
 };
 template <>
 struct HT<T_Q8_0> {
     static constexpr uint32_t UNIT = 272, UNITS = 1, VEC = 8;
-    static constexpr bool TWO = true, MIN = false;
+    static constexpr bool TWO = true, MIN = false, LOSES = true;
 };
 template <>
 struct HT<T_Q6_K> {
     static constexpr uint32_t UNIT = 210, UNITS = 2, VEC = 4;
-    static constexpr bool TWO = true, MIN = false;
+    static constexpr bool TWO = true, MIN = false, LOSES = false;
 };
 // Row stride of the staged bytes in words.  Rows copied by the word: odd, so that 32 lanes reading the same word of their
 // rows hit 32 banks.  Q4_K rows are read as 16-byte vectors, which 36 words spread over the banks; rows copied by
@@ -121,6 +126,7 @@ constexpr uint32_t raw_stride() {
 template <uint32_t TYPE, int N_TILE>
 struct Tile {
     static constexpr bool FINE = N_TILE <= 32;
+    static constexpr int NB = FINE ? 2 : 8;  // blocks of 32 columns behind one accumulator
     static constexpr uint32_t WINDOWS = N_TILE <= 32 && !HT<TYPE>::TWO ? 2 : 1;
     static constexpr uint32_t STAGES = H_STEPS * WINDOWS;
     static constexpr uint32_t ACCS = FINE ? H_STEPS : 2;
@@ -317,52 +323,85 @@ struct RowWin {
     float f;       // result = f * accumulator
     float aux;     // Q4_K / Q2_K: scale of the codes (a power of two); Q8_0: 1 / f; MXFP4: e_max
     float d, dmin; // Q4_K / Q2_K
+    bool lost;     // Q4_K / Q2_K: the window is converted as zeros
 };
 
 // The codes' factor f = d 2^e.  Usually e = 0; where dmin is 32 times d or more the codes are scaled down by 2^-e
 // (exact, f16 has subnormals down to 2^-24) so that the minima stay inside f16: |2^5 dmin / f * m| <= 1024 * 63.
+// Below 2^-9 of d the minima's second terms would end in f16's subnormals, above 2^28 the codes.
 __device__ __forceinline__ RowWin min_factors(uint32_t dd) {
-    const float d = f16_bits_to_f32(dd & 0xFFFF), dmin = f16_bits_to_f32(dd >> 16);
-    if (!(fabsf(dmin) >= 32.0f * fabsf(d)) || dmin == 0.0f) return {d, 1.0f, d, dmin};
-    if (d == 0.0f) return {dmin * (1.0f / 16.0f), 0.0f, d, dmin};
-    const float ratio = fabsf(dmin) / fabsf(d);
-    const int e = (int)(__float_as_uint(ratio) >> 23) - 127 - 4;
-    return {d * pow2_f32(min(e, 100)), e <= 24 ? pow2_f32(-e) : 0.0f, d, dmin};
+    const float d = f16_bits_to_f32(dd & 0xFFFF), dmin = f16_bits_to_f32(dd >> 16), ad = fabsf(d), am = fabsf(dmin);
+    if (dmin == 0.0f || !(am >= 32.0f * ad || am < ad * (1.0f / 512.0f)) || ad > 65504.0f) return {d, 1.0f, d, dmin, false};
+    if (d == 0.0f) return {dmin * (1.0f / 16.0f), 0.0f, d, dmin, false};
+    const int e = (int)(__float_as_uint(am / ad) >> 23) - 127 - 4;
+    if (e < 0 || e > 24) return {d, 0.0f, d, 0.0f, true};
+    return {d * pow2_f32(e), pow2_f32(-e), d, dmin, false};
 }
+// Q8_0: the largest |d| / f lies in [128, 256), codes times it stay below 2^15.  mx: the largest |d|'s bits
+__device__ __forceinline__ int q8_power(uint32_t mx) {
+    return mx == 0 ? 0 : (int)(__float_as_uint(f16_bits_to_f32(mx)) >> 23) - 127 - 7;
+}
+__device__ __forceinline__ bool q8_lost(float ratio) { return ratio != 0.0f && fabsf(ratio) < 6.103515625e-5f; }  // |d| / f < 2^-14
+// MXFP4: 2^(e - e_max + 12) is the unit, half of it the smallest value.
+__device__ __forceinline__ bool mxfp4_lost(uint32_t e, uint32_t mx) { return e + 35 < mx; }
 
-template <uint32_t TYPE>
-__device__ __forceinline__ RowWin row_window(uint32_t u) {  // u: shared address of the row's 256 columns
+// NB blocks of 32 columns have one factor (MXFP4, Q8_0): eight, or the two of a step with its own accumulator.
+// u: shared address of the row's 256 columns, b0: the first of the blocks.
+template <uint32_t TYPE, int NB>
+__device__ __forceinline__ RowWin row_window(uint32_t u, uint32_t b0) {
     if constexpr (TYPE == T_Q4_K) {
         return min_factors(s32(u));
     } else if constexpr (TYPE == T_Q2_K) {
         return min_factors(s32(u + 80));
     } else if constexpr (TYPE == T_IQ2_XXS) {
-        return {f16_bits_to_f32(s16(u)) * 0.125f, 0.0f, 0.0f, 0.0f};
+        return {f16_bits_to_f32(s16(u)) * 0.125f, 0.0f, 0.0f, 0.0f, false};
     } else if constexpr (TYPE == T_Q6_K) {
-        return {f16_bits_to_f32(s16(u + 208)), 0.0f, 0.0f, 0.0f};
+        return {f16_bits_to_f32(s16(u + 208)), 0.0f, 0.0f, 0.0f, false};
     } else if constexpr (TYPE == T_Q8_0) {
         uint32_t mx = 0;
 #pragma unroll
-        for (int b = 0; b < 8; ++b) mx = max(mx, s16(u + 34 * b) & 0x7FFFu);
-        // the largest |d| / f lies in [128, 256): codes times it stay below 2^15
-        const float amax = f16_bits_to_f32(mx);
-        const int p = mx == 0 ? 0 : (int)(__float_as_uint(amax) >> 23) - 127 - 7;
-        return {pow2_f32(p), pow2_f32(-p), 0.0f, 0.0f};
+        for (int b = 0; b < NB; ++b) mx = max(mx, s16(u + 34 * (b0 + b)) & 0x7FFFu);
+        const int p = q8_power(mx);
+        return {pow2_f32(p), pow2_f32(-p), 0.0f, 0.0f, false};
     } else {
         uint32_t mx = 0;
 #pragma unroll
-        for (int b = 0; b < 8; ++b) {
-            const uint32_t e = s8(u + 17 * b);
+        for (int b = 0; b < NB; ++b) {
+            const uint32_t e = s8(u + 17 * (b0 + b));
             mx = max(mx, e == 255u ? 0u : e);
         }
-        return {pow2_f32((int)mx - 139), (float)mx, 0.0f, 0.0f};
+        return {pow2_f32((int)mx - 139), (float)mx, 0.0f, 0.0f, false};
+    }
+}
+// Whether row_window / convert64 leave block b of a row's window, in global memory, to add_lost.
+template <uint32_t TYPE, int NB>
+__device__ bool block_lost(const uint8_t* win, uint32_t b) {
+    const uint32_t b0 = b / NB * NB;
+    if constexpr (TYPE == T_Q4_K || TYPE == T_Q2_K) {
+        return min_factors(ld_u32(win + (TYPE == T_Q4_K ? 0 : 80))).lost;
+    } else if constexpr (TYPE == T_Q8_0) {
+        uint32_t mx = 0;
+#pragma unroll 1
+        for (uint32_t i = b0; i < b0 + NB; ++i) mx = max(mx, ld_u16(win + 34 * i) & 0x7FFFu);
+        return q8_lost(f16_bits_to_f32(ld_u16(win + 34 * b)) * pow2_f32(-q8_power(mx)));
+    } else {
+        uint32_t mx = 0;
+#pragma unroll 1
+        for (uint32_t i = b0; i < b0 + NB; ++i) {
+            const uint32_t e = ld_u8(win + 17 * i);
+            mx = max(mx, e == 255u ? 0u : e);
+        }
+        return mxfp4_lost(ld_u8(win + 17 * b), mx);
     }
 }
 
 // Columns 64 g .. 64 g + 63 of the window: h = 0, 1 are its two groups of 32; put(h, a, b) takes 16 packed first terms
-// and (two-term types) 16 second terms.
+// and (two-term types) 16 second terms.  *lost (shared memory) is set where a block was converted as zeros.
 template <uint32_t TYPE, class Put>
-__device__ __forceinline__ void convert64(uint32_t u, uint32_t g, const RowWin& rw, const uint2* s_grid, Put put) {
+__device__ __forceinline__ void convert64(uint32_t u, uint32_t g, const RowWin& rw, const uint2* s_grid, volatile int* lost, Put put) {
+    if constexpr (TYPE == T_Q4_K || TYPE == T_Q2_K) {
+        if (rw.lost) *lost = 1;
+    }
     if constexpr (TYPE == T_Q4_K) {
         const uint4 hd = s128(u), v0 = s128(u + 16 + 32 * g), v1 = s128(u + 32 + 32 * g);
         const uint32_t w[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
@@ -435,8 +474,9 @@ __device__ __forceinline__ void convert64(uint32_t u, uint32_t g, const RowWin& 
             const uint32_t blk = u + 17 * (2 * g + h), e = s8(blk);
             uint32_t w[4];
             s_words<4>(blk + 1, w);
-            const int ex = (int)e - (int)rw.aux + 12;  // <= 12; below 2^-24 the block is less than 2^-35 of the largest
-            const __half2 s2 = __float2half2_rn(e == 255u || ex < -24 ? 0.0f : pow2_f32(ex));
+            const bool gone = mxfp4_lost(e, (uint32_t)rw.aux);
+            const __half2 s2 = __float2half2_rn(e == 255u || gone ? 0.0f : pow2_f32((int)e - (int)rw.aux + 12));
+            if (gone && ((w[0] | w[1] | w[2] | w[3]) & 0x77777777u)) *lost = 1;  // a block of zeros has exponent 0
             uint32_t a[16];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -457,7 +497,10 @@ __device__ __forceinline__ void convert64(uint32_t u, uint32_t g, const RowWin& 
 #pragma unroll
         for (uint32_t h = 0; h < 2; ++h) {
             const uint32_t blk = u + 34 * (2 * g + h);
-            const __half2 r2 = __float2half2_rn(f16_bits_to_f32(s16(blk)) * rw.aux);
+            const float r = f16_bits_to_f32(s16(blk)) * rw.aux;
+            const bool gone = q8_lost(r);
+            const __half2 r2 = __float2half2_rn(gone ? 0.0f : r);
+            if (gone) *lost = 1;
             uint32_t w[8], a[16], b[16];
             s_words<8>(blk + 2, w);
 #pragma unroll
@@ -500,6 +543,41 @@ __device__ __forceinline__ void convert64(uint32_t u, uint32_t g, const RowWin& 
     }
 }
 
+// The products that the tensor core did not form: blocks converted as zeros, their weights in f32 as the float kernels
+// decode them, times the split activations.  One warp: its lanes' rows, n_chunks windows from win0 on, steps S0 .. S1 - 1 of
+// each, tokens tok0 .. tok0 + n_tok - 1; add(t, v) takes token t's share in units of the row's scale.  Inlined and rolled
+// up: as a call it cost the kernel seven per cent where it never ran (Q4_K 28672 x 4096, 8 rows 53.5 us instead of 50.4).
+template <uint32_t TYPE, int NB, class Add>
+__device__ __forceinline__ void add_lost(const uint8_t* row, uint32_t win0, uint32_t n_chunks, uint32_t S0, uint32_t S1, uint64_t k,
+                                      const __half* __restrict__ x_hi, const __half* __restrict__ x_lo,
+                                      const float* __restrict__ rel, uint64_t m_rows, uint64_t tok0, uint32_t n_tok, Add add) {
+#pragma unroll 1
+    for (uint32_t c = win0; c < win0 + n_chunks; ++c) {
+        const uint8_t* win = row + (uint64_t)c * HT<TYPE>::UNIT;
+#pragma unroll 1
+        for (uint32_t b = 2 * S0; b < 2 * S1; ++b) {
+            const bool mine = block_lost<TYPE, NB>(win, b);
+            if (!__any_sync(0xFFFFFFFFu, mine)) continue;
+#pragma unroll 1
+            for (uint32_t u = 4 * b; u < 4 * b + 4; ++u) {
+                float w[8];
+                decode_unit<TYPE>(win, u, w, false);
+#pragma unroll 1
+                for (uint32_t t = 0; t < n_tok; ++t) {
+                    const uint64_t at = (tok0 + t) * k + (uint64_t)c * 256 + u * 8;
+                    float v = 0.0f;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const int o = TYPE == T_MXFP4 ? j : (j & 4) | ((j & 1) << 1) | ((j >> 1) & 1);  // 0, 2, 1, 3
+                        v = fmaf(w[j], __half2float(x_hi[at + o]) + __half2float(x_lo[at + o]), v);
+                    }
+                    if (mine) add(t, v * rel[c * m_rows + tok0 + t]);
+                }
+            }
+        }
+    }
+}
+
 // The window's 16 minima, -2^5 (dmin / f) m, as eight packed first and eight packed second terms.  The ratio is two f16
 // terms, m at most six bits: the first products' remainders are exact.
 template <uint32_t TYPE>
@@ -526,7 +604,8 @@ template <uint32_t TYPE, int N_TILE>
 __global__ void __launch_bounds__(H_THREADS, 1)
     gemm_f16_kernel(const uint8_t* __restrict__ w_a, uint64_t n, uint64_t k, const __grid_constant__ CUtensorMap map_hi,
                     const __grid_constant__ CUtensorMap map_lo, const __grid_constant__ CUtensorMap map_sums,
-                    const float* __restrict__ inv, const float* __restrict__ rel, uint64_t m_rows, float* dst_a, const float* residual, int* __restrict__ error_flag,
+                    const float* __restrict__ inv, const float* __restrict__ rel, const __half* __restrict__ x_hi,
+                    const __half* __restrict__ x_lo, uint64_t m_rows, float* dst_a, const float* residual, int* __restrict__ error_flag,
                     const GemmTile* __restrict__ tiles, const uint32_t* __restrict__ n_tiles, uint64_t expert_bytes,
                     const uint8_t* __restrict__ w_b, float* dst_b, uint32_t split) {
     using T = HT<TYPE>;
@@ -544,7 +623,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
     // full[s]: the step's four converter warps + the TMA thread (and the tiles' bytes); empty[s]: the MMAs' commit
     __shared__ uint64_t full[S::STAGES], empty[S::STAGES], acc_full[2], acc_empty[S::ACCS];
     __shared__ uint32_t tmem_base_slot;
-    __shared__ int abort_flag;
+    __shared__ int abort_flag, lost_flag;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     pdl_trigger();
@@ -580,7 +659,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
             if (!S::FINE) mbar_init(&acc_full[b & 1], 1);
             mbar_init(&acc_empty[b], S::FINE ? 4 : H_CONV);
         }
-        abort_flag = 0;
+        abort_flag = lost_flag = 0;
         mbar_fence_init();
     }
     if (warp == H_CONV) {
@@ -693,14 +772,14 @@ __global__ void __launch_bounds__(H_THREADS, 1)
             for (uint32_t cc = 0; cc < T::UNITS && ok; ++cc) {
                 const uint32_t c = wn * T::UNITS + cc;
                 const uint32_t u = raw_q + buf * RAW_BUF + lane * RAW_STRIDE * 4 + cc * T::UNIT;
-                const RowWin rw = row_window<TYPE>(u);
+                const RowWin rw = row_window<TYPE, S::NB>(u, S::FINE ? 2 * g : 0);
                 // the stage's columns must have been read by the MMAs that used them last
                 const uint32_t ph = c % S::WINDOWS, st = ph * H_STEPS + g;
                 ok = __all_sync(0xFFFFFFFFu, mbar_wait_polling(&empty[st], ((c / S::WINDOWS) & 1) ^ 1));
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t acol = tmem_d + lane_base + S::ACC_COLS + st * S::A_COLS;
-                convert64<TYPE>(u, g, rw, s_grid, [&](uint32_t h, const uint32_t (&a)[16], const uint32_t (&b)[16]) {
+                convert64<TYPE>(u, g, rw, s_grid, &lost_flag, [&](uint32_t h, const uint32_t (&a)[16], const uint32_t (&b)[16]) {
                     tmem_st16(acol + 16 * h, a);
                     if constexpr (T::TWO) tmem_st16(acol + 32 + 16 * h, b);
                 });
@@ -735,8 +814,12 @@ __global__ void __launch_bounds__(H_THREADS, 1)
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         if (!ok) abort_flag = 1;
         pdl_wait();  // (a warp that gave up in its first window)
+        // The ring and the staged bytes are idle once every converter is here: the last read-back waited for this CTA's
+        // last products.
+        asm volatile("bar.sync 1, %0;" ::"n"(H_CONV * 32) : "memory");
+        const uint64_t out_row = row0 + q * 32 + lane, first_tok = tok0 + (S::FINE ? 0 : g * MY_COLS);
+        float* red = reinterpret_cast<float*>(smem);
         if (!S::FINE && split == 1) {
-            const uint64_t out_row = row0 + q * 32 + lane;
             if (ok && out_row < n) {
 #pragma unroll
                 for (int c = 0; c < MY_COLS; ++c) {
@@ -749,12 +832,21 @@ __global__ void __launch_bounds__(H_THREADS, 1)
             }
         } else {
             // leave the partial tile in shared memory, [token][row] (four of them where the warps of a quarter hold sums
-            // of their own steps).  The ring and the staged bytes are idle once every converter is here: the last
-            // read-back waited for this CTA's last products.
-            asm volatile("bar.sync 1, %0;" ::"n"(H_CONV * 32) : "memory");
-            float* red = reinterpret_cast<float*>(smem);
+            // of their own steps)
 #pragma unroll
             for (int c = 0; c < MY_COLS; ++c) red[(g * MY_COLS + c) * HM + q * 32 + lane] = sums[c];
+        }
+        if constexpr (T::LOSES) {
+            if (lost_flag && ok && first_tok < m) {  // each thread adds to what it has just stored
+                add_lost<TYPE, S::NB>(w + min(out_row, n - 1) * row_bytes, win0 * T::UNITS, n_chunks, S::FINE ? g : 0,
+                                      S::FINE ? g + 1 : H_STEPS, k, x_hi, x_lo, rel, m_rows, first_tok,
+                                      (uint32_t)min((uint64_t)MY_COLS, m - first_tok), [&](uint32_t t, float v) {
+                                          if (S::FINE || split > 1)
+                                              red[(g * MY_COLS + t) * HM + q * 32 + lane] += v;
+                                          else if (out_row < n)
+                                              dst[(first_tok + t) * n + out_row] += v * fabsf(__ldg(inv + first_tok + t));
+                                      });
+            }
         }
     } else {
         // ── issuers (their waits sleep: polling warps take issue slots from the converters) ──
@@ -979,7 +1071,7 @@ cudaError_t launch_f16_tile(const F16Launch& l, cudaStream_t s) {
             cfg.numAttrs = 2;
         }
     }
-    e = cudaLaunchKernelEx(&cfg, kern, l.w_a, l.n, l.k, hi, lo, sums, (const float*)l.x.inv, (const float*)l.x.rel, l.rows, l.dst_a, l.residual, l.error_flag,
+    e = cudaLaunchKernelEx(&cfg, kern, l.w_a, l.n, l.k, hi, lo, sums, (const float*)l.x.inv, (const float*)l.x.rel, (const __half*)l.x.hi, (const __half*)l.x.lo, l.rows, l.dst_a, l.residual, l.error_flag,
                            l.tiles, l.n_tiles, l.expert_bytes, l.w_b, l.dst_b, split);
     return e != cudaSuccess ? e : cudaGetLastError();
 }

@@ -149,6 +149,50 @@ def test_one_large_value_costs_the_others_no_bits(type_id, m, n, outlier):
     assert np.linalg.norm(got - want) <= 3e-6 * np.linalg.norm(want)
 
 
+@pytest.mark.parametrize("type_id,kind", [(synth.MXFP4, "blocks"), (synth.Q8_0, "blocks"), (synth.Q4_K, "codes"), (synth.Q2_K, "codes"),
+                                          (synth.Q4_K, "minima"), (synth.Q2_K, "minima")])
+@pytest.mark.parametrize("m,n,k", [(9, 130, 1024), (20, 70, 4096), (40, 300, 1024), (70, 129, 4096), (130, 19000, 512)])
+def test_small_weights_beside_large_ones_keep_their_bits(type_id, kind, m, n, k):
+    """Scales further apart than f16 reaches inside one factor, and activations that are zero where the large ones are: the
+    result is the small ones' alone.  Blocks: the first of every window is 2^50 (MXFP4) or 2^33 (Q8_0) above the rest.
+    Codes: dmin = 2^32 d, only columns with a minimum of 0 count.  Minima: dmin = 2^-12 d, only columns with a code of 0
+    count.  Exact tiles, 128-row tiles, one and several CTAs along k.  The bound is that of the test above."""
+    elems, nbytes = synth.BLOCK[type_id]
+    if type_id == synth.Q8_0:
+        m = max(m, 17)
+    raw = synth.random_weight(type_id, n, k, seed=n).reshape(n, k // elems, nbytes).copy()
+    lhs = np.random.default_rng(m).standard_normal((m, k)).astype(np.float32)
+    cols = np.arange(k) % 256
+
+    def f16(v):
+        return np.float16(v).view(np.uint16).reshape(1).view(np.uint8)
+
+    if kind == "blocks":
+        lhs[:, cols < 32] = 0
+        if type_id == synth.MXFP4:
+            raw[:, :, 0] = 100 + raw[:, :, 0] % 8
+            raw[:, ::8, 0] = 158
+        else:
+            raw[:, :, :2] = f16(2.0 ** -20)
+            raw[:, ::8, :2] = f16(2.0 ** 13)
+    else:
+        lhs[:, cols >= 32] = 0
+        at = 0 if type_id == synth.Q4_K else 80
+        raw[:, :, at:at + 2] = f16(2.0 ** -20 if kind == "codes" else 2.0 ** 4)
+        raw[:, :, at + 2:at + 4] = f16(2.0 ** 12 if kind == "codes" else 2.0 ** -8)
+        if kind == "codes" and type_id == synth.Q4_K:
+            raw[:, :, 8] &= 0xC0
+        elif kind == "codes":
+            raw[:, :, 0:2] &= 0x0F
+        elif type_id == synth.Q4_K:
+            raw[:, :, 16:48] &= 0xF0
+        else:
+            raw[:, :, 16:48] &= 0xFC
+    got = QTensor.from_bytes(type_id, raw.reshape(-1)).matmul_t((m, k, n), lhs).astype(np.float64)
+    want = lhs.astype(np.float64) @ oracle.dequantize(type_id, raw.reshape(-1)).reshape(n, k).astype(np.float64).T
+    assert np.linalg.norm(got - want) <= 3e-6 * np.linalg.norm(want)
+
+
 @pytest.mark.parametrize("m", [5, 8, 9, 40])
 def test_a_stream_under_capture_without_scratch_takes_the_older_route(m):
     """The tile GEMM needs scratch; a capture on a stream that has none yet must not allocate, so the decode kernel runs
