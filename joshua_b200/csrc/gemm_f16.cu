@@ -600,7 +600,8 @@ __device__ __forceinline__ void convert_minima(uint32_t u, const RowWin& rw, uin
     }
 }
 
-template <uint32_t TYPE, int N_TILE>
+// VEC: bytes a copy of raw weights, HT's or (a tensor that starts on a word boundary only) 4.
+template <uint32_t TYPE, int N_TILE, uint32_t VEC>
 __global__ void __launch_bounds__(H_THREADS, 1)
     gemm_f16_kernel(const uint8_t* __restrict__ w_a, uint64_t n, uint64_t k, const __grid_constant__ CUtensorMap map_hi,
                     const __grid_constant__ CUtensorMap map_lo, const __grid_constant__ CUtensorMap map_sums,
@@ -732,7 +733,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
         };
         // this warp's 8 of the quarter's 32 rows of window wn, as one run of vectors over the lanes
         const uint32_t raw_q = smem_u32(raw) + q * 32 * RAW_STRIDE * 4;
-        constexpr uint32_t VEC = T::VEC, ROW_VECS = WIN_WORDS * 4 / VEC, COPIES = (8 * ROW_VECS + 31) / 32;
+        constexpr uint32_t ROW_VECS = WIN_WORDS * 4 / VEC, COPIES = (8 * ROW_VECS + 31) / 32;
         const uint64_t gr0 = min(row0 + q * 32 + g * 8, n - 1);
         const uint32_t rows_left = (uint32_t)min((uint64_t)8, n - gr0);  // rows past n repeat the last one
         const uint8_t* src0 = w + gr0 * row_bytes + (uint64_t)win0 * (WIN_WORDS * 4);
@@ -1025,10 +1026,12 @@ struct F16Launch {
     int* error_flag;
 };
 
-template <uint32_t TYPE, int N_TILE>
+template <uint32_t TYPE, int N_TILE, uint32_t VEC = HT<TYPE>::VEC>
 cudaError_t launch_f16_tile(const F16Launch& l, cudaStream_t s) {
+    if constexpr (VEC == 8)
+        if ((reinterpret_cast<uintptr_t>(l.w_a) | reinterpret_cast<uintptr_t>(l.w_b)) % 8 != 0) return launch_f16_tile<TYPE, N_TILE, 4>(l, s);
     constexpr size_t smem = Tile<TYPE, N_TILE>::SMEM;
-    auto kern = gemm_f16_kernel<TYPE, N_TILE>;
+    auto kern = gemm_f16_kernel<TYPE, N_TILE, VEC>;
     static bool configured[MAX_DEVICES] = {};
     if (cudaError_t ce = set_max_smem_once(kern, 226 * 1024, configured); ce != cudaSuccess) return ce;
     CUtensorMap hi, lo, sums;
@@ -1103,14 +1106,15 @@ cudaError_t split_activations_f16(uint32_t type, const float* x, uint64_t m, uin
 // Q6_K always does (no 128-row form of it was built).
 static uint32_t tile_rows(uint32_t type, uint64_t m) { return m <= 16 ? 16 : m <= 64 || type == T_Q6_K ? 32 : 128; }
 
-// Whole staged windows in every row, made of the vectors they are copied by; the tiles of lhs fit grid.y.
+// Whole staged windows in every row, made of the vectors they are copied by (Q4_K tensors and slices always start on 16
+// bytes); the tiles of lhs fit grid.y.
 bool gemm_f16_supports(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, uint64_t m) {
     if (m == 0 || n == 0 || k == 0 || k % 256 != 0 || k > 0x7FFFFFFFu || m > 65535ull * tile_rows(type, m)) return false;
     const uintptr_t a = reinterpret_cast<uintptr_t>(w);
     switch (type) {
         case T_Q4_K: return a % 16 == 0;
         case T_Q8_0:
-        case T_MXFP4: return a % 8 == 0;
+        case T_MXFP4:
         case T_Q2_K: return a % 4 == 0;
         case T_IQ2_XXS:
         case T_Q6_K: return a % 4 == 0 && k % 512 == 0;

@@ -193,6 +193,26 @@ def test_small_weights_beside_large_ones_keep_their_bits(type_id, kind, m, n, k)
     assert np.linalg.norm(got - want) <= 3e-6 * np.linalg.norm(want)
 
 
+@pytest.mark.parametrize("type_id", [synth.Q8_0, synth.MXFP4, synth.IQ2_XXS, synth.Q6_K, synth.Q2_K])
+@pytest.mark.parametrize("m,n", [(20, 70), (70, 130), (200, 96)])
+def test_slices_that_start_on_a_word_boundary(type_id, m, n):
+    """A slice of blocks may start anywhere in its tensor: four bytes past an eight-byte boundary here, two past a word for
+    the second one (which takes the older routes).  The same blocks in a tensor of their own give the reference."""
+    k, (elems, nbytes) = 1024, synth.BLOCK[type_id]
+    count = n * (k // elems)
+    lhs = synth.random_activations(m, k, seed=m)
+    whole = synth.random_weight(type_id, n + 8, k, seed=n)
+    parent = QTensor.from_bytes(type_id, whole)
+    for want_mod in (4, 2):
+        skip = next((s for s in range(1, 33) if s * nbytes % 8 == want_mod), None)
+        if skip is None:
+            continue
+        raw = whole[skip * nbytes:(skip + count) * nbytes]
+        got = parent.slice_blocks(skip, count).matmul_t((m, k, n), lhs).astype(np.float64).reshape(m, n)
+        want = lhs.reshape(m, k).astype(np.float64) @ oracle.dequantize(type_id, raw).reshape(n, k).astype(np.float64).T
+        assert np.linalg.norm(got - want) <= 3e-6 * np.linalg.norm(want)   # the sums' bound of the tests above
+
+
 @pytest.mark.parametrize("m", [5, 8, 9, 40])
 def test_a_stream_under_capture_without_scratch_takes_the_older_route(m):
     """The tile GEMM needs scratch; a capture on a stream that has none yet must not allocate, so the decode kernel runs
