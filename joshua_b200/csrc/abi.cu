@@ -106,12 +106,15 @@ int32_t jq_matmul_device(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n,
         JQ_CUDA(jq::launch_gemv_mma(w->type, w->dev, n, k, lhs, m, dst, scratch, ctx->status_dev, s));
         return jq::OK;
     }
-    // What the f16 tiles do not take (k not a whole number of their windows).  Batches a little above the decode
-    // kernel's eight rows: eight rows at a time through the decode kernel (the weights are read once per slice, from
-    // L2 when they fit) still beats the TF32 tile GEMM, whose K loop costs the same at any batch.  Q6_K has no TF32
-    // form: any batch goes in slices, which read packed bytes at terabytes per second where the exact-decode float
-    // kernel (the other route) reaches half of one.
-    if (!ctx->force_f32 && m > jq::GEMV_MMA_MAX_M && (m <= ctx->sliced_max_m || w->type == jq::T_Q6_K) &&
+    // What the f16 tiles do not take: k not a whole number of their windows, tensors off the word boundary, 9 to 16 rows of
+    // Q8_0, a capture without scratch.  Batches a little above the decode kernel's eight rows: eight rows at a time
+    // through the decode kernel (the weights are read once per slice, from L2 when they fit) still beats the TF32 tile
+    // GEMM, whose K loop costs the same at any batch.  Types without a TF32 form, and captures that have no scratch for
+    // it, go in slices at any batch: they read packed bytes at terabytes per second where the exact-decode float kernel
+    // (the other route) reaches half of one.
+    const bool tf32 = !ctx->force_f32 && m > jq::GEMV_MMA_MAX_M && jq::gemm_tc_supports(w->type, w->dev, n, k, m) &&
+                      ctx->scratch_available(s, SLOT_TILES, jq::gemm_tc_scratch_bytes(m, k));
+    if (!ctx->force_f32 && m > jq::GEMV_MMA_MAX_M && (m <= ctx->sliced_max_m || !tf32) &&
         jq::gemv_mma_dense_supports(w->type, w->dev, n, k, jq::GEMV_MMA_MAX_M)) {
         void* scratch = nullptr;
         JQ_CUDA(ctx->scratch_for(s, SLOT_PLANES, jq::gemv_mma_scratch_bytes(jq::GEMV_MMA_MAX_M, k), &scratch));
@@ -122,7 +125,7 @@ int32_t jq_matmul_device(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n,
         }
         return jq::OK;
     }
-    if (!ctx->force_f32 && m > jq::GEMV_MMA_MAX_M && jq::gemm_tc_supports(w->type, w->dev, n, k, m)) {
+    if (tf32) {
         void* scratch = nullptr;
         JQ_CUDA(ctx->scratch_for(s, SLOT_TILES, jq::gemm_tc_scratch_bytes(m, k), &scratch));
         JQ_CUDA(jq::launch_gemm_tc(w->type, w->dev, n, k, lhs, m, dst, scratch, ctx->status_dev, s));

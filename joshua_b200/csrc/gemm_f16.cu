@@ -1082,7 +1082,9 @@ cudaError_t launch_f16_tile(const F16Launch& l, cudaStream_t s) {
 template <int N_TILE>
 cudaError_t launch_f16_typed(uint32_t type, const F16Launch& l, cudaStream_t s) {
     switch (type) {
-        case T_Q8_0: return launch_f16_tile<T_Q8_0, N_TILE>(l, s);
+        case T_Q8_0:
+            if constexpr (N_TILE > 16) return launch_f16_tile<T_Q8_0, N_TILE>(l, s);
+            return cudaErrorInvalidValue;
         case T_Q2_K: return launch_f16_tile<T_Q2_K, N_TILE>(l, s);
         case T_Q4_K: return launch_f16_tile<T_Q4_K, N_TILE>(l, s);
         case T_IQ2_XXS: return launch_f16_tile<T_IQ2_XXS, N_TILE>(l, s);
@@ -1103,8 +1105,8 @@ cudaError_t split_activations_f16(uint32_t type, const float* x, uint64_t m, uin
 }  // namespace
 
 // Rows of a tile for m rows of lhs.  Up to 64 rows the other route is the decode kernel: they stay on the exact tiles.
-// Q6_K always does (no 128-row form of it was built).
-static uint32_t tile_rows(uint32_t type, uint64_t m) { return m <= 16 ? 16 : m <= 64 || type == T_Q6_K ? 32 : 128; }
+// Q6_K always does (no 128-row form of it was built).  Q8_0 comes with 17 rows and more.
+static uint32_t tile_rows(uint32_t type, uint64_t m) { return m <= 16 && type != T_Q8_0 ? 16 : m <= 64 || type == T_Q6_K ? 32 : 128; }
 
 // Whole staged windows in every row, made of the vectors they are copied by (Q4_K tensors and slices always start on 16
 // bytes); the tiles of lhs fit grid.y.

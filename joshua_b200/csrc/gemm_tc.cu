@@ -371,8 +371,6 @@ bool gemm_tc_supports(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, u
     uintptr_t a = reinterpret_cast<uintptr_t>(w);
     // decode_unit's alignment needs hold for every row
     switch (type) {
-        case T_Q4_K: return a % 4 == 0;
-        case T_Q2_K: return a % 4 == 0;
         case T_Q8_0: return a % 2 == 0 && row_bytes % 2 == 0;
         case T_IQ2_XXS: return a % 2 == 0;
         case T_MXFP4: return true;
@@ -389,8 +387,6 @@ cudaError_t launch_gemm_tc(uint32_t type, const uint8_t* w, uint64_t n, uint64_t
     float* scratch = static_cast<float*>(scratch_v);
     switch (type) {
         case T_Q8_0: return launch_type<T_Q8_0, 32, 34>(w, n, k, lhs, m, dst, scratch, error_flag, s);
-        case T_Q2_K: return launch_type<T_Q2_K, 256, 84>(w, n, k, lhs, m, dst, scratch, error_flag, s);
-        case T_Q4_K: return launch_type<T_Q4_K, 256, 144>(w, n, k, lhs, m, dst, scratch, error_flag, s);
         case T_IQ2_XXS: return launch_type<T_IQ2_XXS, 256, 66>(w, n, k, lhs, m, dst, scratch, error_flag, s);
         case T_MXFP4: return launch_type<T_MXFP4, 32, 17>(w, n, k, lhs, m, dst, scratch, error_flag, s);
         default: return cudaErrorInvalidValue;

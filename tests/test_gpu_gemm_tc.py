@@ -193,6 +193,32 @@ def test_small_weights_beside_large_ones_keep_their_bits(type_id, kind, m, n, k)
     assert np.linalg.norm(got - want) <= 3e-6 * np.linalg.norm(want)
 
 
+# Shapes the f16 tiles leave to the older routes: rows that are no whole number of windows (Q8_0, MXFP4: 256 columns,
+# IQ2_XXS: 512) on the TF32 kernel, all its tile widths and ragged edges; Q8_0 of 9 to 16 rows and IQ2_XXS batches in slices.
+OLDER = [(t, (m, 4128, n)) for t in (synth.Q8_0, synth.MXFP4) for m, n in ((20, 130), (40, 257), (65, 130), (130, 257))] + \
+        [(synth.IQ2_XXS, (m, k, n)) for k in (768, 2304) for m, n in ((20, 130), (65, 257), (130, 130))] + \
+        [(synth.Q8_0, (m, 2048, 257)) for m in (9, 12, 16)]
+
+
+@pytest.mark.parametrize("type_id,mkn", OLDER)
+@pytest.mark.parametrize("sliced", [True, False])
+def test_routes_the_f16_tiles_leave_to_others(type_id, mkn, sliced, tc_ctx):
+    """The default context and the one without slices, against the oracle, run to run identical."""
+    m, k, n = mkn
+    raw = synth.random_weight(type_id, n, k, seed=n + k)
+    lhs = synth.random_activations(m, k, seed=m)
+    q = QTensor.from_bytes(type_id, raw) if sliced else QTensor.from_bytes(type_id, raw, tc_ctx)
+    got = q.matmul_t(mkn, lhs)
+    assert_close(got, oracle.matmul_t(type_id, mkn, lhs, raw), what=f"{synth.NAMES[type_id]} {mkn}")
+    assert np.array_equal(bits(got), bits(q.matmul_t(mkn, lhs)))
+
+
+@pytest.mark.parametrize("mkn,kind", [((17, 512, 16), "minima"), ((40, 512, 600), "signs")])
+def test_scales_at_the_edges_of_q8_0_tiles(mkn, kind, tc_ctx):
+    """As test_scales_and_rows_at_the_edges, with the row counts from which Q8_0 takes the f16 tiles."""
+    test_scales_and_rows_at_the_edges(synth.Q8_0, mkn, kind, tc_ctx)
+
+
 @pytest.mark.parametrize("type_id", [synth.Q8_0, synth.MXFP4, synth.IQ2_XXS, synth.Q6_K, synth.Q2_K])
 @pytest.mark.parametrize("m,n", [(20, 70), (70, 130), (200, 96)])
 def test_slices_that_start_on_a_word_boundary(type_id, m, n):
@@ -213,7 +239,7 @@ def test_slices_that_start_on_a_word_boundary(type_id, m, n):
         assert np.linalg.norm(got - want) <= 3e-6 * np.linalg.norm(want)   # the sums' bound of the tests above
 
 
-@pytest.mark.parametrize("m", [5, 8, 9, 40])
+@pytest.mark.parametrize("m", [5, 8, 9, 40, 100])
 def test_a_stream_under_capture_without_scratch_takes_the_older_route(m):
     """The tile GEMM needs scratch; a capture on a stream that has none yet must not allocate, so the decode kernel runs
     there (its planes fit shared memory at this k) as it did before the tiles took these batches."""
