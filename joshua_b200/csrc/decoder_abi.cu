@@ -12,18 +12,18 @@ int32_t check_vectors(const char* who, const float* lhs, const float* norm_w) {
 size_t swiglu_scratch_bytes(uint64_t m, uint64_t n) { return 2 * m * n * 4 + 512; }
 bool pair_uses_tiles(const jq_weight* gate, const jq_weight* up, uint64_t m, uint64_t k, uint64_t n, cudaStream_t s) {
     return jq_uses_tiles(gate, m, k, n, s) && jq_uses_tiles(up, m, k, n, s) &&
-           gate->ctx->scratch_available(s, SLOT_PAIR, swiglu_scratch_bytes(m, n));
+           gate->ctx->scratch_available(s, SLOT_PAIR, m * n * 4);
 }
 
-// silu(clamp(gate x)) * clamp(up x) on the tile GEMM: one launch for both tensors into scratch, then the combine.
+// silu(clamp(gate x)) * clamp(up x) on the tile GEMM: one launch for both tensors, gate into dst and up into scratch (which
+// stays with the stream: a prompt's up products, not both), then the combine.  lhs is split before dst is written.
 int32_t swiglu_tiles(const jq_weight* gate, const jq_weight* up, uint64_t m, uint64_t k, uint64_t n, const float* lhs,
                      const float* norm_w, float eps, float* dst, float clamp, cudaStream_t s) {
     void* scratch = nullptr;
-    JQ_CUDA(gate->ctx->scratch_for(s, SLOT_PAIR, swiglu_scratch_bytes(m, n), &scratch));
-    float* g = static_cast<float*>(scratch);
-    float* u = g + ((m * n + 63) & ~(uint64_t)63);
-    if (int32_t rc = jq_matmul_tiles(gate, up, m, k, n, lhs, norm_w, eps, nullptr, g, u, s)) return rc;
-    JQ_CUDA(jq::launch_swiglu(g, u, m * n, clamp, dst, s));
+    JQ_CUDA(gate->ctx->scratch_for(s, SLOT_PAIR, m * n * 4, &scratch));
+    float* u = static_cast<float*>(scratch);
+    if (int32_t rc = jq_matmul_tiles(gate, up, m, k, n, lhs, norm_w, eps, nullptr, dst, u, s)) return rc;
+    JQ_CUDA(jq::launch_swiglu(dst, u, m * n, clamp, dst, s));
     return jq::OK;
 }
 

@@ -658,8 +658,8 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restric
 
 // out = silu(clamp(g)) * clamp(u), element-wise (the dense shared-expert path at batches the grouped kernel
 // does not take)
-__global__ void __launch_bounds__(256) swiglu_kernel(const float* __restrict__ g, const float* __restrict__ u,
-                                                     uint64_t n, float clamp, float* __restrict__ out) {
+// out may be g
+__global__ void __launch_bounds__(256) swiglu_kernel(const float* g, const float* __restrict__ u, uint64_t n, float clamp, float* out) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {

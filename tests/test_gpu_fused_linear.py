@@ -103,3 +103,32 @@ def test_bad_buffers_are_refused_before_a_launch(type_id, m):
     assert norm(X, N, R) == 0 and pair(X, N) == 0
     torch.cuda.synchronize()
     assert torch.equal(out, torch.zeros_like(out))
+
+
+@pytest.mark.parametrize("m", [16, 700])
+def test_pair_on_tiles_with_its_output_over_its_input(m):
+    """From five rows on the gate product goes to dst and the up product to scratch: dst may be lhs (k = n), and the scratch
+    that stays with the context holds m * n values beside the split activations, not twice that."""
+    import torch
+
+    from joshua_b200 import _lib
+    from joshua_b200.qtensor import Context, QTensor
+
+    L, n, ctx = _lib.lib(), 4096, Context(0)
+    gate, up = (QTensor.from_bytes(synth.Q4_K, synth.random_weight(synth.Q4_K, n, n, seed), ctx) for seed in (1, 2))
+    x = torch.randn(m, n, device="cuda", generator=torch.Generator(device="cuda").manual_seed(m))
+    s = torch.cuda.current_stream().cuda_stream
+    g, u, want = torch.empty_like(x), torch.empty_like(x), torch.empty_like(x)
+    _lib.check(L.jq_matmul_t_dev(gate._h, m, n, n, x.data_ptr(), g.data_ptr(), s))
+    _lib.check(L.jq_matmul_t_dev(up._h, m, n, n, x.data_ptr(), u.data_ptr(), s))
+    _lib.check(L.jq_swiglu_dev(g.data_ptr(), u.data_ptr(), m * n, 0.0, want.data_ptr(), s))
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    _lib.check(L.jq_matmul_swiglu_dev(gate._h, up._h, m, n, n, x.data_ptr(), x.data_ptr(), 0.0, s))
+    torch.cuda.synchronize()
+    # one launch for both tensors may cut k into other pieces: products differ by 3e-6 of their 2-norm, six times that at
+    # most for one value; silu's slope is below 1.1
+    dg, du = 2e-5 * g.square().mean().sqrt(), 2e-5 * u.square().mean().sqrt()
+    assert bool(((x - want).abs() <= 1.1 * dg * u.abs() + torch.nn.functional.silu(g).abs() * du + 1.1 * dg * du).all())
+    # the split is there already; allocations come in pieces of at most 32 MB
+    assert free - torch.cuda.mem_get_info()[0] <= m * n * 4 + (32 << 20)
