@@ -70,22 +70,13 @@ __device__ __forceinline__ void att_trace(const AttnArgs& a, bool on, int slot) 
     }
 }
 
-// BAR == 0: the 256 threads are the whole CTA; otherwise they meet on named barrier BAR.
-template <int BAR>
-__device__ __forceinline__ void att_sync() {
-    if (BAR == 0)
-        __syncthreads();
-    else
-        asm volatile("bar.sync %0, %1;" ::"r"(BAR), "r"(ATT_FUSED_THREADS) : "memory");
-}
-
-// One (chunk, kv head, sequence) item.  tid = 0..255 inside the group of threads; s_f: the item's shared
+// One (chunk, kv head, sequence) item.  tid = 0..255, the whole CTA; s_f: the item's shared
 // memory (attention_fused_smem_floats floats); s_last: one shared word.
 //
 // MANY: the launch holds more items than SMs.  An item then looks at the position first and leaves, without a load, if
 // its chunk lies behind it: with one wave the extra trip to L2 costs more than the loads, with several the dead items'
 // rows are most of the traffic (16 of 17 chunks of a 1056-position cache at the start of a sequence).
-template <int BAR, uint32_t HD, uint32_t G, bool MANY>
+template <uint32_t HD, uint32_t G, bool MANY>
 __device__ __forceinline__ void attention_fused_item_t(const AttnArgs& a, uint32_t chunk, uint32_t kvh, uint32_t sg,
                                                        uint32_t b, uint32_t tid, float* s_f, uint32_t* s_last) {
     constexpr uint32_t NW = ATT_FUSED_THREADS / 32;
@@ -168,7 +159,7 @@ __device__ __forceinline__ void attention_fused_item_t(const AttnArgs& a, uint32
             for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
             if (lane == 0) s_nrm[r][warp] = ss;
         }
-        att_sync<BAR>();
+        __syncthreads();
         constexpr uint32_t WPH = HALF / 32;  // warps per head
 #pragma unroll
         for (uint32_t r = 0; r < ROT_PER; ++r) {
@@ -205,7 +196,7 @@ __device__ __forceinline__ void attention_fused_item_t(const AttnArgs& a, uint32
         }
     }
     if (tid < HD) sv[tid] = vnew;
-    att_sync<BAR>();
+    __syncthreads();
     if (newest && sg == 0 && tid < HD) {
         Kc[(uint64_t)p * HD + tid] = sk[tid];
         Vc[(uint64_t)p * HD + tid] = sv[tid];
@@ -232,7 +223,7 @@ __device__ __forceinline__ void attention_fused_item_t(const AttnArgs& a, uint32
             }
         }
     }
-    att_sync<BAR>();
+    __syncthreads();
     att_trace(a, tr, 2);
     // per head: maximum, exponentials, their sum (one warp per head; a lane holds positions lane, lane + 32)
     for (uint32_t g = warp; g < G; g += NW) {
@@ -256,7 +247,7 @@ __device__ __forceinline__ void attention_fused_item_t(const AttnArgs& a, uint32
             ssum[g] = s0 + s1;
         }
     }
-    att_sync<BAR>();
+    __syncthreads();
     att_trace(a, tr, 3);
     // weighted V sum: thread = (position group, output dimension); a V element is read once for the group
     if (v_thread) {
@@ -275,7 +266,7 @@ __device__ __forceinline__ void attention_fused_item_t(const AttnArgs& a, uint32
 #pragma unroll
         for (uint32_t g = 0; g < G; ++g) spv[(vpg * G + g) * HD + vi] = acc[g];
     }
-    att_sync<BAR>();
+    __syncthreads();
 #pragma unroll
     for (uint32_t r = 0; r < OUT_PER; ++r) {
         const uint32_t idx = tid + r * ATT_FUSED_THREADS;
@@ -295,7 +286,7 @@ __device__ __forceinline__ void attention_fused_item_t(const AttnArgs& a, uint32
     att_trace(a, tr, 4);
     // count in; the last item of this (sequence, kv head) merges.  The barrier orders the threads' stores
     // before thread 0's fence and atomic (the grid-barrier pattern).
-    att_sync<BAR>();
+    __syncthreads();
     if (tid == 0) {
         __threadfence();
         const uint32_t old = atomicAdd(&a.counters[cix], 1u);
@@ -305,7 +296,7 @@ __device__ __forceinline__ void attention_fused_item_t(const AttnArgs& a, uint32
             __threadfence();
         }
     }
-    att_sync<BAR>();
+    __syncthreads();
     att_trace(a, tr, 5);
     if (!*s_last) return;
     // merge: the first batch of partial rows of every output element is requested before the weights exist
@@ -341,7 +332,7 @@ __device__ __forceinline__ void attention_fused_item_t(const AttnArgs& a, uint32
         }
         if (lane == 0) sden[g] = den;
     }
-    att_sync<BAR>();
+    __syncthreads();
 #pragma unroll
     for (uint32_t r = 0; r < OUT_PER; ++r) {
         const uint32_t idx = tid + r * ATT_FUSED_THREADS;

@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(ATT_FUSED_THREADS, MANY && HD <= 128 ? 2 : 1) 
     __shared__ uint32_t s_last;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     pdl_wait_();
-    attention_fused_item_t<0, HD, G, MANY>(a, blockIdx.x, blockIdx.y / a.gsplit, blockIdx.y % a.gsplit, blockIdx.z,
+    attention_fused_item_t<HD, G, MANY>(a, blockIdx.x, blockIdx.y / a.gsplit, blockIdx.y % a.gsplit, blockIdx.z,
                                            threadIdx.x, s_f, &s_last);
 }
 

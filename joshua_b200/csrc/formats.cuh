@@ -91,12 +91,6 @@ __device__ __forceinline__ uint32_t ld_u32(const uint8_t* p) {  // p 4-byte alig
 }
 __device__ __forceinline__ uint32_t ld_u16_bytes(const uint8_t* p) { return ld_u8(p) | (ld_u8(p + 1) << 8); }
 
-// How a decoder reads its block bytes: global memory, read-only path.
-struct LdGlobal {
-    static __device__ __forceinline__ uint32_t u8(const uint8_t* p) { return ld_u8(p); }
-    static __device__ __forceinline__ uint32_t u16(const uint8_t* p) { return ld_u16(p); }
-    static __device__ __forceinline__ uint32_t u32(const uint8_t* p) { return ld_u32(p); }
-};
 // The 8-bit sign pattern of a 7-bit IQ2_XXS sign index: bit 7 makes the
 // population count even (the reference's KSIGNS table, src/iq2xxs.rs:441-449).
 __device__ __forceinline__ uint32_t iq2_signs(uint32_t idx7) { return idx7 | ((__popc(idx7) & 1u) << 7); }
@@ -115,31 +109,29 @@ __device__ __forceinline__ float e2m1_value(uint32_t code) {
 template <uint32_t TYPE>
 __device__ __forceinline__ void decode_unit_generic(const uint8_t* row, uint32_t u, float w[8], bool two_step);
 
-template <class LD>
 __device__ __forceinline__ void decode_q8_0(const uint8_t* row, uint32_t u, float w[8], bool) {
     const uint8_t* blk = row + (size_t)(u >> 2) * 34;
-    float d = f16_bits_to_f32(LD::u16(blk));
+    float d = f16_bits_to_f32(ld_u16(blk));
     const uint8_t* q = blk + 2 + 8 * (u & 3);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        uint32_t v = LD::u16(q + 2 * i);
+        uint32_t v = ld_u16(q + 2 * i);
         w[2 * i] = __fmul_rn((float)(int8_t)(v & 0xFF), d);
         w[2 * i + 1] = __fmul_rn((float)(int8_t)(v >> 8), d);
     }
 }
 
-template <class LD>
 __device__ __forceinline__ void decode_q2_k(const uint8_t* row, uint32_t u, float w[8], bool two_step) {
     const uint8_t* blk = row + (size_t)(u >> 5) * 84;
     uint32_t v0 = (u & 31) * 8;  // first value inside the block
     uint32_t sg = v0 >> 7, r = v0 & 127;
-    uint32_t sc = LD::u8(blk + sg * 8 + (r >> 4));
-    uint32_t dd = LD::u32(blk + 80);
+    uint32_t sc = ld_u8(blk + sg * 8 + (r >> 4));
+    uint32_t dd = ld_u32(blk + 80);
     float d1 = __fmul_rn(f16_bits_to_f32(dd & 0xFFFF), (float)(sc & 15));
     float m1 = __fmul_rn(f16_bits_to_f32(dd >> 16), (float)(sc >> 4));
     const uint8_t* q = blk + 16 + sg * 32 + (r & 31);
     uint32_t shift = 2 * (r >> 5);
-    uint32_t lo = LD::u32(q), hi = LD::u32(q + 4);
+    uint32_t lo = ld_u32(q), hi = ld_u32(q + 4);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         uint32_t word = i < 4 ? lo : hi;
@@ -148,30 +140,28 @@ __device__ __forceinline__ void decode_q2_k(const uint8_t* row, uint32_t u, floa
     }
 }
 
-template <class LD>
 __device__ __forceinline__ void q4k_scale_min(const uint8_t* s, uint32_t j, uint32_t* sc, uint32_t* mn) {
     if (j < 4) {
-        *sc = LD::u8(s + j) & 63;
-        *mn = LD::u8(s + j + 4) & 63;
+        *sc = ld_u8(s + j) & 63;
+        *mn = ld_u8(s + j + 4) & 63;
     } else {
-        uint32_t a = LD::u8(s + j + 4), b = LD::u8(s + j - 4), c = LD::u8(s + j);
+        uint32_t a = ld_u8(s + j + 4), b = ld_u8(s + j - 4), c = ld_u8(s + j);
         *sc = (a & 0xF) | ((b >> 6) << 4);
         *mn = (a >> 4) | ((c >> 6) << 4);
     }
 }
 
-template <class LD>
 __device__ __forceinline__ void decode_q4_k(const uint8_t* row, uint32_t u, float w[8], bool two_step) {
     const uint8_t* blk = row + (size_t)(u >> 5) * 144;
     uint32_t pair = (u & 31) >> 2;  // 32-value group
     uint32_t sc, mn;
-    q4k_scale_min<LD>(blk + 4, pair, &sc, &mn);
-    uint32_t dd = LD::u32(blk);
+    q4k_scale_min(blk + 4, pair, &sc, &mn);
+    uint32_t dd = ld_u32(blk);
     float d1 = __fmul_rn(f16_bits_to_f32(dd & 0xFFFF), (float)sc);
     float m1 = __fmul_rn(f16_bits_to_f32(dd >> 16), (float)mn);
     const uint8_t* q = blk + 16 + 32 * (pair >> 1) + 8 * (u & 3);
     uint32_t shift = 4 * (pair & 1);
-    uint32_t lo = LD::u32(q), hi = LD::u32(q + 4);
+    uint32_t lo = ld_u32(q), hi = ld_u32(q + 4);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         uint32_t word = i < 4 ? lo : hi;
@@ -180,14 +170,13 @@ __device__ __forceinline__ void decode_q4_k(const uint8_t* row, uint32_t u, floa
     }
 }
 
-template <class LD>
 __device__ __forceinline__ void decode_iq2_xxs(const uint8_t* row, uint32_t u, float w[8], bool) {
     const uint8_t* blk = row + (size_t)(u >> 5) * 66;
     uint32_t ib32 = (u & 31) >> 2, l = u & 3;
     const uint8_t* p = blk + 2 + ib32 * 8;
-    float d = f16_bits_to_f32(LD::u16(blk));
-    uint32_t code = LD::u8(p + l);
-    uint32_t hi = LD::u16(p + 4) | (LD::u16(p + 6) << 16);
+    float d = f16_bits_to_f32(ld_u16(blk));
+    uint32_t code = ld_u8(p + l);
+    uint32_t hi = ld_u16(p + 4) | (ld_u16(p + 6) << 16);
     float db = __fmul_rn(__fmul_rn(d, __fadd_rn(0.5f, (float)(hi >> 28))), 0.25f);
     uint32_t signs = iq2_signs((hi >> (7 * l)) & 127u);
     uint2 g = g_iq2xxs_grid[code];
@@ -200,17 +189,16 @@ __device__ __forceinline__ void decode_iq2_xxs(const uint8_t* row, uint32_t u, f
     }
 }
 
-template <class LD>
 __device__ __forceinline__ void decode_mxfp4(const uint8_t* row, uint32_t u, float w[8], bool) {
     const uint8_t* blk = row + (size_t)(u >> 2) * 17;
-    uint32_t e = LD::u8(blk);
+    uint32_t e = ld_u8(blk);
     uint32_t part = u & 3;  // values 8*part .. 8*part+7 of the block
     const uint8_t* q = blk + 1 + 8 * (part & 1);
     uint32_t shift = 4 * (part >> 1);  // split-half: high nibbles hold values 16..31
     float scale = __uint_as_float(e == 0 ? 0x00400000u : e << 23);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        uint32_t code = (LD::u8(q + i) >> shift) & 15u;
+        uint32_t code = (ld_u8(q + i) >> shift) & 15u;
         w[i] = e == 0xFFu ? 0.0f : __fmul_rn(scale, e2m1_value(code));
     }
 }
@@ -311,7 +299,7 @@ __device__ __forceinline__ void decode_unit_generic<T_Q5_K>(const uint8_t* row, 
     const uint8_t* blk = row + (size_t)(u >> 5) * 176;
     const uint32_t pair = (u & 31) >> 2, l0 = 8 * (u & 3);
     uint32_t sc, mn;
-    q4k_scale_min<LdGlobal>(blk + 4, pair, &sc, &mn);
+    q4k_scale_min(blk + 4, pair, &sc, &mn);
     const float d1 = __fmul_rn(ld_f16(blk), (float)sc), m1 = __fmul_rn(ld_f16(blk + 2), (float)mn);
     const uint8_t* q = blk + 48 + 32 * (pair >> 1) + l0;
     const uint32_t shift = 4 * (pair & 1);
@@ -340,14 +328,14 @@ __device__ __forceinline__ void decode_unit_generic<T_Q6_K>(const uint8_t* row, 
     }
 }
 
-// One decoder per block type; LD says where the block bytes are read from.
-template <uint32_t TYPE, class LD = LdGlobal>
+// One decoder per block type; block bytes are read from global memory, read-only path.
+template <uint32_t TYPE>
 __device__ __forceinline__ void decode_unit(const uint8_t* row, uint32_t u, float w[8], bool two_step) {
-    if constexpr (TYPE == T_Q8_0) decode_q8_0<LD>(row, u, w, two_step);
-    else if constexpr (TYPE == T_Q2_K) decode_q2_k<LD>(row, u, w, two_step);
-    else if constexpr (TYPE == T_Q4_K) decode_q4_k<LD>(row, u, w, two_step);
-    else if constexpr (TYPE == T_IQ2_XXS) decode_iq2_xxs<LD>(row, u, w, two_step);
-    else if constexpr (TYPE == T_MXFP4) decode_mxfp4<LD>(row, u, w, two_step);
+    if constexpr (TYPE == T_Q8_0) decode_q8_0(row, u, w, two_step);
+    else if constexpr (TYPE == T_Q2_K) decode_q2_k(row, u, w, two_step);
+    else if constexpr (TYPE == T_Q4_K) decode_q4_k(row, u, w, two_step);
+    else if constexpr (TYPE == T_IQ2_XXS) decode_iq2_xxs(row, u, w, two_step);
+    else if constexpr (TYPE == T_MXFP4) decode_mxfp4(row, u, w, two_step);
     else decode_unit_generic<TYPE>(row, u, w, two_step);
 }
 
