@@ -126,3 +126,21 @@ def lib() -> ctypes.CDLL:
 def check(rc: int) -> None:
     if rc != 0:
         raise JoshuaB200Error(rc, lib().jq_last_error().decode())
+
+
+def graph_kernels(graph) -> int:
+    """Kernel launches in a captured `torch.cuda.CUDAGraph(keep_graph=True)`: what a replay launches, whatever routes
+    the captured calls took."""
+    cu = ctypes.CDLL("libcuda.so.1")
+    handle, n = ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t()
+    if cu.cuGraphGetNodes(handle, None, ctypes.byref(n)):
+        raise RuntimeError("cuGraphGetNodes failed")
+    nodes = (ctypes.c_void_p * n.value)()
+    if cu.cuGraphGetNodes(handle, nodes, ctypes.byref(n)):
+        raise RuntimeError("cuGraphGetNodes failed")
+    kernels, kind = 0, ctypes.c_int()
+    for node in nodes:
+        if cu.cuGraphNodeGetType(ctypes.c_void_p(node), ctypes.byref(kind)):
+            raise RuntimeError("cuGraphNodeGetType failed")
+        kernels += kind.value == 0   # CU_GRAPH_NODE_TYPE_KERNEL
+    return kernels

@@ -20,7 +20,7 @@ import time
 
 import numpy as np
 
-from . import synth
+from . import _lib, synth
 from .llama import LlamaConfig, LlamaDecoder
 
 
@@ -55,9 +55,10 @@ def run(args, emit=True):
             fn()
             fn()
             stream.synchronize()
-            g = torch.cuda.CUDAGraph()
+            g = torch.cuda.CUDAGraph(keep_graph=True)
             with torch.cuda.graph(g, stream=stream):
                 fn()
+            g.instantiate()
         return g
 
     step_graph = capture(model.step)
@@ -169,13 +170,13 @@ def run(args, emit=True):
             "metric": "decode_tok_s", "value": world * batch / dt, "unit": "tok/s", "n_gpus": world,
             "steps": args.steps, "warmup": warmup, "ms_per_step": dt * 1e3, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None,
-            "dtype": "int8 codes x int8 activation planes -> int32, f32 scales and glue", "data": "synthetic",
+            "dtype": "int8 codes x int8 activation planes -> int32, f32 scales and glue" if batch < 5 else
+                     "f16 terms of codes x f16 hi / lo terms of activations -> f32, f32 scales and glue", "data": "synthetic",
             "config": {"workload": f"llama8b_q4k_decode_b{batch}", "layers": c.layers, "hidden": c.hidden,
                        "q_heads": c.q_heads, "kv_heads": c.kv_heads, "head_dim": c.head_dim, "ffn": c.ffn,
                        "vocab": c.vocab, "batch": batch, "prefill": args.prefill,
                        "step": "full decode step on the device (embedding, norms, RoPE, attention over the KV cache, "
-                               "quantized matmuls, greedy arg-max), one CUDA graph; "
-                               "five launches per layer",
+                               f"quantized matmuls, greedy arg-max), one CUDA graph of {_lib.graph_kernels(step_graph)} kernels",
                        "l2": "4.22 GB of weights per step, far larger than L2", "parallelism": f"replicas x{world}"},
             "e2e": {"value": world * batch / e2e_dt, "unit": "tok/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                     "how": "model-level call with host buffers (LlamaDecoder.forward_host, the shape of the "
@@ -191,7 +192,7 @@ def run(args, emit=True):
                          "peak_source": which, "kernel": "gemv_mma_kernel<Q4_K>",
                          "launches_per_step": launches, "avg_launch_us": dt_mm / launches * 1e6,
                          "bytes_per_step": alg},
-            "gpu_launches": model.launches_per_step * args.steps, "clocks": clocks.summary(),
+            "gpu_launches": _lib.graph_kernels(step_graph) * args.steps, "clocks": clocks.summary(),
             "prefill": prefill_info,
         }
         try:

@@ -14,7 +14,7 @@ from __future__ import annotations
 import json
 import os
 
-from . import synth
+from . import _lib, synth
 from .moe_decoder import MoeDecoder, MoeDecoderConfig
 
 
@@ -69,9 +69,10 @@ def measure(args, batch: int, group, sample_load: bool = True, with_e2e: bool = 
         model.step()
         stream.synchronize()
         barrier()
-        graph = torch.cuda.CUDAGraph()
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
         with torch.cuda.graph(graph, stream=stream):
             model.step()
+        graph.instantiate()
         stream.synchronize()
         for _ in range(prefill + warmup):
             graph.replay()
@@ -121,7 +122,7 @@ def measure(args, batch: int, group, sample_load: bool = True, with_e2e: bool = 
                     "rows_per_rank_mean": float(a.mean()), "sampled": "last layer of 8 steps"}
     model.check_flags()
     out = {"dt": dt, "mm_dt": mm_dt, "clocks": clocks.summary(), "load": load, "cfg": cfg, "warmup": warmup,
-           "launches_per_step": model.launches_per_step, "weight_bytes": model.weight_bytes}
+           "launches_per_step": _lib.graph_kernels(graph), "weight_bytes": model.weight_bytes}
     if prompt > 0:
         # the prompt in one pass (`forward(input [1, seq_len], 0)`): batched linears and the experts' buckets on the
         # tile GEMM, causal attention; the reference's bench feeds a repeated token (examples/bench_qwen3moe.rs:148-162)

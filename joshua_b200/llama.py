@@ -116,16 +116,17 @@ class LlamaDecoder:
         fused_bytes = _lib.lib().jq_attention_fused_scratch_bytes(B, cfg.q_heads, cfg.kv_heads, cfg.head_dim, max_ctx)
         self.att_fused_scratch = torch.zeros(fused_bytes // 4 + 1, **f32)   # holds arrival counters: starts at zero
         self.argmax_scratch = torch.empty(_lib.lib().jq_argmax_scratch_bytes(B) // 4 + 1, **f32)
-        self.launches_per_step = 5 * cfg.layers + 4
+        self.launches_per_step = 5 * cfg.layers + 4   # one sequence; larger batches take other routes
         self.matmuls_per_step = 4 * cfg.layers + 1
 
     # ── one token ───────────────────────────────────────────────────────
     def step(self, stream=None) -> None:
         """Decode one token per sequence: reads self.token / self.pos, writes self.logits, the next
-        self.token and advances self.pos.  Launches only.  Five launches per layer: the RMS norms ride in the
-        prologue of the matmul that consumes them, the residual adds in the epilogue of the matmul that
-        produces the branch, and rope + cache append + attention + merge are one kernel.  self.x is the
-        residual stream, updated in place."""
+        self.token and advances self.pos.  Launches only.  Five launches per layer for one sequence: the RMS
+        norms ride in the prologue of the matmul that consumes them, the residual adds in the epilogue of the
+        matmul that produces the branch, and rope + cache append + attention + merge are one kernel.  (From five
+        sequences on Q4_K linears run on the tile GEMM: a split and a product each, ten launches per layer.)
+        self.x is the residual stream, updated in place."""
         L, c, B = _lib.lib(), self.cfg, self.batch
         s = self.torch.cuda.current_stream(self.dev).cuda_stream if stream is None else stream
         h, P = c.hidden, lambda t: t.data_ptr()
@@ -152,8 +153,8 @@ class LlamaDecoder:
     # ── prefill: many tokens of one sequence in one pass ────────────────
     def prefill(self, token_ids, stream=None) -> None:
         """`forward(input [1, seq_len], offset)` of the reference's loaders (src/quantized_qwen3_moe.rs:793-819): the
-        prompt's tokens in ONE pass from the current position - batched matmuls (the tensor-core tile GEMM above
-        64 tokens), rotary embedding + cache append for all positions, causal attention - then the logits of the
+        prompt's tokens in ONE pass from the current position - batched matmuls (the tensor-core tile GEMM from
+        five tokens on, Q8_0 from 17), rotary embedding + cache append for all positions, causal attention - then the logits of the
         last token, the sampled next token and the advanced position, exactly as `step` leaves them.  One
         sequence (batch 1).  Buffers are allocated per call."""
         torch, L, c, P = self.torch, _lib.lib(), self.cfg, lambda t: t.data_ptr()

@@ -391,3 +391,29 @@ def test_forward_host_matches_device_steps():
         assert np.array_equal(logits, b.logits.cpu().numpy()), step
         tok = logits.argmax(axis=1).astype(np.int32)
     assert a.pos.tolist() == [10, 10]
+
+
+@pytest.mark.parametrize("batch,per_layer,rest", [(1, 5, 4), (8, 10, 5)])
+def test_launches_of_a_step_are_those_of_its_graph(batch, per_layer, rest):
+    """What the benchmarks report as launches is counted in the captured step: five kernels a layer for one sequence; with
+    Q4_K tiles a split and a product per linear, the pair's combine, and a split more in front of the head."""
+    import torch
+
+    from joshua_b200 import _lib
+    from joshua_b200.llama import LlamaConfig, LlamaDecoder
+
+    cfg = LlamaConfig(hidden=512, layers=2, q_heads=4, kv_heads=2, head_dim=128, ffn=512, vocab=512)
+    dec = LlamaDecoder(cfg, torch.device("cuda", 0), batch=batch, max_ctx=16, seed=1, weights=_small_weights(synth.Q4_K))
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        dec.step()
+        s.synchronize()
+        g = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(g, stream=s):
+            dec.step()
+        g.instantiate()
+        g.replay()
+        s.synchronize()
+    assert _lib.graph_kernels(g) == per_layer * cfg.layers + rest
+    if batch == 1:
+        assert dec.launches_per_step == per_layer * cfg.layers + rest
