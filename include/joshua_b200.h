@@ -81,7 +81,10 @@ int32_t jq_device_status(const jq_ctx* ctx);
  * when `nbytes` is not a whole number of blocks. */
 int32_t jq_weight_upload(jq_ctx* ctx, uint32_t type, const void* bytes, uint64_t nbytes, jq_weight** out);
 
-/* Adopt blocks that already sit in device memory (not copied, not freed). */
+/* Adopt blocks that already sit in device memory (not copied, not freed), from
+ * a 16-byte boundary on.  Copies run over whole 16-byte vectors: up to 15 bytes
+ * behind the last block are read, and not used, so they must lie in the same
+ * allocation (any that cudaMalloc or a caching allocator rounds to 16 does). */
 int32_t jq_weight_from_device(jq_ctx* ctx, uint32_t type, const void* device_bytes, uint64_t nbytes,
                               jq_weight** out);
 
@@ -183,7 +186,10 @@ int32_t jq_weight_from_float(jq_weight* w, const float* xs, uint64_t len);
 
 /* `Mlp::forward` up to the down projection: dst = silu(gate x) * up x, with the
  * optional clamp of src/quantized_deepseek4.rs:445-462 (clamp <= 0: none)
- * (src/quantized_qwen3_moe.rs:396-402).  One launch for batches of 1..8. */
+ * (src/quantized_qwen3_moe.rs:396-402).  One launch of the decode kernel, or
+ * one of the tile GEMM for both tensors and the combine (gate passes through
+ * dst_dev, up through the stream's scratch), by the rows of jq_matmul_norm_dev.
+ * lhs_dev 16-byte aligned. */
 int32_t jq_matmul_swiglu_dev(const jq_weight* gate, const jq_weight* up, uint64_t m, uint64_t k, uint64_t n,
                              const float* lhs_dev, float* dst_dev, float clamp, void* stream);
 
@@ -208,8 +214,12 @@ int32_t jq_matmul_swiglu_norm_dev(const jq_weight* gate, const jq_weight* up, ui
  * RMS norm in front of it and the residual add behind it in the same launch
  * (the `RmsNorm` -> `QMatMul::forward` -> `xs + residual` pattern of
  * src/quantized_qwen3_moe.rs:793-819).  norm_w_dev and residual_dev are each
- * optional; residual_dev may be dst_dev.  One launch when m <= 8 and the
- * activation planes fit shared memory, otherwise the separate kernels. */
+ * optional; residual_dev may be dst_dev; lhs_dev and norm_w_dev 16-byte
+ * aligned.  One launch of the decode kernel for up to eight rows whose
+ * activation planes fit its shared memory; a split and a product of the tile
+ * GEMM, norm and residual inside, from five rows of Q4_K (or of planes that do
+ * not fit), nine of the other types and 17 of Q8_0 on; the separate kernels for
+ * what neither takes. */
 int32_t jq_matmul_norm_dev(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, const float* lhs_dev,
                            const float* norm_w_dev, float eps, const float* residual_dev, float* dst_dev,
                            void* stream);

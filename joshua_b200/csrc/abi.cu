@@ -73,13 +73,14 @@ int32_t validate_matmul(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, 
 // From nine rows on the other route is the decode kernel once per eight rows.  From five rows on, where the decode
 // kernel's activation planes do not fit its shared memory, it reads them from L2 for every 16 weight rows; Q4_K, bound
 // by its consumers' instructions, is behind the tiles from five rows on in any case.  Measured, eight rows, tiles /
-// decode kernel: Q4_K 28672 x 4096 53 / 66 us, 4096 x 14336 31 / 35 us, 7168 x 2048 12 / 19 us; five rows, planes in
-// shared memory: Q4_K 28672 x 4096 52 / 64 us; four rows: 53 / 28 us.
+// decode kernel: Q4_K 28672 x 4096 50 / 66 us, 4096 x 14336 29 / 36 us, 7168 x 2048 11 / 19 us, Q2_K 4096 x 14336 30 / 54,
+// MXFP4 31 / 36; five rows, planes in shared memory: Q4_K 28672 x 4096 50 / 64 us; four rows: 50 / 28 us.
 bool jq_uses_tiles(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, cudaStream_t s) {
     if (w->ctx->force_f32 || m < 5 || !jq::gemm_f16_supports(w->type, w->dev, n, k, m)) return false;
-    // Q8_0 stays on the decode kernel up to 16 rows, although the tiles are ahead (4096 x 4096, 16 rows: 14 / 40 us): it is
-    // the attention of the routed-expert files, and a decode step of a few sequences that rounds differently lets experts
-    // in a near tie change places (logits 2 % off in a third of the batches tried).
+    // Q8_0 stays on the decode kernel up to 16 rows, although the tiles are ahead (4096 x 4096: 16 rows there 42 us, 17 rows
+    // on tiles 16 us): it is the attention of the routed-expert files, and a decode step of a few sequences that rounds
+    // differently lets experts in a near tie change places (logits 2 % off in a third of the batches tried).  Dense Q8_0
+    // files pay for that; a flag on the products in front of a router would spare them.
     if (w->type == jq::T_Q8_0 && m <= 2 * jq::GEMV_MMA_MAX_M) return false;
     if (m <= jq::GEMV_MMA_MAX_M && w->type != jq::T_Q4_K && jq::gemv_mma_scratch_bytes(m, k) == 0) return false;
     return w->ctx->scratch_available(s, SLOT_TILES, jq::gemm_f16_scratch_bytes(m, k));

@@ -77,7 +77,7 @@ cudaError_t tables_gemv_f32();
 cudaError_t launch_matmul_f32(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, const float* lhs, uint64_t m,
                               float* dst, cudaStream_t s);
 
-// gemm_f16.cu: tcgen05 tile GEMM in half-precision terms for m > 8 (prefill, batched decode)
+// gemm_f16.cu: tcgen05 tile GEMM in half-precision terms, from five rows on (prefill, batched decode)
 cudaError_t tables_gemm_f16();
 bool gemm_f16_supports(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, uint64_t m);
 // scratch: gemm_f16_scratch_bytes(m, k) bytes (the activations' two terms, group sums and scales), 256-byte aligned

@@ -1,5 +1,5 @@
-// Prefill / batched matmul (m > 8) over raw GGUF blocks on the 5th-generation tensor cores, in half precision terms
-// that lose nothing against f32.
+// Prefill / batched matmul (from five rows on) over raw GGUF blocks on the 5th-generation tensor cores, in half precision
+// terms that keep f32's precision.
 //
 // dst[m, n] = lhs[m, k] . W[n, k]^T with W left in its GGUF bytes.  A CTA owns 128 rows of W and up to N_TILE rows of
 // lhs.  Per window of 256 columns (one super-block of the K formats) the weights of a row are one f32 factor times
@@ -21,9 +21,9 @@
 // absolute error below 2^-39 of it otherwise.  A window whose own largest value lies more than 2^8 below the row's (an
 // outlier elsewhere) is scaled further by itself, so the error stays below 2^-31 of the window's largest value (the int8
 // planes of the decode kernel, scaled over the same 256 values: 2^-24 of it), and the read-back undoes that scale token
-// by token.  Rows with such a window say so by the sign of their scale; a tile without one, the usual one, never asks.  The tensor core's products of f16
-// terms are exact; two or three products (hi*hi, hi*lo, lo*hi) replace three TF32 products (gemm_tc.cu) at twice their
-// rate: 32 to 48 instructions per window instead of 96.
+// by token.  Rows with such a window say so by the sign of their scale; a tile without one, the usual one, never asks.
+// The tensor core's products of f16 terms are exact; two or three products (hi*hi, hi*lo, lo*hi) replace three TF32
+// products (gemm_tc.cu) at twice their rate: 32 to 48 instructions per window instead of 96.
 //
 // Minima (Q4_K, Q2_K): sum_c dmin m_g x_c = sum_g (dmin m_g) (sum of x over the group), an inner product of 16 terms per
 // window.  The split kernel also writes the sums of each 16 values, times 2^-5 so that they fit, as two f16 terms, the
@@ -60,7 +60,8 @@
 // shared memory), so results do not depend on timing.
 //
 // Every wait on an mbarrier is bounded; a wait that runs out raises the device status flag, and every thread still
-// reaches the common exit where tensor memory is released.
+// reaches the common exit where tensor memory is released.  Running out takes seconds; copies and products that were in
+// flight when progress stopped have landed long before.
 #include <algorithm>
 #include <type_traits>
 

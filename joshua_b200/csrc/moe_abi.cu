@@ -20,7 +20,7 @@ constexpr uint64_t BUCKET_MIN_TOKENS = 128;      // tokens from which the prefil
 constexpr uint64_t TILES_MIN_TOKENS = 32;        // the same for the types whose experts all run on tiles
 
 // Banks whose experts run on the tile GEMM whatever their row count.  Measured, 384 MXFP4 experts of 7168 x 2048, eight a
-// token, tiles / decode kernel: 3.87 / 4.85 ms at 100 tokens, 2.13 / 2.17 at 32, 1.35 / 1.19 at 16; 48 layers of 128
+// token, tiles / decode kernel: 3.65 / 4.89 ms at 100 tokens, 2.00 / 2.18 at 32, 1.35 / 1.20 at 16; 48 layers of 128
 // Q4_K experts of 2048 x 768: 14.0 / 27.6 ms at 100 tokens, 11.6 / 14.5 at 40, 13.8 / 10.1 (a decode step) at 16.
 bool all_experts_on_tiles(const jq_moe* m) {
     auto one = [](const jq_weight* w) { return w->type == jq::T_Q4_K || w->type == jq::T_MXFP4; };
