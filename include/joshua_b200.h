@@ -390,7 +390,7 @@ int32_t jq_moe_reserve(jq_moe* m, uint64_t n_tokens, uint64_t n_rows);
 /* The same with DEVICE buffers on a caller stream, without synchronisation: routing, job lists and tile lists stay on the
  * device.  Only banks that the grouped tile GEMM does not take (IQ2_XXS with a width that is no multiple of 512) read the
  * job list back from 128 tokens on, which synchronises the stream; such batches cannot be captured in a CUDA graph.
- * A capture of 32 to 127 tokens on a stream without scratch takes the decode kernel instead of the tile GEMM (another
+ * A capture of 32 and more tokens on a stream without scratch takes the decode kernel instead of the tile GEMM (another
  * summation order). */
 int32_t jq_moe_forward_dev(jq_moe* m, const float* x_dev, uint64_t n_tokens, const uint32_t* forced_ids_dev,
                            float* y_dev, void* stream);

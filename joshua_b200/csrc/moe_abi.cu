@@ -598,8 +598,7 @@ int32_t jq_moe_forward_norm_add_dev(jq_moe* m, const float* x_dev, uint64_t T, c
     // decided per expert on the device.  From TILES_MIN_TOKENS on where every expert takes tiles, unless that would
     // allocate the stream's scratch while it is captured (the decode form needs nothing beyond jq_moe_reserve).
     uint64_t min_tokens = bucket_min_tokens(m, P);
-    if (T >= min_tokens && T < BUCKET_MIN_TOKENS && !m->ctx->scratch_available(s, SLOT_TILES, bucket_scratch_bytes(c, P)))
-        min_tokens = BUCKET_MIN_TOKENS;
+    if (T >= min_tokens && !m->ctx->scratch_available(s, SLOT_TILES, bucket_scratch_bytes(c, P))) min_tokens = ~0ull;
 #ifdef JQ_PROFILING
     if (const char* thr_env = std::getenv("JQ_MOE_BUCKET_TOKENS")) min_tokens = std::strtoull(thr_env, nullptr, 10);  // measurement switch
 #endif

@@ -1,4 +1,4 @@
-"""The tensor-core tile GEMM (m > 8: prefill and batched decode) against the oracle."""
+"""The tensor-core tile GEMMs (prefill and batched decode, from five rows on) against the oracle."""
 import numpy as np
 import pytest
 
@@ -12,8 +12,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.fixture(scope="module")
 def tc_ctx():
-    """A context that sends every batch above 8 to the tile GEMM (by default batches up to 64 run as 8-row
-    slices of the decode kernel)."""
+    """A context without slices of the decode kernel: what the f16 tiles do not take runs on the TF32 tile GEMM (by default
+    batches of up to 64 of those go in slices of eight rows)."""
     import os
 
     from joshua_b200.qtensor import Context
@@ -64,7 +64,7 @@ def test_assigns_and_leaves_neighbours_alone(tc_ctx):
 @pytest.mark.parametrize("type_id,mkn", [(synth.Q4_K, (9, 256, 16)), (synth.Q4_K, (20, 4096, 130)), (synth.Q8_0, (64, 2048, 96)),
                                          (synth.MXFP4, (33, 1024, 40)), (synth.IQ2_XXS, (17, 1024, 23)), (synth.Q2_K, (40, 1024, 129))])
 def test_sliced_batches_match_oracle(type_id, mkn):
-    """Batches 9..64 through the default context: 8-row slices of the decode kernel."""
+    """Batches 9..64 through the default context: f16 tiles of 16 and 32 rows (what still goes in slices: OLDER below)."""
     m, k, n = mkn
     raw = synth.random_weight(type_id, n, k, seed=n + k)
     lhs = synth.random_activations(m, k, seed=m)

@@ -375,3 +375,44 @@ def test_a_captured_layer_survives_larger_batches(kind, tokens_):
     assert all(bool(torch.isnan(j).all()) for j in junk)
     _, _, ref = oracle_forward(cfg, x[:tokens_].cpu().numpy(), router, banks, types)
     assert_close(want.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("kind", [synth.Q4_K, synth.MXFP4])
+@pytest.mark.parametrize("tokens_", [40, 150])
+def test_tokens_with_one_large_value_on_tiles(kind, tokens_):
+    """Every seventh token carries a value a thousand times the others: its other windows have scales of their own, in tiles
+    that they share with tokens that have none."""
+    cfg = MoeConfig(gating=GATE_SOFTMAX, n_expert=8, n_used=4, hidden=1024, inter=512)
+    moe, router, banks, types, _ = build(cfg, kind, seed=71)
+    x = tokens(tokens_, cfg.hidden, 8)
+    x[::7, 5] = 20.0
+    _, _, want = oracle_forward(cfg, x, router, banks, types)
+    assert_close(moe.forward(x), want, tol=1e-3 * max(1.0, float(np.abs(want[::7]).mean())))
+
+
+@pytest.mark.parametrize("tokens_", [40, 150])
+def test_a_layer_captured_on_a_stream_without_scratch(tokens_):
+    """The tile GEMM's scratch cannot be allocated during a capture: the decode kernel runs there, at any batch."""
+    import torch
+
+    from joshua_b200.qtensor import Context
+
+    cfg = MoeConfig(gating=GATE_SOFTMAX, n_expert=16, n_used=4, hidden=512, inter=256)
+    warm, router, banks, types, _ = build(cfg, synth.Q4_K, seed=81)
+    x = tokens(tokens_, cfg.hidden, 10)
+    want = warm.forward(x)                      # kernels of this process are loaded (tile form)
+    for T in (9, 31):
+        warm.forward(x[:T])                     # and those of the decode form
+    ctx = Context(0)
+    moe = Moe(cfg, router, *[QTensor.from_bytes(t, b, ctx) for t, b in zip(types, banks)], ctx=ctx)
+    moe.reserve(tokens_)
+    xd = torch.from_numpy(x).cuda()
+    out = torch.zeros_like(xd)
+    s, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g, stream=s):
+        moe.forward_dev(xd, out, stream=s.cuda_stream)
+    g.replay()
+    torch.cuda.synchronize()
+    moe.status()
+    assert_close(out.cpu().numpy(), want)
