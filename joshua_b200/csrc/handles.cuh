@@ -201,8 +201,8 @@ struct jq_moe {
 };
 
 // Expert MLPs over n_rows rows with given local expert ids (an id out of range marks an unused row).
-// `live_rows` is the caller's estimate of how many rows carry a valid id: from 12 per expert on, the rows run
-// in buckets on the tile GEMM (which reads the job list back and so synchronises the stream).
+// `live_rows` is the caller's estimate of how many rows carry a valid id: from 128 on the rows run in the prefill form
+// (the tile GEMM, and the decode kernel for experts with few rows of the types that are not all on tiles).
 int32_t jq_moe_experts_list(jq_moe* m, const float* x_dev, uint64_t n_rows, const uint32_t* expert_ids_dev,
                             uint64_t live_rows, cudaStream_t s);
 // Rows per job for about `live_rows` rows with valid ids: one while two rows rarely share an expert (the decode

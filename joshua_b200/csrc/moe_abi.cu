@@ -189,7 +189,6 @@ int32_t run_experts(jq_moe* m, const float* x, uint64_t R, uint64_t P, uint32_t 
     return jq::OK;
 }
 
-// sh_out[T, hidden] = shared expert MLP over all tokens
 // The prefill form of the expert MLPs, as the reference buckets tokens per expert and runs one matmul per
 // bucket (src/quantized_qwen3_moe.rs:455-520): when an expert sees dozens of rows, its rows are gathered into
 // bucket order and the experts' gate / up / down products run on the tile GEMM (tensor cores), as one grouped
@@ -327,6 +326,7 @@ bool shared_mma_ok(jq_moe* m, uint64_t T) {
            fits_smem(T, c.hidden) && fits_smem(T, c.inter) && m->sh_gate->type == m->sh_up->type;
 }
 
+// sh_out[T, hidden] = shared expert MLP over all tokens
 int32_t run_shared(jq_moe* m, const float* x, uint64_t T, cudaStream_t s, const float* norm_w = nullptr, float eps = 0.0f) {
     const jq_moe_config& c = m->cfg;
     const bool mma_ok = T <= 8 && !m->ctx->force_f32 &&
