@@ -75,7 +75,7 @@ struct jq_ctx {
     // Scratch of `stream` in a role, at least `bytes` large.  Growing it frees the old buffer (cudaFree waits for the
     // device), unless it was handed out while the stream was being captured: then a graph may replay into it, so it stays
     // until the context goes, and the new one is at least twice as large (the retired ones together stay below the live one).
-    cudaError_t scratch_for(cudaStream_t stream, ScratchSlot slot, size_t bytes, void** out) {
+    cudaError_t scratch_for(cudaStream_t stream, ScratchSlot slot, size_t bytes, void** out) try {
         *out = nullptr;
         if (bytes == 0) return cudaSuccess;
         cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
@@ -108,6 +108,8 @@ struct jq_ctx {
         sc.in_graph |= st != cudaStreamCaptureStatusNone;
         *out = sc.dev;
         return cudaSuccess;
+    } catch (const std::bad_alloc&) {  // host memory; nothing was changed
+        return cudaErrorMemoryAllocation;
     }
 
     // Whether that scratch can be had now: it is large enough, or may be allocated because the stream is not being

@@ -60,10 +60,15 @@ int32_t reserve(jq_moe* m, uint64_t T, uint64_t P) {
     T = T > m->cap_tokens ? std::max(T, m->cap_tokens + m->cap_tokens / 4) : m->cap_tokens;
     P = P > m->cap_pairs ? std::max(P, m->cap_pairs + m->cap_pairs / 4) : m->cap_pairs;
     const jq_moe_config& c = m->cfg;
-    if (m->in_graph)
-        m->retired.push_back(m->ws);
-    else if (m->ws)
+    if (m->in_graph) {
+        try {
+            m->retired.push_back(m->ws);
+        } catch (const std::bad_alloc&) {
+            return jq_fail(jq::E_NOMEM, "moe: out of host memory");
+        }
+    } else if (m->ws) {
         cudaFree(m->ws);
+    }
     m->ws = nullptr;
     m->in_graph = false;
     m->cap_tokens = m->cap_pairs = m->bucket_pairs = 0;
