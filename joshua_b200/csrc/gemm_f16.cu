@@ -151,23 +151,6 @@ struct Tile {
     static_assert(SMEM <= 226 * 1024, "shared memory");
 };
 
-// Instruction descriptor: D f32, A and B f16, both K-major, M = 128, N = n_tile.
-__device__ __forceinline__ constexpr uint32_t h_idesc(uint32_t n_tile) {
-    return (1u << 4) | ((n_tile >> 3) << 17) | ((uint32_t)(HM >> 4) << 24);
-}
-// D (tensor memory) += A (tensor memory, 16 columns of k in 8 columns) * B (shared memory)
-__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
-                                            uint32_t accumulate) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t"
-        "}\n" ::"r"(tmem_d),
-        "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
-        : "memory");
-}
-
 // ── activations ──
 // One CTA per row; a thread takes 16 consecutive values at a time, half a warp a window.  hi / lo [m][k];
 // sums [m][k / 256][32]: the 16 group sums of a window, first terms then second terms; inv[m]: the inverse of the row's
@@ -852,7 +835,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
         }
     } else {
         // ── issuers (their waits sleep: polling warps take issue slots from the converters) ──
-        constexpr uint32_t idesc = h_idesc(N_TILE);
+        constexpr uint32_t idesc = umma_idesc_f16(N_TILE);
         const uint32_t base0 = smem_u32(smem);
         const uint64_t d0_hi = umma_desc(base0), d0_lo = umma_desc(base0 + PLANE_B);
         [[maybe_unused]] const uint64_t d_sums = umma_desc(smem_u32(s_sums));
