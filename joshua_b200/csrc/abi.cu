@@ -70,6 +70,7 @@ int32_t validate_matmul(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, 
 
 }  // namespace
 
+// (Batches of three to eight rows that gemv_f16.cu takes never ask.)
 // From nine rows on the other route is the decode kernel once per eight rows.  From five rows on, where the decode
 // kernel's activation planes do not fit its shared memory, it reads them from L2 for every 16 weight rows; Q4_K, bound
 // by its consumers' instructions, is behind the tiles from five rows on in any case.  Measured, eight rows, tiles /
@@ -86,6 +87,10 @@ bool jq_uses_tiles(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, cudaS
     return w->ctx->scratch_available(s, SLOT_TILES, jq::gemm_f16_scratch_bytes(m, k));
 }
 
+bool jq_uses_gemv_f16(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, bool pair) {
+    return !w->ctx->force_f32 && jq::gemv_f16_supports(w->type, w->dev, n, k, m, pair);
+}
+
 int32_t jq_matmul_tiles(const jq_weight* w, const jq_weight* w_b, uint64_t m, uint64_t k, uint64_t n, const float* lhs,
                         const float* norm_w, float eps, const float* residual, float* dst, float* dst_b, cudaStream_t s) {
     jq_ctx* ctx = w->ctx;
@@ -100,6 +105,10 @@ int32_t jq_matmul_tiles(const jq_weight* w, const jq_weight* w_b, uint64_t m, ui
 int32_t jq_matmul_device(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, const float* lhs, float* dst,
                          cudaStream_t s) {
     jq_ctx* ctx = w->ctx;
+    if (jq_uses_gemv_f16(w, m, k, n, false)) {
+        JQ_CUDA(jq::launch_gemv_f16(w->type, w->dev, nullptr, n, k, lhs, m, nullptr, 0.0f, nullptr, 0.0f, dst, ctx->status_dev, s));
+        return jq::OK;
+    }
     if (jq_uses_tiles(w, m, k, n, s)) return jq_matmul_tiles(w, nullptr, m, k, n, lhs, nullptr, 0.0f, nullptr, dst, nullptr, s);
     if (!ctx->force_f32 && jq::gemv_mma_dense_supports(w->type, w->dev, n, k, m)) {
         void* scratch = nullptr;

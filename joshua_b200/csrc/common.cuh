@@ -88,6 +88,15 @@ cudaError_t launch_gemm_f16(uint32_t type, const uint8_t* w_a, const uint8_t* w_
                             uint64_t m, const float* norm_w, float eps, const float* residual, float* dst_a, float* dst_b,
                             void* scratch, int* error_flag, cudaStream_t s);
 
+// gemv_f16.cu: decode matmul of 3 .. 8 rows in half-precision terms (mma.sync), no scratch; Q4_K and MXFP4.
+// dst = residual + norm(lhs) . W^T (norm_w, residual optional; residual may be dst); with w_b, a tensor of the same type and
+// shape, dst = silu(clamp(norm(lhs) . W_a^T)) * clamp(norm(lhs) . W_b^T) (no residual).
+constexpr uint64_t GEMV_F16_MIN_M = 3, GEMV_F16_MAX_M = 8;
+bool gemv_f16_supports(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, uint64_t m, bool pair);
+cudaError_t launch_gemv_f16(uint32_t type, const uint8_t* w_a, const uint8_t* w_b, uint64_t n, uint64_t k, const float* lhs,
+                            uint64_t m, const float* norm_w, float eps, const float* residual, float clamp, float* dst,
+                            int* error_flag, cudaStream_t s);
+
 // gemm_tc.cu: the same for the shapes gemm_f16.cu does not take
 cudaError_t tables_gemm_tc();
 bool gemm_tc_supports(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, uint64_t m);

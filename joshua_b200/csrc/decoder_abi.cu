@@ -45,6 +45,11 @@ int32_t jq_matmul_swiglu_dev(const jq_weight* gate, const jq_weight* up, uint64_
     if (int32_t rc = check_vectors("jq_matmul_swiglu_dev", lhs_dev, nullptr)) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     jq_ctx* ctx = gate->ctx;
+    if (jq_uses_gemv_f16(gate, m, k, n, true) && jq_uses_gemv_f16(up, m, k, n, true)) {
+        JQ_CUDA(jq::launch_gemv_f16(gate->type, gate->dev, up->dev, n, k, lhs_dev, m, nullptr, 0.0f, nullptr, clamp, dst_dev,
+                                    ctx->status_dev, s));
+        return jq::OK;
+    }
     if (pair_uses_tiles(gate, up, m, k, n, s))
         return swiglu_tiles(gate, up, m, k, n, lhs_dev, nullptr, 0.0f, dst_dev, clamp, s);
     if (!ctx->force_f32 && jq::gemv_mma_supports(gate->type, gate->dev, n, k, m) &&
@@ -76,6 +81,11 @@ int32_t jq_matmul_swiglu_norm_dev(const jq_weight* gate, const jq_weight* up, ui
     // the plain entry names the fault (or finds nothing to do) before anything is launched
     if (!shapes_ok) return jq_matmul_swiglu_dev(gate, up, m, k, n, lhs_dev, dst_dev, clamp, stream);
     if (int32_t rc = check_vectors("jq_matmul_swiglu_norm_dev", lhs_dev, norm_w_dev)) return rc;
+    if (jq_uses_gemv_f16(gate, m, k, n, true) && jq_uses_gemv_f16(up, m, k, n, true)) {
+        JQ_CUDA(jq::launch_gemv_f16(gate->type, gate->dev, up->dev, n, k, lhs_dev, m, norm_w_dev, eps, nullptr, clamp, dst_dev,
+                                    ctx->status_dev, s));
+        return jq::OK;
+    }
     if (pair_uses_tiles(gate, up, m, k, n, s))
         return swiglu_tiles(gate, up, m, k, n, lhs_dev, norm_w_dev, eps, dst_dev, clamp, s);
     if (!ctx->force_f32 && jq::gemv_mma_supports(gate->type, gate->dev, n, k, m) &&
@@ -102,6 +112,11 @@ int32_t jq_matmul_norm_dev(const jq_weight* w, uint64_t m, uint64_t k, uint64_t 
                            lhs_dev && dst_dev;
     if (!shapes_ok) return jq_matmul_t_dev(w, m, k, n, lhs_dev, dst_dev, stream);  // as above
     if (int32_t rc = check_vectors("jq_matmul_norm_dev", lhs_dev, norm_w_dev)) return rc;
+    if (jq_uses_gemv_f16(w, m, k, n, false)) {
+        JQ_CUDA(jq::launch_gemv_f16(w->type, w->dev, nullptr, n, k, lhs_dev, m, norm_w_dev, eps, residual_dev, 0.0f, dst_dev,
+                                    ctx->status_dev, s));
+        return jq::OK;
+    }
     if (jq_uses_tiles(w, m, k, n, s))
         return jq_matmul_tiles(w, nullptr, m, k, n, lhs_dev, norm_w_dev, eps, residual_dev, dst_dev, nullptr, s);
     if (!ctx->force_f32 && jq::gemv_mma_dense_supports(w->type, w->dev, n, k, m) &&

@@ -1,0 +1,88 @@
+"""The half-precision decode kernel (batches of 3 to 8 rows of Q4_K and MXFP4) against float64 products of the decoded
+weights: row counts around its tiles of 16, columns that give four to 112 units a row (teams of two to eight warps, idle
+warps, several stages a tile, k split over clusters of up to eight CTAs), the gate / up pair, norm and residual, activations
+decades apart."""
+import numpy as np
+import pytest
+
+from joshua_b200 import synth
+from joshua_b200.qtensor import QMatMul, QTensor
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(1, 1024), (17, 1024), (100, 1280), (48, 1536), (4097, 2048), (33, 4096), (5000, 4096), (333, 7168), (40, 14336),
+          (700, 14336), (20, 16384), (31, 28672)]
+
+
+def setup(type_id, n, k, m, seed, spread=False):
+    import torch
+
+    raw = synth.random_weight(type_id, n, k, seed)
+    q = QTensor.from_bytes(type_id, raw)
+    w = torch.empty(n * k, device="cuda")
+    q.dequantize_dev(w, two_step=False)
+    x = torch.from_numpy(np.random.default_rng(seed + 1).standard_normal((m, k), dtype=np.float32)).cuda()
+    if spread:  # a unit 1e4 times the others, one 1e-6 of them, a row of zeros
+        x[:, :256] *= 1e4
+        x[m - 1] *= 1e-6
+        x[1] = 0
+    return q, w.reshape(n, k).double(), x
+
+
+def bound(w, x, units):
+    """Terms hold 2^-22 of a unit's largest value; a group's four instructions add with truncation (2^-23 of the largest
+    partial sum each), sums go on in f32: a few 2^-23 of sum |w| max|x| over each unit, and of the magnitudes added."""
+    import torch
+
+    m, k = x.shape
+    ax = x.double().abs().reshape(m, units, 256)
+    aw = w.abs().reshape(w.shape[0], units, 256)
+    peak = torch.einsum("mu,nu->mn", ax.amax(-1), aw.sum(-1))
+    return 2.0 ** -21 * peak + 1e-30
+
+
+@pytest.mark.parametrize("type_id", [synth.Q4_K, synth.MXFP4])
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("m", [3, 4, 5, 8])
+def test_products_match_float64(type_id, shape, m):
+    n, k = shape
+    q, w, x = setup(type_id, n, k, m, n + k + m, spread=m == 4)
+    got = QMatMul(q, n, k).forward(x)
+    err = (got.double() - x.double() @ w.T).abs()
+    assert bool((err <= bound(w, x, k // 256)).all()), float((err / bound(w, x, k // 256)).max())
+    assert bool((QMatMul(q, n, k).forward(x) == got).all())  # the order of the sums does not depend on timing
+
+
+@pytest.mark.parametrize("type_id", [synth.Q4_K, synth.MXFP4])
+@pytest.mark.parametrize("shape", [(40, 1024), (1000, 2048), (333, 4096), (70, 14336)])
+@pytest.mark.parametrize("m", [3, 8])
+def test_norm_residual_and_pair(type_id, shape, m):
+    import torch
+
+    from joshua_b200 import _lib
+
+    n, k = shape
+    L, st = _lib.lib(), torch.cuda.current_stream().cuda_stream
+    q, w, x = setup(type_id, n, k, m, 3 * n + m)
+    up, wu, _ = setup(type_id, n, k, m, 3 * n + m + 50)
+    norm = torch.rand(k, device="cuda") + 0.5
+    xn = x.double() * torch.rsqrt(x.double().pow(2).mean(1, keepdim=True) + 1e-6) * norm.double()
+    scale = 2.0  # the f32 norm rounds its values as much again
+    tol = scale * bound(w, xn.float(), k // 256)
+    out = torch.randn(m, n, device="cuda")
+    want = out.double() + xn @ w.T
+    tol_r = tol + 2.0 ** -23 * want.abs()
+    _lib.check(L.jq_matmul_norm_dev(q._h, m, k, n, x.data_ptr(), norm.data_ptr(), 1e-6, out.data_ptr(), out.data_ptr(), st))
+    assert bool(((out.double() - want).abs() <= tol_r).all())
+    for clamp in (0.0, 0.7):
+        g, u = xn @ w.T, xn @ wu.T
+        tol_u = scale * bound(wu, xn.float(), k // 256)
+        if clamp:
+            g, u = g.clamp(max=clamp), u.clamp(-clamp, clamp)
+        s = g * torch.sigmoid(g)
+        # silu changes by at most 1.1 of its argument's change
+        tol_p = 1.1 * tol * u.abs() + (s.abs() + 1.1 * tol) * tol_u + 2.0 ** -20 * (s * u).abs() + 1e-30
+        dst = torch.empty(m, n, device="cuda")
+        _lib.check(L.jq_matmul_swiglu_norm_dev(q._h, up._h, m, k, n, x.data_ptr(), norm.data_ptr(), 1e-6, dst.data_ptr(),
+                                               clamp, st))
+        assert bool(((dst.double() - s * u).abs() <= tol_p).all()), float(((dst.double() - s * u).abs() / tol_p).max())
