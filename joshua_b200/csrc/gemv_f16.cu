@@ -459,55 +459,73 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_f16_kernel(const __grid_const
             store(held_tile, gate, v);
         };
         uint32_t at = 0, par = 0, rb = 0;  // the team's next stage, its buffer of partial sums
+        // Activations: a warp takes one unit (or every 16th) of every row (of every pn-th, where the units are few), four rows'
+        // loads ahead of their use.
+        const uint32_t pn = U < NCW ? NCW / U : 1, pu = U < NCW ? cw % U : cw, pr = cw / max(U, 1u) * (U < NCW ? 1 : 0);
+        const uint32_t p_rows = U < NCW && pr >= pn ? 0 : TOK;  // 16 is no multiple of U: the last warps rest
+        float row_scale = 1.0f;                                 // of row `lane`
         if (ga.norm_w != nullptr) {
             // the rows' sums of squares: units in unit order (in the idle buffers of partial sums), ranks in rank order
-            for (uint32_t i = cw; i < U * ga.m; i += NCW) {
-                const uint32_t row = i / U, u = i - row * U;
-                float v[8], ss = 0.0f;
-                load_run<TYPE>(ga.x + (uint64_t)row * k + (uint64_t)(unit0 + u) * 256, lane, v);
+            for (uint32_t u = pu; u < U; u += NCW > U ? U : NCW)
+                for (uint32_t r0 = pr; r0 < min(p_rows, ga.m); r0 += 4 * pn) {
+                    float v[4][8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) ss = fmaf(v[j], v[j], ss);
+                    for (uint32_t j = 0; j < 4; ++j)
+                        load_run<TYPE>(ga.x + (uint64_t)min(r0 + j * pn, ga.m - 1) * k + (uint64_t)(unit0 + u) * 256, lane, v[j]);
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
-                if (lane == 0) s_red[u * TOK + row] = ss;
-            }
-            asm volatile("bar.sync 1, %0;" ::"n"(NCW * 32) : "memory");
-            if (warp == 1) {
-                if (lane < ga.m) {
-                    float ss = 0.0f;
-                    for (uint32_t u = 0; u < U; ++u) ss += s_red[u * TOK + lane];
-                    const uint32_t at = smem_u32(s_rs + rank * GEMV_F16_MAX_M + lane);
-                    if (split == 1) s_rs[lane] = ss;
-                    else
-                        for (uint32_t r = 0; r < split; ++r)
-                            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(map_rank(at, r)), "f"(ss) : "memory");
+                    for (uint32_t j = 0; j < 4; ++j) {
+                        float ss = 0.0f;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) ss = fmaf(v[j][i], v[j][i], ss);
+#pragma unroll
+                        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
+                        if (lane == 0 && r0 + j * pn < ga.m) s_red[u * TOK + r0 + j * pn] = ss;
+                    }
                 }
-                if (split > 1) {
+            asm volatile("bar.sync 1, %0;" ::"n"(NCW * 32) : "memory");
+            float ss = 0.0f;
+            if (lane < ga.m)
+#pragma unroll 4
+                for (uint32_t u = 0; u < U; ++u) ss += s_red[u * TOK + lane];
+            if (split > 1) {
+                if (warp == 1) {
+                    if (lane < ga.m)
+                        for (uint32_t r = 0; r < split; ++r)
+                            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(map_rank(smem_u32(s_rs + rank * GEMV_F16_MAX_M + lane), r)), "f"(ss) : "memory");
                     asm volatile("fence.acq_rel.cluster;" ::: "memory");
                     __syncwarp();
                     if (lane < split) arrive_rank(&norm_full, lane);
-                } else {
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&norm_full);
                 }
+                check(__all_sync(0xFFFFFFFFu, mbar_wait_cluster(&norm_full, 0)));
+                ss = 0.0f;
+                if (lane < ga.m)
+                    for (uint32_t r = 0; r < split; ++r) ss += s_rs[r * GEMV_F16_MAX_M + lane];
             }
-            check(__all_sync(0xFFFFFFFFu, split > 1 ? mbar_wait_cluster(&norm_full, 0) : mbar_wait(&norm_full, 0)));
+            row_scale = rsqrtf(ss / (float)k + ga.norm_eps);
         }
-        for (uint32_t i = cw; i < U * TOK; i += NCW) {
-            const uint32_t row = i / U, u = i - row * U;
-            float v[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-            if (row < ga.m) {
-                load_run<TYPE>(ga.x + (uint64_t)row * k + (uint64_t)(unit0 + u) * 256, lane, v);
-                if (ga.norm_w != nullptr) {
-                    float w[8], ss = 0.0f;
-                    load_run<TYPE>(ga.norm_w + (uint64_t)(unit0 + u) * 256, lane, w);
-                    for (uint32_t r = 0; r < split; ++r) ss += s_rs[r * GEMV_F16_MAX_M + row];
-                    const float rs = rsqrtf(ss / (float)k + ga.norm_eps);
+        for (uint32_t u = pu; u < U; u += NCW > U ? U : NCW) {
+            float w[8];
+            if (ga.norm_w != nullptr) load_run<TYPE>(ga.norm_w + (uint64_t)(unit0 + u) * 256, lane, w);
+            for (uint32_t r0 = pr; r0 < p_rows; r0 += 4 * pn) {
+                float v[4][8];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) v[j] = v[j] * rs * w[j];
+                for (uint32_t j = 0; j < 4; ++j)
+                    load_run<TYPE>(ga.x + (uint64_t)min(r0 + j * pn, ga.m - 1) * k + (uint64_t)(unit0 + u) * 256, lane, v[j]);
+#pragma unroll
+                for (uint32_t j = 0; j < 4; ++j) {
+                    const uint32_t row = r0 + j * pn;
+                    if (row >= TOK) break;
+                    if (row >= ga.m) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) v[j][i] = 0.0f;
+                    } else if (ga.norm_w != nullptr) {
+                        const float rs = __shfl_sync(0xFFFFFFFFu, row_scale, row);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) v[j][i] = v[j][i] * rs * w[i];
+                    }
+                    split_unit<TYPE, PACK>(v[j], lane, row, smem + u * S::ACT_UNIT);
                 }
             }
-            split_unit<TYPE, PACK>(v, lane, row, smem + u * S::ACT_UNIT);
         }
         asm volatile("bar.sync 1, %0;" ::"n"(NCW * 32) : "memory");
         for (uint32_t ti = team < n_teams ? team : tiles; ti < tiles; ti += n_teams) {  // (warps that do not fill a team: none)
