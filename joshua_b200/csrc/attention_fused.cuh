@@ -70,13 +70,19 @@ __device__ __forceinline__ void att_trace(const AttnArgs& a, bool on, int slot) 
     }
 }
 
+// What an item requests before it knows its position (see below), from the number of items.
+enum AttLoad { ATT_ALL, ATT_LIVE, ATT_LATE };
+
 // One (chunk, kv head, sequence) item.  tid = 0..255, the whole CTA; s_f: the item's shared
 // memory (attention_fused_smem_floats floats); s_last: one shared word.
 //
-// MANY: the launch holds more items than SMs.  An item then looks at the position first and leaves, without a load, if
+// LOAD: ATT_LIVE and ATT_LATE: the launch holds more items than SMs.  An item then looks at the position first and leaves, without a load, if
 // its chunk lies behind it: with one wave the extra trip to L2 costs more than the loads, with several the dead items'
 // rows are most of the traffic (16 of 17 chunks of a 1056-position cache at the start of a sequence).
-template <uint32_t HD, uint32_t G, bool MANY>
+// ATT_LATE: more than two items an SM.  The V rows are requested behind the scores, in the registers that held K: four CTAs
+// an SM instead of two hide the second trip.  Measured, decode steps of the dense model, eight sequences at 512: the kernel
+// 27.8 -> 20 us; with few live items (three sequences of the routed-expert model at 100) the step is 1 % slower that way.
+template <uint32_t HD, uint32_t G, AttLoad LOAD>
 __device__ __forceinline__ void attention_fused_item_t(const AttnArgs& a, uint32_t chunk, uint32_t kvh, uint32_t sg,
                                                        uint32_t b, uint32_t tid, float* s_f, uint32_t* s_last) {
     constexpr uint32_t NW = ATT_FUSED_THREADS / 32;
@@ -110,7 +116,7 @@ __device__ __forceinline__ void attention_fused_item_t(const AttnArgs& a, uint32
 
     // ── every independent load first: position, rotary inputs, the chunk's K rows and V rows ──
     const int32_t p_raw = __ldcg(a.pos + b);
-    if (MANY && p_raw >= 0 && (uint32_t)p_raw < max_ctx && t0 > (uint32_t)p_raw) return;
+    if (LOAD != ATT_ALL && p_raw >= 0 && (uint32_t)p_raw < max_ctx && t0 > (uint32_t)p_raw) return;
     float ra[ROT_PER], rb[ROT_PER];
 #pragma unroll
     for (uint32_t r = 0; r < ROT_PER; ++r) {
@@ -135,11 +141,14 @@ __device__ __forceinline__ void attention_fused_item_t(const AttnArgs& a, uint32
     const bool v_thread = tid < PG * HD;
     const uint32_t vpg = tid / HD, vi = tid - vpg * HD;
     float vreg[VN];
+    auto load_v = [&] {
 #pragma unroll
-    for (uint32_t u = 0; u < VN; ++u) {
-        const uint32_t t = t0 + vpg + u * PG;
-        vreg[u] = (v_thread && t < max_ctx) ? Vc[(uint64_t)t * HD + vi] : 0.0f;
-    }
+        for (uint32_t u = 0; u < VN; ++u) {
+            const uint32_t t = t0 + vpg + u * PG;
+            vreg[u] = (v_thread && t < max_ctx) ? Vc[(uint64_t)t * HD + vi] : 0.0f;
+        }
+    };
+    if (LOAD != ATT_LATE) load_v();
 
     // A position outside [0, max_ctx) has no cache row: store nothing, attend to nothing, say so.  Every item of
     // the sequence takes this exit, so the arrival counters stay at zero.
@@ -223,6 +232,7 @@ __device__ __forceinline__ void attention_fused_item_t(const AttnArgs& a, uint32
             }
         }
     }
+    if (LOAD == ATT_LATE) load_v();
     __syncthreads();
     att_trace(a, tr, 2);
     // per head: maximum, exponentials, their sum (one warp per head; a lane holds positions lane, lane + 32)

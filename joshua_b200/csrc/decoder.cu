@@ -251,16 +251,15 @@ __global__ void __launch_bounds__(128) attention_merge_kernel(const float* __res
 
 // Decode attention in ONE launch, straight from the fused qkv row (attention_fused.cuh): one CTA per
 // (chunk, kv head, sequence).  One kernel per head size and heads per item, so that small shapes do not pay for the
-// registers of the largest; with more items than SMs two CTAs share an SM.  Measured on the Llama-8B heads, eight
-// sequences at position 512: 27.8 us, against 46 us with one kernel of 254 registers for all shapes, which also loaded
-// dead chunks.
-template <uint32_t HD, uint32_t G, bool MANY>
-__global__ void __launch_bounds__(ATT_FUSED_THREADS, MANY && HD <= 128 ? 2 : 1) attention_fused_kernel(AttnArgs a) {
+// registers of the largest; with more items than SMs two CTAs share an SM, with more than twice as many four.
+template <uint32_t HD, uint32_t G, AttLoad LOAD>
+__global__ void __launch_bounds__(ATT_FUSED_THREADS, HD > 128 || LOAD == ATT_ALL ? 1 : LOAD == ATT_LIVE ? 2 : 4)
+    attention_fused_kernel(AttnArgs a) {
     extern __shared__ float s_f[];
     __shared__ uint32_t s_last;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     pdl_wait_();
-    attention_fused_item_t<HD, G, MANY>(a, blockIdx.x, blockIdx.y / a.gsplit, blockIdx.y % a.gsplit, blockIdx.z,
+    attention_fused_item_t<HD, G, LOAD>(a, blockIdx.x, blockIdx.y / a.gsplit, blockIdx.y % a.gsplit, blockIdx.z,
                                            threadIdx.x, s_f, &s_last);
 }
 
@@ -514,13 +513,15 @@ cudaError_t launch_attention_fused(const float* qkv, const int32_t* pos, uint32_
     a.qk_eps = qk_eps;
     size_t smem = (size_t)attention_fused_smem_floats(nq / a.gsplit, nkv, hd, a.n_chunks) * 4;
     const dim3 grid(a.n_chunks, nkv * a.gsplit, batch);
-    const bool many = (uint64_t)a.n_chunks * grid.y * batch > (uint64_t)num_sms();
+    const uint64_t items = (uint64_t)a.n_chunks * grid.y * batch, sms = (uint64_t)num_sms();
     const uint32_t G = nq / nkv / a.gsplit;
     cudaError_t e = cudaErrorInvalidValue;
 #define JQ_ATT_CASE(HD, GV)                                                                                            \
     if (hd == HD && G == GV)                                                                                           \
-        e = many ? launch_pdl(attention_fused_kernel<HD, GV, true>, grid, ATT_FUSED_THREADS, smem, s, a)               \
-                 : launch_pdl(attention_fused_kernel<HD, GV, false>, grid, ATT_FUSED_THREADS, smem, s, a);
+        e = items <= sms ? launch_pdl(attention_fused_kernel<HD, GV, ATT_ALL>, grid, ATT_FUSED_THREADS, smem, s, a)    \
+            : items <= 2 * sms || HD > 128                                                                             \
+                ? launch_pdl(attention_fused_kernel<HD, GV, ATT_LIVE>, grid, ATT_FUSED_THREADS, smem, s, a)            \
+                : launch_pdl(attention_fused_kernel<HD, GV, (HD > 128 ? ATT_LIVE : ATT_LATE)>, grid, ATT_FUSED_THREADS, smem, s, a);
     JQ_ATT_CASE(64, 1)
     JQ_ATT_CASE(64, 2)
     JQ_ATT_CASE(64, 4)
