@@ -43,17 +43,26 @@
 // narrow tiles keep two windows in flight, because their products take less time than a conversion.
 //
 // Order of k inside four columns: 0, 2, 1, 3, for the activations and the weights alike, so that a mask picks two
-// codes out of a word of nibbles or bytes (MXFP4, which looks its values up, keeps the plain order).
+// codes out of a word of nibbles or bytes.  MXFP4: i, i + 16 of a block, the two nibbles of a byte, which one instruction
+// converts.
 //
-// What bounds it: the converters' instruction issue (2 to 3 instructions per weight at first, all in address arithmetic
-// and unpacking; the masks and the flattened copies brought that to about 1.5), the tensor pipe from 128 rows on.
+// What bounds it: the converters' instruction issue (1.5 to 2.5 instructions a weight, waits included, at 2.6 to 3.0 a cycle on
+// narrow tiles), the tensor pipe from 128 rows on (70 % while a tile runs).
 //
-// Warps: 16 converters, warp (q = w % 4, g = w / 4) owns weight rows 32q .. 32q+31 (the tensor-memory lanes it may
-// touch) and the columns 64g .. 64g+63 of every window; the four warps of a quarter share the staged raw bytes of a
-// window and meet once per window on a named barrier (an mbarrier round trip costs some 200 cycles here).  Warps 16 to
-// 19 issue the MMAs and the TMA copies: an instruction takes about 30 cycles to issue, so narrow tiles have an issuer per
-// step, which also copies its step's activation tiles; wide ones, whose steps share an accumulator, have one, and another
-// warp copies.
+// Warps: 16 converters, warp (q = w % 4, g = w / 4) owns weight rows 32q .. 32q+31 (the tensor-memory lanes it may touch) and
+// the columns 64g .. 64g+63 of every window.  Warps 16 to 19 issue the MMAs and the TMA copies: an instruction takes about 30
+// cycles to issue, so narrow tiles have an issuer per step, which also copies its step's activation tiles; wide ones, whose
+// steps share an accumulator, have one, and another warp copies.  Warps 20 to 23 copy raw weights (cp.async, eight lanes a
+// row, so that an address serves all of a row's vectors; a whole window completes on one mbarrier): when the converters
+// copied their own rows and met on a named barrier, that was an eighth of their instructions and a fifth of their waits.
+// Against that form, and with the issuer of wide tiles waiting for its next step between the halves of the one it issues:
+// Q2_K 4096 x 14336, 333 rows 146 -> 121 us, Q4_K 28672 x 4096, 512 rows 250 -> 239 (at 1.4 GHz under the power cap) and
+// 4096 x 14336 127 -> 122, Q8_0 5120 x 2048, 1000 rows 86 -> 81, Q4_K 28672 x 4096, 16 rows 50.5 -> 47.3.  MXFP4, whose nibbles
+// one conversion instruction a pair now unpacks (64 a cycle and SM) instead of three byte permutes and masks: 28672 x 7168,
+// 20 / 64 / 200 rows 102 / 203 / 252 -> 76 / 150 / 206 us.  It costs launches of one or two windows a CTA 0.2 to 0.5 us
+// (Q4_K 5000 x 1536, 13 rows 8.8 -> 9.1; Q6_K, whose rows are copied by the word, 2048 x 4096, 33 rows 15.8 -> 17.1).
+// Two further forms were slower: an owner per window instead of per step (half the instructions, but a chain of single warps:
+// 28672 x 4096, 16 rows 56 us) and a persistent loop over tiles on top of it.
 //
 // Few tiles (small n, or few rows of lhs) leave SMs idle: then a cluster of S CTAs splits k, every CTA leaves its
 // partial tile in its shared memory, and each adds a share of the tile over the cluster in rank order (distributed
@@ -79,7 +88,11 @@ namespace {
 constexpr int HM = 128;           // weight rows per CTA = MMA M = TMEM lanes
 constexpr int H_CONV = 16;        // converter / epilogue warps
 constexpr int H_ISSUE = 4;        // issuing warps: one per 64-column step where the steps have their own accumulators
-constexpr int H_THREADS = (H_CONV + H_ISSUE) * 32;  // five warps a scheduler: 96 registers a thread (six: 80, and spills)
+constexpr int H_COPY = 4;         // warps that copy raw weights
+constexpr int H_THREADS = (H_CONV + H_ISSUE + H_COPY) * 32;
+// Registers a thread: the launch has 768 x 80 = 61440; the converters take 512 x 96 of them, the others 256 x 48.
+constexpr int H_REGS_CONV = 96, H_REGS_REST = 48;
+static_assert(H_CONV * 32 * H_REGS_CONV + (H_ISSUE + H_COPY) * 32 * H_REGS_REST <= H_THREADS * 80, "registers");
 constexpr uint32_t H_STEPS = 4;   // 64-column steps per 256-column window = ring stages
 
 template <uint32_t TYPE>
@@ -156,7 +169,7 @@ struct Tile {
 // sums [m][k / 256][32]: the 16 group sums of a window, first terms then second terms; inv[m]: the inverse of the row's
 // scale, negative where some window has one of its own; rel[k / 256][m]: the inverse of that.  With norm_w the rows are RMS-normalised first: the values split are x * rs * norm_w.
 __global__ void __launch_bounds__(256) split_f16_kernel(const float* __restrict__ x, uint32_t k,
-                                                        const float* __restrict__ norm_w, float eps, int plain_order,
+                                                        const float* __restrict__ norm_w, float eps, int nibble_pairs,
                                                         __half* __restrict__ hi,
                                                         __half* __restrict__ lo, __half* __restrict__ sums,
                                                         float* __restrict__ inv, float* __restrict__ rel) {
@@ -201,9 +214,11 @@ __global__ void __launch_bounds__(256) split_f16_kernel(const float* __restrict_
         float amax = 0.0f;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            float4 v = __ldg(xr + 4 * g + j);
+            // 16 values in a row, or 0 .. 7 and 16 .. 23 (8 .. 15 and 24 .. 31) of 32
+            const uint32_t at = nibble_pairs ? 8 * (g >> 1) + 2 * (g & 1) + 4 * (j >> 1) + (j & 1) : 4 * g + j;
+            float4 v = __ldg(xr + at);
             if (norm_w) {
-                const float4 w = __ldg(nr + 4 * g + j);
+                const float4 w = __ldg(nr + at);
                 v.x = v.x * rs * w.x, v.y = v.y * rs * w.y, v.z = v.z * rs * w.z, v.w = v.w * rs * w.w;
             }
             amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
@@ -218,20 +233,21 @@ __global__ void __launch_bounds__(256) split_f16_kernel(const float* __restrict_
         if ((g & 15) == 0) rel[(uint64_t)(g >> 4) * gridDim.x + row] = __uint_as_float((uint32_t)(127 - extra) << 23);
         uint32_t h[8], l[8];
         float sum = 0.0f;
+        float f[16];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            float4 v = val[j];
-            v.x *= scale, v.y *= scale, v.z *= scale, v.w *= scale;
-            sum += (v.x + v.y) + (v.z + v.w);
-            if (!plain_order) {
-                const float t = v.y;
-                v.y = v.z, v.z = t;
-            }
-            const __half2 h0 = __floats2half2_rn(v.x, v.y), h1 = __floats2half2_rn(v.z, v.w);
-            const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
-            const __half2 l0 = __floats2half2_rn(v.x - f0.x, v.y - f0.y), l1 = __floats2half2_rn(v.z - f1.x, v.w - f1.y);
-            h[2 * j] = *reinterpret_cast<const uint32_t*>(&h0), h[2 * j + 1] = *reinterpret_cast<const uint32_t*>(&h1);
-            l[2 * j] = *reinterpret_cast<const uint32_t*>(&l0), l[2 * j + 1] = *reinterpret_cast<const uint32_t*>(&l1);
+            const float4 v = val[j];
+            f[4 * j] = v.x * scale, f[4 * j + 1] = v.y * scale, f[4 * j + 2] = v.z * scale, f[4 * j + 3] = v.w * scale;
+            sum += (f[4 * j] + f[4 * j + 1]) + (f[4 * j + 2] + f[4 * j + 3]);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int p = 4 * (j >> 1) + (j & 1);  // 0, 2 and 1, 3 of four
+            const float x0 = nibble_pairs ? f[j] : f[p], x1 = nibble_pairs ? f[8 + j] : f[p + 2];
+            const __half2 t = __floats2half2_rn(x0, x1);
+            const float2 back = __half22float2(t);
+            const __half2 rest = __floats2half2_rn(x0 - back.x, x1 - back.y);
+            h[j] = *reinterpret_cast<const uint32_t*>(&t), l[j] = *reinterpret_cast<const uint32_t*>(&rest);
         }
         uint4* hp = reinterpret_cast<uint4*>(hi + (uint64_t)row * k + 16 * g);
         uint4* lp = reinterpret_cast<uint4*>(lo + (uint64_t)row * k + 16 * g);
@@ -293,6 +309,17 @@ __device__ __forceinline__ uint32_t and_or(uint32_t w, uint32_t mask, uint32_t b
     uint32_t r;
     asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(w), "r"(mask), "r"(bits));
     return r;
+}
+// The two E2M1 values of every byte (low nibble, high nibble) as halves.
+__device__ __forceinline__ void e2m1_pairs(uint32_t w, uint32_t (&v)[4]) {
+    asm("{\n\t.reg .b8 a, b, c, d;\n\t"
+        "mov.b32 {a, b, c, d}, %4;\n\t"
+        "cvt.rn.f16x2.e2m1x2 %0, a;\n\t"
+        "cvt.rn.f16x2.e2m1x2 %1, b;\n\t"
+        "cvt.rn.f16x2.e2m1x2 %2, c;\n\t"
+        "cvt.rn.f16x2.e2m1x2 %3, d;\n\t}"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+        : "r"(w));
 }
 // a small integer (0..255) in both halves, exact
 __device__ __forceinline__ __half2 int_h2(uint32_t v) {
@@ -451,8 +478,6 @@ __device__ __forceinline__ void convert64(uint32_t u, uint32_t g, const RowWin& 
             put(h, a, a);
         }
     } else if constexpr (TYPE == T_MXFP4) {
-        // f16 of 0, .5, 1, 1.5, 2, 3, 4, 6 has a zero low byte: the table holds the high bytes
-        const uint32_t T0 = 0x3E3C3800u, T1 = 0x46444240u;
 #pragma unroll
         for (uint32_t h = 0; h < 2; ++h) {
             const uint32_t blk = u + 17 * (2 * g + h), e = s8(blk);
@@ -463,17 +488,11 @@ __device__ __forceinline__ void convert64(uint32_t u, uint32_t g, const RowWin& 
             if (gone && ((w[0] | w[1] | w[2] | w[3]) & 0x77777777u)) *lost = 1;  // a block of zeros has exponent 0
             uint32_t a[16];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const uint32_t m = w[q] & 0x77777777u, w4 = w[q] << 4;
+            for (int q = 0; q < 4; ++q) {  // a byte: values i and i + 16
+                uint32_t v[4];
+                e2m1_pairs(w[q], v);
 #pragma unroll
-                for (int hw = 0; hw < 2; ++hw) {  // two code bytes: values 4q + 2hw, + 1 (low nibbles) and those + 16
-                    // bytes {low of byte 0, high of byte 0, low of byte 1, high of byte 1}, then their sign bits (the top
-                    // bits of the bytes of w << 4 and w)
-                    const uint32_t mag = __byte_perm(T0, T1, hw ? m >> 16 : m & 0xFFFFu);
-                    const uint32_t v = and_or(__byte_perm(w[q], w4, hw ? 0x3726 : 0x1504), 0x80808080u, mag);
-                    a[2 * q + hw] = as_u32(__hmul2(as_h2(__byte_perm(v, 0, 0x2404)), s2));
-                    a[8 + 2 * q + hw] = as_u32(__hmul2(as_h2(__byte_perm(v, 0, 0x3414)), s2));
-                }
+                for (int j = 0; j < 4; ++j) a[4 * q + j] = as_u32(__hmul2(as_h2(v[j]), s2));
             }
             put(h, a, a);
         }
@@ -548,11 +567,12 @@ __device__ __forceinline__ void add_lost(const uint8_t* row, uint32_t win0, uint
                 decode_unit<TYPE>(win, u, w, false);
 #pragma unroll 1
                 for (uint32_t t = 0; t < n_tok; ++t) {
-                    const uint64_t at = (tok0 + t) * k + (uint64_t)c * 256 + u * 8;
+                    // where the split kernel put the values: 0, 2, 1, 3 of four, or value i of a block's half at 2 i (+ 1)
+                    const uint64_t at = (tok0 + t) * k + (uint64_t)c * 256 + (TYPE == T_MXFP4 ? (u & ~3u) * 8 + (u & 1) * 16 + (u >> 1 & 1) : u * 8);
                     float v = 0.0f;
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        const int o = TYPE == T_MXFP4 ? j : (j & 4) | ((j & 1) << 1) | ((j >> 1) & 1);  // 0, 2, 1, 3
+                        const int o = TYPE == T_MXFP4 ? 2 * j : (j & 4) | ((j & 1) << 1) | ((j >> 1) & 1);
                         v = fmaf(w[j], __half2float(x_hi[at + o]) + __half2float(x_lo[at + o]), v);
                     }
                     if (mine) add(t, v * rel[c * m_rows + tok0 + t]);
@@ -606,7 +626,8 @@ __global__ void __launch_bounds__(H_THREADS, 1)
     const uint32_t scales = smem_u32(raw + BUFS * RAW_BUF);
     uint2* s_grid = reinterpret_cast<uint2*>(raw + BUFS * RAW_BUF + S::SCALE_B);
     // full[s]: the step's four converter warps + the TMA thread (and the tiles' bytes); empty[s]: the MMAs' commit
-    __shared__ uint64_t full[S::STAGES], empty[S::STAGES], acc_full[2], acc_empty[S::ACCS];
+    // raw_full / raw_empty: the copying threads, the converter warps
+    __shared__ uint64_t full[S::STAGES], empty[S::STAGES], acc_full[2], acc_empty[S::ACCS], raw_full[BUFS], raw_empty[BUFS];
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag, lost_flag;
 
@@ -635,6 +656,40 @@ __global__ void __launch_bounds__(H_THREADS, 1)
     const uint32_t n_windows = (uint32_t)((uint64_t)all_windows * (rank + 1) / split) - win0;
     const uint32_t n_chunks = n_windows * T::UNITS;  // accumulated windows of 256 columns
 
+    // A staged window of the tile's rows: eight lanes a row, a warp 32 rows, four at a time; the rest of a row of vectors that
+    // is no multiple of eight falls to the first lanes.
+    constexpr uint32_t ROW_VECS = WIN_WORDS * 4 / VEC, COPIERS = H_COPY * 32;
+    static_assert(COPIERS == HM, "a copying warp takes 32 rows");
+    auto copy_window = [&](uint32_t wn) {
+        const uint32_t buf = wn % BUFS, r0 = (warp & 3) * 32 + (lane >> 3), v0 = lane & 7;
+        const uint32_t last = (uint32_t)min((uint64_t)HM, n - row0) - 1;  // rows past n repeat the last one
+        const uint8_t* base = w + row0 * row_bytes + (uint64_t)(win0 + wn) * (WIN_WORDS * 4) + v0 * VEC;
+        const uint32_t dst0 = smem_u32(raw) + buf * RAW_BUF + r0 * (RAW_STRIDE * 4) + v0 * VEC;
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) {
+            const uint8_t* src = base + (uint64_t)min(r0 + 4 * j, last) * (uint32_t)row_bytes;
+            const uint32_t dst = dst0 + 4 * j * (RAW_STRIDE * 4);
+#pragma unroll
+            for (uint32_t c = 0; c < (ROW_VECS + 7) / 8; ++c) {
+                if (8 * c + 8 > ROW_VECS && v0 >= ROW_VECS - 8 * c) continue;
+                if constexpr (VEC == 16)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 8 * c * VEC), "l"(src + 8 * c * VEC) : "memory");
+                else
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst + 8 * c * VEC), "l"(src + 8 * c * VEC), "n"(VEC) : "memory");
+            }
+        }
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&raw_full[buf])) : "memory");
+    };
+    // the first window is on its way before anything else is set up (more of them would hold up the rest: Q6_K, 4096 x 4096, 20
+    // rows 16.6 -> 18.0 us)
+    if (warp >= H_CONV + H_ISSUE) {
+        if (tid == (H_CONV + H_ISSUE) * 32) {
+            for (uint32_t b = 0; b < BUFS; ++b) mbar_init(&raw_full[b], COPIERS), mbar_init(&raw_empty[b], H_CONV);
+            mbar_fence_init();
+        }
+        asm volatile("bar.sync 2, %0;" ::"n"(COPIERS) : "memory");
+        copy_window(0);
+    }
     if (tid == 0) {
         for (uint32_t s = 0; s < S::STAGES; ++s) {
             mbar_init(&full[s], 4 + 1);
@@ -661,6 +716,9 @@ __global__ void __launch_bounds__(H_THREADS, 1)
     const uint32_t tmem_d = tmem_base_slot;
 
     if (warp < H_CONV) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(H_REGS_CONV));
+        // narrow tiles: polls, a chain of short waits is what they spend their time on; wide ones sleep and leave the issue slots
+        auto converter_wait = [](uint64_t* bar, uint32_t parity) { return S::FINE ? mbar_wait_polling(bar, parity) : mbar_wait(bar, parity); };
         const uint32_t q = warp & 3, g = warp >> 2;
         const uint32_t lane_base = (q * 32) << 16;  // this warp's quarter of the tensor-memory lanes
         float sums[MY_COLS];
@@ -707,7 +765,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
         // read back window c: this warp's columns of its accumulator, or all columns of the accumulator of its own step
         auto drain = [&](uint32_t c, float f) -> bool {
             uint64_t* ready = S::FINE ? &empty[(c % S::WINDOWS) * H_STEPS + g] : &acc_full[c & 1];
-            if (!__all_sync(0xFFFFFFFFu, mbar_wait_polling(ready, (S::FINE ? c / S::WINDOWS : c >> 1) & 1))) return false;
+            if (!__all_sync(0xFFFFFFFFu, converter_wait(ready, (S::FINE ? c / S::WINDOWS : c >> 1) & 1))) return false;
             tc_fence_after();
             add_acc(S::FINE ? g * N_TILE : (c & 1) * N_TILE + g * MY_COLS, f);
             tc_fence_before();
@@ -715,44 +773,12 @@ __global__ void __launch_bounds__(H_THREADS, 1)
             if (lane == 0) mbar_arrive(&acc_empty[S::FINE ? g : c & 1]);
             return true;
         };
-        // this warp's 8 of the quarter's 32 rows of window wn, as one run of vectors over the lanes
         const uint32_t raw_q = smem_u32(raw) + q * 32 * RAW_STRIDE * 4;
-        constexpr uint32_t ROW_VECS = WIN_WORDS * 4 / VEC, COPIES = (8 * ROW_VECS + 31) / 32;
-        const uint64_t gr0 = min(row0 + q * 32 + g * 8, n - 1);
-        const uint32_t rows_left = (uint32_t)min((uint64_t)8, n - gr0);  // rows past n repeat the last one
-        const uint8_t* src0 = w + gr0 * row_bytes + (uint64_t)win0 * (WIN_WORDS * 4);
-        const uint32_t row_bytes32 = (uint32_t)row_bytes;
-        auto copy_window = [&](uint32_t wn) {
-            if (wn < n_windows) {
-                const uint32_t dst0 = raw_q + (wn % BUFS) * RAW_BUF + g * 8 * RAW_STRIDE * 4;
-                const uint8_t* src = src0 + (uint64_t)wn * (WIN_WORDS * 4);
-                auto one = [&](uint32_t i) {
-                    const uint32_t rr = i / ROW_VECS, c = i - rr * ROW_VECS;
-                    const uint8_t* sp = src + ((uint64_t)min(rr, rows_left - 1) * row_bytes32 + c * VEC);
-                    const uint32_t dp = dst0 + rr * (RAW_STRIDE * 4) + c * VEC;
-                    if constexpr (VEC == 16)
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dp), "l"(sp) : "memory");
-                    else
-                        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dp), "l"(sp), "n"(VEC) : "memory");
-                };
-#pragma unroll
-                for (uint32_t j = 0; j < COPIES; ++j)
-                    if (32 * j + 32 <= 8 * ROW_VECS || lane + 32 * j < 8 * ROW_VECS) one(lane + 32 * j);
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");  // an empty group past the last window
-        };
         bool ok = true;
         float f_prev = 0.0f;
-#pragma unroll
-        for (uint32_t b = 0; b + 1 < BUFS; ++b) copy_window(b);
         auto window = [&](uint32_t wn, auto with_scales) {
             const uint32_t buf = wn % BUFS;
-            // my copies of this window have landed; meet the quarter's other warps, which also means that all four are
-            // through with the window before: its buffer takes a later one.  A warp whose wait ran out keeps coming
-            // here, so that no other waits for it.
-            asm volatile("cp.async.wait_group %0;" ::"n"(BUFS - 2) : "memory");
-            asm volatile("bar.sync %0, 128;" ::"r"(2 + q) : "memory");
-            copy_window(wn + BUFS - 1);
+            ok = __all_sync(0xFFFFFFFFu, converter_wait(&raw_full[buf], (wn / BUFS) & 1));
 #pragma unroll 1
             for (uint32_t cc = 0; cc < T::UNITS && ok; ++cc) {
                 const uint32_t c = wn * T::UNITS + cc;
@@ -760,7 +786,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
                 const RowWin rw = row_window<TYPE, S::NB>(u, S::FINE ? 2 * g : 0);
                 // the stage's columns must have been read by the MMAs that used them last
                 const uint32_t ph = c % S::WINDOWS, st = ph * H_STEPS + g;
-                ok = __all_sync(0xFFFFFFFFu, mbar_wait_polling(&empty[st], ((c / S::WINDOWS) & 1) ^ 1));
+                ok = __all_sync(0xFFFFFFFFu, converter_wait(&empty[st], ((c / S::WINDOWS) & 1) ^ 1));
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t acol = tmem_d + lane_base + S::ACC_COLS + st * S::A_COLS;
@@ -774,6 +800,10 @@ __global__ void __launch_bounds__(H_THREADS, 1)
                         convert_minima<TYPE>(u, rw, a);
                         tmem_st16(tmem_d + lane_base + S::MIN_COL0 + 16 * ph, a);
                     }
+                }
+                if (cc == T::UNITS - 1) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&raw_empty[buf]);
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 tc_fence_before();
@@ -791,12 +821,11 @@ __global__ void __launch_bounds__(H_THREADS, 1)
             }
         };
         uint32_t wn = 0;
-        for (; wn < n_windows && !scaled; ++wn) window(wn, std::false_type{});  // the first window tells
-        for (; wn < n_windows; ++wn) window(wn, std::true_type{});
+        for (; wn < n_windows && !scaled && ok; ++wn) window(wn, std::false_type{});  // the first window tells
+        for (; wn < n_windows && ok; ++wn) window(wn, std::true_type{});
         if (scaled) rescale(n_chunks - 1);
         if (ok && n_chunks > 0) ok = drain(n_chunks - 1, f_prev);
         if (scaled) rescale(n_chunks);
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
         if (!ok) abort_flag = 1;
         pdl_wait();  // (a warp that gave up in its first window)
         // The ring and the staged bytes are idle once every converter is here: the last read-back waited for this CTA's
@@ -833,7 +862,8 @@ __global__ void __launch_bounds__(H_THREADS, 1)
                                       });
             }
         }
-    } else {
+    } else if (warp < H_CONV + H_ISSUE) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(H_REGS_REST));
         // ── issuers (their waits sleep: polling warps take issue slots from the converters) ──
         constexpr uint32_t idesc = umma_idesc_f16(N_TILE);
         const uint32_t base0 = smem_u32(smem);
@@ -857,29 +887,33 @@ __global__ void __launch_bounds__(H_THREADS, 1)
             __syncwarp();
             return true;
         };
-        // steps G0 .. G1 - 1 of every window; compile-time, so that the descriptors need no arithmetic but a stage's offset
+        // Steps G0 .. G1 - 1 of every window; compile-time, so that the descriptors need no arithmetic but a stage's offset.
+        // The tensor pipe takes few instructions ahead: on wide tiles the waits for the next step stand between the two halves of
+        // this one's, or the pipe runs dry at every step (some 220 cycles, 600 at a new window).
         auto issue = [&](auto G0, auto G1) {
+            // whether step g of window c can start: its accumulator's last contents have been read back, its operands are there
+            auto can_start = [&](uint32_t c, uint32_t g) {
+                if (S::FINE ? c >= 1 : g == 0 && c >= 2)
+                    if (!mbar_wait(&acc_empty[S::FINE ? g : c & 1], (S::FINE ? c - 1 : (c >> 1) - 1) & 1)) return false;
+                return mbar_wait(&full[c % S::WINDOWS * H_STEPS + g], (c / S::WINDOWS) & 1);
+            };
             if (S::FINE) {
                 pdl_wait();
                 for (uint32_t c = 0; c < S::WINDOWS && c < n_chunks && ok; ++c) ok = load(c, G0.value);
             }
+            if (ok && n_chunks > 0) ok = __all_sync(0xFFFFFFFFu, can_start(0, G0.value));
+            const bool leader = elect_one();
             for (uint32_t c = 0; c < n_chunks && ok; ++c) {
                 const uint32_t ph = c % S::WINDOWS;
 #pragma unroll
                 for (uint32_t g = G0.value; g < G1.value; ++g) {
                     const uint32_t st = ph * H_STEPS + g, acc = S::FINE ? g : c & 1, d = tmem_d + acc * N_TILE;
-                    // the accumulator's last contents must have been read back
-                    if (S::FINE ? c >= 1 : g == 0 && c >= 2) {
-                        ok = __all_sync(0xFFFFFFFFu, mbar_wait(&acc_empty[acc], (S::FINE ? c - 1 : (c >> 1) - 1) & 1));
-                        if (!ok) break;
-                    }
-                    ok = __all_sync(0xFFFFFFFFu, mbar_wait(&full[st], (c / S::WINDOWS) & 1));
-                    if (!ok) break;
+                    const uint64_t so = (uint64_t)st * (STAGE >> 4);
+                    const uint32_t a1 = tmem_d + S::ACC_COLS + st * S::A_COLS;
+                    [[maybe_unused]] const uint32_t a2 = a1 + 32;
+                    const bool fresh = S::FINE || g == 0;
                     tc_fence_after();  // the converters' tcgen05.st / .ld
-                    if (elect_one()) {
-                        const uint64_t so = (uint64_t)st * (STAGE >> 4);
-                        const uint32_t a1 = tmem_d + S::ACC_COLS + st * S::A_COLS, a2 = a1 + 32;
-                        const bool fresh = S::FINE || g == 0;
+                    if (leader) {
                         // small products first, while the accumulator is small.  16 columns an instruction: 8 columns of A,
                         // 32 bytes of B's swizzled rows.
 #pragma unroll
@@ -897,15 +931,28 @@ __global__ void __launch_bounds__(H_THREADS, 1)
                                 umma_f16_ts(d, am, ds, idesc, 1);
                             }
                         }
+                    }
+                    bool next = true;
+                    if (!S::FINE) {  // the next step does not depend on this one's products
+                        __syncwarp();
+                        if (!(g == G1.value - 1 && c + 1 == n_chunks))
+                            next = g + 1 < G1.value ? can_start(c, g + 1) : can_start(c + 1, G0.value);
+                        next = __all_sync(0xFFFFFFFFu, next);
+                    }
+                    if (leader) {
 #pragma unroll
                         for (uint32_t kk = 0; kk < 4; ++kk) umma_f16_ts(d, a1 + kk * 8, d0_hi + so + kk * 2, idesc, 1);
                         umma_commit(&empty[st]);  // the weight columns and the activation tiles of the stage are free
                         if (!S::FINE && g == H_STEPS - 1) umma_commit(&acc_full[acc]);
                     }
                     __syncwarp();
+                    ok = next;
+                    if (!ok) break;
                 }
+                if (!S::FINE) continue;
                 // the next window's tiles: its stage's last products are a window behind, or (one window) the ones above
-                if (S::FINE && ok && c + 1 >= S::WINDOWS && c + 1 < n_chunks) ok = load(c + 1, G0.value);
+                if (ok && c + 1 >= S::WINDOWS && c + 1 < n_chunks) ok = load(c + 1, G0.value);
+                if (ok && c + 1 < n_chunks) ok = __all_sync(0xFFFFFFFFu, can_start(c + 1, G0.value));
             }
         };
         using std::integral_constant;
@@ -922,6 +969,16 @@ __global__ void __launch_bounds__(H_THREADS, 1)
             for (uint32_t c = 0; c < n_chunks && ok; ++c)
                 for (uint32_t g = 0; g < H_STEPS && ok; ++g) ok = load(c, g);
         }
+        if (!ok && lane == 0) abort_flag = 1;
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(H_REGS_REST));
+        // ── copies of raw weights ──
+        bool ok = true;
+        for (uint32_t wn = 1; wn < n_windows && ok; ++wn) {
+            ok = __all_sync(0xFFFFFFFFu, mbar_wait(&raw_empty[wn % BUFS], ((wn / BUFS) & 1) ^ 1));
+            if (ok) copy_window(wn);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
         if (!ok && lane == 0) abort_flag = 1;
     }
     tc_fence_before();
