@@ -310,17 +310,6 @@ __device__ __forceinline__ uint32_t and_or(uint32_t w, uint32_t mask, uint32_t b
     asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(w), "r"(mask), "r"(bits));
     return r;
 }
-// The two E2M1 values of every byte (low nibble, high nibble) as halves.
-__device__ __forceinline__ void e2m1_pairs(uint32_t w, uint32_t (&v)[4]) {
-    asm("{\n\t.reg .b8 a, b, c, d;\n\t"
-        "mov.b32 {a, b, c, d}, %4;\n\t"
-        "cvt.rn.f16x2.e2m1x2 %0, a;\n\t"
-        "cvt.rn.f16x2.e2m1x2 %1, b;\n\t"
-        "cvt.rn.f16x2.e2m1x2 %2, c;\n\t"
-        "cvt.rn.f16x2.e2m1x2 %3, d;\n\t}"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
-        : "r"(w));
-}
 // a small integer (0..255) in both halves, exact
 __device__ __forceinline__ __half2 int_h2(uint32_t v) {
     return __hsub2(as_h2(__byte_perm(v, 0x64646464u, 0x4040)), __float2half2_rn(1024.0f));

@@ -6,7 +6,7 @@
 //     sum_c x_c (s_g q_c - o_g)  =  s_g sum_c x_c q_c  -  o_g sum_c x_c     (per group of 32 columns g)
 //
 // but the products are mma.sync.m16n8k16 on f16: the codes are exact f16 numbers (Q4_K: a nibble left in place under the
-// exponent of 1024 or 64, less that; MXFP4: the high byte of the E2M1 value from a byte permute), and an activation is two f16
+// exponent of 1024 or 64, less that; MXFP4: one conversion instruction a pair), and an activation is two f16
 // terms under a power-of-two scale of its 256 columns (largest value just below 2^15): 22 to 24 bits of every value within 2^17
 // of the largest.  A group is four chained instructions, low terms first, whose exact products the tensor core adds with
 // truncation; its sum is scaled and added round-to-nearest.  The minima of Q4_K are one more instruction per 256 columns:
@@ -204,8 +204,6 @@ __device__ __forceinline__ void f16_unit(const uint8_t* u0, const uint8_t* u1, c
         acc[2] = fmaf(fmaf(cm[2], e1, us[2] * f1.x), sx.x, acc[2]);
         acc[3] = fmaf(fmaf(cm[3], e1, us[3] * f1.x), sx.y, acc[3]);
     } else {
-        // f16 of 0, .5, 1, 1.5, 2, 3, 4, 6 has a zero low byte: the table holds the high bytes
-        const uint32_t T0 = 0x3E3C3800u, T1 = 0x46444240u;
         auto block_scale = [](uint32_t e) {  // 2^(e - 127); e = 255 zeroes the block, e = 0 is subnormal
             return e == 255u ? 0.0f : __uint_as_float(e ? e << 23 : 0x00400000u);
         };
@@ -221,16 +219,9 @@ __device__ __forceinline__ void f16_unit(const uint8_t* u0, const uint8_t* u1, c
                     const uint8_t* p = (r ? u1 : u0) + at - mis + 4 * t;
                     uint32_t w = lds32(p);
                     if (mis) w = __funnelshift_r(w, lds32(p + 4), 8 * mis);
-                    const uint32_t m = w & 0x77777777u, w4 = w << 4;
-#pragma unroll
-                    for (uint32_t hw = 0; hw < 2; ++hw) {
-                        // bytes {low, high of byte 2 hw, low, high of byte 2 hw + 1}, then their sign bits; a low and a high
-                        // pair of halves
-                        const uint32_t mag = __byte_perm(T0, T1, hw ? m >> 16 : m);
-                        const uint32_t v = and_or(__byte_perm(w, w4, hw ? 0x3726 : 0x1504), 0x80808080u, mag);
-                        a[j][hw][r] = (v << 8) & 0xFF00FF00u;
-                        a[j][hw][2 + r] = v & 0xFF00FF00u;
-                    }
+                    uint32_t v[4];
+                    e2m1_pairs(w, v);  // values 4t + i and 16 + 4t + i of the block
+                    a[j][0][r] = v[0], a[j][0][2 + r] = v[1], a[j][1][r] = v[2], a[j][1][2 + r] = v[3];
                     s[r][j] = block_scale((r ? u1 : u0)[17 * (G0 + j)]);
                 }
             }
@@ -269,8 +260,8 @@ __device__ __forceinline__ void split_unit(float (&v)[8], uint32_t lane, uint32_
     uint32_t hi[4], lo[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        // pairs as the weights come: Q4_K 0 2, 1 3, 4 6, 5 7; MXFP4 0 1, 16 17, 2 3, 18 19 (the run is 0 .. 3, 16 .. 19)
-        const int p = TYPE == T_MXFP4 ? (j & 1) * 4 + (j >> 1) * 2 : (j >> 1) * 4 + (j & 1), q = p + (TYPE == T_MXFP4 ? 1 : 2);
+        // pairs as the weights come: Q4_K 0 2, 1 3, 4 6, 5 7; MXFP4 0 16, 1 17, 2 18, 3 19 (the run is 0 .. 3, 16 .. 19)
+        const int p = TYPE == T_MXFP4 ? j : (j >> 1) * 4 + (j & 1), q = p + (TYPE == T_MXFP4 ? 4 : 2);
         const __half2 h = __floats2half2_rn(v[p], v[q]);
         const float2 f = __half22float2(h);
         const __half2 l = __floats2half2_rn(v[p] - f.x, v[q] - f.y);

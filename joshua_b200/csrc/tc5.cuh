@@ -118,6 +118,17 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t r[16]) 
         : "memory");
 }
 
+// The two E2M1 values of every byte (low nibble, high nibble) as halves.
+__device__ __forceinline__ void e2m1_pairs(uint32_t w, uint32_t (&v)[4]) {
+    asm("{\n\t.reg .b8 a, b, c, d;\n\t"
+        "mov.b32 {a, b, c, d}, %4;\n\t"
+        "cvt.rn.f16x2.e2m1x2 %0, a;\n\t"
+        "cvt.rn.f16x2.e2m1x2 %1, b;\n\t"
+        "cvt.rn.f16x2.e2m1x2 %2, c;\n\t"
+        "cvt.rn.f16x2.e2m1x2 %3, d;\n\t}"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+        : "r"(w));
+}
 // Barrier over all threads of the cluster (every thread of every CTA takes part).
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
