@@ -249,6 +249,46 @@ def test_rotary_append_of_a_long_prompt_equals_short_pieces(nq, nkv, hd, norms):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("nq,nkv,hd,norms", [(3, 1, 256, True), (10, 2, 64, False), (16, 8, 128, True), (2, 1, 96, True)])
+def test_rotary_append_by_rows_equals_by_heads(nq, nkv, hd, norms):
+    """Hundreds of sequences take one CTA a row (heads of 64, 128 and 256), a few one a head: the same bits; a position outside
+    the cache stores nothing either way."""
+    import torch
+
+    from joshua_b200 import _lib
+
+    L = _lib.lib()
+    B, max_ctx, theta = 320, 40, 10000.0
+    g = torch.Generator(device="cuda").manual_seed(hd)
+    qkv = torch.randn(B, (nq + 2 * nkv) * hd, device="cuda", generator=g)
+    pos = torch.randint(0, max_ctx, (B,), dtype=torch.int32, device="cuda", generator=g)
+    pos[7], pos[301] = max_ctx, -1
+    s = torch.cuda.current_stream().cuda_stream
+    if norms:   # the entry with norms takes one sequence: rows are the tokens of a prompt
+        w, p0, ctx = torch.rand(2, hd, device="cuda", generator=g), torch.zeros(1, dtype=torch.int32, device="cuda"), B - 3
+    outs = []
+    for piece in (B, 32):
+        q = torch.full((B, nq * hd), 9.0, device="cuda")
+        flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+        k = torch.full((nkv, B - 3, hd) if norms else (B, nkv, max_ctx, hd), 9.0, device="cuda")
+        v = k.clone()
+        for a in range(0, B, piece):
+            if norms:
+                p0.fill_(a)
+                _lib.check(L.jq_rope_append_prefill_dev(qkv[a:].data_ptr(), p0.data_ptr(), piece, nq, nkv, hd, ctx, theta,
+                                                        w[0].data_ptr(), w[1].data_ptr(), 1e-6, q[a:].data_ptr(), k.data_ptr(),
+                                                        v.data_ptr(), flag.data_ptr(), s))
+            else:
+                _lib.check(L.jq_rope_append_dev(qkv[a:].data_ptr(), pos[a:].data_ptr(), piece, nq, nkv, hd, max_ctx, theta,
+                                                q[a:].data_ptr(), k[a:].data_ptr(), v[a:].data_ptr(), flag.data_ptr(), s))
+        torch.cuda.synchronize()
+        assert int(flag.item()) == 1
+        outs.append((q, k, v))
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
+    assert bool((outs[0][0][[-1] if norms else [7, 301]] == 9.0).all())
+
+
 def test_positions_beyond_the_cache_store_nothing_and_raise_the_flag():
     """Stepping past max_ctx: the kernels skip the append and the attention for that sequence, the flag is set,
     the memory behind the cache is untouched (the cache is the front part of a larger canary-filled buffer),
