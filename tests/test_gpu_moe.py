@@ -316,6 +316,25 @@ def test_routing_of_many_tokens_equals_small_batches(hidden, n_expert):
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
 
 
+@pytest.mark.parametrize("hidden,n_expert,T", [(256, 130, 16), (512, 5, 17), (1280, 384, 45)])
+def test_router_tiles_add_like_the_warp_per_token(hidden, n_expert, T):
+    """From 16 tokens on the logits come from tiles of 16 tokens and 16 experts: the sums of the kernel for fewer, bit for bit."""
+    import torch
+
+    rng = np.random.default_rng(T)
+    layer = Moe(MoeConfig(gating=GATE_SOFTMAX, n_expert=n_expert, n_used=4, hidden=hidden, inter=256),
+                rng.standard_normal((n_expert, hidden)).astype(np.float32), None, None, None)
+    layer.reserve(T)
+    x = torch.randn(T, hidden, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+    got = []
+    for starts, piece in (([0], T), (list(range(0, T - 9, 9)) + [T - 9], 9)):
+        ids, wts = torch.zeros(T, 4, dtype=torch.int32, device="cuda"), torch.zeros(T, 4, device="cuda")
+        for a in starts:
+            layer.route_dev(x[a:a + piece], ids[a:a + piece], wts[a:a + piece])
+        got.append((ids, wts))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
 @pytest.mark.parametrize("tokens", [31, 32, 90])
 def test_experts_on_tiles_match_the_oracle_and_replay(tokens):
     """From 32 tokens the experts of Q4_K and MXFP4 banks run on tiles; the replay entry still finds the job list."""
