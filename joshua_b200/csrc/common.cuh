@@ -112,7 +112,8 @@ cudaError_t launch_gemm_tc(uint32_t type, const uint8_t* w, uint64_t n, uint64_t
 // banks in one launch (gate and up).  dst[row, n] is written for the tiles' rows only.  Two lists on the device:
 // `narrow` (tiles of at most 32 rows, run as 32-token tiles) and `wide`, their lengths in counts[0] and counts[1]
 // (device memory, read by the kernels: the launches cover max_narrow / max_wide entries and the surplus CTAs
-// leave at once), so that no host read stands between the routing and the products.  False from
+// leave at once), so that no host read stands between the routing and the products.  With a list, row r of the product is
+// row list[r] of x, for r below *n_list.  False from
 // gemm_f16_grouped_supports = shapes this form does not take (the caller then runs one product per expert).
 struct GemmTile {
     uint32_t expert;
@@ -122,8 +123,8 @@ struct GemmTile {
 };
 bool gemm_f16_grouped_supports(uint32_t type, const uint8_t* bank, uint64_t n, uint64_t k);
 cudaError_t launch_gemm_f16_grouped(uint32_t type, const uint8_t* bank_a, const uint8_t* bank_b, uint64_t expert_bytes,
-                                   uint64_t n, uint64_t k, const float* x, uint64_t rows, float* dst_a, float* dst_b,
-                                   const GemmTile* narrow, uint32_t max_narrow, const GemmTile* wide, uint32_t max_wide,
+                                   uint64_t n, uint64_t k, const float* x, const uint32_t* list, const uint32_t* n_list,
+                                   uint64_t rows, float* dst_a, float* dst_b, const GemmTile* narrow, uint32_t max_narrow, const GemmTile* wide, uint32_t max_wide,
                                    const uint32_t* counts, void* scratch, int* error_flag, cudaStream_t s);
 
 // One unit of grouped (MoE) work: up to 8 consecutive positions of the expert-sorted activation list,

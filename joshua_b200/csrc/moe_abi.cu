@@ -226,16 +226,15 @@ int32_t run_experts_bucketed(jq_moe* m, const float* x, uint64_t T, uint64_t P, 
             (reinterpret_cast<uintptr_t>(small_jobs + max_small) + 15) & ~(uintptr_t)15);
         void* scratch = nullptr;
         JQ_CUDA(m->ctx->scratch_for(s, SLOT_TILES, bucket_scratch_bytes(c, P), &scratch));
-        JQ_CUDA(jq::launch_moe_gather(x, m->list_token, m->n_list, (uint32_t)P, c.hidden, xs, s));
         JQ_CUDA(jq::launch_moe_tiles(m->jobs, m->n_jobs, m->n_list, c.n_expert, min_rows, narrow, wide, small_jobs, counts, s));
-        JQ_CUDA(jq::launch_gemm_f16_grouped(m->gate->type, m->gate->dev, m->up->dev, m->gate_expert_bytes, c.inter, c.hidden, xs, P,
-                                           gbuf, ubuf, narrow, max_narrow, wide, max_wide, counts, scratch, m->ctx->status_dev, s));
+        JQ_CUDA(jq::launch_gemm_f16_grouped(m->gate->type, m->gate->dev, m->up->dev, m->gate_expert_bytes, c.inter, c.hidden, x,
+                                           m->list_token, m->n_list, P, gbuf, ubuf, narrow, max_narrow, wide, max_wide, counts, scratch, m->ctx->status_dev, s));
         // SwiGLU over every list row (rows of the small experts hold nothing yet; the decode kernel writes them next)
         JQ_CUDA(jq::launch_swiglu_rows(gbuf, ubuf, counts + 2, (uint32_t)P, c.inter, c.clamp, m->hidden, s));
         if (!all_tiles)
             if (int32_t rc = run_experts(m, x, T, P, rows_per_job, s, nullptr, 0.0f, small_jobs, counts + 3, 1)) return rc;
         JQ_CUDA(jq::launch_gemm_f16_grouped(m->down->type, m->down->dev, nullptr, m->down_expert_bytes, c.hidden, c.inter,
-                                           m->hidden, P, m->out, nullptr, narrow, max_narrow, wide, max_wide, counts, scratch,
+                                           m->hidden, nullptr, nullptr, P, m->out, nullptr, narrow, max_narrow, wide, max_wide, counts, scratch,
                                            m->ctx->status_dev, s));
         return all_tiles ? jq::OK : run_experts(m, x, T, P, rows_per_job, s, nullptr, 0.0f, small_jobs, counts + 3, 2);
     }
