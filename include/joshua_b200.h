@@ -186,7 +186,7 @@ int32_t jq_weight_from_float(jq_weight* w, const float* xs, uint64_t len);
 
 /* `Mlp::forward` up to the down projection: dst = silu(gate x) * up x, with the
  * optional clamp of src/quantized_deepseek4.rs:445-462 (clamp <= 0: none)
- * (src/quantized_qwen3_moe.rs:396-402).  One launch of the decode kernel, or
+ * (src/quantized_qwen3_moe.rs:396-402).  One launch of a decode kernel, or
  * one of the tile GEMM for both tensors and the combine (gate passes through
  * dst_dev, up through the stream's scratch), by the rows of jq_matmul_norm_dev.
  * lhs_dev 16-byte aligned. */
@@ -215,11 +215,12 @@ int32_t jq_matmul_swiglu_norm_dev(const jq_weight* gate, const jq_weight* up, ui
  * (the `RmsNorm` -> `QMatMul::forward` -> `xs + residual` pattern of
  * src/quantized_qwen3_moe.rs:793-819).  norm_w_dev and residual_dev are each
  * optional; residual_dev may be dst_dev; lhs_dev and norm_w_dev 16-byte
- * aligned.  One launch of the decode kernel for up to eight rows whose
- * activation planes fit its shared memory; a split and a product of the tile
- * GEMM, norm and residual inside, from five rows of Q4_K (or of planes that do
- * not fit), nine of the other types and 17 of Q8_0 on; the separate kernels for
- * what neither takes. */
+ * aligned.  One launch of a decode kernel for three to eight rows of Q4_K and
+ * MXFP4 with k >= 1024 (dst_dev not over lhs_dev) and for up to eight rows whose
+ * activation planes fit the other one's shared memory; a split and a product of
+ * the tile GEMM, norm and residual inside, from five rows of Q4_K (or of planes
+ * that do not fit) that no decode kernel took, nine of the other types and 17 of
+ * Q8_0 on; the separate kernels for what none takes. */
 int32_t jq_matmul_norm_dev(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, const float* lhs_dev,
                            const float* norm_w_dev, float eps, const float* residual_dev, float* dst_dev,
                            void* stream);

@@ -45,7 +45,7 @@ int32_t jq_matmul_swiglu_dev(const jq_weight* gate, const jq_weight* up, uint64_
     if (int32_t rc = check_vectors("jq_matmul_swiglu_dev", lhs_dev, nullptr)) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     jq_ctx* ctx = gate->ctx;
-    if (jq_uses_gemv_f16(gate, m, k, n, true) && jq_uses_gemv_f16(up, m, k, n, true)) {
+    if (jq_uses_gemv_f16(gate, m, k, n, lhs_dev, dst_dev, true) && jq_uses_gemv_f16(up, m, k, n, lhs_dev, dst_dev, true)) {
         JQ_CUDA(jq::launch_gemv_f16(gate->type, gate->dev, up->dev, n, k, lhs_dev, m, nullptr, 0.0f, nullptr, clamp, dst_dev,
                                     ctx->status_dev, s));
         return jq::OK;
@@ -81,7 +81,7 @@ int32_t jq_matmul_swiglu_norm_dev(const jq_weight* gate, const jq_weight* up, ui
     // the plain entry names the fault (or finds nothing to do) before anything is launched
     if (!shapes_ok) return jq_matmul_swiglu_dev(gate, up, m, k, n, lhs_dev, dst_dev, clamp, stream);
     if (int32_t rc = check_vectors("jq_matmul_swiglu_norm_dev", lhs_dev, norm_w_dev)) return rc;
-    if (jq_uses_gemv_f16(gate, m, k, n, true) && jq_uses_gemv_f16(up, m, k, n, true)) {
+    if (jq_uses_gemv_f16(gate, m, k, n, lhs_dev, dst_dev, true) && jq_uses_gemv_f16(up, m, k, n, lhs_dev, dst_dev, true)) {
         JQ_CUDA(jq::launch_gemv_f16(gate->type, gate->dev, up->dev, n, k, lhs_dev, m, norm_w_dev, eps, nullptr, clamp, dst_dev,
                                     ctx->status_dev, s));
         return jq::OK;
@@ -112,7 +112,7 @@ int32_t jq_matmul_norm_dev(const jq_weight* w, uint64_t m, uint64_t k, uint64_t 
                            lhs_dev && dst_dev;
     if (!shapes_ok) return jq_matmul_t_dev(w, m, k, n, lhs_dev, dst_dev, stream);  // as above
     if (int32_t rc = check_vectors("jq_matmul_norm_dev", lhs_dev, norm_w_dev)) return rc;
-    if (jq_uses_gemv_f16(w, m, k, n, false)) {
+    if (jq_uses_gemv_f16(w, m, k, n, lhs_dev, dst_dev, false)) {
         JQ_CUDA(jq::launch_gemv_f16(w->type, w->dev, nullptr, n, k, lhs_dev, m, norm_w_dev, eps, residual_dev, 0.0f, dst_dev,
                                     ctx->status_dev, s));
         return jq::OK;

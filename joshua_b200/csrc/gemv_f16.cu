@@ -25,7 +25,7 @@
 // Error against float64 (2-norm, N(0, 1) rows): Q4_K 1.8e-7 to 2.1e-7, MXFP4 0.9e-7 to 1.1e-7; the routes before 2.4e-7 to
 // 3.8e-7 and 1.2e-7 to 1.5e-7.  Algorithmic bytes per launch: n*k/B*S (weights) + 4*m*(k + n).  What bounds it: the consumers'
 // instructions, 460 (four rows) to 600 (eight) per 16 x 256 unit at 1.8 to 2.8 a cycle.  Measured, four / eight rows, before (the
-// integer kernel / the tile GEMM and its split) and now: Q4_K 28672 x 4096 27.4 / 49.5 and 22.2 / 28.3 us, 6144 x 4096 11.4 /
+// integer kernel / the tile GEMM and its split) and now: Q4_K 28672 x 4096 27.4 / 49.5 and 22.2 / 27.5 us, 6144 x 4096 11.4 /
 // 25.9 and 9.2 / 12.2, 4096 x 4096 9.8 / 11.5 and 7.4 / 10.2, 4096 x 14336 24.6 / 28.5 and 18.3 / 22.8, 128256 x 4096 94 / 169 and
 // 73 / 96; MXFP4 28672 x 4096 41.5 (three rows) / 54.7 and 30.1 / 36.3, 7168 x 2048 11.6 / 18.2 and 7.2 / 9.2.
 //

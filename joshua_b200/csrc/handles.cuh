@@ -164,7 +164,7 @@ int32_t jq_matmul_device(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n,
                          cudaStream_t s);
 
 // Whether a product of m rows (pair: gate and up) runs on the f16 decode kernel.
-bool jq_uses_gemv_f16(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, bool pair);
+bool jq_uses_gemv_f16(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, const float* lhs, const float* dst, bool pair);
 
 // Whether a product of m rows runs on the f16 tile GEMM, and that product: dst = residual + norm(lhs) . W^T, with w_b (a
 // tensor of the same type and shape) also dst_b = norm(lhs) . W_b^T.  norm_w, residual and w_b may be NULL (abi.cu).

@@ -122,9 +122,9 @@ class LlamaDecoder:
     # ── one token ───────────────────────────────────────────────────────
     def step(self, stream=None) -> None:
         """Decode one token per sequence: reads self.token / self.pos, writes self.logits, the next
-        self.token and advances self.pos.  Launches only.  Five launches per layer for one sequence: the RMS
+        self.token and advances self.pos.  Launches only.  Five launches per layer for one to eight sequences of Q4_K: the RMS
         norms ride in the prologue of the matmul that consumes them, the residual adds in the epilogue of the
-        matmul that produces the branch, and rope + cache append + attention + merge are one kernel.  (From five
+        matmul that produces the branch, and rope + cache append + attention + merge are one kernel.  (From nine
         sequences on Q4_K linears run on the tile GEMM: a split and a product each, ten launches per layer.)
         self.x is the residual stream, updated in place."""
         L, c, B = _lib.lib(), self.cfg, self.batch
