@@ -27,7 +27,7 @@
 // instructions, 460 (four rows) to 600 (eight) per 16 x 256 unit at 1.8 to 2.8 a cycle.  Measured, four / eight rows, before (the
 // integer kernel / the tile GEMM and its split) and now: Q4_K 28672 x 4096 27.4 / 49.5 and 22.2 / 27.5 us, 6144 x 4096 11.4 /
 // 25.9 and 9.2 / 12.2, 4096 x 4096 9.8 / 11.5 and 7.4 / 10.2, 4096 x 14336 24.6 / 28.5 and 18.3 / 22.8, 128256 x 4096 94 / 169 and
-// 73 / 96; MXFP4 28672 x 4096 41.5 (three rows) / 54.7 and 30.1 / 36.3, 7168 x 2048 11.6 / 18.2 and 7.2 / 9.2.
+// 73 / 96; MXFP4 28672 x 4096 41.5 (three rows) / 54.7 and 23.7 / 30.3, 7168 x 2048 11.6 / 18.2 and 6.8 / 8.6.
 //
 // Every wait is bounded and raises the device status flag; threads that gave up still take part in the CTA's and the
 // cluster's barriers.
@@ -707,7 +707,8 @@ bool gemv_f16_supports(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, 
     };
     switch (type) {
         case T_Q4_K: return a % 16 == 0 && fits(std::integral_constant<uint32_t, T_Q4_K>{});
-        // five to eight rows with k split: 4096 x 7168 18.6 us, on tiles 17.2 (7168 x 16384 52.4 / 56.2)
+        // five to eight rows with k split: 4096 x 7168 18.6 us, on tiles 17.2 (7168 x 16384 52.4 / 56.2), both before the
+        // conversion instruction; the tiles take 14.6 with it
         case T_MXFP4: return a % 16 == 0 && fits(std::integral_constant<uint32_t, T_MXFP4>{}) && (m <= 4 || p.split == 1);
         default: return false;
     }
