@@ -67,7 +67,8 @@ void jq_free(jq_ctx* ctx);
 /* Every wait inside a kernel (on a copy in flight) is bounded; a kernel whose
  * wait runs out sets a device-visible flag and returns.  Host-buffer entries
  * check the flag themselves; callers of the *_dev entries poll it here after
- * synchronising their stream.  JQ_OK or JQ_E_TIMEOUT; a reported timeout is
+ * synchronising their stream (entries without a handle report to every context
+ * of their device).  JQ_OK or JQ_E_TIMEOUT; a reported timeout is
  * cleared, so the next call answers for the work after it.  (The reference's
  * counterpart is the deadline handling of its plugin shim, src/npu/shim.rs:1-8.) */
 int32_t jq_device_status(const jq_ctx* ctx);
@@ -262,7 +263,8 @@ int32_t jq_attention_fused_qknorm_dev(const float* qkv, const int32_t* pos, uint
  * jq_rope_append_prefill_dev: qkv [seq, (n_q + 2 n_kv) * head_dim] -> q_out [seq, n_q * head_dim] rotated (after the
  * optional per-head q / k norm), k and v appended to the cache of sequence 0 ([n_kv, max_ctx, head_dim]).
  * jq_attention_prefill_dev: out[s] = attention of token s over cache positions 0 .. pos0 + s (causal); head_dim 64
- * or 128.  Tokens that would run past max_ctx store nothing / the whole call does nothing, and *bad_pos_dev is set. */
+ * or 128.  Tokens that would run past max_ctx store nothing / the whole call does nothing, and *bad_pos_dev is set.
+ * A wait that ran out leaves NaN in the rows that it concerns, and jq_device_status reports it. */
 int32_t jq_rope_append_prefill_dev(const float* qkv, const int32_t* pos0, uint32_t seq, uint32_t n_q, uint32_t n_kv,
                                    uint32_t head_dim, uint32_t max_ctx, float theta, const float* q_norm_w,
                                    const float* k_norm_w, float qk_eps, float* q_out, float* cache_k, float* cache_v,

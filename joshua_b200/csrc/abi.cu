@@ -4,6 +4,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "handles.cuh"
 
@@ -68,7 +69,14 @@ int32_t validate_matmul(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, 
     return jq::OK;
 }
 
+struct EntryStatus {
+    std::atomic<int*> host{nullptr}, dev{nullptr};
+};
+EntryStatus g_entry_status[jq::MAX_DEVICES];  // by device
+
 }  // namespace
+
+int* jq_entry_status_flag() { return g_entry_status[jq::current_device()].dev.load(); }
 
 // (Batches of three to eight rows that gemv_f16.cu takes never ask.)
 // From nine rows on the other route is the decode kernel once per eight rows.  From five rows on, where the decode
@@ -160,12 +168,29 @@ namespace {
 // Reports a kernel wait that gave up, once: the flag is cleared as it is reported, so that one late peer or one
 // lost copy does not fail every later call on the context.
 int32_t check_device_status(const jq_ctx* ctx) {
-    volatile int* flag = static_cast<volatile int*>(ctx->status_host);
-    if (flag && *flag != 0) {
-        *flag = 0;
-        return jq_fail(jq::E_TIMEOUT, "a bounded wait inside a kernel gave up (device status flag was set)");
+    bool raised = false;
+    for (volatile int* flag : {static_cast<volatile int*>(ctx->status_host), static_cast<volatile int*>(g_entry_status[ctx->device % jq::MAX_DEVICES].host.load())})
+        if (flag && *flag != 0) *flag = 0, raised = true;
+    return raised ? jq_fail(jq::E_TIMEOUT, "a bounded wait inside a kernel gave up (device status flag was set)") : jq::OK;
+}
+
+// Makes the device's flag for entries without a context, once.
+cudaError_t make_entry_status(int device) {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> g(mu);
+    EntryStatus& st = g_entry_status[device % jq::MAX_DEVICES];
+    if (st.host.load()) return cudaSuccess;
+    int *host = nullptr, *dev = nullptr;
+    cudaError_t e = cudaHostAlloc(&host, sizeof(int), cudaHostAllocMapped);
+    if (e != cudaSuccess) return e;
+    if (e = cudaHostGetDevicePointer(&dev, host, 0); e != cudaSuccess) {
+        cudaFreeHost(host);
+        return e;
     }
-    return jq::OK;
+    *host = 0;
+    st.dev.store(dev);
+    st.host.store(host);
+    return cudaSuccess;
 }
 
 __global__ void f16_to_f32_kernel(const __half* in, float* out, uint64_t n) {
@@ -223,6 +248,7 @@ int32_t jq_init(int32_t device, jq_ctx** out) {
     if (const char* sm = std::getenv("JQ_SLICED_MAX_M")) c->sliced_max_m = std::strtoull(sm, nullptr, 10);
     cudaError_t he = cudaHostAlloc(&c->status_host, sizeof(int), cudaHostAllocMapped);
     if (he == cudaSuccess) he = cudaHostGetDevicePointer(&c->status_dev, c->status_host, 0);
+    if (he == cudaSuccess) he = make_entry_status(device);
     if (he != cudaSuccess) {
         delete c;
         return jq_fail_cuda(he, "jq_init: status flag");

@@ -27,8 +27,9 @@
 // 128 13.7 (27.0), 16 6.0 (10.8), one 5.8 (10.3); heads of 64, 1000 tokens 33.1 (152): ahead at every size, so it is the
 // only route.
 //
-// Every wait on an mbarrier is bounded; one that runs out raises bad_pos, leaves NaN in the rows of its CTA, and every
-// thread still reaches the common exit where tensor memory is released.
+// Every wait on an mbarrier is bounded.  A warp whose wait ran out hands nothing on (the waits that depend on it run out in
+// turn) but still comes to every named barrier that others expect it at, so that all warps reach the common exit, where
+// tensor memory is released.  The status flag is raised and the rows of the CTA are NaN.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -103,7 +104,7 @@ template <uint32_t HD>
 __global__ void __launch_bounds__(A_THREADS, 1)
     attention_prefill_kernel(const float* __restrict__ q, const float* __restrict__ cache_k, const float* __restrict__ cache_v,
                              const int32_t* __restrict__ pos, uint32_t seq, uint32_t nq, uint32_t nkv, uint32_t max_ctx,
-                             float* __restrict__ out, int32_t* __restrict__ bad_pos) {
+                             float* __restrict__ out, int32_t* __restrict__ bad_pos, int* __restrict__ error_flag) {
     using T = AttTile<HD>;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -115,6 +116,7 @@ __global__ void __launch_bounds__(A_THREADS, 1)
     __shared__ float s_row[2][2][AQ];                         // row maxima of the two halves
     __shared__ uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2], s_full, s_free, p_full, o_full;
     __shared__ uint64_t rk_full, rk_empty, rv_full, rv_empty;  // the raw rows
+    __shared__ uint64_t drained;                               // the products of a CTA that gives up
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
 
@@ -135,6 +137,7 @@ __global__ void __launch_bounds__(A_THREADS, 1)
         mbar_init(&rv_full, 1);
         mbar_init(&rk_empty, A_CONV);
         mbar_init(&rv_empty, A_CONV);
+        mbar_init(&drained, 1);
         abort_flag = 0;
         mbar_fence_init();
     }
@@ -156,9 +159,16 @@ __global__ void __launch_bounds__(A_THREADS, 1)
     if (!in_cache && tid == 0 && bad_pos) atomicExch(bad_pos, 1);
     const uint32_t n_keys = in_cache ? (uint32_t)p0 + min(seq, s0 + AQ) : 0;  // keys the newest query of the tile sees
     const uint32_t n_tiles = (n_keys + AK - 1) / AK;
-    bool ok = true;
+    bool ok = true;  // the same in all lanes of a warp; once false, the warp waits for nothing more
     auto wait_all = [&](uint64_t* bar, uint32_t parity) {
-        ok = __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity)) && ok;
+        return ok = __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity));
+    };
+    // The common exit, where all warps meet: whether some wait of the CTA ran out.
+    auto leave = [&] {
+        if (!ok && lane == 0) *static_cast<volatile int*>(&abort_flag) = 1;
+        tc_fence_before();
+        asm volatile("bar.sync 6, %0;" ::"n"(A_THREADS) : "memory");
+        return *static_cast<volatile int*>(&abort_flag) != 0;
     };
 
     if (warp < A_SOFT) {
@@ -209,7 +219,7 @@ __global__ void __launch_bounds__(A_THREADS, 1)
 #pragma unroll
                     for (uint32_t i = 0; i < DN; ++i) o[i] *= alpha;
                 }
-                wait_all(&o_full, j & 1);
+                if (!wait_all(&o_full, j & 1)) return;
                 tc_fence_after();
 #pragma unroll
                 for (uint32_t c = 0; c < DN / 32; ++c) {
@@ -227,10 +237,11 @@ __global__ void __launch_bounds__(A_THREADS, 1)
                     }
                 }
             };
-            for (uint32_t j = 0; j < n_tiles && ok; ++j) {
+            uint32_t j = 0;  // tiles whose barrier this warp has come to
+            while (j < n_tiles) {
                 const uint32_t t0 = j * AK + half * 32;  // this thread's first key
                 float sc[32];
-                wait_all(&s_full, j & 1);
+                if (!wait_all(&s_full, j & 1)) break;
                 tc_fence_after();
                 {
                     uint32_t r[32];
@@ -276,7 +287,8 @@ __global__ void __launch_bounds__(A_THREADS, 1)
                 }
                 sum = sum * alpha + ps;
                 mx = nm;
-                if (j > 0) add_tile(j - 1, alpha_prev);  // its products have read the probabilities before these
+                if (j++ > 0) add_tile(j - 2, alpha_prev);  // its products have read the probabilities before these
+                if (!ok) break;
                 alpha_prev = alpha;
                 tmem_st16(lanes + T::P_HI + half * 16, hi);
                 tmem_st16(lanes + T::P_LO + half * 16, lo);
@@ -285,18 +297,21 @@ __global__ void __launch_bounds__(A_THREADS, 1)
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&p_full);
             }
+            for (; j < n_tiles; ++j) pair_bar();  // the other half of the rows may not have given up
             if (ok) add_tile(n_tiles - 1, alpha_prev);
             s_row[n_tiles & 1][half][row] = sum;
             pair_bar();
             const float inv = 1.0f / (sum + s_row[n_tiles & 1][half ^ 1][row]);
+            const float bad = leave() ? NAN : 0.0f;
             if (sr < seq) {
                 float4* dst = reinterpret_cast<float4*>(out + ((uint64_t)sr * nq + head) * HD + half * DN);
-                const float bad = ok ? 0.0f : NAN;
 #pragma unroll
                 for (uint32_t i = 0; i < DN / 4; ++i)
                     dst[i] = make_float4(fmaf(o[4 * i], inv, bad), fmaf(o[4 * i + 1], inv, bad), fmaf(o[4 * i + 2], inv, bad),
                                          fmaf(o[4 * i + 3], inv, bad));
             }
+        } else {
+            leave();
         }
     } else if (warp < A_SOFT + A_CONV) {
         // ── converters ──
@@ -316,11 +331,7 @@ __global__ void __launch_bounds__(A_THREADS, 1)
             __syncwarp();
             if (lane == 0) mbar_arrive(bar);
         };
-        for (uint32_t j = 0; j < n_tiles && ok; ++j) {
-            const uint32_t st = j & 1, freed = ((j >> 1) & 1) ^ 1;
-            const uint32_t live = n_keys - j * AK;  // rows of the tile that hold keys; the others are zeros
-            wait_all(&k_empty[st], freed);
-            wait_all(&rk_full, j & 1);
+        auto convert_keys = [&](uint32_t j, uint32_t st, uint32_t live) {
             // all loads, then all row maxima, then the terms: rows after one another took three times as long
             float4 kr[KIT][2];
             float row_max[KIT];
@@ -361,7 +372,15 @@ __global__ void __launch_bounds__(A_THREADS, 1)
                 if (chunk == 0) s_ks[j & 3][r] = bits_inverse(bits);
             }
             publish(&k_full[st]);
-            wait_all(&rv_full, j & 1);
+        };
+        auto meet = [&] { asm volatile("bar.sync 5, %0;" ::"n"(A_CONV * 32) : "memory"); };
+        uint32_t j = 0;  // tiles whose barrier this warp has come to
+        while (j < n_tiles) {
+            const uint32_t st = j & 1, freed = ((j >> 1) & 1) ^ 1;
+            const uint32_t live = n_keys - j * AK;  // rows of the tile that hold keys; the others are zeros
+            if (!wait_all(&k_empty[st], freed) || !wait_all(&rk_full, j & 1)) break;
+            convert_keys(j, st, live);
+            if (!wait_all(&rv_full, j & 1)) break;
             float amax = 0.0f, vr[KN];
 #pragma unroll
             for (uint32_t i = 0; i < KN; ++i) {
@@ -371,12 +390,13 @@ __global__ void __launch_bounds__(A_THREADS, 1)
             __syncwarp();
             if (lane == 0) mbar_arrive(&rv_empty);
             s_vmax[st][part * HD + vd] = amax;
-            asm volatile("bar.sync 5, %0;" ::"n"(A_CONV * 32) : "memory");
+            meet();
+            const uint32_t vs_at = j++ & 3;
+            if (!wait_all(&v_empty[st], freed)) break;
 #pragma unroll
             for (uint32_t p = 0; p < KP; ++p) amax = fmaxf(amax, s_vmax[st][p * HD + vd]);
             const uint32_t bits = term_scale_bits(amax);
             const float sc = bits_scale(bits);
-            wait_all(&v_empty[st], freed);
 #pragma unroll
             for (uint32_t c = 0; c < KN / 8; ++c) {
                 uint32_t hi[4], lo[4];
@@ -387,84 +407,95 @@ __global__ void __launch_bounds__(A_THREADS, 1)
                 st_shared_v4(at, hi);
                 st_shared_v4(at + T::V_PLANE, lo);
             }
-            if (part == 0) s_vs[j & 3][vd] = bits_inverse(bits);
+            if (part == 0) s_vs[vs_at][vd] = bits_inverse(bits);
             publish(&v_full[st]);
         }
+        for (; j < n_tiles; ++j) meet();  // the others may not have given up
+        leave();
     } else {
         // ── issuer (one warp issues, one copies, two have nothing to do) ──
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(A_REGS_ISSUE));
         if (warp == A_SOFT + A_CONV) {
-        constexpr uint32_t idesc_s = umma_idesc_f16(AK), idesc_o = umma_idesc_f16(HD);
-        const uint64_t dk = umma_desc(k_base), dv = umma_desc(v_base);
-        auto scores = [&](uint32_t j) {  // one accumulator per 64 dimensions, small products first
-            wait_all(&s_free, j & 1);    // the scores before have been read (the first: the query is in place)
-            wait_all(&k_full[j & 1], (j >> 1) & 1);
-            if (!ok) return;
-            tc_fence_after();
-            if (elect_one()) {
-                const uint64_t d0 = dk + (uint64_t)(j & 1) * (T::K_STAGE >> 4);
+            constexpr uint32_t idesc_s = umma_idesc_f16(AK), idesc_o = umma_idesc_f16(HD);
+            const uint64_t dk = umma_desc(k_base), dv = umma_desc(v_base);
+            auto scores = [&](uint32_t j) {  // one accumulator per 64 dimensions, small products first
+                // the scores before have been read (the first: the query is in place)
+                if (!wait_all(&s_free, j & 1) || !wait_all(&k_full[j & 1], (j >> 1) & 1)) return;
+                tc_fence_after();
+                if (elect_one()) {
+                    const uint64_t d0 = dk + (uint64_t)(j & 1) * (T::K_STAGE >> 4);
 #pragma unroll
-                for (uint32_t h = 0; h < T::HALVES; ++h) {
-                    const uint64_t hi = d0 + h * (T::K_PLANE >> 4), lo = hi + T::HALVES * (T::K_PLANE >> 4);
-                    const uint32_t d = tmem + T::S0 + 64 * h, a_hi = tmem + T::Q_HI + 32 * h, a_lo = tmem + T::Q_LO + 32 * h;
+                    for (uint32_t h = 0; h < T::HALVES; ++h) {
+                        const uint64_t hi = d0 + h * (T::K_PLANE >> 4), lo = hi + T::HALVES * (T::K_PLANE >> 4);
+                        const uint32_t d = tmem + T::S0 + 64 * h, a_hi = tmem + T::Q_HI + 32 * h, a_lo = tmem + T::Q_LO + 32 * h;
+#pragma unroll
+                        for (uint32_t kk = 0; kk < 4; ++kk) {
+                            umma_f16_ts(d, a_lo + 8 * kk, hi + 2 * kk, idesc_s, kk != 0);
+                            umma_f16_ts(d, a_hi + 8 * kk, lo + 2 * kk, idesc_s, 1);
+                        }
+#pragma unroll
+                        for (uint32_t kk = 0; kk < 4; ++kk) umma_f16_ts(d, a_hi + 8 * kk, hi + 2 * kk, idesc_s, 1);
+                    }
+                    umma_commit(&k_empty[j & 1]);
+                    umma_commit(&s_full);
+                }
+                __syncwarp();
+            };
+            if (n_tiles) scores(0);
+            for (uint32_t j = 0; j < n_tiles && ok; ++j) {
+                if (j + 1 < n_tiles) scores(j + 1);
+                // the probabilities are in place, the output before has been read
+                if (!ok || !wait_all(&v_full[j & 1], (j >> 1) & 1) || !wait_all(&p_full, j & 1)) break;
+                tc_fence_after();
+                if (elect_one()) {
+                    const uint64_t hi = dv + (uint64_t)(j & 1) * (T::V_STAGE >> 4), lo = hi + (T::V_PLANE >> 4);
+                    const uint32_t d = tmem + T::O, a_hi = tmem + T::P_HI, a_lo = tmem + T::P_LO;
 #pragma unroll
                     for (uint32_t kk = 0; kk < 4; ++kk) {
-                        umma_f16_ts(d, a_lo + 8 * kk, hi + 2 * kk, idesc_s, kk != 0);
-                        umma_f16_ts(d, a_hi + 8 * kk, lo + 2 * kk, idesc_s, 1);
+                        umma_f16_ts(d, a_lo + 8 * kk, hi + 2 * kk, idesc_o, kk != 0);
+                        umma_f16_ts(d, a_hi + 8 * kk, lo + 2 * kk, idesc_o, 1);
                     }
 #pragma unroll
-                    for (uint32_t kk = 0; kk < 4; ++kk) umma_f16_ts(d, a_hi + 8 * kk, hi + 2 * kk, idesc_s, 1);
+                    for (uint32_t kk = 0; kk < 4; ++kk) umma_f16_ts(d, a_hi + 8 * kk, hi + 2 * kk, idesc_o, 1);
+                    umma_commit(&v_empty[j & 1]);
+                    umma_commit(&o_full);
                 }
-                umma_commit(&k_empty[j & 1]);
-                umma_commit(&s_full);
+                __syncwarp();
             }
-            __syncwarp();
-        };
-        if (n_tiles) scores(0);
-        for (uint32_t j = 0; j < n_tiles && ok; ++j) {
-            if (j + 1 < n_tiles) scores(j + 1);
-            wait_all(&v_full[j & 1], (j >> 1) & 1);
-            wait_all(&p_full, j & 1);  // the probabilities are in place, the output before has been read
-            if (!ok) break;
-            tc_fence_after();
-            if (elect_one()) {
-                const uint64_t hi = dv + (uint64_t)(j & 1) * (T::V_STAGE >> 4), lo = hi + (T::V_PLANE >> 4);
-                const uint32_t d = tmem + T::O, a_hi = tmem + T::P_HI, a_lo = tmem + T::P_LO;
-#pragma unroll
-                for (uint32_t kk = 0; kk < 4; ++kk) {
-                    umma_f16_ts(d, a_lo + 8 * kk, hi + 2 * kk, idesc_o, kk != 0);
-                    umma_f16_ts(d, a_hi + 8 * kk, lo + 2 * kk, idesc_o, 1);
-                }
-#pragma unroll
-                for (uint32_t kk = 0; kk < 4; ++kk) umma_f16_ts(d, a_hi + 8 * kk, hi + 2 * kk, idesc_o, 1);
-                umma_commit(&v_empty[j & 1]);
-                umma_commit(&o_full);
+            if (!ok) {  // products in flight still use tensor memory and the tiles
+                if (elect_one()) umma_commit(&drained);
+                __syncwarp();
+                mbar_wait(&drained, 0);
             }
-            __syncwarp();
-        }
         } else if (warp == A_SOFT + A_CONV + 1) {
             // ── loader: a tile's rows are one run of memory ──
             const float* K = cache_k + (uint64_t)kvh * max_ctx * HD;
             const float* V = cache_v + (uint64_t)kvh * max_ctx * HD;
+            uint32_t k_sent = 0, v_sent = 0;
             for (uint32_t j = 0; j < n_tiles && ok; ++j) {
                 const uint32_t bytes = min(n_keys - j * AK, AK) * (HD * 4);
-                wait_all(&rk_empty, (j & 1) ^ 1);
-                if (ok && lane == 0) {
+                if (!wait_all(&rk_empty, (j & 1) ^ 1)) break;
+                ++k_sent;
+                if (lane == 0) {
                     mbar_arrive_expect_tx(&rk_full, bytes);
                     bulk_g2s(raw_k, K + (uint64_t)j * AK * HD, bytes, &rk_full);
                 }
-                wait_all(&rv_empty, (j & 1) ^ 1);
-                if (ok && lane == 0) {
+                if (!wait_all(&rv_empty, (j & 1) ^ 1)) break;
+                ++v_sent;
+                if (lane == 0) {
                     mbar_arrive_expect_tx(&rv_full, bytes);
                     bulk_g2s(raw_v, V + (uint64_t)j * AK * HD, bytes, &rv_full);
                 }
             }
+            if (!ok) {  // copies in flight still write to shared memory
+                if (k_sent) mbar_wait(&rk_full, (k_sent - 1) & 1);
+                if (v_sent) mbar_wait(&rv_full, (v_sent - 1) & 1);
+            }
         }
+        leave();
     }
-    if (!ok && lane == 0) abort_flag = 1;
-    tc_fence_before();
-    __syncthreads();
-    if (abort_flag && tid == 0 && bad_pos) atomicExch(bad_pos, 1);
+    if (tid == 0 && abort_flag) *reinterpret_cast<volatile int*>(error_flag) = 1;
+    tc_fence_after();
     if (warp == A_SOFT + A_CONV)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }
@@ -473,11 +504,12 @@ __global__ void __launch_bounds__(A_THREADS, 1)
 
 cudaError_t launch_attention_prefill(const float* q, const float* cache_k, const float* cache_v, const int32_t* pos,
                                      uint32_t seq, uint32_t nq, uint32_t nkv, uint32_t hd, uint32_t max_ctx, float* out,
-                                     int32_t* bad_pos, cudaStream_t s) {
+                                     int32_t* bad_pos, int* error_flag, cudaStream_t s) {
     const dim3 grid(nq, (seq + AQ - 1) / AQ);
     auto launch = [&](auto kern, size_t smem, bool* configured) {
         if (cudaError_t ce = set_max_smem_once(kern, (int)smem, configured); ce != cudaSuccess) return ce;
-        cudaError_t e = launch_pdl(kern, grid, A_THREADS, smem, s, q, cache_k, cache_v, pos, seq, nq, nkv, max_ctx, out, bad_pos);
+        cudaError_t e = launch_pdl(kern, grid, A_THREADS, smem, s, q, cache_k, cache_v, pos, seq, nq, nkv, max_ctx, out, bad_pos,
+                                   error_flag);
         return e != cudaSuccess ? e : cudaGetLastError();
     };
     static bool configured[2][MAX_DEVICES] = {};

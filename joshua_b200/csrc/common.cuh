@@ -244,7 +244,7 @@ cudaError_t launch_rope_append(const float* qkv, const int32_t* pos, uint32_t ba
 // causal attention of `seq` new tokens of one sequence (positions pos[0] ..) over the cache; hd 64 or 128
 cudaError_t launch_attention_prefill(const float* q, const float* cache_k, const float* cache_v, const int32_t* pos,
                                      uint32_t seq, uint32_t nq, uint32_t nkv, uint32_t hd, uint32_t max_ctx, float* out,
-                                     int32_t* bad_pos, cudaStream_t s);
+                                     int32_t* bad_pos, int* error_flag, cudaStream_t s);
 // rope + cache append + attention + merge in one launch, from the fused qkv row (decoder.cu)
 struct AttnArgs;
 bool attention_fused_args(const float* qkv, const int32_t* pos, uint32_t batch, uint32_t nq, uint32_t nkv, uint32_t hd,

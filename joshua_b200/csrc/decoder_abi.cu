@@ -264,7 +264,7 @@ int32_t jq_attention_prefill_dev(const float* q, const float* cache_k, const flo
     if (head_dim != 64 && head_dim != 128)
         return jq_fail(jq::E_INVALID, "jq_attention_prefill_dev: head_dim 64 or 128");
     JQ_CUDA(jq::launch_attention_prefill(q, cache_k, cache_v, pos0, seq, n_q, n_kv, head_dim, max_ctx, out, bad_pos_dev,
-                                         static_cast<cudaStream_t>(stream)));
+                                         jq_entry_status_flag(), static_cast<cudaStream_t>(stream)));
     return jq::OK;
 }
 

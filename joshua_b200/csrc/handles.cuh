@@ -159,6 +159,11 @@ struct jq_weight {
     bool owns;
 };
 
+// Status flag of the current device for kernels behind entries that are given no context: device memory's view of a pinned
+// word that lives as long as the process, made by the first jq_init of the device (NULL before it); jq_device_status of any
+// context of the device reports it (abi.cu).
+int* jq_entry_status_flag();
+
 // Picks the kernel for a device-resident product (abi.cu).
 int32_t jq_matmul_device(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, const float* lhs, float* dst,
                          cudaStream_t s);

@@ -215,11 +215,13 @@ class LlamaDecoder:
         self.window_state.copy_(torch.tensor([[len(tail), len(tail) % 64]] * self.batch, dtype=torch.int32))
 
     def check_flags(self) -> None:
-        """Raises if a token id was out of range or a position ran past the KV cache (synchronises)."""
+        """Raises if a token id was out of range, a position ran past the KV cache or a wait inside a kernel gave up
+        (synchronises)."""
         if int(self.bad.item()) != 0:
             raise _lib.JoshuaB200Error(_lib.E_INVALID, "embedding id out of range")
         if int(self.bad_pos.item()) != 0:
             raise _lib.JoshuaB200Error(_lib.E_TOO_LARGE, f"a position ran past the KV cache of {self.max_ctx} positions")
+        check(_lib.lib().jq_device_status(self.embed.ctx._h))
 
     def step_unfused(self, stream=None) -> None:
         """The same step from the separate kernels (norm, rope, attention partial + merge as their own
