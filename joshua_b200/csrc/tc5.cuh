@@ -50,7 +50,9 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
 __device__ __forceinline__ constexpr uint32_t umma_idesc_f16(uint32_t n) {
     return (1u << 4) | ((n >> 3) << 17) | ((128u >> 4) << 24);
 }
-// D (tensor memory) += A (tensor memory, 16 columns of k in 8 columns) * B (shared memory)
+// The same for A and B in bf16.
+__device__ __forceinline__ constexpr uint32_t umma_idesc_bf16(uint32_t n) { return umma_idesc_f16(n) | (1u << 7) | (1u << 10); }
+// D (tensor memory) += A (tensor memory, 16 columns of k in 8 columns) * B (shared memory), 16-bit A and B
 __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
                                             uint32_t accumulate) {
     asm volatile(

@@ -1,6 +1,6 @@
-"""`jq_attention_prefill_dev` (f16 terms on the tensor cores) against float64 attention: query and key counts around the
+"""`jq_attention_prefill_dev` (16-bit terms on the tensor cores) against float64 attention: query and key counts around the
 tiles of 128 queries and 64 keys, both head sizes, grouped heads, earlier positions in the cache, rows behind the last key
-that hold NaN, values and keys decades apart."""
+that hold NaN, values and keys decades apart, infinities."""
 import math
 
 import pytest
@@ -63,6 +63,77 @@ def test_prefill_attention_matches_float64(shape, spread):
     # Terms hold 2^-22 of a row's or column's largest values and a chain of 12 products adds a few 2^-24; a score's error
     # is that of its size and makes a relative error of its probability, above and below the fraction line.
     tol = 2.0 ** -20 * (1.0 + s_max) * v[:, :p0 + S].abs().amax((0, 1)).double()
+    assert bool(((got.double() - want).abs() <= tol).all()), float(((got.double() - want).abs() / tol).max())
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("S, p0", [(16, 0), (130, 0), (200, 37)])
+def test_later_tokens_do_not_reach_earlier_ones(S, p0, hd):
+    """Bit for bit, whatever the keys and values of tokens behind a query hold."""
+    import torch
+
+    dev = torch.device("cuda", 0)
+    gen = torch.Generator(device=dev).manual_seed(S + hd)
+    q = torch.randn(S, 4, hd, device=dev, generator=gen)
+    k = torch.randn(2, p0 + S, hd, device=dev, generator=gen)
+    v = torch.randn(2, p0 + S, hd, device=dev, generator=gen)
+    first, _ = run(q, k, v, p0, p0 + S)
+    for cut in (1, S // 2, S - 1):  # tokens cut .. S - 1 change
+        for later in (0.0, 1e6, 3e38, 1e-30, math.inf, -math.inf, math.nan):
+            k2, v2 = k.clone(), v.clone()
+            k2[:, p0 + cut:, ::3] = later
+            v2[:, p0 + cut:, ::2] = later
+            got, bad = run(q, k2, v2, p0, p0 + S)
+            assert bad == 0 and bool((got[:cut] == first[:cut]).all()), (cut, later)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+def test_infinities_reach_the_queries_that_see_them(hd):
+    import torch
+
+    S, at, dev = 150, 70, torch.device("cuda", 0)
+    gen = torch.Generator(device=dev).manual_seed(hd)
+    q = torch.randn(S, 2, hd, device=dev, generator=gen)
+    k = torch.randn(1, S, hd, device=dev, generator=gen)
+    v = torch.randn(1, S, hd, device=dev, generator=gen)
+    first, _ = run(q, k, v, 0, S)
+    v[0, at, 3], v[0, at, hd - 1], v[0, at + 1, 5] = math.inf, -math.inf, math.nan
+    got, _ = run(q, k, v, 0, S)
+    assert bool((got[at:, :, 3] == math.inf).all()) and bool((got[at:, :, hd - 1] == -math.inf).all())
+    assert bool(got[at + 1:, :, 5].isnan().all())
+    for t in (got, first):
+        t[at:, :, [3, 5, hd - 1]] = 0
+    assert bool((got == first).all())
+    # a key of minus infinity in a dimension where the query is positive has no weight, one of plus infinity no result
+    v[0, at:at + 2] = 1.0
+    q[:, :, 7] = q[:, :, 7].abs() + 0.1
+    k[0, at, 7] = -math.inf
+    got, _ = run(q, k, v, 0, S)
+    want, _ = reference(q, k, v, 0)
+    assert float((got.double() - want).norm() / want.norm()) <= 1e-6
+    k[0, at, 7] = math.inf
+    got, _ = run(q, k, v, 0, S)
+    assert bool(got[at:].isnan().all()) and bool(got[:at].isfinite().all())
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("S", [16, 64, 200])
+def test_values_decades_apart_keep_their_bits(S, hd):
+    """One value of 1e6 and a dimension of 1e-6 beside N(0, 1): each output to the size of what it adds up."""
+    import torch
+
+    dev = torch.device("cuda", 0)
+    gen = torch.Generator(device=dev).manual_seed(S + hd)
+    q = torch.randn(S, 4, hd, device=dev, generator=gen)
+    k = torch.randn(1, S, hd, device=dev, generator=gen)
+    v = torch.randn(1, S, hd, device=dev, generator=gen)
+    v[0, S // 2, 3], v[0, :, 9] = 1e6, v[0, :, 9] * 1e-6
+    got, _ = run(q, k, v, 0, S)
+    want, s_max = reference(q, k, v, 0)
+    size, _ = reference(q, k, v.abs(), 0)
+    # a score's error is 2^-22 of its size and makes a relative error of its probability, above and below the fraction line;
+    # the terms of probabilities and values hold 2^-24, their chain of 24 products adds a few 2^-24 of the sum of magnitudes
+    tol = 2.0 ** -20 * (1.0 + s_max) * size
     assert bool(((got.double() - want).abs() <= tol).all()), float(((got.double() - want).abs() / tol).max())
 
 
