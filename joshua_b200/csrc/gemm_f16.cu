@@ -631,6 +631,20 @@ __device__ __forceinline__ void convert_minima(uint32_t u, const RowWin& rw, uin
     }
 }
 
+// Loads of what a kernel in front wrote, for places directly behind pdl_wait: read-only loads (__ldg, or plain ones through
+// __restrict__) may be moved above the wait, volatile ones stay.  (The sign of a row's scale, read too early: in one call out
+// of eight of 200 rows x 14336 columns a window with a scale of its own, where the call before had none, counted some 500 times.)
+__device__ __forceinline__ float ld_behind_wait(const float* p) {
+    float v;
+    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t ld_behind_wait(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
 // VEC: bytes a copy of raw weights, HT's or (a tensor that starts on a word boundary only) 4.
 template <uint32_t TYPE, int N_TILE, uint32_t VEC>
 __global__ void __launch_bounds__(H_THREADS, 1)
@@ -669,11 +683,11 @@ __global__ void __launch_bounds__(H_THREADS, 1)
     float* dst = bank ? dst_b : dst_a;
     if (tiles != nullptr) {
         pdl_wait();
-        if (blockIdx.y >= *n_tiles) return;
-        const GemmTile t = tiles[blockIdx.y];
-        w += (uint64_t)t.expert * expert_bytes;
-        tok0 = t.row0;
-        m = (uint64_t)t.row0 + t.cnt;
+        if (blockIdx.y >= ld_behind_wait(n_tiles)) return;
+        const GemmTile* t = tiles + blockIdx.y;
+        w += (uint64_t)ld_behind_wait(&t->expert) * expert_bytes;
+        tok0 = ld_behind_wait(&t->row0);
+        m = tok0 + ld_behind_wait(&t->cnt);
     }
     const uint64_t row0 = (uint64_t)blockIdx.x * HM;
     const uint64_t row_bytes = k / 256 * T::UNIT;
@@ -759,16 +773,16 @@ __global__ void __launch_bounds__(H_THREADS, 1)
         const uint32_t slot = scales + warp * 32 * 16;  // per token: its address in rel, its scale so far, its change
         auto find_scales = [&] {
             const uint64_t tok = min(tok0 + (S::FINE ? 0 : g * MY_COLS) + lane % MY_COLS, m_rows - 1);  // the last row, past it
-            scaled = __any_sync(0xFFFFFFFFu, __ldg(inv + tok) < 0.0f);
+            scaled = __any_sync(0xFFFFFFFFu, ld_behind_wait(inv + tok) < 0.0f);
             if (!scaled) return;
             const float* p = rel + (uint64_t)win0 * T::UNITS * m_rows + tok;
             asm volatile("st.shared.u64 [%0], %1;" ::"r"(slot + lane * 8), "l"(p) : "memory");
-            asm volatile("st.shared.f32 [%0], %1;" ::"r"(slot + 256 + lane * 4), "f"(__ldg(p)) : "memory");
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(slot + 256 + lane * 4), "f"(ld_behind_wait(p)) : "memory");
         };
         auto rescale = [&](uint32_t c) {  // to window c's scales; c = n_chunks: to the rows'
             const float* p;
             asm volatile("ld.shared.u64 %0, [%1];" : "=l"(p) : "r"(slot + lane * 8));
-            const float was = __uint_as_float(s32(slot + 256 + lane * 4)), now = c < n_chunks ? __ldg(p + (uint64_t)c * m_rows) : 1.0f;
+            const float was = __uint_as_float(s32(slot + 256 + lane * 4)), now = c < n_chunks ? ld_behind_wait(p + (uint64_t)c * m_rows) : 1.0f;
             if (!__any_sync(0xFFFFFFFFu, was != now)) return;
             asm volatile("st.shared.f32 [%0], %1;" ::"r"(slot + 256 + lane * 4), "f"(now) : "memory");
             asm volatile("st.shared.f32 [%0], %1;" ::"r"(slot + 384 + lane * 4), "f"(was / now) : "memory");  // powers of two
