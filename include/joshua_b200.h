@@ -133,7 +133,9 @@ int32_t jq_matmul_t_f16(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, 
  * the stream runs later.  A graph replays into the scratch of the stream it was
  * captured on, so work on that stream, and other graphs captured on it, must not
  * run at the same time on another stream.  Growth allocates: warm a stream up
- * before capturing it. */
+ * before capturing it.
+ *   dst_dev may lie over lhs_dev, here and in the fused entries: the rows are
+ * then split or copied into scratch first. */
 int32_t jq_matmul_t_dev(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, const float* lhs_dev,
                         float* dst_dev, void* stream);
 
@@ -217,11 +219,11 @@ int32_t jq_matmul_swiglu_norm_dev(const jq_weight* gate, const jq_weight* up, ui
  * src/quantized_qwen3_moe.rs:793-819).  norm_w_dev and residual_dev are each
  * optional; residual_dev may be dst_dev; lhs_dev and norm_w_dev 16-byte
  * aligned.  One launch of a decode kernel for three to eight rows of Q4_K and
- * MXFP4 with k >= 1024 (dst_dev not over lhs_dev) and for up to eight rows whose
- * activation planes fit the other one's shared memory; a split and a product of
- * the tile GEMM, norm and residual inside, from five rows of Q4_K (or of planes
- * that do not fit) that no decode kernel took, nine of the other types and 17 of
- * Q8_0 on; the separate kernels for what none takes. */
+ * MXFP4 with k >= 1024 and for up to eight rows whose activation planes fit the
+ * other one's shared memory (neither with dst_dev over lhs_dev); a split and a
+ * product of the tile GEMM, norm and residual inside, from five rows of Q4_K (or
+ * of planes that do not fit) that no decode kernel took, nine of the other types
+ * and 17 of Q8_0 on; the separate kernels for what none takes. */
 int32_t jq_matmul_norm_dev(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, const float* lhs_dev,
                            const float* norm_w_dev, float eps, const float* residual_dev, float* dst_dev,
                            void* stream);

@@ -95,11 +95,13 @@ bool jq_uses_tiles(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, cudaS
     return w->ctx->scratch_available(s, SLOT_TILES, jq::gemm_f16_scratch_bytes(m, k));
 }
 
-// A CTA of that kernel may read lhs after another has stored: a result over its input stays with the routes that split lhs first.
-bool jq_uses_gemv_f16(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, const float* lhs, const float* dst, bool pair) {
-    if (w->ctx->force_f32 || !jq::gemv_f16_supports(w->type, w->dev, n, k, m, pair)) return false;
+bool jq_overlaps(const float* lhs, const float* dst, uint64_t m, uint64_t k, uint64_t n) {
     const uintptr_t a = reinterpret_cast<uintptr_t>(lhs), d = reinterpret_cast<uintptr_t>(dst);
-    return a + 4 * m * k <= d || d + 4 * m * n <= a;
+    return a < d + 4 * m * n && d < a + 4 * m * k;
+}
+
+bool jq_uses_gemv_f16(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, const float* lhs, const float* dst, bool pair) {
+    return !w->ctx->force_f32 && !jq_overlaps(lhs, dst, m, k, n) && jq::gemv_f16_supports(w->type, w->dev, n, k, m, pair);
 }
 
 int32_t jq_matmul_tiles(const jq_weight* w, const jq_weight* w_b, uint64_t m, uint64_t k, uint64_t n, const float* lhs,
@@ -116,6 +118,15 @@ int32_t jq_matmul_tiles(const jq_weight* w, const jq_weight* w_b, uint64_t m, ui
 int32_t jq_matmul_device(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, const float* lhs, float* dst,
                          cudaStream_t s) {
     jq_ctx* ctx = w->ctx;
+    if (jq_overlaps(lhs, dst, m, k, n) && !jq_uses_tiles(w, m, k, n, s)) {  // the tile GEMM splits lhs before it stores
+        if (!ctx->scratch_available(s, SLOT_LHS, m * k * 4))
+            return jq_fail(jq::E_INVALID, "matmul: a result over its input needs scratch, which a capture cannot allocate: "
+                                          "run the call once on the stream before capturing it");
+        void* copy = nullptr;
+        JQ_CUDA(ctx->scratch_for(s, SLOT_LHS, m * k * 4, &copy));
+        JQ_CUDA(cudaMemcpyAsync(copy, lhs, m * k * 4, cudaMemcpyDeviceToDevice, s));
+        lhs = static_cast<const float*>(copy);
+    }
     if (jq_uses_gemv_f16(w, m, k, n, lhs, dst, false)) {
         JQ_CUDA(jq::launch_gemv_f16(w->type, w->dev, nullptr, n, k, lhs, m, nullptr, 0.0f, nullptr, 0.0f, dst, ctx->status_dev, s));
         return jq::OK;

@@ -52,7 +52,7 @@ int32_t jq_matmul_swiglu_dev(const jq_weight* gate, const jq_weight* up, uint64_
     }
     if (pair_uses_tiles(gate, up, m, k, n, s))
         return swiglu_tiles(gate, up, m, k, n, lhs_dev, nullptr, 0.0f, dst_dev, clamp, s);
-    if (!ctx->force_f32 && jq::gemv_mma_supports(gate->type, gate->dev, n, k, m) &&
+    if (!ctx->force_f32 && !jq_overlaps(lhs_dev, dst_dev, m, k, n) && jq::gemv_mma_supports(gate->type, gate->dev, n, k, m) &&
         jq::gemv_mma_supports(up->type, up->dev, n, k, m) && jq::gemv_mma_scratch_bytes(m, k) == 0) {
         JQ_CUDA(jq::launch_gemv_mma_swiglu(gate->type, gate->dev, up->dev, n, k, lhs_dev, m, dst_dev, clamp,
                                            ctx->status_dev, s));
@@ -88,7 +88,7 @@ int32_t jq_matmul_swiglu_norm_dev(const jq_weight* gate, const jq_weight* up, ui
     }
     if (pair_uses_tiles(gate, up, m, k, n, s))
         return swiglu_tiles(gate, up, m, k, n, lhs_dev, norm_w_dev, eps, dst_dev, clamp, s);
-    if (!ctx->force_f32 && jq::gemv_mma_supports(gate->type, gate->dev, n, k, m) &&
+    if (!ctx->force_f32 && !jq_overlaps(lhs_dev, dst_dev, m, k, n) && jq::gemv_mma_supports(gate->type, gate->dev, n, k, m) &&
         jq::gemv_mma_supports(up->type, up->dev, n, k, m) && jq::gemv_mma_fusable(gate->type, m, k)) {
         JQ_CUDA(jq::launch_gemv_mma_swiglu(gate->type, gate->dev, up->dev, n, k, lhs_dev, m, dst_dev, clamp,
                                            ctx->status_dev, s, norm_w_dev, eps));
@@ -119,7 +119,7 @@ int32_t jq_matmul_norm_dev(const jq_weight* w, uint64_t m, uint64_t k, uint64_t 
     }
     if (jq_uses_tiles(w, m, k, n, s))
         return jq_matmul_tiles(w, nullptr, m, k, n, lhs_dev, norm_w_dev, eps, residual_dev, dst_dev, nullptr, s);
-    if (!ctx->force_f32 && jq::gemv_mma_dense_supports(w->type, w->dev, n, k, m) &&
+    if (!ctx->force_f32 && !jq_overlaps(lhs_dev, dst_dev, m, k, n) && jq::gemv_mma_dense_supports(w->type, w->dev, n, k, m) &&
         jq::gemv_mma_fusable(w->type, m, k)) {
         JQ_CUDA(jq::launch_gemv_mma_fused(w->type, w->dev, n, k, lhs_dev, m, dst_dev, norm_w_dev, eps, residual_dev,
                                           ctx->status_dev, s));

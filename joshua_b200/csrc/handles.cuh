@@ -49,6 +49,7 @@ enum ScratchSlot : uint32_t {
     SLOT_PAIR,    // gate and up products in front of their combine
     SLOT_NORM,    // normalised rows and the product of the separate kernels
     SLOT_TILES,   // split activations of the tile GEMMs
+    SLOT_LHS,     // rows whose product goes over them
 };
 struct StreamScratch {
     void* dev = nullptr;
@@ -167,6 +168,10 @@ int* jq_entry_status_flag();
 // Picks the kernel for a device-resident product (abi.cu).
 int32_t jq_matmul_device(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, const float* lhs, float* dst,
                          cudaStream_t s);
+
+// Whether a product of m rows is to be stored over (part of) them.  CTAs of the decode kernels and of the exact-decode one
+// read rows after others have stored: such calls take a route that splits or copies the rows first.
+bool jq_overlaps(const float* lhs, const float* dst, uint64_t m, uint64_t k, uint64_t n);
 
 // Whether a product of m rows (pair: gate and up) runs on the f16 decode kernel.
 bool jq_uses_gemv_f16(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, const float* lhs, const float* dst, bool pair);

@@ -107,3 +107,38 @@ def test_a_result_over_its_input_splits_the_input_first(m):
         _lib.check(call(y.data_ptr()))
         # 2-norm of the tile GEMM's error below 1e-6, three times that for a product of two and silu
         assert float((y.double() - ref).norm() / ref.norm()) <= 3e-6
+
+
+@pytest.mark.parametrize("type_id", [synth.Q4_K, synth.MXFP4, synth.Q8_0, synth.Q4_0])
+@pytest.mark.parametrize("m", [1, 3, 4, 6, 20])
+def test_a_result_over_its_input_at_every_batch(type_id, m):
+    """dst = lhs, or one row behind it, on the routes whose CTAs would read lhs while others store: the rows go through scratch.
+    Plain, with norm and residual, and as a gate / up pair."""
+    import torch
+
+    from joshua_b200 import _lib
+
+    n = 2048
+    L, st = _lib.lib(), torch.cuda.current_stream().cuda_stream
+    q, w, x = setup(type_id, n, n, m, m)
+    up, wu, _ = setup(type_id, n, n, m, m + 50)
+    norm, res = torch.rand(n, device="cuda") + 0.5, torch.randn(m, n, device="cuda")
+    xn = x.double() * torch.rsqrt(x.double().pow(2).mean(1, keepdim=True) + 1e-6) * norm.double()
+
+    def pair(v):
+        g = v @ w.T
+        return g * torch.sigmoid(g) * (v @ wu.T)
+
+    for call, ref in (
+            (lambda a, d: L.jq_matmul_t_dev(q._h, m, n, n, a, d, st), x.double() @ w.T),
+            (lambda a, d: L.jq_matmul_norm_dev(q._h, m, n, n, a, norm.data_ptr(), 1e-6, res.data_ptr(), d, st), xn @ w.T + res.double()),
+            (lambda a, d: L.jq_matmul_norm_dev(q._h, m, n, n, a, None, 0.0, res.data_ptr(), d, st), x.double() @ w.T + res.double()),
+            (lambda a, d: L.jq_matmul_swiglu_dev(q._h, up._h, m, n, n, a, d, 0.0, st), pair(x.double())),
+            (lambda a, d: L.jq_matmul_swiglu_norm_dev(q._h, up._h, m, n, n, a, norm.data_ptr(), 1e-6, d, 0.0, st), pair(xn))):
+        for behind in (0, 1):
+            buf = torch.zeros(m + 1, n, device="cuda")
+            buf[:m] = x
+            _lib.check(call(buf.data_ptr(), buf[behind:].data_ptr()))
+            got = buf[behind:behind + m]
+            # as above: 1e-6 for one product, three times that for two of them and silu
+            assert float((got.double() - ref).norm() / ref.norm()) <= 3e-6
