@@ -22,8 +22,9 @@
 // teams send their partial tiles to one of the ranks in turn (distributed shared memory, an mbarrier a slot), which adds them
 // in rank order, so that results do not depend on timing.
 //
-// Error against float64 (2-norm, N(0, 1) rows): Q4_K 1.8e-7 to 2.1e-7, MXFP4 0.9e-7 to 1.1e-7; the routes before 2.4e-7 to
-// 3.8e-7 and 1.2e-7 to 1.5e-7.  Algorithmic bytes per launch: n*k/B*S (weights) + 4*m*(k + n).  What bounds it: the consumers'
+// Error against float64 (2-norm, N(0, 1) rows): Q4_K 2.1e-7 to 2.9e-7, MXFP4 0.9e-7 to 1.1e-7; the routes before 3.3e-7 to
+// 3.8e-7 and 1.3e-7 to 1.5e-7.  Positive rows (1 + |N(0, 1)|), Q4_K weights of mean zero: up to four rows 1.2e-6, before 1.8e-6 to
+// 2.8e-6; five to eight 1.4e-6 to 1.6e-6, before 2.4e-6 to 5.6e-6.  Algorithmic bytes per launch: n*k/B*S (weights) + 4*m*(k + n).  What bounds it: the consumers'
 // instructions, 460 (four rows) to 600 (eight) per 16 x 256 unit at 1.8 to 2.8 a cycle.  Measured, four / eight rows, before (the
 // integer kernel / the tile GEMM and its split) and now: Q4_K 28672 x 4096 27.4 / 49.5 and 22.2 / 27.5 us, 6144 x 4096 11.4 /
 // 25.9 and 9.2 / 12.2, 4096 x 4096 9.8 / 11.5 and 7.4 / 10.2, 4096 x 14336 24.6 / 28.5 and 18.3 / 22.8, 128256 x 4096 94 / 169 and
@@ -277,8 +278,12 @@ __device__ __forceinline__ void split_unit(float (&v)[8], uint32_t lane, uint32_
             sum *= 0.03125f;  // 32 values below 2^15
             const __half h = __float2half_rn(sum), l = __float2half_rn(sum - __half2float(h));
             __half* s = reinterpret_cast<__half*>(act + S::UNIT_B + col * 32 + (G >> 1) * 8) + (G & 1);
-            s[0] = h, s[2] = l;
-            if constexpr (PACK) s[4 * 16] = s[4 * 16 + 2] = __float2half_rn(0.0f);  // the low terms' columns: their sums are in s
+            // Second terms: behind the first ones, or (PACK) in the low terms' columns, which keeps the first ones' products
+            // exact.  Beside them the tensor core cuts off the second ones' last bits, a bias that the codes' exact products
+            // do not share.
+            const __half zero = __float2half_rn(0.0f);
+            s[0] = h, s[2] = PACK ? zero : l;
+            if constexpr (PACK) s[4 * 16] = l, s[4 * 16 + 2] = zero;
         }
     }
     if (lane == 0) {
