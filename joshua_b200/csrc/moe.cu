@@ -11,50 +11,68 @@ namespace jq {
 
 namespace {
 
-// logits[t, e] = sum_j x[t, j] * router[e, j], f32: one warp per (token, four consecutive experts), so that a token's row is
-// read once for four dot products; each dot product sums its lane's strided pieces in column order and then across the
-// lanes, the same order for every batch size.  For the few tokens that fill no tile of the next kernel.
+// logits[t, e] = sum_j x[t, j] * router[e, j], f32: one warp per (TT consecutive tokens, four consecutive experts), so
+// that a token's row is read once for four dot products and an expert's for TT; each dot product sums its lane's
+// strided pieces in column order and then across the lanes, the same order for every batch size.  Bound by the loads
+// from L1 and L2: with one token a warp five vectors feed 16 multiply-adds a lane, with four eight feed 64.
+template <int TT>
 __global__ void __launch_bounds__(256) moe_logits_kernel(const float* __restrict__ x, const float* __restrict__ router,
                                                          uint32_t T, uint32_t E, uint32_t h,
                                                          float* __restrict__ logits) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const uint32_t lane = threadIdx.x & 31, E4 = (E + 3) / 4;
-    const uint64_t total = (uint64_t)T * E4;
+    const uint32_t lane = threadIdx.x & 31, E4 = (E + 3) / 4, TG = (T + TT - 1) / TT;
+    const uint64_t total = (uint64_t)TG * E4;
     for (uint64_t p = blockIdx.x * 8ull + (threadIdx.x >> 5); p < total; p += gridDim.x * 8ull) {
-        const uint32_t t = (uint32_t)(p / E4), e0 = (uint32_t)(p % E4) * 4;
-        const float4* a = reinterpret_cast<const float4*>(x + (uint64_t)t * h);
+        const uint32_t t0 = (uint32_t)(p / E4) * TT, e0 = (uint32_t)(p % E4) * 4;
+        const float4* a[TT];
+#pragma unroll
+        for (int r = 0; r < TT; ++r) a[r] = reinterpret_cast<const float4*>(x + (uint64_t)min(t0 + r, T - 1) * h);
         const float4* b[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) b[q] = reinterpret_cast<const float4*>(router + (uint64_t)min(e0 + q, E - 1) * h);
-        float acc[4] = {};
+        float acc[TT][4];
+#pragma unroll
+        for (int r = 0; r < TT; ++r)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[r][q] = 0.0f;
         for (uint32_t j = lane; j < h / 4; j += 32) {
-            const float4 u = __ldg(a + j);
+            float4 u[TT];
+#pragma unroll
+            for (int r = 0; r < TT; ++r) u[r] = __ldg(a[r] + j);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const float4 v = __ldg(b[q] + j);
-                acc[q] = fmaf(u.x, v.x, acc[q]);
-                acc[q] = fmaf(u.y, v.y, acc[q]);
-                acc[q] = fmaf(u.z, v.z, acc[q]);
-                acc[q] = fmaf(u.w, v.w, acc[q]);
+#pragma unroll
+                for (int r = 0; r < TT; ++r) {
+                    acc[r][q] = fmaf(u[r].x, v.x, acc[r][q]);
+                    acc[r][q] = fmaf(u[r].y, v.y, acc[r][q]);
+                    acc[r][q] = fmaf(u[r].z, v.z, acc[r][q]);
+                    acc[r][q] = fmaf(u[r].w, v.w, acc[r][q]);
+                }
             }
         }
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            float v = acc[q];
+        for (int r = 0; r < TT; ++r)
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-            if (lane == 0 && e0 + q < E) logits[(uint64_t)t * E + e0 + q] = v;
-        }
+            for (int q = 0; q < 4; ++q) {
+                float v = acc[r][q];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+                if (lane == 0 && t0 + r < T && e0 + q < E) logits[(uint64_t)(t0 + r) * E + e0 + q] = v;
+            }
     }
 }
 
 // The same for many tokens, the same sums in the same order: a CTA takes 16 tokens and 16 experts, a warp eight of each
 // (64 multiply-adds a lane for sixteen 16-byte loads), and the rows pass through shared memory in pieces of 512 bytes, three
 // of them on the way, so that the L2 hands each row to a sixteenth of the warps that the kernel above sends for it.
-// 256 tokens x 384 experts x 7168 with the routing behind it: 132 -> 58 us; 512 x 128 x 2048: 38 -> 21.5.
+// With the routing behind it, the kernel above and this one: 256 tokens x 384 experts x 7168 81 and 56 us, 64 tokens 33 and 27,
+// 512 x 128 x 2048 22 and 20.
 constexpr int LG_STAGES = 4, LG_ROWS = 32;
 constexpr size_t LG_SMEM = (size_t)LG_STAGES * LG_ROWS * 512;
+constexpr uint64_t LG_MIN_LOGITS = 6144;
+constexpr size_t LG_SMEM_ALONE = 116 * 1024;  // more than half of an SM's: a CTA has it to itself
 __global__ void __launch_bounds__(128) moe_logits_tile_kernel(const float* __restrict__ x, const float* __restrict__ router,
                                                               uint32_t T, uint32_t E, uint32_t h, float* __restrict__ logits) {
     extern __shared__ __align__(16) float4 s_rows[];  // [stage][16 tokens, 16 experts][32]
@@ -817,16 +835,24 @@ unsigned blocks_for(uint64_t work, unsigned per_block) {
 
 cudaError_t launch_moe_logits(const float* x, const float* router, uint32_t T, uint32_t E, uint32_t h, float* logits,
                               cudaStream_t s) {
-    // from one whole tile of tokens on: 16 tokens, 384 x 7168, 35.8 -> 29.8 us with the routing behind it (128 x 2048: 15.4 ->
-    // 13.4, 64 tokens 17.4 -> 15.4)
-    if (T >= LG_ROWS / 2 && h % 128 == 0) {
+    // Up to one CTA an SM the tiles take the same time however many there are (h = 2048 / 4096 / 7168 with the routing: 9.7 / 15 /
+    // 22 to 27 us), the other kernel grows with the logits, and at every width from 8 to 384 experts the lines cross near
+    // 6144 of them: 128 x 2048, 40 / 48 / 64 tokens 10.8 / 11.2 / 11.7 us there and 10.3 / 10.5 / 10.2 here; 8 x 4096, 512 / 1000
+    // tokens 11.9 / 15.8 and 15 / 16.3; 384 x 7168, 16 / 32 tokens 27.7 / 37.5 and 26.6 / 27.7.  An SM to a CTA as long as they
+    // last: two on one SM take twice as long beside SMs that stand idle (256 x 7168, 128 tokens 41 -> 25 us).
+    if (T >= LG_ROWS / 2 && (uint64_t)T * E >= LG_MIN_LOGITS && h % 128 == 0) {
         static bool configured[MAX_DEVICES] = {};
-        if (cudaError_t ce = set_max_smem_once(moe_logits_tile_kernel, LG_SMEM, configured); ce != cudaSuccess) return ce;
-        const cudaError_t e = launch_pdl(moe_logits_tile_kernel, dim3((T + 15) / 16, (E + 15) / 16), 128, LG_SMEM, s, x, router, T,
-                                         E, h, logits);
+        if (cudaError_t ce = set_max_smem_once(moe_logits_tile_kernel, LG_SMEM_ALONE, configured); ce != cudaSuccess) return ce;
+        const dim3 grid((T + 15) / 16, (E + 15) / 16);
+        const size_t smem = grid.x * grid.y <= (uint32_t)num_sms() ? LG_SMEM_ALONE : LG_SMEM;
+        const cudaError_t e = launch_pdl(moe_logits_tile_kernel, grid, 128, smem, s, x, router, T, E, h, logits);
         return e != cudaSuccess ? e : cudaGetLastError();
     }
-    cudaError_t le1__ = launch_pdl(moe_logits_kernel, blocks_for((uint64_t)T * ((E + 3) / 4), 8), 256, 0, s, x, router, T, E, h, logits);
+    // four tokens a warp once that still leaves every SM eight warps
+    const uint64_t e4 = (E + 3) / 4, groups4 = (uint64_t)((T + 3) / 4) * e4;
+    cudaError_t le1__ = groups4 >= 8ull * num_sms()
+                            ? launch_pdl(moe_logits_kernel<4>, blocks_for(groups4, 8), 256, 0, s, x, router, T, E, h, logits)
+                            : launch_pdl(moe_logits_kernel<1>, blocks_for((uint64_t)T * e4, 8), 256, 0, s, x, router, T, E, h, logits);
     if (le1__ != cudaSuccess) return le1__;
     return cudaGetLastError();
 }

@@ -435,3 +435,11 @@ def test_a_layer_captured_on_a_stream_without_scratch(tokens_):
     torch.cuda.synchronize()
     moe.status()
     assert_close(out.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("hidden,n_expert,T", [(1280, 384, 16), (256, 130, 47), (256, 130, 48), (512, 5, 1229), (512, 24, 257),
+                                               (256, 512, 90)])
+def test_router_tiles_around_their_line_add_like_the_warp_per_token(hidden, n_expert, T):
+    """From 6144 logits on they come from tiles of 16 tokens and 16 experts (an SM to a CTA up to 148 of them): the sums of
+    the kernel for fewer, bit for bit."""
+    test_router_tiles_add_like_the_warp_per_token(hidden, n_expert, T)
