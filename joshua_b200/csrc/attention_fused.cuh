@@ -8,7 +8,8 @@
 // chunks in chunk order and resets the counter.
 //
 // The function is written for latency, which is all a decode step sees of it: every global load that does
-// not depend on another (the position, the qkv row, the chunk's K and V rows) is requested up front, the
+// not depend on another (the position, the qkv row, the chunk's K and V rows) is requested up front (with many
+// live items V rows behind the scores, see AttLoad), the
 // partials of the merge are requested before their weights are known, and the code is specialised on the
 // head size and the group size so that it stays small.
 #pragma once
@@ -79,9 +80,8 @@ enum AttLoad { ATT_ALL, ATT_LIVE, ATT_LATE };
 // LOAD: ATT_LIVE and ATT_LATE: the launch holds more items than SMs.  An item then looks at the position first and leaves, without a load, if
 // its chunk lies behind it: with one wave the extra trip to L2 costs more than the loads, with several the dead items'
 // rows are most of the traffic (16 of 17 chunks of a 1056-position cache at the start of a sequence).
-// ATT_LATE: more than two items an SM.  The V rows are requested behind the scores, in the registers that held K: four CTAs
-// an SM instead of two hide the second trip.  Measured, decode steps of the dense model, eight sequences at 512: the kernel
-// 27.8 -> 20 us; with few live items (three sequences of the routed-expert model at 100) the step is 1 % slower that way.
+// ATT_LATE: more than two items an SM, many of them live.  The V rows are requested behind the scores, in the registers that
+// held K: four CTAs an SM instead of two hide the second trip.
 template <uint32_t HD, uint32_t G, AttLoad LOAD>
 __device__ __forceinline__ void attention_fused_item_t(const AttnArgs& a, uint32_t chunk, uint32_t kvh, uint32_t sg,
                                                        uint32_t b, uint32_t tid, float* s_f, uint32_t* s_last) {

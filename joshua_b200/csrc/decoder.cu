@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(128) attention_merge_kernel(const float* __res
 
 // Decode attention in ONE launch, straight from the fused qkv row (attention_fused.cuh): one CTA per
 // (chunk, kv head, sequence).  One kernel per head size and heads per item, so that small shapes do not pay for the
-// registers of the largest; with more items than SMs two CTAs share an SM, with more than twice as many four.
+// registers of the largest; with more items than SMs two CTAs share an SM, with many live ones four.
 template <uint32_t HD, uint32_t G, AttLoad LOAD>
 __global__ void __launch_bounds__(ATT_FUSED_THREADS, HD > 128 || LOAD == ATT_ALL ? 1 : LOAD == ATT_LIVE ? 2 : 4)
     attention_fused_kernel(AttnArgs a) {
@@ -594,12 +594,18 @@ cudaError_t launch_attention_fused(const float* qkv, const int32_t* pos, uint32_
     size_t smem = (size_t)attention_fused_smem_floats(nq / a.gsplit, nkv, hd, a.n_chunks) * 4;
     const dim3 grid(a.n_chunks, nkv * a.gsplit, batch);
     const uint64_t items = (uint64_t)a.n_chunks * grid.y * batch, sms = (uint64_t)num_sms();
+    // Items count the cache's capacity, and how many are live is not known here.  Four CTAs an SM pay where the live ones alone
+    // keep the SMs busy (eight sequences of the dense model at 512: the kernel 25 -> 19 us), and cost where few are live, which
+    // then share SMs and merge with half the registers (one sequence at 1000 of 4096: 12.7 -> 15.2 us, the step 2002 -> 2137).
+    // Taken for live: 512 positions a sequence.
+    const uint64_t live = (uint64_t)std::min(a.n_chunks, 512 / ATT_FUSED_CHUNK) * grid.y * batch;
+    const bool late = items > 2 * sms && live > sms;
     const uint32_t G = nq / nkv / a.gsplit;
     cudaError_t e = cudaErrorInvalidValue;
 #define JQ_ATT_CASE(HD, GV)                                                                                            \
     if (hd == HD && G == GV)                                                                                           \
         e = items <= sms ? launch_pdl(attention_fused_kernel<HD, GV, ATT_ALL>, grid, ATT_FUSED_THREADS, smem, s, a)    \
-            : items <= 2 * sms || HD > 128                                                                             \
+            : !late || HD > 128                                                                                        \
                 ? launch_pdl(attention_fused_kernel<HD, GV, ATT_LIVE>, grid, ATT_FUSED_THREADS, smem, s, a)            \
                 : launch_pdl(attention_fused_kernel<HD, GV, (HD > 128 ? ATT_LIVE : ATT_LATE)>, grid, ATT_FUSED_THREADS, smem, s, a);
     JQ_ATT_CASE(64, 1)

@@ -457,3 +457,40 @@ def test_launches_of_a_step_are_those_of_its_graph(batch, per_layer, rest):
     assert _lib.graph_kernels(g) == per_layer * cfg.layers + rest
     if batch == 1:
         assert dec.launches_per_step == per_layer * cfg.layers + rest
+
+
+@pytest.mark.parametrize("nq,nkv,hd,batch,max_ctx,off", [(32, 8, 128, 1, 4096, 0), (32, 4, 128, 1, 4097, 1), (16, 16, 64, 1, 2049, 3),
+                                                         (8, 8, 128, 5, 1057, 2), (8, 4, 64, 2, 8000, 0)])
+def test_fused_attention_over_a_large_cache_of_few_live_positions(nq, nkv, hd, batch, max_ctx, off):
+    """More than two items an SM by the cache's capacity, on both sides of the line between two and four CTAs an SM; caches off
+    every boundary but the word's; positions at the ends of chunks, few and many live, NaN behind them."""
+    import torch
+
+    from joshua_b200 import _lib
+
+    L, theta, s = _lib.lib(), 10000.0, torch.cuda.current_stream().cuda_stream
+    g = torch.Generator(device="cuda").manual_seed(hd + off)
+    qkv = torch.randn(batch, (nq + 2 * nkv) * hd, device="cuda", generator=g)
+    size = batch * nkv * max_ctx * hd
+    full = [torch.randn(size + 4, device="cuda", generator=g) for _ in range(2)]
+    for p in (0, 63, 64, 100, 1000, max_ctx - 1):
+        pos = torch.tensor([min(max(p - i, 0), max_ctx - 1) for i in range(batch)], dtype=torch.int32, device="cuda")
+        k, v = (f.clone()[off:off + size].view(batch, nkv, max_ctx, hd) for f in full)
+        for b in range(batch):
+            k[b, :, int(pos[b]):] = v[b, :, int(pos[b]):] = float("nan")
+        k2, v2 = (torch.cat([t.flatten(), t.new_zeros(4)])[:size].view_as(t) for t in (k, v))
+        q, want = torch.empty(batch, nq * hd, device="cuda"), torch.empty(batch, nq * hd, device="cuda")
+        scratch = torch.empty(L.jq_attention_scratch_bytes(batch, nq, hd, max_ctx) // 4 + 1, device="cuda")
+        flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+        _lib.check(L.jq_rope_append_dev(qkv.data_ptr(), pos.data_ptr(), batch, nq, nkv, hd, max_ctx, theta, q.data_ptr(),
+                                        k2.data_ptr(), v2.data_ptr(), flag.data_ptr(), s))
+        _lib.check(L.jq_attention_decode_dev(q.data_ptr(), k2.data_ptr(), v2.data_ptr(), pos.data_ptr(), batch, nq, nkv, hd,
+                                             max_ctx, want.data_ptr(), scratch.data_ptr(), flag.data_ptr(), s))
+        got = torch.full((batch, nq * hd), 123.0, device="cuda")
+        fscratch = torch.zeros(L.jq_attention_fused_scratch_bytes(batch, nq, nkv, hd, max_ctx) // 4 + 1, device="cuda")
+        _lib.check(L.jq_attention_fused_dev(qkv.data_ptr(), pos.data_ptr(), batch, nq, nkv, hd, max_ctx, theta, k.data_ptr(),
+                                            v.data_ptr(), got.data_ptr(), fscratch.data_ptr(), flag.data_ptr(), s))
+        torch.cuda.synchronize()
+        assert int(flag.item()) == 0
+        # f32 sums of up to 8000 terms in another order: eight times the terms of the test above
+        assert float((got - want).abs().max()) <= 8 * 2e-5 * max(1.0, float(want.abs().max()))
