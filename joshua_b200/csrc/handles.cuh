@@ -203,7 +203,7 @@ struct jq_moe {
     uint32_t* one = nullptr;
     uint32_t* counter = nullptr;  // arrival counter of the fused router kernel (zero between calls)
     float* xn = nullptr;          // normalised tokens, for the paths that cannot fold the norm in
-    float* bucket = nullptr;      // prefill path: gathered rows [P, hidden] + gate and up products [2][P, inter]
+    float* bucket = nullptr;      // prefill path: gate and up products [2][P, inter], then rows [P, hidden] where the form gathers them
     uint64_t bucket_pairs = 0;    // P the prefill path's buffers (in ws, like the rest) are sized for
     bool in_graph = false;        // a capture has used ws: a graph may hold its addresses
     std::vector<void*> retired;   // outgrown workspaces of captured graphs; freed with the layer

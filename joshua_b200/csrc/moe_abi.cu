@@ -90,7 +90,9 @@ int32_t reserve(jq_moe* m, uint64_t T, uint64_t P) {
 #ifdef JQ_PROFILING
     bucket |= m->gate != nullptr;  // the measurement switch of the forward entry sends any batch to the prefill form
 #endif
-    if (bucket) o_bucket = take(P * (c.hidden + 2ull * c.inter) * sizeof(float)), o_tiles = take(bucket_lists_bytes(m, P));
+    // gathered rows for the form that gathers; a smaller batch may take the other one, never the other way round
+    const uint64_t gathered = bucket && !grouped_tiles_ok(m, P) ? P * c.hidden : 0;
+    if (bucket) o_bucket = take((2 * P * c.inter + gathered) * sizeof(float)), o_tiles = take(bucket_lists_bytes(m, P));
     JQ_CUDA(cudaMalloc(&m->ws, off));
     uint8_t* b = m->ws;
     m->logits = (float*)(b + o_logits);
@@ -195,14 +197,13 @@ int32_t run_experts(jq_moe* m, const float* x, uint64_t R, uint64_t P, uint32_t 
 }
 
 // The prefill form of the expert MLPs, as the reference buckets tokens per expert and runs one matmul per
-// bucket (src/quantized_qwen3_moe.rs:455-520): when an expert sees dozens of rows, its rows are gathered into
-// bucket order and the experts' gate / up / down products run on the tile GEMM (tensor cores), as one grouped
-// launch per phase over a list of (expert, row range) tiles built on the device.
+// bucket (src/quantized_qwen3_moe.rs:455-520): when an expert sees dozens of rows, its rows are split for the tile
+// GEMM (tensor cores) in bucket order, straight from the routed list, and the experts' gate / up / down products are
+// one grouped launch per phase over a list of (expert, row range) tiles built on the device.
 // P is at most m->bucket_pairs.
 int32_t run_experts_bucketed(jq_moe* m, const float* x, uint64_t T, uint64_t P, uint32_t rows_per_job, cudaStream_t s) {
     const jq_moe_config& c = m->cfg;
-    float* xs = m->bucket;
-    float* gbuf = xs + P * c.hidden;
+    float* gbuf = m->bucket;
     float* ubuf = gbuf + P * c.inter;
     // Usual form, all on the device (`moe_tiles_kernel`): an expert with at least BUCKET_ROWS_PER_EXPERT rows has
     // them cut into tiles of up to 128 rows and runs on the tile GEMM, one grouped launch per phase and tile class
@@ -245,6 +246,7 @@ int32_t run_experts_bucketed(jq_moe* m, const float* x, uint64_t T, uint64_t P, 
     JQ_CUDA(cudaStreamSynchronize(s));
     std::vector<jq::MoeJob> jobs(n_jobs);
     if (n_jobs) JQ_CUDA(cudaMemcpyAsync(jobs.data(), m->jobs, n_jobs * sizeof(jq::MoeJob), cudaMemcpyDeviceToHost, s));
+    float* xs = ubuf + P * c.inter;
     JQ_CUDA(jq::launch_moe_gather(x, m->list_token, m->n_list, (uint32_t)P, c.hidden, xs, s));
     JQ_CUDA(cudaStreamSynchronize(s));
     // consecutive jobs of one expert form its bucket

@@ -443,3 +443,20 @@ def test_router_tiles_around_their_line_add_like_the_warp_per_token(hidden, n_ex
     """From 6144 logits on they come from tiles of 16 tokens and 16 experts (an SM to a CTA up to 148 of them): the sums of
     the kernel for fewer, bit for bit."""
     test_router_tiles_add_like_the_warp_per_token(hidden, n_expert, T)
+
+
+def test_a_prompts_workspace_holds_no_gathered_rows():
+    """Banks that run on the grouped tiles split their rows straight from the routed list: 32768 rows of 2048 values less."""
+    import torch
+
+    cfg = MoeConfig(gating=GATE_SOFTMAX, n_expert=16, n_used=8, hidden=2048, inter=256)
+    rng = np.random.default_rng(3)
+    banks = [QTensor.from_bytes(synth.Q4_K, synth.random_weight(synth.Q4_K, 16 * r, c, i))
+             for i, (r, c) in enumerate([(256, 2048), (256, 2048), (2048, 256)])]
+    layer = Moe(cfg, rng.standard_normal((16, 2048)).astype(np.float32), *banks)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    layer.reserve(4096)
+    rows = 4096 * 8 * 2048 * 4
+    # the result rows, the products of 256 columns (three times an eighth), tokens and planes (three quarters of the rows)
+    assert free - torch.cuda.mem_get_info()[0] <= rows * (1 + 3 / 8 + 3 / 4 + 1 / 8)
