@@ -535,7 +535,7 @@ __global__ void __launch_bounds__(A_THREADS, 1)
         }
         leave();
     }
-    if (tid == 0 && sh.abort_flag) *reinterpret_cast<volatile int*>(error_flag) = 1;
+    if (tid == 0 && sh.abort_flag && error_flag) *reinterpret_cast<volatile int*>(error_flag) = 1;
     tc_fence_after();
     if (warp == A_SOFT + A_CONV)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");

@@ -60,3 +60,11 @@ def test_a_failed_wait_leaves_nobody_at_a_named_barrier(path):
         if held and own_breaks(body):
             rest = re.match(r"\s*for \(; [^;]*; [^)]*\) (\w+\()\);", behind)
             assert rest and rest.group(1) in meeting, f"{path.name}:{line}: left by break, comes to {held}"
+
+
+def test_an_entry_without_a_context_may_have_no_status_flag():
+    """The prompt attention takes no context: its flag is NULL until a context exists on the device, so every store through it
+    is guarded."""
+    text = (ROOT / "joshua_b200" / "csrc" / "attention_prefill.cu").read_text()
+    stores = [line for line in text.splitlines() if "volatile int*>(error_flag) = 1" in line]
+    assert len(stores) == 2 and all("&& error_flag)" in line for line in stores)
