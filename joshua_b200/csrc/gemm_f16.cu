@@ -59,8 +59,9 @@
 // Q2_K 4096 x 14336, 333 rows 146 -> 121 us, Q4_K 28672 x 4096, 512 rows 250 -> 239 (at 1.4 GHz under the power cap) and
 // 4096 x 14336 127 -> 122, Q8_0 5120 x 2048, 1000 rows 86 -> 81, Q4_K 28672 x 4096, 16 rows 50.5 -> 47.3.  MXFP4, whose nibbles
 // one conversion instruction a pair now unpacks (64 a cycle and SM) instead of three byte permutes and masks: 28672 x 7168,
-// 20 / 64 / 200 rows 102 / 203 / 252 -> 76 / 150 / 206 us.  It costs launches of one or two windows a CTA 0.2 to 0.5 us
-// (Q4_K 5000 x 1536, 13 rows 8.8 -> 9.1; Q6_K, whose rows are copied by the word, 2048 x 4096, 33 rows 15.8 -> 17.1).
+// 20 / 64 / 200 rows 102 / 203 / 252 -> 76 / 150 / 206 us.  It costs launches of one or two windows a CTA 0.2 to 0.9 us
+// (Q4_K 2048 x 4096, 33 rows 13.3 -> 13.8; Q6_K, whose rows are copied by the word, 2048 x 4096, 33 rows 15.4 -> 16.3, 4096 x 4096
+// 20 rows 15.4 -> 15.9, 128 rows 46.7 -> 43.4).
 // Two further forms were slower: an owner per window instead of per step (half the instructions, but a chain of single warps:
 // 28672 x 4096, 16 rows 56 us) and a persistent loop over tiles on top of it.
 //
@@ -701,13 +702,14 @@ __global__ void __launch_bounds__(H_THREADS, 1)
     // is no multiple of eight falls to the first lanes.
     constexpr uint32_t ROW_VECS = WIN_WORDS * 4 / VEC, COPIERS = H_COPY * 32;
     static_assert(COPIERS == HM, "a copying warp takes 32 rows");
-    auto copy_window = [&](uint32_t wn) {
-        const uint32_t buf = wn % BUFS, r0 = (warp & 3) * 32 + (lane >> 3), v0 = lane & 7;
+    // rows r0, r0 + 4, .. of window wn by a warp whose lanes' first row is r0
+    auto copy_rows = [&](uint32_t wn, uint32_t r0, auto n_rows) {
+        const uint32_t buf = wn % BUFS, v0 = lane & 7;
         const uint32_t last = (uint32_t)min((uint64_t)HM, n - row0) - 1;  // rows past n repeat the last one
         const uint8_t* base = w + row0 * row_bytes + (uint64_t)(win0 + wn) * (WIN_WORDS * 4) + v0 * VEC;
         const uint32_t dst0 = smem_u32(raw) + buf * RAW_BUF + r0 * (RAW_STRIDE * 4) + v0 * VEC;
 #pragma unroll
-        for (uint32_t j = 0; j < 8; ++j) {
+        for (uint32_t j = 0; j < n_rows.value; ++j) {
             const uint8_t* src = base + (uint64_t)min(r0 + 4 * j, last) * (uint32_t)row_bytes;
             const uint32_t dst = dst0 + 4 * j * (RAW_STRIDE * 4);
 #pragma unroll
@@ -719,17 +721,28 @@ __global__ void __launch_bounds__(H_THREADS, 1)
                     asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst + 8 * c * VEC), "l"(src + 8 * c * VEC), "n"(VEC) : "memory");
             }
         }
-        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&raw_full[buf])) : "memory");
     };
-    // the first window is on its way before anything else is set up (more of them would hold up the rest: Q6_K, 4096 x 4096, 20
-    // rows 16.6 -> 18.0 us)
+    auto copy_window = [&](uint32_t wn) {
+        copy_rows(wn, (warp & 3) * 32 + (lane >> 3), std::integral_constant<uint32_t, 8>{});
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&raw_full[wn % BUFS])) : "memory");
+    };
+    // The first window is on its way before anything else is set up (more of them would hold up the rest: Q6_K, 4096 x 4096, 20
+    // rows 16.6 -> 18.0 us).  A window of Q6_K, 512 columns copied by the word, is a hundred instructions a copying thread, which
+    // launches of one or two windows a CTA wait for: there the converters, idle until it arrives, copy it among themselves
+    // (4096 x 4096, 64 rows 26.8 -> 25.9 us, 2048 x 4096 19.0 -> 18.6; Q2_K and IQ2_XXS, half of it, lose up to 0.6 us).
+    constexpr bool SHARED_FIRST = TYPE == T_Q6_K;
+    if (SHARED_FIRST && warp < H_CONV) {
+        copy_rows(0, warp * 8 + (lane >> 3), std::integral_constant<uint32_t, 2>{});
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
     if (warp >= H_CONV + H_ISSUE) {
         if (tid == (H_CONV + H_ISSUE) * 32) {
             for (uint32_t b = 0; b < BUFS; ++b) mbar_init(&raw_full[b], COPIERS), mbar_init(&raw_empty[b], H_CONV);
             mbar_fence_init();
         }
         asm volatile("bar.sync 2, %0;" ::"n"(COPIERS) : "memory");
-        copy_window(0);
+        if (SHARED_FIRST) asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&raw_full[0])) : "memory");
+        else copy_window(0);
     }
     if (tid == 0) {
         for (uint32_t s = 0; s < S::STAGES; ++s) {
@@ -815,6 +828,10 @@ __global__ void __launch_bounds__(H_THREADS, 1)
             return true;
         };
         const uint32_t raw_q = smem_u32(raw) + q * 32 * RAW_STRIDE * 4;
+        if (SHARED_FIRST) {  // the first window, which they copied
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            asm volatile("bar.sync 1, %0;" ::"n"(H_CONV * 32) : "memory");
+        }
         bool ok = true;
         float f_prev = 0.0f;
         auto window = [&](uint32_t wn, auto with_scales) {
