@@ -115,7 +115,7 @@ cudaError_t launch_gemm_tc(uint32_t type, const uint8_t* w, uint64_t n, uint64_t
 // leave at once), so that no host read stands between the routing and the products.  With a list, row r of the product is
 // row list[r] of x, for r below *n_list.  False from
 // gemm_f16_grouped_supports = shapes this form does not take (the caller then runs one product per expert).
-struct GemmTile {
+struct alignas(16) GemmTile {  // the kernels read it as one vector
     uint32_t expert;
     uint32_t row0;  // first row of the tile in x / dst
     uint32_t cnt;   // rows, 1..128

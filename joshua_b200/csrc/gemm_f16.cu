@@ -46,8 +46,8 @@
 // codes out of a word of nibbles or bytes.  MXFP4: i, i + 16 of a block, the two nibbles of a byte, which one instruction
 // converts.
 //
-// What bounds it: the converters' instruction issue (1.5 to 2.5 instructions a weight, waits included, at 2.6 to 3.0 a cycle on
-// narrow tiles), the tensor pipe from 128 rows on (70 % while a tile runs).
+// What bounds it: the converters' chain and its issue slots; a window of a tile is 7 700 warp instructions at 128 rows, at 2.0 a
+// cycle (Q4_K 28672 x 4096, 512 rows: the tensor pipe 59 % of the active cycles).
 //
 // Warps: 16 converters, warp (q = w % 4, g = w / 4) owns weight rows 32q .. 32q+31 (the tensor-memory lanes it may touch) and
 // the columns 64g .. 64g+63 of every window.  Warps 16 to 19 issue the MMAs and the TMA copies: an instruction takes about 30
@@ -640,9 +640,16 @@ __device__ __forceinline__ float ld_behind_wait(const float* p) {
     asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ uint32_t ld_behind_wait(const uint32_t* p) {
+// The same for the list of expert tiles, which every CTA of an SM reads: kept in L1 (the lists of two launches that could overlap are
+// one layer's, and equal).  Through L2 the routed-expert model's prompt of 1000 tokens took 36.7 ms instead of 34.9.
+__device__ __forceinline__ uint32_t ld_list(const uint32_t* p) {
     uint32_t v;
-    asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint4 ld_list(const GemmTile* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
     return v;
 }
 
@@ -670,25 +677,26 @@ __global__ void __launch_bounds__(H_THREADS, 1)
     // full[s]: the step's four converter warps + the TMA thread (and the tiles' bytes); empty[s]: the MMAs' commit
     // raw_full / raw_empty: the copying threads, the converter warps
     __shared__ uint64_t full[S::STAGES], empty[S::STAGES], acc_full[2], acc_empty[S::ACCS], raw_full[BUFS], raw_empty[BUFS];
-    __shared__ uint32_t tmem_base_slot;
+    __shared__ uint64_t scales_known;  // wide tiles: scaled_groups, by converter group, whether some token has windows with own scales
+    __shared__ uint32_t scaled_groups, tmem_base_slot;
     __shared__ int abort_flag, lost_flag;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     pdl_trigger();
     // blockIdx.z: the bank (gate and up in one launch) and this CTA's place in its cluster along k.
-    // Grouped form: tile blockIdx.y of the list, its expert's slice of the bank; rows of the tile box beyond the tile's count belong to other experts, are multiplied along and
-    // never stored.  The launch covers the list's capacity, not its length.
+    // Grouped form: tile blockIdx.y of the list, its expert's slice of the bank; rows of the tile box beyond the tile's count
+    // belong to other experts, are multiplied along and never stored.  The launch covers the list's capacity, not its length.
     uint64_t tok0 = (uint64_t)blockIdx.y * N_TILE, m = m_rows;
     const uint32_t bank = blockIdx.z / split, rank = blockIdx.z - bank * split;
     const uint8_t* w = bank ? w_b : w_a;
     float* dst = bank ? dst_b : dst_a;
     if (tiles != nullptr) {
         pdl_wait();
-        if (blockIdx.y >= ld_behind_wait(n_tiles)) return;
-        const GemmTile* t = tiles + blockIdx.y;
-        w += (uint64_t)ld_behind_wait(&t->expert) * expert_bytes;
-        tok0 = ld_behind_wait(&t->row0);
-        m = tok0 + ld_behind_wait(&t->cnt);
+        if (blockIdx.y >= ld_list(n_tiles)) return;
+        const uint4 t = ld_list(tiles + blockIdx.y);  // expert, row0, cnt
+        w += (uint64_t)t.x * expert_bytes;
+        tok0 = t.y;
+        m = tok0 + t.z;
     }
     const uint64_t row0 = (uint64_t)blockIdx.x * HM;
     const uint64_t row_bytes = k / 256 * T::UNIT;
@@ -753,6 +761,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
             if (!S::FINE) mbar_init(&acc_full[b & 1], 1);
             mbar_init(&acc_empty[b], S::FINE ? 4 : H_CONV);
         }
+        mbar_init(&scales_known, 1);
         abort_flag = lost_flag = 0;
         mbar_fence_init();
     }
@@ -784,10 +793,20 @@ __global__ void __launch_bounds__(H_THREADS, 1)
         // registers on it (in one loop Q6_K, 28672 x 4096, 40 rows took 202 us instead of 172).
         bool scaled = false;
         const uint32_t slot = scales + warp * 32 * 16;  // per token: its address in rel, its scale so far, its change
+        // On wide tiles an idle issuer reads the signs and tells: the load in the converters' chain cost Q2_K 4096 x 14336, 333 rows
+        // 2.8 of 125 us.  On narrow ones, whose issuers have no time, waiting for one costs more than the load (Q4_K 512 x 2048, 33
+        // rows 10.4 and 9.9 us).
         auto find_scales = [&] {
+            if constexpr (!S::FINE) {
+                scaled = scaled_groups >> g & 1;
+                if (!scaled) return;
+            }
+            pdl_wait();  // the scales belong to the kernel in front
             const uint64_t tok = min(tok0 + (S::FINE ? 0 : g * MY_COLS) + lane % MY_COLS, m_rows - 1);  // the last row, past it
-            scaled = __any_sync(0xFFFFFFFFu, ld_behind_wait(inv + tok) < 0.0f);
-            if (!scaled) return;
+            if constexpr (S::FINE) {
+                scaled = __any_sync(0xFFFFFFFFu, ld_behind_wait(inv + tok) < 0.0f);
+                if (!scaled) return;
+            }
             const float* p = rel + (uint64_t)win0 * T::UNITS * m_rows + tok;
             asm volatile("st.shared.u64 [%0], %1;" ::"r"(slot + lane * 8), "l"(p) : "memory");
             asm volatile("st.shared.f32 [%0], %1;" ::"r"(slot + 256 + lane * 4), "f"(ld_behind_wait(p)) : "memory");
@@ -872,8 +891,8 @@ __global__ void __launch_bounds__(H_THREADS, 1)
                     if constexpr (with_scales.value) rescale(c - 1);
                     ok = drain(c - 1, f_prev);
                 } else {
-                    pdl_wait();  // the scales, and dst, belong to the kernels before this one
-                    find_scales();
+                    if constexpr (!S::FINE) ok = __all_sync(0xFFFFFFFFu, converter_wait(&scales_known, 0));
+                    if (ok) find_scales();
                 }
                 f_prev = rw.f;
             }
@@ -885,7 +904,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
         if (ok && n_chunks > 0) ok = drain(n_chunks - 1, f_prev);
         if (scaled) rescale(n_chunks);
         if (!ok) abort_flag = 1;
-        pdl_wait();  // (a warp that gave up in its first window)
+        pdl_wait();  // dst and the rows' scales belong to the kernels before this one
         // The ring and the staged bytes are idle once every converter is here: the last read-back waited for this CTA's
         // last products.
         asm volatile("bar.sync 1, %0;" ::"n"(H_CONV * 32) : "memory");
@@ -1026,6 +1045,18 @@ __global__ void __launch_bounds__(H_THREADS, 1)
             pdl_wait();
             for (uint32_t c = 0; c < n_chunks && ok; ++c)
                 for (uint32_t g = 0; g < H_STEPS && ok; ++g) ok = load(c, g);
+        } else if (mine == 2) {
+            pdl_wait();
+            uint32_t bits = 0;
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+                const uint64_t tok = min(tok0 + i * (N_TILE / 4) + lane, m_rows - 1);  // the last row, past it
+                bits |= (uint32_t)(__any_sync(0xFFFFFFFFu, ld_behind_wait(inv + tok) < 0.0f) != 0) << i;
+            }
+            if (lane == 0) {
+                *static_cast<volatile uint32_t*>(&scaled_groups) = bits;
+                mbar_arrive(&scales_known);
+            }
         }
         if (!ok && lane == 0) abort_flag = 1;
     } else {
@@ -1173,8 +1204,9 @@ cudaError_t launch_f16_tile(const F16Launch& l, cudaStream_t s) {
             cfg.numAttrs = 2;
         }
     }
-    e = cudaLaunchKernelEx(&cfg, kern, l.w_a, l.n, l.k, hi, lo, sums, (const float*)l.x.inv, (const float*)l.x.rel, (const __half*)l.x.hi, (const __half*)l.x.lo, l.rows, l.dst_a, l.residual, l.error_flag,
-                           l.tiles, l.n_tiles, l.expert_bytes, l.w_b, l.dst_b, split);
+    e = cudaLaunchKernelEx(&cfg, kern, l.w_a, l.n, l.k, hi, lo, sums, (const float*)l.x.inv, (const float*)l.x.rel,
+                           (const __half*)l.x.hi, (const __half*)l.x.lo, l.rows, l.dst_a, l.residual, l.error_flag, l.tiles,
+                           l.n_tiles, l.expert_bytes, l.w_b, l.dst_b, split);
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
