@@ -24,9 +24,10 @@
 //
 // Error against float64 (2-norm, N(0, 1) rows): Q4_K 2.1e-7 to 2.9e-7, MXFP4 0.9e-7 to 1.1e-7; the routes before 3.3e-7 to
 // 3.8e-7 and 1.3e-7 to 1.5e-7.  Positive rows (1 + |N(0, 1)|), Q4_K weights of mean zero: up to four rows 1.2e-6, before 1.8e-6 to
-// 2.8e-6; five to eight 1.4e-6 to 1.6e-6, before 2.4e-6 to 5.6e-6.  Algorithmic bytes per launch: n*k/B*S (weights) + 4*m*(k + n).  What bounds it: the consumers'
-// instructions, 460 (four rows) to 600 (eight) per 16 x 256 unit at 1.8 to 2.8 a cycle.  Measured, four / eight rows, before (the
-// integer kernel / the tile GEMM and its split) and now: Q4_K 28672 x 4096 27.4 / 49.5 and 22.2 / 27.5 us, 6144 x 4096 11.4 /
+// 2.8e-6; five to eight 1.4e-6 to 1.6e-6, before 2.4e-6 to 5.6e-6.
+// Algorithmic bytes per launch: n*k/B*S (weights) + 4*m*(k + n).  What bounds it: the consumers' instructions, 460 (four rows) to 600 (eight)
+// per 16 x 256 unit at 1.8 to 2.8 a cycle.  Measured, four / eight rows, before (the integer kernel / the tile GEMM and its
+// split) and now: Q4_K 28672 x 4096 27.4 / 49.5 and 22.2 / 27.5 us, 6144 x 4096 11.4 /
 // 25.9 and 9.2 / 12.2, 4096 x 4096 9.8 / 11.5 and 7.4 / 10.2, 4096 x 14336 24.6 / 28.5 and 18.3 / 22.8, 128256 x 4096 94 / 169 and
 // 73 / 96; MXFP4 28672 x 4096 41.5 (three rows) / 54.7 and 23.7 / 30.3, 7168 x 2048 11.6 / 18.2 and 6.8 / 8.6.
 //
@@ -54,8 +55,9 @@ constexpr uint32_t SLOTS = 2;      // partial tiles a rank can hold of every oth
 constexpr uint32_t MAX_SPLIT = 8;
 constexpr uint32_t SMEM_MAX = 225 * 1024;
 constexpr uint32_t MAX_STAGES = 48;  // of all teams
-// Shorter rows stay with the routes they had: three units or less keep two or three of a team's warps busy.  One and two
-// rows of x stay with the integer kernel in any case: 28672 x 4096 17.0 and 18.7 us there, 21.9 and 22.0 here.
+// Shorter rows stay with the routes they had, although they lose there: k = 512, four / eight rows, Q4_K 4096 rows 5.0 / 6.3 us
+// (here 4.5 / 5.1), 28672 rows 16.4 / 13.1 (6.6 / 7.5), MXFP4 5.9 / 8.4 (5.0 / 5.7) and 22.4 / 35.1 (7.0 / 8.4).  One and two
+// rows of x stay with the integer kernel: 28672 x 4096 17.0 and 18.7 us there, 21.9 and 22.0 here.
 constexpr uint64_t MIN_K = 1024;
 
 template <uint32_t TYPE>
@@ -321,11 +323,6 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
     }
     return false;
 }
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
-}
-
 template <uint32_t TYPE, bool PACK, bool PAIR>
 __global__ void __launch_bounds__(THREADS, 1) gemv_f16_kernel(const __grid_constant__ F16Args ga, const __grid_constant__ CUtensorMap map_a,
                                                               const __grid_constant__ CUtensorMap map_b) {
@@ -341,10 +338,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_f16_kernel(const __grid_const
     const uint32_t unit0 = (uint32_t)((uint64_t)(units / STEP) * rank / split) * STEP,
                    U = (uint32_t)((uint64_t)(units / STEP) * (rank + 1) / split) * STEP - unit0;
     const uint32_t u_max = (units / STEP + split - 1) / split * STEP;
-    // A stage is `cu` units of a tile.  The consumers form teams of cu warps; a team takes every n_teams-th tile of an
-    // item, a warp one unit of each of the tile's stages; the stages of a round of teams come chunk by chunk.  Every team has a ring of its own, `depth` stages that it takes one after another:
-    // with one ring for all, a team's wait for a stage's next round could find the round before still on its way, whose
-    // parity an mbarrier cannot tell from the one asked for.
+    // A stage is `cu` units of a tile.  The consumers form teams of cu warps; a team takes every n_teams-th tile of an item, a warp
+    // one unit of each of the tile's stages; the stages of a round of teams come chunk by chunk.  Every team has a ring of its
+    // own, `depth` stages that it takes one after another: with one ring for all, a team's wait for a stage's next round could
+    // find the round before still on its way, whose parity an mbarrier cannot tell from the one asked for.
     const uint32_t cu = ga.cu, n_teams = min(NCW / cu, MAX_TEAMS), n_chunks = (u_max + cu - 1) / cu, depth = NS / n_teams;
     const uint32_t stage_bytes = ROWS * ga.row_stride;
     // layout: activations | ring | two buffers of the warps' partial sums | partial tiles of the cluster's ranks | mbarriers
@@ -369,7 +366,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_f16_kernel(const __grid_const
         mbar_fence_init();
     }
     __syncthreads();
-    if (split > 1) cluster_barrier();  // the ranks' mbarriers exist
+    if (split > 1) cluster_sync_all();  // the ranks' mbarriers exist
     pdl_trigger();
     if (warp != 0) pdl_wait();  // the weights do not depend on the kernel in front
     const uint32_t tiles = cid < row_tiles ? (row_tiles - cid + n_clusters - 1) / n_clusters : 0;  // cid, cid + n_clusters, ...
@@ -487,7 +484,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_f16_kernel(const __grid_const
                 if (warp == 1) {
                     if (lane < ga.m)
                         for (uint32_t r = 0; r < split; ++r)
-                            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(map_rank(smem_u32(s_rs + rank * GEMV_F16_MAX_M + lane), r)), "f"(ss) : "memory");
+                            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(map_rank(smem_u32(s_rs + rank * GEMV_F16_MAX_M + lane), r)),
+                                         "f"(ss)
+                                         : "memory");
                     asm volatile("fence.acq_rel.cluster;" ::: "memory");
                     __syncwarp();
                     if (lane < split) arrive_rank(&norm_full, lane);
@@ -593,7 +592,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_f16_kernel(const __grid_const
     }
     if (split > 1) {
         __syncthreads();
-        cluster_barrier();  // no CTA leaves while another writes to its shared memory
+        cluster_sync_all();  // no CTA leaves while another writes to its shared memory
     }
 }
 
@@ -664,7 +663,11 @@ cudaError_t f16_launch(F16Args& ga, const uint8_t* w_a, const uint8_t* w_b, cuda
     CUtensorMap map_a, map_b;
     const uint64_t row_bytes = ga.k / 256 * FT<TYPE>::UNIT;
     if (cudaError_t e = f16_weight_map(w_a, ga.n, row_bytes, p.row_stride, &map_a); e != cudaSuccess) return e;
-    if (cudaError_t e = f16_weight_map(PAIR ? w_b : w_a, ga.n, row_bytes, p.row_stride, &map_b); e != cudaSuccess) return e;
+    if constexpr (PAIR) {
+        if (cudaError_t e = f16_weight_map(w_b, ga.n, row_bytes, p.row_stride, &map_b); e != cudaSuccess) return e;
+    } else {
+        map_b = map_a;  // not read
+    }
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -712,8 +715,9 @@ bool gemv_f16_supports(uint32_t type, const uint8_t* w, uint64_t n, uint64_t k, 
     };
     switch (type) {
         case T_Q4_K: return a % 16 == 0 && fits(std::integral_constant<uint32_t, T_Q4_K>{});
-        // five to eight rows with k split: 4096 x 7168 18.6 us, on tiles 17.2 (7168 x 16384 52.4 / 56.2), both before the
-        // conversion instruction; the tiles take 14.6 with it
+        // five to eight rows with k split stay on tiles: 4096 x 7168 14.2 us there and 16.8 here, 7168 x 16384 40.7 and 46.1,
+        // 4096 x 14336 23.8 and 25.6 (the other way round for few rows of weights and very many: 1536 x 7168 13.9 and 12.7,
+        // 24576 x 7168 61.2 and 57.5)
         case T_MXFP4: return a % 16 == 0 && fits(std::integral_constant<uint32_t, T_MXFP4>{}) && (m <= 4 || p.split == 1);
         default: return false;
     }

@@ -169,3 +169,46 @@ def test_rows_of_one_sign_are_as_exact_in_four_columns_as_in_eight(k, m):
         for rows in total:
             total[rows] += float((lin.forward(x[:rows])[:m].double() - ref).square().sum())
     assert total[m] <= 1.1 ** 2 * total[8]
+
+
+def kernels_of(call):
+    """Names of the kernels that a call launches."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    call()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
+        call()
+        torch.cuda.synchronize()
+    return [e.key for e in p.key_averages() if "_kernel" in e.key]
+
+
+@pytest.mark.parametrize("type_id,n,k,m,mine", [
+    (synth.Q4_K, 100, 1280, 3, True), (synth.Q4_K, 100, 1280, 8, True), (synth.Q4_K, 700, 14336, 8, True),
+    (synth.Q4_K, 100, 1024, 5, True), (synth.Q4_K, 100, 768, 5, False), (synth.Q4_K, 100, 1280, 2, False),
+    (synth.Q4_K, 100, 1280, 9, False), (synth.MXFP4, 48, 1536, 3, True), (synth.MXFP4, 48, 1536, 8, True),
+    (synth.MXFP4, 100, 1280, 3, False), (synth.MXFP4, 40, 14336, 4, True), (synth.MXFP4, 40, 14336, 5, False),
+    (synth.Q8_0, 100, 1280, 4, False)])
+def test_the_route_by_type_columns_and_rows(type_id, n, k, m, mine):
+    q, _, x = setup(type_id, n, k, m, 1)
+    names = kernels_of(lambda: QMatMul(q, n, k).forward(x))
+    assert any("gemv_f16_kernel" in v for v in names) == mine, names
+    assert names
+
+
+@pytest.mark.parametrize("type_id,k", [(synth.Q4_K, 1280), (synth.Q4_K, 4096), (synth.Q4_K, 14336), (synth.MXFP4, 1536),
+                                       (synth.MXFP4, 4096)])
+@pytest.mark.parametrize("m", [3, 4, 5, 6, 7, 8])
+def test_units_and_rows_decades_apart(type_id, k, m):
+    """Both layouts of the terms: a unit 1e4 times the others, one 1e-6 of them, a row 1e-6 of the others, a row of zeros."""
+    n = 100
+    q, w, x = setup(type_id, n, k, m, k + m)
+    x[:, :256] *= 1e4
+    x[:, 512:768] *= 1e-6
+    x[m - 1] *= 1e-6
+    x[1] = 0
+    got = QMatMul(q, n, k).forward(x)
+    err = (got.double() - x.double() @ w.T).abs()
+    assert bool((err <= bound(w, x, k // 256)).all()), float((err / bound(w, x, k // 256)).max())
+    assert bool((got[1] == 0).all())
