@@ -83,7 +83,8 @@ int* jq_entry_status_flag() { return g_entry_status[jq::current_device()].dev.lo
 // kernel's activation planes do not fit its shared memory, it reads them from L2 for every 16 weight rows; Q4_K, bound
 // by its consumers' instructions, is behind the tiles from five rows on in any case.  Measured, eight rows, tiles /
 // decode kernel: Q4_K 28672 x 4096 50 / 66 us, 4096 x 14336 29 / 36 us, 7168 x 2048 11 / 19 us, Q2_K 4096 x 14336 30 / 54,
-// MXFP4 31 / 36; five rows, planes in shared memory: Q4_K 28672 x 4096 50 / 64 us; four rows: 50 / 28 us.
+// MXFP4 31 / 36; five rows, planes in shared memory: Q4_K 28672 x 4096 50 / 64 us; four rows: 50 / 28 us.  (The tiles' figures
+// are from before their copying warps, which put them further ahead: Q4_K 28672 x 4096, 16 rows 50.5 -> 47.3 us.)
 bool jq_uses_tiles(const jq_weight* w, uint64_t m, uint64_t k, uint64_t n, cudaStream_t s) {
     if (w->ctx->force_f32 || m < 5 || !jq::gemm_f16_supports(w->type, w->dev, n, k, m)) return false;
     // Q8_0 stays on the decode kernel up to 16 rows, although the tiles are ahead (4096 x 4096: 16 rows there 42 us, 17 rows
@@ -180,7 +181,8 @@ namespace {
 // lost copy does not fail every later call on the context.
 int32_t check_device_status(const jq_ctx* ctx) {
     bool raised = false;
-    for (volatile int* flag : {static_cast<volatile int*>(ctx->status_host), static_cast<volatile int*>(g_entry_status[ctx->device % jq::MAX_DEVICES].host.load())})
+    volatile int* const flags[2] = {ctx->status_host, g_entry_status[ctx->device % jq::MAX_DEVICES].host.load()};
+    for (volatile int* flag : flags)
         if (flag && *flag != 0) *flag = 0, raised = true;
     return raised ? jq_fail(jq::E_TIMEOUT, "a bounded wait inside a kernel gave up (device status flag was set)") : jq::OK;
 }

@@ -154,7 +154,7 @@ class LlamaDecoder:
     def prefill(self, token_ids, stream=None) -> None:
         """`forward(input [1, seq_len], offset)` of the reference's loaders (src/quantized_qwen3_moe.rs:793-819): the
         prompt's tokens in ONE pass from the current position - batched matmuls (the tensor-core tile GEMM from
-        five tokens on, Q8_0 from 17), rotary embedding + cache append for all positions, causal attention - then the logits of the
+        nine tokens on, Q8_0 from 17), rotary embedding + cache append for all positions, causal attention - then the logits of the
         last token, the sampled next token and the advanced position, exactly as `step` leaves them.  One
         sequence (batch 1).  Buffers are allocated per call."""
         torch, L, c, P = self.torch, _lib.lib(), self.cfg, lambda t: t.data_ptr()
