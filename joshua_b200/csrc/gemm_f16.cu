@@ -641,7 +641,7 @@ __device__ __forceinline__ float ld_behind_wait(const float* p) {
     return v;
 }
 // The same for the list of expert tiles, which every CTA of an SM reads: kept in L1 (the lists of two launches that could overlap are
-// one layer's, and equal).  Through L2 the routed-expert model's prompt of 1000 tokens took 36.7 ms instead of 34.9.
+// one layer's, and equal).  Through L2 the routed-expert model's prompt of 1000 tokens took 36.7 ms instead of 35.7.
 __device__ __forceinline__ uint32_t ld_list(const uint32_t* p) {
     uint32_t v;
     asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -964,6 +964,21 @@ __global__ void __launch_bounds__(H_THREADS, 1)
             __syncwarp();
             return true;
         };
+        // wide tiles: whether some token of a converter warp's columns has windows with scales of their own
+        auto tell_scales = [&] {
+            constexpr uint32_t COLS = S::FINE ? N_TILE : N_TILE / 4;
+            uint32_t bits = 0;
+#pragma unroll
+            for (uint32_t i = 0; i < N_TILE / COLS; ++i) {
+                const uint64_t tok = min(tok0 + i * COLS + lane % COLS, m_rows - 1);  // the last row, past it
+                bits |= (__any_sync(0xFFFFFFFFu, ld_behind_wait(inv + tok) < 0.0f) ? 1u : 0u) << i;
+            }
+            if (lane == 0) {
+                *static_cast<volatile uint32_t*>(&scaled_groups) = bits;
+                mbar_arrive(&scales_known);
+            }
+            __syncwarp();
+        };
         // Steps G0 .. G1 - 1 of every window; compile-time, so that the descriptors need no arithmetic but a stage's offset.
         // The tensor pipe takes few instructions ahead: on wide tiles the waits for the next step stand between the two halves of
         // this one's, or the pipe runs dry at every step (some 220 cycles, 600 at a new window).
@@ -1047,16 +1062,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
                 for (uint32_t g = 0; g < H_STEPS && ok; ++g) ok = load(c, g);
         } else if (mine == 2) {
             pdl_wait();
-            uint32_t bits = 0;
-#pragma unroll
-            for (uint32_t i = 0; i < 4; ++i) {
-                const uint64_t tok = min(tok0 + i * (N_TILE / 4) + lane, m_rows - 1);  // the last row, past it
-                bits |= (uint32_t)(__any_sync(0xFFFFFFFFu, ld_behind_wait(inv + tok) < 0.0f) != 0) << i;
-            }
-            if (lane == 0) {
-                *static_cast<volatile uint32_t*>(&scaled_groups) = bits;
-                mbar_arrive(&scales_known);
-            }
+            tell_scales();
         }
         if (!ok && lane == 0) abort_flag = 1;
     } else {
