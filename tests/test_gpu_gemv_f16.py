@@ -212,3 +212,37 @@ def test_units_and_rows_decades_apart(type_id, k, m):
     err = (got.double() - x.double() @ w.T).abs()
     assert bool((err <= bound(w, x, k // 256)).all()), float((err / bound(w, x, k // 256)).max())
     assert bool((got[1] == 0).all())
+
+
+def test_a_result_over_its_input_under_capture():
+    """The copy's scratch is the stream's, and a capture cannot allocate it: refused with nothing launched on a stream that has
+    none, captured and replayed on one that has run the call before."""
+    import torch
+
+    from joshua_b200 import _lib
+    from joshua_b200.qtensor import Context
+
+    L, n, m = _lib.lib(), 1024, 3
+    raw, ctx = synth.random_weight(synth.Q4_K, n, n, 9), Context(0)
+    q = QTensor.from_bytes(synth.Q4_K, raw, ctx)
+    w = torch.empty(n * n, device="cuda")
+    q.dequantize_dev(w, two_step=False)
+    x = torch.randn(m, n, device="cuda", generator=torch.Generator(device="cuda").manual_seed(2))
+    y, st = x.clone(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    refused, graph = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
+    call = lambda: L.jq_matmul_t_dev(q._h, m, n, n, y.data_ptr(), y.data_ptr(), st.cuda_stream)
+    with torch.cuda.stream(st):
+        with torch.cuda.graph(refused, stream=st):
+            assert call() == _lib.E_INVALID
+            y.mul_(2.0)  # the capture goes on
+        _lib.check(call())
+        with torch.cuda.graph(graph, stream=st):
+            _lib.check(call())
+        y.copy_(x)
+        refused.replay()
+        graph.replay()
+        st.synchronize()
+    want = 2.0 * x.double() @ w.reshape(n, n).double().T
+    assert float((y.double() - want).norm() / want.norm()) <= 1e-6
+    del refused, graph
